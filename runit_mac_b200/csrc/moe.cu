@@ -36,6 +36,10 @@ struct MoeScratch {
     size_t bytes;
 };
 
+// Tokens from which the slots are sorted by expert (moe_slots.cu), and up to which the scratch size asks for its staging area.
+constexpr uint32_t kSlotsMinTokens = 4, kSlotsMaxTokens = 4096;
+static bool moe_by_expert(uint32_t T) { return T >= kSlotsMinTokens && T <= kSlotsMaxTokens; }
+
 // Expert-parallel decode block, replicated tokens.  This rank's weighted sum over the slots whose expert it owns
 // (routing order), stored into slot `rank` of the partial buffer of every rank: plain stores into peer memory.
 struct EpPeers {
@@ -136,6 +140,16 @@ int32_t moe_layer_q4k_impl(runit_ctx* ctx, const void* router_w, const void* gat
         if (st != RUNIT_OK) return st;
     }
     const uint32_t slots = T * k;
+    // a scratch without the staging area (the built-in region at larger shapes) keeps the launches per slot
+    if (moe_by_expert(T) && !fused_route && scratch_bytes >= s.bytes + moe_slots_bytes(T, h, ff, E, k) && ctx->encode_tiled && ctx->tune.gemv_math != 1 &&
+        ctx->tune.gemv_variant != 1 && runit_aligned(gate, 16) && runit_aligned(up, 16) && runit_aligned(down, 16)) {
+        st = moe_slots_experts(ctx, gate, up, down, (const float*)x, idx, s.act, s.y, (uint8_t*)scratch + s.bytes, T, h, ff, E, k);
+        if (st != RUNIT_OK) return st;
+        runit_launch_chain(ctx, moe_combine_kernel, dim3((h + 255) / 256, T), dim3(256), (const float*)s.y, (const float*)wts, (const float*)residual, (float*)out, T, h, k);
+        st = runit_after_launch(ctx, "moe_combine");
+        if (st != RUNIT_OK || !next_gamma) return st;
+        return launch_rms_norm(ctx, (const float*)out, next_xn, next_gamma, false, next_eps, h, T);
+    }
     // gate+up+SiLU for every (token, expert) slot: act[s][ff]
     const bool fused_sum = fused_route && h <= 32 * 960;
     st = gemv_grouped(ctx, "moe_gate_up", RUNIT_FMT_Q4K, gate, up, E, ff, h, x, k, s.act, idx, slots, 0, nullptr, nullptr, nullptr,
@@ -305,7 +319,7 @@ int32_t runit_moe_layer_q4k_static(runit_ctx_t* ctx, const void* router_w, const
 }
 
 size_t runit_moe_scratch_bytes(uint32_t T, uint32_t h, uint32_t ff, uint32_t E, uint32_t k) {
-    return moe_carve(nullptr, T, h, ff, E, k).bytes;
+    return moe_carve(nullptr, T, h, ff, E, k).bytes + (moe_by_expert(T) ? moe_slots_bytes(T, h, ff, E, k) : 0);
 }
 
 int32_t runit_moe_router_f32(runit_ctx_t* ctx, const void* router_w, const void* x, void* logits, uint32_t E, uint32_t h,
