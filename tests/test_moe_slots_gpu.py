@@ -17,8 +17,12 @@ def run(ctx, R, weights, x, res, h, ff, E, k, nbytes):
     T = x.shape[0]
     out, idx, w = ctx.new_buffer(T * h * 4), ctx.new_buffer(T * k * 4), ctx.new_buffer(T * k * 4)
     scratch = ctx.new_buffer(nbytes)
-    R.moe_layer_q4k(ctx, *weights, ctx.buffer_from(x), ctx.buffer_from(res), out, idx, w, scratch, nbytes, T, h, ff, E, k, 0)
-    ctx.flush()
+    ctx.set_tuning("moe_slots", 1)                  # small layers, too
+    try:
+        R.moe_layer_q4k(ctx, *weights, ctx.buffer_from(x), ctx.buffer_from(res), out, idx, w, scratch, nbytes, T, h, ff, E, k, 0)
+        ctx.flush()
+    finally:
+        ctx.set_tuning("moe_slots", 0)
     return out.download(np.float32, T * h).reshape(T, h), idx.download(np.int32, T * k).reshape(T, k)
 
 
