@@ -1,0 +1,282 @@
+// Causal attention of the prefill on the tcgen05 tensor cores: softmax(q.K^T / sqrt(hd)) . V over the f16 cache with key <=
+// start + query (attention.metal:36-158), head dim 64 or 128.
+//
+// A CTA owns 128 queries of one head and walks the keys in blocks of 128.  Warp 4's first lane issues every copy and MMA; warps
+// 0..3 hold one query per thread (thread = tensor-memory lane):
+//   S = Q.K^T     Q rounded to f16 once (shared memory, 128-byte swizzle), K by TMA; f32 accumulator, 128 columns
+//   P             row maximum, exp2 and sum from tensor memory, two passes over S so that no row lives in registers; P is rounded to
+//                 f16 into the columns of S that the thread has already read, which makes it the A operand of the second product
+//   O_blk = P.V   V by TMA as it lies in the cache (hd contiguous: B is MN-major); the block's result is added to the thread's f32
+//                 registers with the factor of the moved maximum while S of the next block is being computed
+// The K buffer is free once S is there and V once O_blk is, so one buffer each suffices: 96 KB and 256 tensor-memory columns a CTA,
+// two CTAs per SM, which overlap each other's softmax and products.  Query blocks go from the most keys to the fewest.
+// Bound: the chain of a row's blocks (product, softmax, product) and the exponentials (16 a clock and SM: 1024 clocks a block).
+// Measured, 2048 queries x 16 heads x 128: 102 -> 58 us (mma.sync, 64 queries of 4 warps, 167 TFLOP/s of useful products before);
+// the error against 64 bits is the bf16 output's, 1.7e-3, on both.
+// Rows of the tensor maps end at start + T, so that what the cache holds behind the data (NaN included) reads as zeros.
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include "gemv_common.cuh"
+#include "runit_internal.h"
+#include "tcgen05.cuh"
+#include "tma.cuh"
+
+namespace runit {
+namespace atc {
+
+constexpr int kRows = 128, kKeys = 128;
+constexpr uint32_t kCols = 256;                    // tensor memory: S | P in columns 0..127, O_blk from 128
+
+template <int HD> struct Shape {
+    static constexpr uint32_t kPanel = 128 * 128;  // 64 elements of 128 rows
+    static constexpr uint32_t kTile = HD / 64 * kPanel;
+    static constexpr uint32_t kSmem = 3 * kTile + 1024;
+};
+
+// kind::f16 with f16 operands (formats 0), f32 accumulator; bit 16: B is MN-major
+__host__ __device__ constexpr uint32_t idesc_f16(uint32_t m, uint32_t n, uint32_t b_mn) {
+    return (1u << 4) | (b_mn << 16) | ((n >> 3) << 17) | ((m >> 4) << 24);
+}
+// MN-major tile in the 128-byte swizzled layout: 64 elements (128 bytes) per row of K, groups of 8 K rows 1024 bytes apart (stride
+// byte offset), the next 64 elements a panel further (leading byte offset)
+__device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t addr, uint32_t panel) {
+    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)(panel >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+// A in tensor memory: 128 lanes, 32-bit column c = K elements 2c, 2c + 1
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int32_t c0, int32_t c1, int32_t c2, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ float exp2_approx(float v) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+struct Args {
+    const float* q;
+    __nv_bfloat16* out;
+    uint32_t T, heads, group, start;               // group: query heads per key head
+    float scale_log2;                              // log2(e) / sqrt(hd)
+    int32_t* status;
+};
+
+template <int HD>
+__global__ void __launch_bounds__(160, 2) attention_tc_kernel(const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mv, const Args a) {
+    using S = Shape<HD>;
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t bars[5];
+    __shared__ uint32_t tmem_holder;
+    __shared__ volatile int abort_flag;
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t qs = base, ks = base + S::kTile, vs = base + 2 * S::kTile;
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t k_full = smem_u32(&bars[0]), v_full = smem_u32(&bars[1]), s_full = smem_u32(&bars[2]), p_full = smem_u32(&bars[3]), o_full = smem_u32(&bars[4]);
+    const uint32_t head = blockIdx.x, q0 = (gridDim.y - 1 - blockIdx.y) * kRows;
+    if (tid == 0) {
+        abort_flag = 0;
+        for (int i = 0; i < 5; i++) mbar_init(smem_u32(&bars[i]), i == 3 ? 128 : 1);
+        fence_mbar_init();
+    }
+    if (warp == 0) {
+        tmem_alloc(smem_u32(&tmem_holder), kCols);
+        tmem_relinquish();
+    }
+    grid_dependency_wait();
+    grid_launch_dependents();
+    // queries of this CTA as f16 into the swizzled K-major tile; rows behind the last query are zeros
+    if (warp < 4) {
+        constexpr uint32_t CH = HD / 8;            // 16-byte chunks of a row
+        for (uint32_t i = tid; i < kRows * CH; i += 128) {
+            const uint32_t r = i / CH, c = i % CH;
+            float4 x0 = make_float4(0.f, 0.f, 0.f, 0.f), x1 = x0;
+            if (q0 + r < a.T) {
+                const float4* src = reinterpret_cast<const float4*>(a.q + ((size_t)(q0 + r) * a.heads + head) * HD + c * 8);
+                x0 = src[0];
+                x1 = src[1];
+            }
+            const __half2 h[4] = {__floats2half2_rn(x0.x, x0.y), __floats2half2_rn(x0.z, x0.w), __floats2half2_rn(x1.x, x1.y), __floats2half2_rn(x1.z, x1.w)};
+            uint8_t* dst = smem_raw + (qs - smem_u32(smem_raw)) + (c >> 3) * S::kPanel + r * 128 + (((c & 7) ^ (r & 7)) << 4);
+            *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(h);
+        }
+        fence_proxy_async();
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem = tmem_holder;
+    const uint32_t last_q = min(a.T, q0 + kRows) - 1, n_blocks = (a.start + last_q) / kKeys + 1;
+    bool ok = true;
+
+    if (warp == 4) {
+        if (lane == 0) {
+            const int32_t kvh = (int32_t)(head / a.group);
+            auto load = [&](const CUtensorMap* m, uint32_t dst, uint32_t bar, uint32_t i) {
+                mbar_expect_tx(bar, S::kTile);
+                for (int p = 0; p < HD / 64; p++) tma_load_3d(dst + p * S::kPanel, m, 64 * p, (int32_t)(i * kKeys), kvh, bar);
+            };
+            load(&mk, ks, k_full, 0);
+            load(&mv, vs, v_full, 0);
+            for (uint32_t i = 0; i < n_blocks && ok; i++) {
+                const uint32_t ph = i & 1;
+                // the columns of S hold P of the block before until its product is done; V's buffer is free then, too
+                if (i > 0) {
+                    if (!(ok = mbar_wait_timed(o_full, ph ^ 1, &abort_flag))) break;
+                    load(&mv, vs, v_full, i);
+                }
+                if (!(ok = mbar_wait_timed(k_full, ph, &abort_flag))) break;
+                tc_fence_after_sync();
+#pragma unroll
+                for (int s = 0; s < HD / 16; s++) {
+                    const uint32_t off = (s >> 2) * S::kPanel + (s & 3) * 32;
+                    umma_bf16(tmem, umma_desc_sw128(qs + off), umma_desc_sw128(ks + off), idesc_f16(kRows, kKeys, 0), s > 0);
+                }
+                umma_commit(s_full);
+                if (!(ok = mbar_wait_timed(s_full, ph, &abort_flag))) break;
+                if (i + 1 < n_blocks) load(&mk, ks, k_full, i + 1);
+                if (!(ok = mbar_wait_timed(v_full, ph, &abort_flag))) break;
+                if (!(ok = mbar_wait_timed(p_full, ph, &abort_flag))) break;
+                tc_fence_after_sync();
+#pragma unroll
+                for (int s = 0; s < kKeys / 16; s++)
+                    umma_f16_ts(tmem + 128, tmem + 8 * s, desc_mn_sw128(vs + s * 2048, S::kPanel), idesc_f16(kRows, HD, 1), s > 0);
+                umma_commit(o_full);
+            }
+            if (ok) ok = mbar_wait_timed(o_full, (n_blocks - 1) & 1, &abort_flag);      // nothing is in flight when the CTA leaves
+        }
+    } else {
+        const uint32_t row = warp * 32 + lane, mine = tmem + ((warp * 32) << 16), qpos = a.start + q0 + row;
+        float o[HD], m = -INFINITY, l = 0.f;       // m in units of the scaled score times log2(e)
+#pragma unroll
+        for (int j = 0; j < HD; j++) o[j] = 0.f;
+        for (uint32_t i = 0; i < n_blocks; i++) {
+            if (!(ok = mbar_wait_timed(s_full, i & 1, &abort_flag))) break;
+            tc_fence_after_sync();
+            const uint32_t key0 = i * kKeys;
+            const bool masked = key0 + kKeys - 1 > a.start + q0;      // some row of the CTA does not see the whole block
+            float mx = -INFINITY;
+#pragma unroll
+            for (int c = 0; c < kKeys / 32; c++) {
+                uint32_t r[32];
+                tmem_ld32(mine + 32 * c, r);
+                tmem_ld_wait();
+                if (masked) {
+#pragma unroll
+                    for (int j = 0; j < 32; j++)
+                        if (key0 + 32 * c + j <= qpos) mx = fmaxf(mx, __uint_as_float(r[j]));
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; j++) mx = fmaxf(mx, __uint_as_float(r[j]));
+                }
+            }
+            const float mn = fmaxf(m, mx * a.scale_log2);
+            const float ref = mn == -INFINITY ? 0.f : mn;               // no finite score yet: every factor is 0
+            const float corr = exp2_approx(m - ref);
+            m = mn;
+            float sum = 0.f;
+#pragma unroll
+            for (int c = 0; c < kKeys / 32; c++) {
+                uint32_t r[32], p[16];
+                tmem_ld32(mine + 32 * c, r);
+                tmem_ld_wait();
+                if (masked) {
+#pragma unroll
+                    for (int j = 0; j < 32; j++)
+                        if (key0 + 32 * c + j > qpos) r[j] = 0xFF800000u;
+                }
+#pragma unroll
+                for (int j = 0; j < 16; j++) {
+                    const float p0 = exp2_approx(fmaf(__uint_as_float(r[2 * j]), a.scale_log2, -ref)), p1 = exp2_approx(fmaf(__uint_as_float(r[2 * j + 1]), a.scale_log2, -ref));
+                    sum += p0 + p1;
+                    const __half2 h = __floats2half2_rn(p0, p1);
+                    p[j] = *reinterpret_cast<const uint32_t*>(&h);
+                }
+                tmem_st16(mine + 16 * c, p);       // behind what has been read: columns 0 .. 16 c + 15
+            }
+            l = fmaf(l, corr, sum);
+            tmem_st_wait();
+            tc_fence_before_sync();
+            mbar_arrive(p_full);
+            if (!(ok = mbar_wait_timed(o_full, i & 1, &abort_flag))) break;
+            tc_fence_after_sync();
+#pragma unroll
+            for (int c = 0; c < HD / 32; c++) {
+                uint32_t r[32];
+                tmem_ld32(mine + 128 + 32 * c, r);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 32; j++) o[32 * c + j] = fmaf(o[32 * c + j], corr, __uint_as_float(r[j]));
+            }
+            tc_fence_before_sync();                // ordered before the next arrival on p_full
+        }
+        if (ok && q0 + row < a.T) {
+            const float inv = l > 0.f || !(l == l) ? 1.0f / l : 0.f;
+            uint4* dst = reinterpret_cast<uint4*>(a.out + ((size_t)(q0 + row) * a.heads + head) * HD);
+#pragma unroll
+            for (int c = 0; c < HD / 8; c++) {
+                __nv_bfloat162 h[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) h[j] = __floats2bfloat162_rn(o[8 * c + 2 * j] * inv, o[8 * c + 2 * j + 1] * inv);
+                dst[c] = *reinterpret_cast<const uint4*>(h);
+            }
+        }
+    }
+    if (!ok) {
+        abort_flag = 1;
+        if (a.status) atomicExch(a.status, 1);
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after_sync();
+        tmem_dealloc(tmem, kCols);
+    }
+}
+
+template <int HD>
+static int32_t run(runit_ctx* ctx, const CUtensorMap& mk, const CUtensorMap& mv, const Args& a) {
+    static bool configured[64] = {false};
+    if (ctx->device >= 64 || !configured[ctx->device]) {
+        RUNIT_CUDA_TRY(ctx, cudaFuncSetAttribute(attention_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<HD>::kSmem));
+        if (ctx->device < 64) configured[ctx->device] = true;
+    }
+    runit_launch_chain_smem(ctx, attention_tc_kernel<HD>, dim3(a.heads, (a.T + kRows - 1) / kRows), dim3(160), Shape<HD>::kSmem, mk, mv, a);
+    return runit_after_launch(ctx, "prefill_attention_tc");
+}
+
+}  // namespace atc
+
+// More than 64 queries: below, half of a tile would be padding (one launch of the mma.sync kernel's 64-query tiles serves them).
+bool attention_tc_applies(const runit_ctx* ctx, const float* q, const void* kcache, const void* vcache, const void* out, uint32_t T, uint32_t hd) {
+    return ctx->encode_tiled && (hd == 64 || hd == 128) && T > 64 && runit_aligned(q, 16) && runit_aligned(kcache, 16) && runit_aligned(vcache, 16) && runit_aligned(out, 16);
+}
+
+int32_t attention_tc(runit_ctx* ctx, const float* q, const void* kcache, const void* vcache, void* out_bf16, uint32_t T, uint32_t heads, uint32_t kv_heads,
+                     uint32_t hd, uint32_t max_seq, uint32_t start_pos) {
+    auto encode = reinterpret_cast<CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
+                                                CUtensorMapFloatOOBfill)>(ctx->encode_tiled);
+    CUtensorMap m[2];
+    for (int i = 0; i < 2; i++) {
+        const cuuint64_t dim[3] = {hd, start_pos + T, kv_heads}, stride[2] = {hd * 2ull, (cuuint64_t)max_seq * hd * 2};
+        const cuuint32_t box[3] = {64, atc::kKeys, 1}, one[3] = {1, 1, 1};
+        const CUresult r = encode(&m[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(i ? vcache : kcache), dim, stride, box, one,
+                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return runit_fail(ctx, RUNIT_ERR_LAUNCH, "cuTensorMapEncodeTiled failed with %d", (int)r);
+    }
+    const atc::Args a{q, (__nv_bfloat16*)out_bf16, T, heads, heads / kv_heads, start_pos, 1.4426950408889634f / sqrtf((float)hd), ctx->d_status};
+    return hd == 128 ? atc::run<128>(ctx, m[0], m[1], a) : atc::run<64>(ctx, m[0], m[1], a);
+}
+
+}  // namespace runit

@@ -331,6 +331,8 @@ int32_t prefill_attention(runit_ctx* ctx, const float* q, const void* kcache, co
                           uint32_t kv_heads, uint32_t hd, uint32_t max_seq, uint32_t start_pos) {
     RUNIT_REQUIRE(ctx, hd == 128 || hd == 64, "prefill_attention: head_dim %u unsupported (64 or 128)", hd);
     RUNIT_REQUIRE(ctx, T > 0 && heads % kv_heads == 0 && (uint64_t)start_pos + T <= max_seq, "prefill_attention: bad shape");
+    if (attention_tc_applies(ctx, q, kcache, vcache, out_bf16, T, hd))
+        return attention_tc(ctx, q, kcache, vcache, out_bf16, T, heads, kv_heads, hd, max_seq, start_pos);
     const float scale = 1.0f / sqrtf((float)hd);
     const dim3 grid(heads, (T + 63) / 64);      // heads fastest: the launch order walks the query blocks from the last (most keys) to the first
     const size_t smem = (size_t)4 * 64 * (hd + 8) * 2;      // two stages of a K and a V block

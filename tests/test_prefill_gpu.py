@@ -38,6 +38,30 @@ def test_causal_attention_kernel(ctx, oracle, hd, T, start):
     assert_close(oracle, ref, got, rel_tol=5e-3, what="prefill attention hd=%d T=%d start=%d" % (hd, T, start))
 
 
+@pytest.mark.parametrize("hd", [128, 64])
+@pytest.mark.parametrize("T,start,heads,kvh", [(65, 63, 2, 2), (127, 1, 4, 1), (128, 0, 2, 1), (129, 127, 2, 2), (257, 300, 6, 3)])
+def test_causal_attention_tensor_core_tiles(ctx, oracle, hd, T, start, heads, kvh):
+    """Edges of the 128-query tiles and 128-key blocks; NaN in the cache behind the data must not show; a large score decides its
+    row.  Bound as above: one bf16 ulp of the output (the f16 roundings of q and P are 2^-11)."""
+    import runit_mac_b200 as R
+    from oracle import prefill as OP
+    n, max_seq = start + T, start + T + 40
+    rng = np.random.default_rng(T * 11 + hd + start)
+    q = rng.normal(0, 1, (T, heads * hd)).astype(np.float32)
+    q[T // 2] *= 12.0
+    kc = np.full((kvh, max_seq, hd), np.nan, np.float16)
+    vc = np.full((kvh, max_seq, hd), np.nan, np.float16)
+    kc[:, :n] = rng.normal(0, 1, (kvh, n, hd)).astype(np.float16)
+    vc[:, :n] = rng.normal(0, 1, (kvh, n, hd)).astype(np.float16)
+    ob = ctx.new_buffer(T * heads * hd * 2)
+    R.prefill_attention_f16kv(ctx, ctx.buffer_from(q), ctx.buffer_from(kc), ctx.buffer_from(vc), ob, T, heads, kvh, hd, max_seq, start)
+    ctx.flush()
+    got = bf16_bits_to_f32(ob.download(np.uint16, T * heads * hd)).reshape(T, heads * hd)
+    kc[:, n:], vc[:, n:] = 0, 0
+    ref = OP.causal_attention_f16(q, kc, vc, heads, kvh, hd, start_pos=start)
+    assert_close(oracle, ref, got, rel_tol=5e-3, what="attention tiles hd=%d T=%d start=%d" % (hd, T, start))
+
+
 def test_small_model_prefill_matches_restatement_and_decode(ctx, oracle):
     import runit_mac_b200 as R
     from oracle import prefill as OP
