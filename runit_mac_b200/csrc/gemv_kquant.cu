@@ -152,27 +152,29 @@ __global__ void __launch_bounds__(kWarps * 32) gemv_kquant_kernel(const Args a) 
     cp_async_wait<0>();
 }
 
-// ───────────────────────── Q6_K, tile kernel ─────────────────────────
-// Lane = row.  Every warp owns a tile of 32 rows and walks all superblocks of K (4 tiles per CTA, no reduction across
-// warps).  Per superblock the warp copies the 32 rows' 210 bytes into its own two-stage ring (4-byte cp.async from the aligned word
-// below each row's start: a row's superblock starts on a 2-byte boundary only) together with the 256 activations, which
-// it then turns into three signed 8-bit limbs per element with one power-of-two scale per 32 (prep_int_block: 23 bits,
-// exact to f32 rounding).  Every lane decodes its own row: a word of ql low nibbles, a word of ql high nibbles and a word
-// of qh give four weights each of the reference's four groups q1..q4 (forward.rs:920-949) as 6-bit fields in bytes,
-// which meet the limbs in dp4a; the "- 32" is taken through the blocks' sums.  About 1.7 instructions per weight instead
-// of 7, and scales, d and the activations are read once per row-lane instead of once per weight.
-namespace q6t {
+// ───────────────────────── Q6_K and Q5_K, tile kernel ─────────────────────────
+// Every warp owns a tile of 32 rows and walks all 256-weight units of K (4 tiles per CTA), or a share of them (split).  Per unit it
+// copies the rows' packed bytes into its own two-stage ring together with the 256 activations, which it turns into three signed
+// 8-bit limbs per element with one power-of-two scale per 32 (prep_int_block: 23 bits, exact to f32 rounding).  The 5- and 6-bit
+// fields, unsigned bytes once their upper bits are merged in, are the A operand of mma.sync.m16n8k32, one MMA per 16 rows x 32 weights:
+//   * the eight columns carry limbs 0 and 1 of FOUR blocks at once: column n holds limb n & 1 of block n >> 1 of a group of four and
+//     zeros in the MMAs of the group's other blocks, so four MMAs add into one register tile;
+//   * limb 2 of all eight blocks goes the same way into a second tile, column n = block (n >> 1) + 4 (n & 1), so that lane
+//     (g, t) ends up with every limb's exact sums of blocks t and t + 4 of its rows g and g + 8.
+// 16 MMAs for 16 rows x 256 weights; integers, combination and error against 64 bits are those of dp4a on the same limbs.
+// Bound: instruction issue (unpacking, the activations' limbs where they are not prepared) at 11 warps per SM, which the stages'
+// shared memory allows.  Measured, lane = row with dp4a before: Q6_K 152064 x 3584 164 -> 127 us (3.5 TB/s), 3584 x 18944 25.6 ->
+// 22.4, 32000 x 2048 26.1 -> 23.5; Q5_K 152064 x 3584 106 -> 100, 3584 x 3584 8.4 -> 7.8.
+namespace kt {
 
-constexpr int kPitch = 220;                       // bytes per row in a stage: 53 words + 2 (an odd number of words)
-constexpr int kXOff = 32 * kPitch;                // activations of the unit: 1024 bytes raw, prepared in place
-constexpr int kStage = kXOff + 1024;
+template <int FMT> struct Tile {
+    static constexpr int kUnit = FMT == RUNIT_FMT_Q6K ? 210 : 176;
+    // Q6_K rows start on even bytes only: the unit arrives as the 16-byte pieces that hold it (14 of them) and is read from its
+    // offset; 240 and 176 are odd multiples of 16, which spreads the eight rows of a fragment over the banks
+    static constexpr int kPitch = FMT == RUNIT_FMT_Q6K ? 240 : 176;
+    static constexpr int kXOff = 32 * kPitch, kStage = kXOff + 1024, kSmem = 4 * 2 * kStage;
+};
 constexpr int kS = 2;
-
-__device__ __forceinline__ int dp4a_u8s8(uint32_t a, uint32_t b, int c) {
-    int d;
-    asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
 
 struct Args {
     const uint8_t* w;
@@ -186,269 +188,242 @@ struct Args {
     uint32_t split;
     float* part;
     uint32_t* tickets;       // one word per tile, zero at rest
+    const uint8_t* xq;       // PRE: the prepared activations, kXq bytes per unit
+};
+constexpr int kXq = IntX<8>::BYTES;                  // 832: a multiple of 16
+
+// The activations' limbs, scales and sums, once per call: one warp per unit.
+__global__ void __launch_bounds__(32) kquant_prepare_kernel(const float* __restrict__ x, uint8_t* __restrict__ xq) {
+    __shared__ __align__(16) uint8_t out[kXq];
+    grid_launch_dependents();                        // the GEMV may request its first weights
+    grid_dependency_wait();
+    const int lane = threadIdx.x;
+    const float4* xr = reinterpret_cast<const float4*>(x + (size_t)blockIdx.x * 256) + 2 * lane;
+    const float4 a = xr[0], b = xr[1];
+    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    prep_int_block<8, 8, 0>(out, v, lane);
+    __syncwarp();
+    uint4* dst = reinterpret_cast<uint4*>(xq + (size_t)blockIdx.x * kXq);
+    dst[lane] = reinterpret_cast<const uint4*>(out)[lane];
+    if (lane < kXq / 16 - 32) dst[32 + lane] = reinterpret_cast<const uint4*>(out)[32 + lane];
+}
+
+__device__ __forceinline__ uint32_t ld32(const uint8_t* p) { return *reinterpret_cast<const uint32_t*>(p); }
+
+// Unpacked words of 16 rows x one block for this lane: a[0], a[1] = first word of rows g and g + 8, a[2], a[3] = second word.
+// Words 2t and 2t + 1 of the block's eight.
+template <int FMT> struct Rows;
+
+template <> struct Rows<RUNIT_FMT_Q6K> {             // forward.rs:920-949
+    const uint8_t* p[2];                             // the rows' units; even addresses
+    uint32_t q[2][4][2];                             // [row][group of 32 of the half][word]
+    __device__ __forceinline__ void init(const uint8_t* r0, const uint8_t* r1) { p[0] = r0; p[1] = r1; }
+    __device__ __forceinline__ void load(int b, int t) {
+        if (b & 3) return;
+        const int h = b >> 2;
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const uint8_t* al = p[r] - (reinterpret_cast<uintptr_t>(p[r]) & 2u);
+            const uint32_t sh = (uint32_t)(reinterpret_cast<uintptr_t>(p[r]) & 2u) * 8u;
+            auto pair = [&](int off, uint32_t& w0, uint32_t& w1) {
+                const uint32_t x0 = ld32(al + off), x1 = ld32(al + off + 4), x2 = ld32(al + off + 8);
+                w0 = __funnelshift_r(x0, x1, sh);
+                w1 = __funnelshift_r(x1, x2, sh);
+            };
+            uint32_t a[2], c[2], u[2];
+            pair(64 * h + 8 * t, a[0], a[1]);
+            pair(64 * h + 32 + 8 * t, c[0], c[1]);
+            pair(128 + 32 * h + 8 * t, u[0], u[1]);
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                q[r][0][i] = (a[i] & 0x0F0F0F0Fu) | ((u[i] << 4) & 0x30303030u);
+                q[r][1][i] = (c[i] & 0x0F0F0F0Fu) | ((u[i] << 2) & 0x30303030u);
+                q[r][2][i] = ((a[i] >> 4) & 0x0F0F0F0Fu) | (u[i] & 0x30303030u);
+                q[r][3][i] = ((c[i] >> 4) & 0x0F0F0F0Fu) | ((u[i] >> 2) & 0x30303030u);
+            }
+        }
+    }
+    __device__ __forceinline__ uint32_t word(int b, int r, int i) const { return q[r][b & 3][i]; }
+    // d * scale * (sum q v - 32 sum v) * s of block b = t + 4 * gr; the reference takes scales[2 b]
+    __device__ __forceinline__ float value(int gr, int r, int t, float dot, float sx, float sv) const {
+        const int b = t + 4 * gr;
+        const float d = __half2float(*reinterpret_cast<const __half*>(p[r] + 208));
+        const float sc = (float)reinterpret_cast<const int8_t*>(p[r])[192 + 2 * b];
+        return d * ((sc * sx) * (dot - 32.f * sv));
+    }
 };
 
-__global__ void __launch_bounds__(128) gemv_q6k_tile_kernel(const Args a) {
-    extern __shared__ __align__(16) uint8_t q6_smem[];
+template <> struct Rows<RUNIT_FMT_Q5K> {             // forward.rs:979-1012
+    const uint8_t* p[2];                             // 16-byte aligned
+    uint32_t q[2][2][2];                             // [row][low, high nibbles of the chunk][word]
+    __device__ __forceinline__ void init(const uint8_t* r0, const uint8_t* r1) { p[0] = r0; p[1] = r1; }
+    __device__ __forceinline__ void load(int b, int t) {
+        if (b & 1) return;
+        const int j = b >> 1;
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const uint2 w = *reinterpret_cast<const uint2*>(p[r] + 48 + 32 * j + 8 * t);
+            // this lane's eight elements of a block have their fifth bits in one byte
+            const uint32_t fl = p[r][16 + 8 * j + t], fh = p[r][16 + 8 * j + 4 + t];
+            q[r][0][0] = (w.x & 0x0F0F0F0Fu) | (((fl & 15u) * 0x02040810u) & 0x10101010u);
+            q[r][0][1] = (w.y & 0x0F0F0F0Fu) | (((fl >> 4) * 0x02040810u) & 0x10101010u);
+            q[r][1][0] = ((w.x >> 4) & 0x0F0F0F0Fu) | (((fh & 15u) * 0x02040810u) & 0x10101010u);
+            q[r][1][1] = ((w.y >> 4) & 0x0F0F0F0Fu) | (((fh >> 4) * 0x02040810u) & 0x10101010u);
+        }
+    }
+    __device__ __forceinline__ uint32_t word(int b, int r, int i) const { return q[r][b & 1][i]; }
+    __device__ __forceinline__ float value(int gr, int r, int t, float dot, float sx, float sv) const {
+        const uint4 hd = *reinterpret_cast<const uint4*>(p[r]);                                // d, dmin, packed scales and mins
+        const float d = half_bits_to_float(hd.x), dmin = half_bits_to_float(hd.x >> 16);
+        const Q4KScales s = q4k_unpack_scales(hd.y, hd.z, hd.w);
+        const uint32_t sel = 0x4440u + (uint32_t)((t >> 1) + 2 * gr);                          // block b: index b / 2, + 4 if odd
+        const float sc = (float)__byte_perm((t & 1) ? s.sh : s.sl, 0u, sel), mn = (float)__byte_perm((t & 1) ? s.mh : s.ml, 0u, sel);
+        return sx * (d * sc * dot - dmin * mn * sv);
+    }
+};
+
+// PRE: the activations were prepared by a launch of their own (their limbs are a sixth of the instructions per unit otherwise).
+template <int FMT, bool PRE>
+__global__ void __launch_bounds__(128) gemv_kquant_tile_kernel(const Args a) {
+    using T = Tile<FMT>;
+    extern __shared__ __align__(16) uint8_t kt_smem[];
     __shared__ float red[4][32];
     __shared__ uint32_t s_last;
     grid_launch_dependents();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint8_t* ring = q6_smem + warp * (kS * kStage);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    uint8_t* ring = kt_smem + warp * (kS * T::kStage);
     // split == 0: every warp owns a tile of 32 rows and walks all of K; else the CTA owns tile blockIdx.x
     const uint32_t row0 = a.split ? blockIdx.x * 32 : (blockIdx.x * 4 + warp) * 32;
     if (row0 >= a.m) return;
     const uint32_t rows_here = min(32u, a.m - row0);
     const uint32_t u0 = a.split ? blockIdx.y * 4 + warp : 0u, ustep = a.split ? 4u * a.split : 1u;
     const int n_it = u0 < a.nb ? (int)((a.nb - u0 + ustep - 1) / ustep) : 0;
+    const size_t first = (size_t)row0 * a.row_bytes, total = (size_t)a.m * a.row_bytes;
 
-    auto issue = [&](int it) {
-        if (it < n_it) {
-            const uint32_t u = u0 + ustep * (uint32_t)it;
-            const uint32_t st = smem_u32(ring + (it % kS) * kStage);
-            // row r: 53 words from the aligned word below its superblock; lane l copies words l and l + 32 (l < 21).  With
-            // shift 0 the last word holds only two bytes of the row (its f16 d): that copy takes two bytes from memory
-            // (the rest is filled with zeros), so nothing is read past the row.  Branch-free: the size is an operand.
-            const uint8_t* p = a.w + (size_t)row0 * a.row_bytes + (size_t)u * 210;
-            uint32_t dst = st + 4 * lane;
-#pragma unroll 4
-            for (uint32_t r = 0; r < rows_here; r++) {
-                const uint32_t shift = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3u);      // 0 or 2
-                const uint8_t* src = p - shift + 4 * lane;
-                cp_async4(dst, src);
-                if (lane < 21) {
-                    const uint32_t nbytes = (lane == 20 && shift == 0) ? 2u : 4u;
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst + 128), "l"(src + 128), "r"(nbytes) : "memory");
-                }
-                p += a.row_bytes;
-                dst += kPitch;
-            }
-            const float* xu = a.x + (size_t)u * 256;
-            cp_async16(st + kXOff + 16 * lane, xu + 4 * lane);
-            cp_async16(st + kXOff + 16 * (32 + lane), xu + 4 * (32 + lane));
-        }
-        cp_async_commit();
-    };
-    grid_dependency_wait();      // x (and the residual) may come from the previous kernel of the chain
+    auto issue_w = [&](int it) {
+        if (it >= n_it) return;
+        const uint32_t u = u0 + ustep * (uint32_t)it;
+        const uint32_t st = smem_u32(ring + (it % kS) * T::kStage);
+        if (FMT == RUNIT_FMT_Q6K) {
+            // four lanes per row, 16-byte pieces 4 i + t from the one that holds the unit's first byte (the matrix itself is
+            // 16-byte aligned); nothing is read past the matrix
+            const bool inner = row0 + 32 < a.m;      // a row follows: whole pieces
 #pragma unroll
-    for (int s = 0; s < kS; s++) issue(s);
-    float acc = 0.f;
-    for (int it = 0; it < n_it; it++) {
-        cp_async_wait<kS - 1>();
-        __syncwarp();
-        uint8_t* stg = ring + (it % kS) * kStage;
-        {   // activations of the unit -> limbs, scales, block sums (in place)
-            float v[8];
-            const float4* xr = reinterpret_cast<const float4*>(stg + kXOff) + 2 * lane;
-            const float4 t0 = xr[0], t1 = xr[1];
-            v[0] = t0.x; v[1] = t0.y; v[2] = t0.z; v[3] = t0.w; v[4] = t1.x; v[5] = t1.y; v[6] = t1.z; v[7] = t1.w;
-            __syncwarp();
-            prep_int_block<8, 8, 0>(stg + kXOff, v, lane);
-            __syncwarp();
-        }
-        if ((uint32_t)lane < rows_here) {
-            const uint32_t u = u0 + ustep * (uint32_t)it;
-            const uint32_t sh8 = (uint32_t)((((size_t)(row0 + lane) * a.row_bytes + (size_t)u * 210) & 3u) * 8u);   // 0 or 16
-            const uint32_t* rw = reinterpret_cast<const uint32_t*>(stg + lane * kPitch);
-            uint32_t rv[54];                     // the row's words, once; word 53 is never part of a result
+            for (int rg = 0; rg < 4; rg++) {
+                const uint32_t r = 8 * rg + g;
+                const size_t from = (first + (size_t)r * a.row_bytes + (size_t)u * 210) & ~(size_t)15;
+                const uint8_t* src = a.w + from + 16 * t;
+                const uint32_t dst = st + r * T::kPitch + 16 * t;
+                if (inner) {
 #pragma unroll
-            for (int j = 0; j < 53; j++) rv[j] = rw[j];
-            rv[53] = 0;
-            auto W = [&](int j) -> uint32_t { return __funnelshift_r(rv[j], rv[j + 1], sh8); };
-            const uint8_t* xq = stg + kXOff;
-            const float* sx = reinterpret_cast<const float*>(xq + IntX<8>::SCALE);
-            const int* sv = reinterpret_cast<const int*>(xq + IntX<8>::VSUM);
-            const uint32_t sc_w[4] = {W(48), W(49), W(50), W(51)};           // 16 signed scales
-            const float d = half_bits_to_float(W(52) & 0xFFFFu);
-            float unit_acc = 0.f;
+                    for (int i = 0; i < 3; i++) cp_async16(dst + 64 * i, src + 64 * i);
+                    if (t < 2) cp_async16(dst + 192, src + 192);
+                } else if (r < rows_here) {
+                    const uint32_t left = (uint32_t)min((size_t)256, total - from);
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                // the 128 weights of this half as 6-bit fields in bytes: q[j][g] = elements 32 j + 4 g .. + 3 of the half
-                uint32_t q[4][8];
-#pragma unroll
-                for (int g = 0; g < 8; g++) {
-                    const uint32_t wa = W(16 * h + g), wc = W(16 * h + 8 + g), wh = W(32 + 8 * h + g);
-                    q[0][g] = (wa & 0x0F0F0F0Fu) | ((wh & 0x03030303u) << 4);
-                    q[1][g] = (wc & 0x0F0F0F0Fu) | ((wh & 0x0C0C0C0Cu) << 2);
-                    q[2][g] = ((wa >> 4) & 0x0F0F0F0Fu) | (wh & 0x30303030u);
-                    q[3][g] = ((wc >> 4) & 0x0F0F0F0Fu) | ((wh >> 2) & 0x30303030u);
-                }
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int b = 4 * h + j;
-                    const uint4* xl = reinterpret_cast<const uint4*>(xq + b * 96);     // limb l of the block: xl[2 l], xl[2 l + 1]
-                    int s0 = 0, s1 = 0, s2 = 0;
-#pragma unroll
-                    for (int hf = 0; hf < 2; hf++) {
-                        const uint4 l0 = xl[hf], l1 = xl[2 + hf], l2 = xl[4 + hf];
-                        const uint32_t x0[4] = {l0.x, l0.y, l0.z, l0.w}, x1[4] = {l1.x, l1.y, l1.z, l1.w}, x2[4] = {l2.x, l2.y, l2.z, l2.w};
-#pragma unroll
-                        for (int c = 0; c < 4; c++) {
-                            s0 = dp4a_u8s8(q[j][4 * hf + c], x0[c], s0);
-                            s1 = dp4a_u8s8(q[j][4 * hf + c], x1[c], s1);
-                            s2 = dp4a_u8s8(q[j][4 * hf + c], x2[c], s2);
-                        }
+                    for (int i = 0; i < 4; i++) {
+                        const uint32_t at = 64 * i + 16 * t;
+                        if (at < left && at < 224)
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst + 64 * i), "l"(src + 64 * i), "r"(min(16u, left - at)) : "memory");
                     }
-                    // sum q * v over the block, exact in every limb; the reference's q - 32 through the block's sum of v
-                    const float dot = fmaf((float)s2, 65536.f, fmaf((float)s1, 256.f, (float)s0)) - 32.f * (float)sv[b];
-                    const int scb = (int)(int8_t)((sc_w[(2 * b) >> 2] >> (8 * ((2 * b) & 3))) & 0xFFu);   // scales[8 half + 2 group]
-                    unit_acc = fmaf((float)scb * sx[b], dot, unit_acc);
                 }
             }
-            acc = fmaf(d, unit_acc, acc);
-        }
-        __syncwarp();
-        issue(it + kS);
-    }
-    cp_async_wait<0>();
-    if (a.split == 0) {
-        if ((uint32_t)lane < rows_here) {
-            const uint32_t row = row0 + lane;
-            a.y[row] = a.res ? a.res[row] + acc : acc;
-        }
-        return;
-    }
-    red[warp][lane] = acc;
-    __syncthreads();
-    if (warp == 0) {
-        const float v = ((red[0][lane] + red[1][lane]) + red[2][lane]) + red[3][lane];
-        if ((uint32_t)lane < rows_here) __stcg(&a.part[(size_t)blockIdx.y * a.m + row0 + lane], v);
-        __threadfence();
-        __syncwarp();
-        if (lane == 0) s_last = atomicAdd(&a.tickets[blockIdx.x], 1u) == a.split - 1;
-    }
-    __syncthreads();
-    if (s_last && warp == 0) {
-        __threadfence();
-        if ((uint32_t)lane < rows_here) {
-            const uint32_t row = row0 + lane;
-            float v = a.res ? a.res[row] : 0.f;
-            for (uint32_t sp = 0; sp < a.split; sp++) v += __ldcg(&a.part[(size_t)sp * a.m + row]);
-            a.y[row] = v;
-        }
-        if (lane == 0) a.tickets[blockIdx.x] = 0;
-    }
-}
-
-}  // namespace q6t
-
-// ───────────────────────── Q5_K, tile kernel ─────────────────────────
-// The same arrangement for Q5_K: superblocks are 176 bytes and rows 16-byte aligned, so a tile's unit arrives by 16-byte
-// cp.async (11 per row) at a pitch of 176 bytes (an odd multiple of 16: lane = row reads 128 bits without bank conflicts).
-// A word of qs gives four low-nibble weights of block 2j and four high-nibble weights of block 2j + 1; their fifth bits
-// are a nibble of qh (bit e % 8 of qh[e / 8], forward.rs:979-1012), spread into bit 4 of four bytes by one multiply.
-namespace q5t {
-
-constexpr int kPitch = 176;
-constexpr int kXOff = 32 * kPitch;
-constexpr int kStage = kXOff + 1024;
-constexpr int kS = 2;
-
-__global__ void __launch_bounds__(128) gemv_q5k_tile_kernel(const q6t::Args a) {
-    extern __shared__ __align__(16) uint8_t q5_smem[];
-    __shared__ float red[4][32];
-    __shared__ uint32_t s_last;
-    grid_launch_dependents();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint8_t* ring = q5_smem + warp * (kS * kStage);
-    const uint32_t row0 = a.split ? blockIdx.x * 32 : (blockIdx.x * 4 + warp) * 32;
-    if (row0 >= a.m) return;
-    const uint32_t rows_here = min(32u, a.m - row0);
-    const uint32_t u0 = a.split ? blockIdx.y * 4 + warp : 0u, ustep = a.split ? 4u * a.split : 1u;
-    const int n_it = u0 < a.nb ? (int)((a.nb - u0 + ustep - 1) / ustep) : 0;
-
-    auto issue = [&](int it) {
-        if (it < n_it) {
-            const uint32_t u = u0 + ustep * (uint32_t)it;
-            const uint32_t st = smem_u32(ring + (it % kS) * kStage);
-            const uint8_t* base = a.w + (size_t)row0 * a.row_bytes + (size_t)u * 176;
+        } else {
+            const uint8_t* base = a.w + first + (size_t)u * 176;
 #pragma unroll
             for (int i = 0; i < 11; i++) {
                 const uint32_t c = (uint32_t)lane + 32u * i, r = c / 11u, col = c - 11u * r;      // 352 chunks of 16 bytes
-                if (r < rows_here) cp_async16(st + r * kPitch + 16 * col, base + (size_t)r * a.row_bytes + 16 * col);
+                if (r < rows_here) cp_async16(st + r * T::kPitch + 16 * col, base + (size_t)r * a.row_bytes + 16 * col);
             }
-            const float* xu = a.x + (size_t)u * 256;
-            cp_async16(st + kXOff + 16 * lane, xu + 4 * lane);
-            cp_async16(st + kXOff + 16 * (32 + lane), xu + 4 * (32 + lane));
+        }
+    };
+    auto issue_x = [&](int it) {
+        if (it < n_it) {
+            const uint32_t u = u0 + ustep * (uint32_t)it, st = smem_u32(ring + (it % kS) * T::kStage) + T::kXOff;
+            const uint8_t* xu = PRE ? a.xq + (size_t)u * kXq : reinterpret_cast<const uint8_t*>(a.x + (size_t)u * 256);
+            cp_async16(st + 16 * lane, xu + 16 * lane);
+            if (!PRE || lane < kXq / 16 - 32) cp_async16(st + 16 * (32 + lane), xu + 16 * (32 + lane));
         }
         cp_async_commit();
     };
+    // the weights do not depend on the kernel before; its output may be x or the residual
+#pragma unroll
+    for (int s = 0; s < kS; s++) issue_w(s);
     grid_dependency_wait();
 #pragma unroll
-    for (int s = 0; s < kS; s++) issue(s);
-    float acc = 0.f;
+    for (int s = 0; s < kS; s++) issue_x(s);
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};             // rows g, g + 8, g + 16, g + 24, this lane's blocks
     for (int it = 0; it < n_it; it++) {
         cp_async_wait<kS - 1>();
         __syncwarp();
-        uint8_t* stg = ring + (it % kS) * kStage;
-        {
+        uint8_t* stg = ring + (it % kS) * T::kStage;
+        if (!PRE) {   // activations of the unit -> limbs, scales, block sums (in place)
             float v[8];
-            const float4* xr = reinterpret_cast<const float4*>(stg + kXOff) + 2 * lane;
+            const float4* xr = reinterpret_cast<const float4*>(stg + T::kXOff) + 2 * lane;
             const float4 t0 = xr[0], t1 = xr[1];
             v[0] = t0.x; v[1] = t0.y; v[2] = t0.z; v[3] = t0.w; v[4] = t1.x; v[5] = t1.y; v[6] = t1.z; v[7] = t1.w;
             __syncwarp();
-            prep_int_block<8, 8, 0>(stg + kXOff, v, lane);
+            prep_int_block<8, 8, 0>(stg + T::kXOff, v, lane);
             __syncwarp();
         }
-        if ((uint32_t)lane < rows_here) {
-            const uint4* ru = reinterpret_cast<const uint4*>(stg + lane * kPitch);
-            const uint8_t* xq = stg + kXOff;
-            const float* sx = reinterpret_cast<const float*>(xq + IntX<8>::SCALE);
-            const int* sv = reinterpret_cast<const int*>(xq + IntX<8>::VSUM);
-            const uint4 hd = ru[0];                                   // d, dmin, 12 bytes of packed 6-bit scales and mins
-            const float d = half_bits_to_float(hd.x), dmin = half_bits_to_float(hd.x >> 16);
-            const Q4KScales sc = q4k_unpack_scales(hd.y, hd.z, hd.w);   // get_scale_min_k4 for j (sl, ml) and j + 4 (sh, mh)
-            const uint4 h0 = ru[1], h1 = ru[2];
-            const uint32_t qh[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-            float unit_acc = 0.f;
+        const uint8_t* xq = stg + T::kXOff;
+        // this lane's column: limb g & 1 of blocks g >> 1 and (g >> 1) + 4; limb 2 of block (g >> 1) + 4 (g & 1)
+        uint32_t bx[2][2], bz[2];
+        {
+            const uint8_t *c0 = xq + (g >> 1) * 96 + (g & 1) * 32, *c1 = c0 + 4 * 96, *cz = xq + ((g >> 1) + 4 * (g & 1)) * 96 + 64;
+            const int o0 = 8 * t, o1 = 8 * t + 4;
+            bx[0][0] = ld32(c0 + o0); bx[0][1] = ld32(c0 + o1);
+            bx[1][0] = ld32(c1 + o0); bx[1][1] = ld32(c1 + o1);
+            bz[0] = ld32(cz + o0); bz[1] = ld32(cz + o1);
+        }
+        uint32_t shift[4];
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const uint4 qa = ru[3 + 2 * j], qb = ru[4 + 2 * j];
-                const uint32_t w[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-                uint32_t lo[8], hi[8];
+        for (int i = 0; i < 4; i++)
+            shift[i] = FMT == RUNIT_FMT_Q6K ? (uint32_t)(first + (size_t)(8 * i + g) * a.row_bytes + (size_t)(u0 + ustep * (uint32_t)it) * 210) & 15u : 0u;
+        const float* sx = reinterpret_cast<const float*>(xq + IntX<8>::SCALE);
+        const int* sv = reinterpret_cast<const int*>(xq + IntX<8>::VSUM);
 #pragma unroll
-                for (int g = 0; g < 8; g++) {
-                    const int sh = 8 * (g >> 1) + 4 * (g & 1);
-                    const uint32_t nl = (qh[2 * j] >> sh) & 15u, nh = (qh[2 * j + 1] >> sh) & 15u;
-                    lo[g] = (w[g] & 0x0F0F0F0Fu) | (((nl * 0x00204081u) & 0x01010101u) << 4);
-                    hi[g] = ((w[g] >> 4) & 0x0F0F0F0Fu) | (((nh * 0x00204081u) & 0x01010101u) << 4);
-                }
+        for (int mt = 0; mt < 2; mt++) {
+            Rows<FMT> rows;
+            rows.init(stg + (16 * mt + g) * T::kPitch + shift[2 * mt], stg + (16 * mt + 8 + g) * T::kPitch + shift[2 * mt + 1]);
+            int c[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}}, z[4] = {0, 0, 0, 0};
 #pragma unroll
-                for (int half = 0; half < 2; half++) {
-                    const int b = 2 * j + half;
-                    const uint32_t* q = half ? hi : lo;
-                    const uint4* xl = reinterpret_cast<const uint4*>(xq + b * 96);
-                    int s0 = 0, s1 = 0, s2 = 0;
-#pragma unroll
-                    for (int hf = 0; hf < 2; hf++) {
-                        const uint4 l0 = xl[hf], l1 = xl[2 + hf], l2 = xl[4 + hf];
-                        const uint32_t x0[4] = {l0.x, l0.y, l0.z, l0.w}, x1[4] = {l1.x, l1.y, l1.z, l1.w}, x2[4] = {l2.x, l2.y, l2.z, l2.w};
-#pragma unroll
-                        for (int c = 0; c < 4; c++) {
-                            s0 = q6t::dp4a_u8s8(q[4 * hf + c], x0[c], s0);
-                            s1 = q6t::dp4a_u8s8(q[4 * hf + c], x1[c], s1);
-                            s2 = q6t::dp4a_u8s8(q[4 * hf + c], x2[c], s2);
-                        }
-                    }
-                    const float dot = fmaf((float)s2, 65536.f, fmaf((float)s1, 256.f, (float)s0));
-                    const float scw = (float)(((half ? sc.sh : sc.sl) >> (8 * j)) & 0xFFu), mnw = (float)(((half ? sc.mh : sc.ml) >> (8 * j)) & 0xFFu);
-                    unit_acc = fmaf(sx[b], d * scw * dot - dmin * mnw * (float)sv[b], unit_acc);
-                }
+            for (int b = 0; b < 8; b++) {
+                rows.load(b, t);
+                const bool mine = (g >> 1) == (b & 3), third = mine && (g & 1) == (b >> 2);
+                const uint32_t a0 = rows.word(b, 0, 0), a1 = rows.word(b, 1, 0), a2 = rows.word(b, 0, 1), a3 = rows.word(b, 1, 1);
+                mma_u8s8_acc(c[b >> 2], a0, a1, a2, a3, mine ? bx[b >> 2][0] : 0u, mine ? bx[b >> 2][1] : 0u);
+                mma_u8s8_acc(z, a0, a1, a2, a3, third ? bz[0] : 0u, third ? bz[1] : 0u);
             }
-            acc += unit_acc;
+#pragma unroll
+            for (int r = 0; r < 2; r++)
+#pragma unroll
+                for (int gr = 0; gr < 2; gr++) {
+                    // sum q * v over the block, exact in every limb
+                    const float dot = fmaf((float)z[2 * r + gr], 65536.f, (float)(c[gr][2 * r + 1] * 256 + c[gr][2 * r]));   // |.| < 63 * 32 * 128 * 257 < 2^27
+                    acc[2 * mt + r] += rows.value(gr, r, t, dot, sx[t + 4 * gr], (float)sv[t + 4 * gr]);
+                }
         }
         __syncwarp();
-        issue(it + kS);
+        issue_w(it + kS);
+        issue_x(it + kS);
     }
     cp_async_wait<0>();
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 1);
+        acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 2);
+        if (t == 0) red[warp][8 * i + g] = acc[i];
+    }
     if (a.split == 0) {
+        __syncwarp();
         if ((uint32_t)lane < rows_here) {
             const uint32_t row = row0 + lane;
-            a.y[row] = a.res ? a.res[row] + acc : acc;
+            const float v = red[warp][lane];
+            a.y[row] = a.res ? a.res[row] + v : v;
         }
         return;
     }
-    red[warp][lane] = acc;
     __syncthreads();
     if (warp == 0) {
         const float v = ((red[0][lane] + red[1][lane]) + red[2][lane]) + red[3][lane];
@@ -470,11 +445,12 @@ __global__ void __launch_bounds__(128) gemv_q5k_tile_kernel(const q6t::Args a) {
     }
 }
 
-}  // namespace q5t
+}  // namespace kt
 
 // ───────────────────────── Q5_0, tile kernel ─────────────────────────
-// Q5_0 with K a multiple of 256: a unit is eight 22-byte blocks (176 bytes, 256 weights), rows are then multiples of
-// 176 bytes and the copy is the Q5_K one (16-byte cp.async, pitch 176).  Inside the unit the blocks alternate between
+// Lane = row, three dp4a per four weights.  (On the MMAs of the kernel above, whose fragments re-read a block's fifth bits in four
+// lanes, 18944 x 3584 took 21.9 us against 18.6.)  K a multiple of 256: a unit is eight 22-byte blocks (176 bytes, 256 weights),
+// rows are then multiples of 176 bytes and the copy is the Q5_K one (16-byte cp.async, pitch 176).  Inside the unit the blocks alternate between
 // word-aligned and two bytes off, which a compile-time funnel shift takes care of.  A word of qs gives four low-nibble weights (elements 4 g ..) and four
 // high-nibble weights (elements 16 + 4 g ..); their fifth bits are nibbles g and 4 + g of qh (forward.rs:900-918); the
 // "- 16" is taken through the block's sum of activations.
@@ -485,7 +461,7 @@ constexpr int kXOff = 32 * kPitch;
 constexpr int kStage = kXOff + 1024;
 constexpr int kS = 2;
 
-__global__ void __launch_bounds__(128) gemv_q5_0_tile_kernel(const q6t::Args a) {
+__global__ void __launch_bounds__(128) gemv_q5_0_tile_kernel(const kt::Args a) {
     extern __shared__ __align__(16) uint8_t q50_smem[];
     __shared__ float red[4][32];
     __shared__ uint32_t s_last;
@@ -562,9 +538,9 @@ __global__ void __launch_bounds__(128) gemv_q5_0_tile_kernel(const q6t::Args a) 
                     for (int g = 0; g < 4; g++) {
                         const uint32_t nib = (qh >> (16 * hf + 4 * g)) & 15u;
                         const uint32_t q = ((hf ? (w[g] >> 4) : w[g]) & 0x0F0F0F0Fu) | (((nib * 0x00204081u) & 0x01010101u) << 4);
-                        s0 = q6t::dp4a_u8s8(q, x0[g], s0);
-                        s1 = q6t::dp4a_u8s8(q, x1[g], s1);
-                        s2 = q6t::dp4a_u8s8(q, x2[g], s2);
+                        s0 = dp4a_us(q, x0[g], s0);
+                        s1 = dp4a_us(q, x1[g], s1);
+                        s2 = dp4a_us(q, x2[g], s2);
                     }
                 }
                 const float dot = fmaf((float)s2, 65536.f, fmaf((float)s1, 256.f, (float)s0)) - 16.f * (float)sv[b];
@@ -618,7 +594,7 @@ static int32_t launch(runit_ctx* ctx, const char* name, const void* w, const voi
     // the tile kernel needs a tile of 32 rows per warp: with fewer than two warps' worth of tiles per scheduler the first
     // kernel (one warp per row) keeps more of the machine busy
     if ((FMT != RUNIT_FMT_Q5_0 || k % 256 == 0) && ctx->tune.kquant_variant != 1) {
-        q6t::Args t;
+        kt::Args t;
         const uint32_t tiles = (m + 31) / 32, sms = (uint32_t)ctx->sm_count, nbk = k / 256;
         // few tiles: shares of K go to different CTAs (2..16 shares, about one superblock per warp at least, fewer than 8 CTAs
         // per SM; measured on 3584 x 3584: 4 shares 15 -> 9 us, and on 18944 x 3584 two shares gain nothing)
@@ -640,12 +616,28 @@ static int32_t launch(runit_ctx* ctx, const char* name, const void* w, const voi
         t.m = m;
         t.nb = k / 256;
         t.row_bytes = (k / 256) * (FMT == RUNIT_FMT_Q6K ? 210u : 176u);
-        constexpr int smem = FMT == RUNIT_FMT_Q6K ? 4 * q6t::kS * q6t::kStage : FMT == RUNIT_FMT_Q5K ? 4 * q5t::kS * q5t::kStage : 4 * q50t::kS * q50t::kStage;
-        auto kern = FMT == RUNIT_FMT_Q6K ? q6t::gemv_q6k_tile_kernel : FMT == RUNIT_FMT_Q5K ? q5t::gemv_q5k_tile_kernel : q50t::gemv_q5_0_tile_kernel;
-        static bool configured[64] = {false};
-        if (ctx->device >= 0 && ctx->device < 64 && !configured[ctx->device]) {
+        // the preparing launch costs 2 us: from 150 MB of weights on it pays (Q6_K 152064 x 3584 147 -> 127 us; Q5_K 50304 x 2048,
+        // 72 MB, 33 us without and 35 with it)
+        const bool pre = FMT != RUNIT_FMT_Q5_0 && split == 0 && ctx->d_xq && (size_t)t.nb * kt::kXq <= ctx->xq_bytes && (uint64_t)m * t.row_bytes >= 150000000ull;
+        t.xq = (const uint8_t*)ctx->d_xq;
+        int smem;
+        void (*kern)(const kt::Args);
+        if constexpr (FMT == RUNIT_FMT_Q5_0) {
+            smem = 4 * q50t::kS * q50t::kStage;
+            kern = q50t::gemv_q5_0_tile_kernel;
+        } else {
+            smem = kt::Tile<FMT>::kSmem;
+            kern = pre ? kt::gemv_kquant_tile_kernel<FMT, true> : kt::gemv_kquant_tile_kernel<FMT, false>;
+        }
+        static bool configured[2][64] = {{false}};
+        if (ctx->device >= 0 && ctx->device < 64 && !configured[pre][ctx->device]) {
             RUNIT_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-            configured[ctx->device] = true;
+            configured[pre][ctx->device] = true;
+        }
+        if (pre) {
+            runit_launch_chain(ctx, kt::kquant_prepare_kernel, dim3(t.nb), dim3(32), t.x, (uint8_t*)ctx->d_xq);
+            const int32_t st = runit_after_launch(ctx, "gemv_kquant_prepare_x");
+            if (st != RUNIT_OK) return st;
         }
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = split ? dim3(tiles, split) : dim3((m + 127) / 128);

@@ -122,3 +122,28 @@ def test_kquant_tile_kernel(ctx, oracle, fmt, tag):
             assert not np.isfinite(yb.download(np.float32, m)).any()
     finally:
         ctx.set_tuning("kquant_variant", 0)
+
+
+@pytest.mark.parametrize("fmt,tag,m,k", [(5, "q6k", 100003, 2048), (5, "q6k", 100001, 1792), (4, "q5k", 110010, 2048)])
+def test_kquant_prepared_activations(ctx, oracle, fmt, tag, m, k):
+    """Matrices large enough for the launch that prepares the activations: last rows of a partial tile, rows of odd half-word
+    offsets (1792 = 7 superblocks), next to the oracle on a sample of rows.  Same integers as without it: the bar above."""
+    import torch
+    import runit_mac_b200 as R
+    O = oracle
+    nb = {5: 210, 4: 176}[fmt] * (k // 256)
+    g = torch.Generator(device="cuda").manual_seed(m)
+    w = torch.randint(0, 256, (m * (k // 256), nb // (k // 256)), generator=g, device="cuda", dtype=torch.uint8)
+    scale = (torch.rand(w.shape[0], generator=g, device="cuda") + 0.5).half().view(torch.uint8).reshape(-1, 2)
+    for at in {5: (208,), 4: (0, 2)}[fmt]:
+        w[:, at:at + 2] = scale
+    x = torch.randn(k, generator=g, device="cuda")
+    x[5] = 500.0
+    y = torch.zeros(m, device="cuda")
+    torch.cuda.synchronize()
+    getattr(R, "gemv_%s_f32in_f32out" % tag)(ctx, w, x, y, m, k)
+    ctx.flush()
+    rows = torch.cat([torch.arange(64), torch.arange(m - 70, m), torch.randint(0, m, (100,))])
+    ref = O.gemv(fmt, w.reshape(m, nb)[rows.cuda()].cpu().numpy(), x.cpu().numpy(), len(rows), k, O.TIER_F64)
+    st = assert_close(O, ref, y[rows.cuda()].cpu().numpy(), what=tag + " prepared activations")
+    assert st.max_rel < 2e-5, st
