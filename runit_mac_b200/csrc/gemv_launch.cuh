@@ -40,9 +40,10 @@ static inline int32_t launch_staged(runit_ctx* ctx, const GemvArgs& a, const Gem
     cudaLaunchAttribute attr[2];
     int na = 0;
     // Dependent launch pays except for grids of about one CTA per SM, which were measured 15-25% slower with it
-    // (the early CTAs of the next grid double up on busy SMs instead of spreading out).
+    // (the early CTAs of the next grid double up on busy SMs instead of spreading out).  The cp.async kernels (Q8_0), whose copies
+    // take a CTA longer to issue, gain at every size: decoding step of a 0.5B model 467 us with that exception, 451 without.
     const uint32_t sms = (uint32_t)ctx->sm_count;
-    const bool pdl = ctx->tune.pdl == 1 || (ctx->tune.pdl == 2 && (grid < (2 * sms) / 3 || grid > (4 * sms) / 3));
+    const bool pdl = ctx->tune.pdl == 1 || (ctx->tune.pdl == 2 && (LD == 0 || grid < (2 * sms) / 3 || grid > (4 * sms) / 3));
     if (pdl) {
         attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[na].val.programmaticStreamSerializationAllowed = 1;
