@@ -1,8 +1,9 @@
 // Causal attention of the prefill on the tcgen05 tensor cores: softmax(q.K^T / sqrt(hd)) . V over the f16 cache with key <=
 // start + query (attention.metal:36-158), head dim 64 or 128.
 //
-// A CTA owns 128 queries of one head and walks the keys in blocks of 128.  Warp 4's first lane issues every copy and MMA; warps
-// 0..3 hold one query per thread (thread = tensor-memory lane):
+// A CTA owns 128 queries of one head and walks the keys in blocks of 128.  Warp 8's first lane issues every copy and MMA; of warps
+// 0..7 two threads share a query (tensor-memory lane): warps 0..3 have keys 0..63 of a block and the first half of the head's
+// dimensions, warps 4..7 the others, and the row maximum meets in shared memory:
 //   S = Q.K^T     Q rounded to f16 once (shared memory, 128-byte swizzle), K by TMA; f32 accumulator, 128 columns
 //   P             row maximum, exp2 and sum from tensor memory, two passes over S so that no row lives in registers; P is rounded to
 //                 f16 into the columns of S that the thread has already read, which makes it the A operand of the second product
@@ -11,7 +12,8 @@
 // The K buffer is free once S is there and V once O_blk is, so one buffer each suffices: 96 KB and 256 tensor-memory columns a CTA,
 // two CTAs per SM, which overlap each other's softmax and products.  Query blocks go from the most keys to the fewest.
 // Bound: the chain of a row's blocks (product, softmax, product) and the exponentials (16 a clock and SM: 1024 clocks a block).
-// Measured, 2048 queries x 16 heads x 128: 102 -> 58 us (mma.sync, 64 queries of 4 warps, 167 TFLOP/s of useful products before);
+// Measured, 2048 queries x 16 heads x 128: 102 us (mma.sync, 64 queries of 4 warps, 167 TFLOP/s of useful products), 58 with one
+// thread per query, 51 with two (half the passes over S in a chain of 16 blocks);
 // the error against 64 bits is the bf16 output's, 1.7e-3, on both.
 // Rows of the tensor maps end at start + T, so that what the cache holds behind the data (NaN included) reads as zeros.
 #include <cuda_bf16.h>
@@ -57,6 +59,20 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
         : "memory");
 }
+// 16 columns at a time: half a thread's row and its 64 accumulators fit the 96 registers that two CTAs of nine warps leave
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+          "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+                 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
 __device__ __forceinline__ float exp2_approx(float v) {
     float r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
@@ -72,12 +88,13 @@ struct Args {
 };
 
 template <int HD>
-__global__ void __launch_bounds__(160, 2) attention_tc_kernel(const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mv, const Args a) {
+__global__ void __launch_bounds__(288, 2) attention_tc_kernel(const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mv, const Args a) {
     using S = Shape<HD>;
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bars[5];
     __shared__ uint32_t tmem_holder;
     __shared__ volatile int abort_flag;
+    __shared__ float part[2][2][kRows];            // [block parity][half]: row maximum of a half; at the end the sums
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t qs = base, ks = base + S::kTile, vs = base + 2 * S::kTile;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -85,7 +102,7 @@ __global__ void __launch_bounds__(160, 2) attention_tc_kernel(const __grid_const
     const uint32_t head = blockIdx.x, q0 = (gridDim.y - 1 - blockIdx.y) * kRows;
     if (tid == 0) {
         abort_flag = 0;
-        for (int i = 0; i < 5; i++) mbar_init(smem_u32(&bars[i]), i == 3 ? 128 : 1);
+        for (int i = 0; i < 5; i++) mbar_init(smem_u32(&bars[i]), i == 3 ? 256 : 1);
         fence_mbar_init();
     }
     if (warp == 0) {
@@ -95,9 +112,9 @@ __global__ void __launch_bounds__(160, 2) attention_tc_kernel(const __grid_const
     grid_dependency_wait();
     grid_launch_dependents();
     // queries of this CTA as f16 into the swizzled K-major tile; rows behind the last query are zeros
-    if (warp < 4) {
+    if (warp < 8) {
         constexpr uint32_t CH = HD / 8;            // 16-byte chunks of a row
-        for (uint32_t i = tid; i < kRows * CH; i += 128) {
+        for (uint32_t i = tid; i < kRows * CH; i += 256) {
             const uint32_t r = i / CH, c = i % CH;
             float4 x0 = make_float4(0.f, 0.f, 0.f, 0.f), x1 = x0;
             if (q0 + r < a.T) {
@@ -118,7 +135,7 @@ __global__ void __launch_bounds__(160, 2) attention_tc_kernel(const __grid_const
     const uint32_t last_q = min(a.T, q0 + kRows) - 1, n_blocks = (a.start + last_q) / kKeys + 1;
     bool ok = true;
 
-    if (warp == 4) {
+    if (warp == 8) {
         if (lane == 0) {
             const int32_t kvh = (int32_t)(head / a.group);
             auto load = [&](const CUtensorMap* m, uint32_t dst, uint32_t bar, uint32_t i) {
@@ -149,81 +166,92 @@ __global__ void __launch_bounds__(160, 2) attention_tc_kernel(const __grid_const
                 tc_fence_after_sync();
 #pragma unroll
                 for (int s = 0; s < kKeys / 16; s++)
-                    umma_f16_ts(tmem + 128, tmem + 8 * s, desc_mn_sw128(vs + s * 2048, S::kPanel), idesc_f16(kRows, HD, 1), s > 0);
+                    umma_f16_ts(tmem + 128, tmem + 8 * s + (s >= 4 ? 32 : 0), desc_mn_sw128(vs + s * 2048, S::kPanel), idesc_f16(kRows, HD, 1), s > 0);
                 umma_commit(o_full);
             }
             if (ok) ok = mbar_wait_timed(o_full, (n_blocks - 1) & 1, &abort_flag);      // nothing is in flight when the CTA leaves
         }
     } else {
-        const uint32_t row = warp * 32 + lane, mine = tmem + ((warp * 32) << 16), qpos = a.start + q0 + row;
-        float o[HD], m = -INFINITY, l = 0.f;       // m in units of the scaled score times log2(e)
+        const uint32_t half = warp >> 2, row = (warp & 3) * 32 + lane, mine = tmem + (((warp & 3) * 32) << 16), qpos = a.start + q0 + row;
+        const uint32_t s_cols = mine + 64 * half, o_cols = mine + 128 + HD / 2 * half;
+        float o[HD / 2], m = -INFINITY, l = 0.f;   // m in units of the scaled score times log2(e); l: this half's sum
 #pragma unroll
-        for (int j = 0; j < HD; j++) o[j] = 0.f;
+        for (int j = 0; j < HD / 2; j++) o[j] = 0.f;
+        // a thread whose wait gave up goes on without waiting: all 256 take the same barriers
         for (uint32_t i = 0; i < n_blocks; i++) {
-            if (!(ok = mbar_wait_timed(s_full, i & 1, &abort_flag))) break;
+            if (ok) ok = mbar_wait_timed(s_full, i & 1, &abort_flag);
+            __syncwarp();
             tc_fence_after_sync();
-            const uint32_t key0 = i * kKeys;
-            const bool masked = key0 + kKeys - 1 > a.start + q0;      // some row of the CTA does not see the whole block
+            const uint32_t key0 = i * kKeys + 64 * half;
+            const bool masked = i * kKeys + kKeys - 1 > a.start + q0;      // some row of the CTA does not see the whole block
             float mx = -INFINITY;
 #pragma unroll
-            for (int c = 0; c < kKeys / 32; c++) {
-                uint32_t r[32];
-                tmem_ld32(mine + 32 * c, r);
+            for (int c = 0; c < 4; c++) {
+                uint32_t r[16];
+                tmem_ld16(s_cols + 16 * c, r);
                 tmem_ld_wait();
                 if (masked) {
 #pragma unroll
-                    for (int j = 0; j < 32; j++)
-                        if (key0 + 32 * c + j <= qpos) mx = fmaxf(mx, __uint_as_float(r[j]));
+                    for (int j = 0; j < 16; j++)
+                        if (key0 + 16 * c + j <= qpos) mx = fmaxf(mx, __uint_as_float(r[j]));
                 } else {
 #pragma unroll
-                    for (int j = 0; j < 32; j++) mx = fmaxf(mx, __uint_as_float(r[j]));
+                    for (int j = 0; j < 16; j++) mx = fmaxf(mx, __uint_as_float(r[j]));
                 }
             }
+            part[i & 1][half][row] = mx;
+            asm volatile("bar.sync 1, 256;" ::: "memory");              // two blocks' slots: nobody is a whole block ahead of another
+            mx = fmaxf(mx, part[i & 1][half ^ 1][row]);
             const float mn = fmaxf(m, mx * a.scale_log2);
             const float ref = mn == -INFINITY ? 0.f : mn;               // no finite score yet: every factor is 0
             const float corr = exp2_approx(m - ref);
             m = mn;
             float sum = 0.f;
 #pragma unroll
-            for (int c = 0; c < kKeys / 32; c++) {
-                uint32_t r[32], p[16];
-                tmem_ld32(mine + 32 * c, r);
+            for (int c = 0; c < 4; c++) {
+                uint32_t r[16], p[8];
+                tmem_ld16(s_cols + 16 * c, r);
                 tmem_ld_wait();
                 if (masked) {
 #pragma unroll
-                    for (int j = 0; j < 32; j++)
-                        if (key0 + 32 * c + j > qpos) r[j] = 0xFF800000u;
+                    for (int j = 0; j < 16; j++)
+                        if (key0 + 16 * c + j > qpos) r[j] = 0xFF800000u;
                 }
 #pragma unroll
-                for (int j = 0; j < 16; j++) {
+                for (int j = 0; j < 8; j++) {
                     const float p0 = exp2_approx(fmaf(__uint_as_float(r[2 * j]), a.scale_log2, -ref)), p1 = exp2_approx(fmaf(__uint_as_float(r[2 * j + 1]), a.scale_log2, -ref));
                     sum += p0 + p1;
                     const __half2 h = __floats2half2_rn(p0, p1);
                     p[j] = *reinterpret_cast<const uint32_t*>(&h);
                 }
-                tmem_st16(mine + 16 * c, p);       // behind what has been read: columns 0 .. 16 c + 15
+                tmem_st8(s_cols + 8 * c, p);       // behind what this thread has read: 8 columns for 16 keys
             }
             l = fmaf(l, corr, sum);
             tmem_st_wait();
             tc_fence_before_sync();
             mbar_arrive(p_full);
-            if (!(ok = mbar_wait_timed(o_full, i & 1, &abort_flag))) break;
+            if (ok) ok = mbar_wait_timed(o_full, i & 1, &abort_flag);
+            __syncwarp();
             tc_fence_after_sync();
 #pragma unroll
             for (int c = 0; c < HD / 32; c++) {
-                uint32_t r[32];
-                tmem_ld32(mine + 128 + 32 * c, r);
+                uint32_t r[16];
+                tmem_ld16(o_cols + 16 * c, r);
                 tmem_ld_wait();
 #pragma unroll
-                for (int j = 0; j < 32; j++) o[32 * c + j] = fmaf(o[32 * c + j], corr, __uint_as_float(r[j]));
+                for (int j = 0; j < 16; j++) o[16 * c + j] = fmaf(o[16 * c + j], corr, __uint_as_float(r[j]));
             }
             tc_fence_before_sync();                // ordered before the next arrival on p_full
         }
+        // the slots of the block after the last one: its predecessor's readers have passed that block's barrier
+        part[n_blocks & 1][half][row] = l;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        l += part[n_blocks & 1][half ^ 1][row];
         if (ok && q0 + row < a.T) {
             const float inv = l > 0.f || !(l == l) ? 1.0f / l : 0.f;
-            uint4* dst = reinterpret_cast<uint4*>(a.out + ((size_t)(q0 + row) * a.heads + head) * HD);
+            uint4* dst = reinterpret_cast<uint4*>(a.out + ((size_t)(q0 + row) * a.heads + head) * HD + HD / 2 * half);
 #pragma unroll
-            for (int c = 0; c < HD / 8; c++) {
+            for (int c = 0; c < HD / 16; c++) {
                 __nv_bfloat162 h[4];
 #pragma unroll
                 for (int j = 0; j < 4; j++) h[j] = __floats2bfloat162_rn(o[8 * c + 2 * j] * inv, o[8 * c + 2 * j + 1] * inv);
@@ -250,7 +278,7 @@ static int32_t run(runit_ctx* ctx, const CUtensorMap& mk, const CUtensorMap& mv,
         RUNIT_CUDA_TRY(ctx, cudaFuncSetAttribute(attention_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<HD>::kSmem));
         if (ctx->device < 64) configured[ctx->device] = true;
     }
-    runit_launch_chain_smem(ctx, attention_tc_kernel<HD>, dim3(a.heads, (a.T + kRows - 1) / kRows), dim3(160), Shape<HD>::kSmem, mk, mv, a);
+    runit_launch_chain_smem(ctx, attention_tc_kernel<HD>, dim3(a.heads, (a.T + kRows - 1) / kRows), dim3(288), Shape<HD>::kSmem, mk, mv, a);
     return runit_after_launch(ctx, "prefill_attention_tc");
 }
 
