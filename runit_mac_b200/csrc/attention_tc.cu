@@ -4,17 +4,20 @@
 // A CTA owns 128 queries of one head and walks the keys in blocks of 128.  Warp 8's first lane issues every copy and MMA; of warps
 // 0..7 two threads share a query (tensor-memory lane): warps 0..3 have keys 0..63 of a block and the first half of the head's
 // dimensions, warps 4..7 the others, and the row maximum meets in shared memory:
-//   S = Q.K^T     Q rounded to f16 once (shared memory, 128-byte swizzle), K by TMA; f32 accumulator, 128 columns
-//   P             row maximum, exp2 and sum from tensor memory, two passes over S so that no row lives in registers; P is rounded to
-//                 f16 into the columns of S that the thread has already read, which makes it the A operand of the second product
-//   O_blk = P.V   V by TMA as it lies in the cache (hd contiguous: B is MN-major); the block's result is added to the thread's f32
-//                 registers with the factor of the moved maximum while S of the next block is being computed
-// The K buffer is free once S is there and V once O_blk is, so one buffer each suffices: 96 KB and 256 tensor-memory columns a CTA,
-// two CTAs per SM, which overlap each other's softmax and products.  Query blocks go from the most keys to the fewest.
-// Bound: the chain of a row's blocks (product, softmax, product) and the exponentials (16 a clock and SM: 1024 clocks a block).
+//   S = Q.K^T     Q rounded to f16 once (shared memory, 128-byte swizzle), K by TMA; f32, two buffers of 128 columns: the product of
+//                 block i + 1 runs under the softmax of block i
+//   P             row maximum, exp2 and sum from tensor memory, two passes over S; P is rounded to f16 into the columns of S that the
+//                 thread has already read, which makes it the A operand of the second product
+//   O += P.V      V by TMA as it lies in the cache (hd contiguous: B is MN-major), accumulated in tensor memory.  P, the sum and O are
+//                 relative to a reference score, which follows the row maximum only when that has risen by more than 2^8 (P
+//                 then stays below 256, and f16 keeps its 11 bits); O and the sum are scaled by then, by the row's own threads.
+//                 The sum is that of the rounded P, because the largest P is no longer exactly 1.
+// One CTA per SM: 160 KB (two buffers of K and V) and all 512 tensor-memory columns.  Query blocks go from the most keys to the fewest.
+// Bound: a block's softmax (two passes, 1024 clocks of exponentials at 16 a clock and SM, the maximum's exchange).
 // Measured, 2048 queries x 16 heads x 128: 102 us (mma.sync, 64 queries of 4 warps, 167 TFLOP/s of useful products), 58 with one
-// thread per query, 51 with two (half the passes over S in a chain of 16 blocks);
-// the error against 64 bits is the bf16 output's, 1.7e-3, on both.
+// thread per query, one buffer of S and the block's output added in registers, 51 with two threads per query, 41 as it is (424
+// TFLOP/s); 1024 queries 45 -> 19 us, 2000 behind 1000 cached ones 156 -> 64.  The error against 64 bits is the bf16 output's, 1.7e-3,
+// on all of them.
 // Rows of the tensor maps end at start + T, so that what the cache holds behind the data (NaN included) reads as zeros.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -28,12 +31,13 @@ namespace runit {
 namespace atc {
 
 constexpr int kRows = 128, kKeys = 128;
-constexpr uint32_t kCols = 256;                    // tensor memory: S | P in columns 0..127, O_blk from 128
+constexpr uint32_t kCols = 512;                    // tensor memory: S | P in columns 0..127 and 128..255, O from 256
+constexpr float kRise = 8.f;                       // log2 of how far the maximum may rise above the reference
 
 template <int HD> struct Shape {
     static constexpr uint32_t kPanel = 128 * 128;  // 64 elements of 128 rows
     static constexpr uint32_t kTile = HD / 64 * kPanel;
-    static constexpr uint32_t kSmem = 3 * kTile + 1024;
+    static constexpr uint32_t kSmem = 5 * kTile + 1024;      // Q, two blocks of K, two of V
 };
 
 // kind::f16 with f16 operands (formats 0), f32 accumulator; bit 16: B is MN-major
@@ -59,19 +63,14 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
         : "memory");
 }
-// 16 columns at a time: half a thread's row and its 64 accumulators fit the 96 registers that two CTAs of nine warps leave
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
-          "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
-                 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        uint32_t v[16];
+#pragma unroll
+        for (int j = 0; j < 16; j++) v[j] = r[16 * h + j];
+        tmem_st16(taddr + 16 * h, v);
+    }
 }
 __device__ __forceinline__ float exp2_approx(float v) {
     float r;
@@ -88,21 +87,22 @@ struct Args {
 };
 
 template <int HD>
-__global__ void __launch_bounds__(288, 2) attention_tc_kernel(const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mv, const Args a) {
+__global__ void __launch_bounds__(288, 1) attention_tc_kernel(const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mv, const Args a) {
     using S = Shape<HD>;
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t bars[5];
+    __shared__ __align__(8) uint64_t bars[8];
     __shared__ uint32_t tmem_holder;
     __shared__ volatile int abort_flag;
     __shared__ float part[2][2][kRows];            // [block parity][half]: row maximum of a half; at the end the sums
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t qs = base, ks = base + S::kTile, vs = base + 2 * S::kTile;
+    const uint32_t qs = base, ks = base + S::kTile, vs = base + 3 * S::kTile;      // two buffers each
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t k_full = smem_u32(&bars[0]), v_full = smem_u32(&bars[1]), s_full = smem_u32(&bars[2]), p_full = smem_u32(&bars[3]), o_full = smem_u32(&bars[4]);
+    // k_full, v_full, s_full: one per buffer; p_full, o_full: one phase per block
+    const uint32_t k_full = smem_u32(&bars[0]), v_full = smem_u32(&bars[2]), s_full = smem_u32(&bars[4]), p_full = smem_u32(&bars[6]), o_full = smem_u32(&bars[7]);
     const uint32_t head = blockIdx.x, q0 = (gridDim.y - 1 - blockIdx.y) * kRows;
     if (tid == 0) {
         abort_flag = 0;
-        for (int i = 0; i < 5; i++) mbar_init(smem_u32(&bars[i]), i == 3 ? 256 : 1);
+        for (int i = 0; i < 8; i++) mbar_init(smem_u32(&bars[i]), i == 6 ? 256 : 1);
         fence_mbar_init();
     }
     if (warp == 0) {
@@ -142,120 +142,154 @@ __global__ void __launch_bounds__(288, 2) attention_tc_kernel(const __grid_const
                 mbar_expect_tx(bar, S::kTile);
                 for (int p = 0; p < HD / 64; p++) tma_load_3d(dst + p * S::kPanel, m, 64 * p, (int32_t)(i * kKeys), kvh, bar);
             };
-            load(&mk, ks, k_full, 0);
-            load(&mv, vs, v_full, 0);
-            for (uint32_t i = 0; i < n_blocks && ok; i++) {
-                const uint32_t ph = i & 1;
-                // the columns of S hold P of the block before until its product is done; V's buffer is free then, too
-                if (i > 0) {
-                    if (!(ok = mbar_wait_timed(o_full, ph ^ 1, &abort_flag))) break;
-                    load(&mv, vs, v_full, i);
-                }
-                if (!(ok = mbar_wait_timed(k_full, ph, &abort_flag))) break;
-                tc_fence_after_sync();
+            auto load_k = [&](uint32_t i) { load(&mk, ks + (i & 1) * S::kTile, k_full + 8 * (i & 1), i); };
+            auto load_v = [&](uint32_t i) { load(&mv, vs + (i & 1) * S::kTile, v_full + 8 * (i & 1), i); };
+            auto scores = [&](uint32_t i) {        // S of block i; its K has been waited for
+                const uint32_t kb = ks + (i & 1) * S::kTile;
 #pragma unroll
                 for (int s = 0; s < HD / 16; s++) {
                     const uint32_t off = (s >> 2) * S::kPanel + (s & 3) * 32;
-                    umma_bf16(tmem, umma_desc_sw128(qs + off), umma_desc_sw128(ks + off), idesc_f16(kRows, kKeys, 0), s > 0);
+                    umma_bf16(tmem + 128 * (i & 1), umma_desc_sw128(qs + off), umma_desc_sw128(kb + off), idesc_f16(kRows, kKeys, 0), s > 0);
                 }
-                umma_commit(s_full);
-                if (!(ok = mbar_wait_timed(s_full, ph, &abort_flag))) break;
-                if (i + 1 < n_blocks) load(&mk, ks, k_full, i + 1);
-                if (!(ok = mbar_wait_timed(v_full, ph, &abort_flag))) break;
-                if (!(ok = mbar_wait_timed(p_full, ph, &abort_flag))) break;
+                umma_commit(s_full + 8 * (i & 1));
+            };
+            load_k(0);
+            load_v(0);
+            if (n_blocks > 1) {
+                load_k(1);
+                load_v(1);
+            }
+            ok = mbar_wait_timed(k_full, 0, &abort_flag);
+            if (ok) {
                 tc_fence_after_sync();
+                scores(0);
+            }
+            for (uint32_t i = 0; i < n_blocks && ok; i++) {
+                const uint32_t ph = (i >> 1) & 1;
+                // block i + 1's columns hold P of block i - 1, whose product also frees V's buffer
+                if (i > 0) {
+                    if (!(ok = mbar_wait_timed(o_full, (i - 1) & 1, &abort_flag))) break;
+                    if (i + 1 < n_blocks) load_v(i + 1);
+                }
+                if (i + 1 < n_blocks) {
+                    if (!(ok = mbar_wait_timed(k_full + 8 * ((i + 1) & 1), ((i + 1) >> 1) & 1, &abort_flag))) break;
+                    tc_fence_after_sync();
+                    scores(i + 1);
+                }
+                if (!(ok = mbar_wait_timed(s_full + 8 * (i & 1), ph, &abort_flag))) break;
+                if (i + 2 < n_blocks) load_k(i + 2);      // S of block i is there: its K buffer is free
+                if (!(ok = mbar_wait_timed(v_full + 8 * (i & 1), ph, &abort_flag))) break;
+                if (!(ok = mbar_wait_timed(p_full, i & 1, &abort_flag))) break;
+                tc_fence_after_sync();
+                const uint32_t vb = vs + (i & 1) * S::kTile, pb = tmem + 128 * (i & 1);
 #pragma unroll
                 for (int s = 0; s < kKeys / 16; s++)
-                    umma_f16_ts(tmem + 128, tmem + 8 * s + (s >= 4 ? 32 : 0), desc_mn_sw128(vs + s * 2048, S::kPanel), idesc_f16(kRows, HD, 1), s > 0);
+                    umma_f16_ts(tmem + 256, pb + 8 * s + (s >= 4 ? 32 : 0), desc_mn_sw128(vb + s * 2048, S::kPanel), idesc_f16(kRows, HD, 1), i > 0 || s > 0);
                 umma_commit(o_full);
             }
             if (ok) ok = mbar_wait_timed(o_full, (n_blocks - 1) & 1, &abort_flag);      // nothing is in flight when the CTA leaves
         }
     } else {
         const uint32_t half = warp >> 2, row = (warp & 3) * 32 + lane, mine = tmem + (((warp & 3) * 32) << 16), qpos = a.start + q0 + row;
-        const uint32_t s_cols = mine + 64 * half, o_cols = mine + 128 + HD / 2 * half;
-        float o[HD / 2], m = -INFINITY, l = 0.f;   // m in units of the scaled score times log2(e); l: this half's sum
-#pragma unroll
-        for (int j = 0; j < HD / 2; j++) o[j] = 0.f;
+        const uint32_t o_cols = mine + 256 + HD / 2 * half;
+        float ref = -INFINITY, l = 0.f;            // reference in units of the scaled score times log2(e); l: this half's sum
         // a thread whose wait gave up goes on without waiting: all 256 take the same barriers
         for (uint32_t i = 0; i < n_blocks; i++) {
-            if (ok) ok = mbar_wait_timed(s_full, i & 1, &abort_flag);
+            if (ok) ok = mbar_wait_timed(s_full + 8 * (i & 1), (i >> 1) & 1, &abort_flag);
             __syncwarp();
             tc_fence_after_sync();
-            const uint32_t key0 = i * kKeys + 64 * half;
+            const uint32_t s_cols = mine + 128 * (i & 1) + 64 * half, key0 = i * kKeys + 64 * half;
             const bool masked = i * kKeys + kKeys - 1 > a.start + q0;      // some row of the CTA does not see the whole block
             float mx = -INFINITY;
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                uint32_t r[16];
-                tmem_ld16(s_cols + 16 * c, r);
+            for (int c = 0; c < 2; c++) {
+                uint32_t r[32];
+                tmem_ld32(s_cols + 32 * c, r);
                 tmem_ld_wait();
                 if (masked) {
 #pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        if (key0 + 16 * c + j <= qpos) mx = fmaxf(mx, __uint_as_float(r[j]));
+                    for (int j = 0; j < 32; j++)
+                        if (key0 + 32 * c + j <= qpos) mx = fmaxf(mx, __uint_as_float(r[j]));
                 } else {
 #pragma unroll
-                    for (int j = 0; j < 16; j++) mx = fmaxf(mx, __uint_as_float(r[j]));
+                    for (int j = 0; j < 32; j++) mx = fmaxf(mx, __uint_as_float(r[j]));
                 }
             }
             part[i & 1][half][row] = mx;
             asm volatile("bar.sync 1, 256;" ::: "memory");              // two blocks' slots: nobody is a whole block ahead of another
-            mx = fmaxf(mx, part[i & 1][half ^ 1][row]);
-            const float mn = fmaxf(m, mx * a.scale_log2);
-            const float ref = mn == -INFINITY ? 0.f : mn;               // no finite score yet: every factor is 0
-            const float corr = exp2_approx(m - ref);
-            m = mn;
+            mx = fmaxf(mx, part[i & 1][half ^ 1][row]) * a.scale_log2;
+            const bool rise = mx > ref + kRise || (ref == -INFINITY && mx > ref);
+            if (__any_sync(0xffffffffu, rise)) {
+                const float to = rise ? mx : ref, corr = rise ? exp2_approx(ref - to) : 1.f;
+                l *= corr;
+                ref = to;
+                if (i > 0) {
+                    if (ok) ok = mbar_wait_timed(o_full, (i - 1) & 1, &abort_flag);
+                    __syncwarp();
+                    tc_fence_after_sync();
+#pragma unroll
+                    for (int c = 0; c < HD / 64; c++) {
+                        uint32_t r[32];
+                        tmem_ld32(o_cols + 32 * c, r);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 32; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) * corr);
+                        tmem_st32(o_cols + 32 * c, r);
+                    }
+                }
+            }
+            const float sub = ref == -INFINITY ? 0.f : ref;             // no finite score yet: every factor is 0
             float sum = 0.f;
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                uint32_t r[16], p[8];
-                tmem_ld16(s_cols + 16 * c, r);
+            for (int c = 0; c < 2; c++) {
+                uint32_t r[32], p[16];
+                tmem_ld32(s_cols + 32 * c, r);
                 tmem_ld_wait();
                 if (masked) {
 #pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        if (key0 + 16 * c + j > qpos) r[j] = 0xFF800000u;
+                    for (int j = 0; j < 32; j++)
+                        if (key0 + 32 * c + j > qpos) r[j] = 0xFF800000u;
                 }
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const float p0 = exp2_approx(fmaf(__uint_as_float(r[2 * j]), a.scale_log2, -ref)), p1 = exp2_approx(fmaf(__uint_as_float(r[2 * j + 1]), a.scale_log2, -ref));
-                    sum += p0 + p1;
+                for (int j = 0; j < 16; j++) {
+                    const float p0 = exp2_approx(fmaf(__uint_as_float(r[2 * j]), a.scale_log2, -sub)), p1 = exp2_approx(fmaf(__uint_as_float(r[2 * j + 1]), a.scale_log2, -sub));
                     const __half2 h = __floats2half2_rn(p0, p1);
+                    const float2 hf = __half22float2(h);
+                    sum += hf.x + hf.y;            // of the rounded values: a row that one key decides comes out as that key's V
                     p[j] = *reinterpret_cast<const uint32_t*>(&h);
                 }
-                tmem_st8(s_cols + 8 * c, p);       // behind what this thread has read: 8 columns for 16 keys
+                tmem_st16(s_cols + 16 * c, p);     // behind what this thread has read: 16 columns for 32 keys
             }
-            l = fmaf(l, corr, sum);
+            l += sum;
             tmem_st_wait();
+            // every phase of o_full is waited for in turn (this one is long over), so that its parity says which
+            if (i > 0 && ok) ok = mbar_wait_timed(o_full, (i - 1) & 1, &abort_flag);
             tc_fence_before_sync();
             mbar_arrive(p_full);
-            if (ok) ok = mbar_wait_timed(o_full, i & 1, &abort_flag);
-            __syncwarp();
-            tc_fence_after_sync();
-#pragma unroll
-            for (int c = 0; c < HD / 32; c++) {
-                uint32_t r[16];
-                tmem_ld16(o_cols + 16 * c, r);
-                tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < 16; j++) o[16 * c + j] = fmaf(o[16 * c + j], corr, __uint_as_float(r[j]));
-            }
-            tc_fence_before_sync();                // ordered before the next arrival on p_full
         }
+        if (ok) ok = mbar_wait_timed(o_full, (n_blocks - 1) & 1, &abort_flag);
+        __syncwarp();
+        tc_fence_after_sync();
         // the slots of the block after the last one: its predecessor's readers have passed that block's barrier
         part[n_blocks & 1][half][row] = l;
         asm volatile("bar.sync 1, 256;" ::: "memory");
         l += part[n_blocks & 1][half ^ 1][row];
-        if (ok && q0 + row < a.T) {
-            const float inv = l > 0.f || !(l == l) ? 1.0f / l : 0.f;
-            uint4* dst = reinterpret_cast<uint4*>(a.out + ((size_t)(q0 + row) * a.heads + head) * HD + HD / 2 * half);
+        const float inv = l > 0.f || !(l == l) ? 1.0f / l : 0.f;
+        uint4* dst = reinterpret_cast<uint4*>(a.out + ((size_t)(q0 + row) * a.heads + head) * HD + HD / 2 * half);
 #pragma unroll
-            for (int c = 0; c < HD / 16; c++) {
-                __nv_bfloat162 h[4];
+        for (int c = 0; c < HD / 64; c++) {
+            uint32_t r[32];
+            tmem_ld32(o_cols + 32 * c, r);
+            tmem_ld_wait();
+            if (ok && q0 + row < a.T) {
 #pragma unroll
-                for (int j = 0; j < 4; j++) h[j] = __floats2bfloat162_rn(o[8 * c + 2 * j] * inv, o[8 * c + 2 * j + 1] * inv);
-                dst[c] = *reinterpret_cast<const uint4*>(h);
+                for (int k = 0; k < 4; k++) {
+                    __nv_bfloat162 h[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        h[j] = __floats2bfloat162_rn(__uint_as_float(r[8 * k + 2 * j]) * inv, __uint_as_float(r[8 * k + 2 * j + 1]) * inv);
+                    dst[4 * c + k] = *reinterpret_cast<const uint4*>(h);
+                }
             }
         }
     }

@@ -42,7 +42,9 @@ def test_causal_attention_kernel(ctx, oracle, hd, T, start):
 @pytest.mark.parametrize("T,start,heads,kvh", [(65, 63, 2, 2), (127, 1, 4, 1), (128, 0, 2, 1), (129, 127, 2, 2), (257, 300, 6, 3)])
 def test_causal_attention_tensor_core_tiles(ctx, oracle, hd, T, start, heads, kvh):
     """Edges of the 128-query tiles and 128-key blocks; NaN in the cache behind the data must not show; a large score decides its
-    row.  Bound as above: one bf16 ulp of the output (the f16 roundings of q and P are 2^-11)."""
+    row.  Bound: q is rounded alike on both sides; P is rounded to f16 relative to another reference score than the restatement's
+    running maximum, so either side's weights are off by 2^-11, which is d = 2 * 2^-11 * (P . |V|) of an output (f32 sums are far
+    below), and the output's rounding to bf16 is half an ulp, 2^-8 of it."""
     import runit_mac_b200 as R
     from oracle import prefill as OP
     n, max_seq = start + T, start + T + 40
@@ -59,7 +61,10 @@ def test_causal_attention_tensor_core_tiles(ctx, oracle, hd, T, start, heads, kv
     got = bf16_bits_to_f32(ob.download(np.uint16, T * heads * hd)).reshape(T, heads * hd)
     kc[:, n:], vc[:, n:] = 0, 0
     ref = OP.causal_attention_f16(q, kc, vc, heads, kvh, hd, start_pos=start)
-    assert_close(oracle, ref, got, rel_tol=5e-3, what="attention tiles hd=%d T=%d start=%d" % (hd, T, start))
+    d = 2.0 ** -10 * OP.causal_attention_f16(q, kc, np.abs(vc), heads, kvh, hd, start_pos=start) + 1e-6
+    assert np.isfinite(got).all()
+    worst = (np.abs(got - ref) / (d + 2.0 ** -8 * (np.abs(ref) + d))).max()
+    assert worst <= 1.0, worst
 
 
 def test_small_model_prefill_matches_restatement_and_decode(ctx, oracle):
