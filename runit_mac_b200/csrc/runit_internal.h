@@ -169,7 +169,6 @@ struct EpWait {          // consumer: the next GEMV that reads the hidden state
     const uint32_t* epoch;
 };
 // attention_tc.cu: causal attention of the prefill on the tcgen05 tensor cores.
-bool attention_tc_applies(const runit_ctx* ctx, const float* q, const void* kcache, const void* vcache, const void* out, uint32_t T, uint32_t hd);
 int32_t attention_tc(runit_ctx* ctx, const float* q, const void* kcache, const void* vcache, void* out_bf16, uint32_t T, uint32_t heads,
                      uint32_t kv_heads, uint32_t hd, uint32_t max_seq, uint32_t start_pos);
 // gemv_imma.cu: batched GEMV of the 4-bit formats on the integer tensor-core path.
