@@ -519,7 +519,7 @@ __global__ void __launch_bounds__(256) latent_value_kernel(const Dims d, const f
 }
 
 // ── expanded attention (prompts) ──
-// Flash attention on mma.sync (four warps of 16 queries, key blocks of 64 by cp.async in two stages) with keys of two sources and separate key and value widths: grid
+// Flash attention with keys of two sources and separate key and value widths: grid
 // (heads, ceil(T / 64)), 4 warps of 16 queries, key blocks of 64 staged two deep by cp.async, mma.sync m16n8k16.
 // QK >= dim + rot_dim and VD >= vdim: the rest is zero.
 template <int QK, int VD>
