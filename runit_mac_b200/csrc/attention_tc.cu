@@ -110,7 +110,6 @@ __global__ void __launch_bounds__(288, 1) attention_tc_kernel(const __grid_const
         tmem_relinquish();
     }
     grid_dependency_wait();
-    grid_launch_dependents();
     // queries of this CTA as f16 into the swizzled K-major tile; rows behind the last query are zeros
     if (warp < 8) {
         constexpr uint32_t CH = HD / 8;            // 16-byte chunks of a row
@@ -131,6 +130,9 @@ __global__ void __launch_bounds__(288, 1) attention_tc_kernel(const __grid_const
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
+    // not before the allocation is known to be done: it waits without a limit, and a block of the next grid, which allocates before its
+    // own dependency wait, must not take the columns first
+    grid_launch_dependents();
     const uint32_t tmem = tmem_holder;
     const uint32_t last_q = min(a.T, q0 + kRows) - 1, n_blocks = (a.start + last_q) / kKeys + 1;
     bool ok = true;

@@ -1,0 +1,40 @@
+"""Order of instructions in kernels that hold tensor memory or copies in flight, read from their sources: what it guards against
+cannot be shown by running it (a grid that waits for another one without a limit, a copy that lands after its block has left)."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "runit_mac_b200" / "csrc"
+
+
+def kernels(path):
+    """(name, body) of every __global__ function of a source file, comments removed."""
+    text = re.sub(r"//[^\n]*", "", path.read_text())
+    for m in re.finditer(r"__global__[^;{]*?\b(\w+_kernel)\s*\(", text):
+        at = text.index("{", text.index(")", m.end()))
+        depth, i = 0, at
+        while True:
+            depth += {"{": 1, "}": -1}.get(text[i], 0)
+            i += 1
+            if depth == 0:
+                break
+        yield m.group(1), text[at:i]
+
+
+def test_dependents_are_released_after_tensor_memory_is_held():
+    """tcgen05.alloc waits without a limit.  A kernel that allocates may let a dependent grid start only when all of its own blocks
+    hold their columns: else a block of the dependent grid, which allocates before it waits for its predecessor, can take the columns
+    that the predecessor still waits for."""
+    seen = 0
+    for path in sorted(CSRC.glob("*.cu")):
+        for name, body in kernels(path):
+            alloc, trigger = re.search(r"\btmem_alloc(_pair)?\(", body), body.find("grid_launch_dependents(")
+            if not alloc:
+                continue
+            seen += 1
+            if trigger < 0:
+                continue
+            barrier = re.compile(r"__syncthreads\(\)|cluster_sync\(\)").search(body, alloc.end())
+            assert barrier and trigger > barrier.end(), "%s (%s) releases its dependents before its allocation is known to be done" % (name, path.name)
+    assert seen >= 3
