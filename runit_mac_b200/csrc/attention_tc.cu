@@ -12,7 +12,7 @@
 //                 relative to a reference score, which follows the row maximum only when that has risen by more than 2^8 (P
 //                 then stays below 256, and f16 keeps its 11 bits); O and the sum are scaled by then, by the row's own threads.
 //                 The sum is that of the rounded P, because the largest P is no longer exactly 1.
-// One CTA per SM: 160 KB (two buffers of K and V) and all 512 tensor-memory columns.  Query blocks go from the most keys to the fewest.
+// One CTA per SM: 161 KB (two buffers of K and V; 116 asked for at head dim 64) and all 512 tensor-memory columns.  Query blocks go from the most keys to the fewest.
 // Bound: a block's softmax (two passes, 1024 clocks of exponentials at 16 a clock and SM, the maximum's exchange).
 // Measured, 2048 queries x 16 heads x 128: 102 us (mma.sync, 64 queries of 4 warps, 167 TFLOP/s of useful products), 58 with one
 // thread per query, one buffer of S and the block's output added in registers, 51 with two threads per query, 41 as it is (424
@@ -32,12 +32,17 @@ namespace atc {
 
 constexpr int kRows = 128, kKeys = 128;
 constexpr uint32_t kCols = 512;                    // tensor memory: S | P in columns 0..127 and 128..255, O from 256
+constexpr uint32_t kOnePerSm = 116 * 1024;         // shared memory that only one CTA of an SM can have
 constexpr float kRise = 8.f;                       // log2 of how far the maximum may rise above the reference
 
 template <int HD> struct Shape {
     static constexpr uint32_t kPanel = 128 * 128;  // 64 elements of 128 rows
     static constexpr uint32_t kTile = HD / 64 * kPanel;
-    static constexpr uint32_t kSmem = 5 * kTile + 1024;      // Q, two blocks of K, two of V
+    // Q, two blocks of K, two of V; at head dim 64 (83 KB) more than it needs: a second CTA of an SM would only sit in its allocation
+    // behind the first, bound to that SM however long the first one's row of blocks is (2048 queries x 16 heads x 64: 36.1 us with two
+    // resident CTAs, 28.9 with one; 2000 behind 1000 cached ones 58.3 and 49.9; 1024 15.4 and 15.1, fewer the same)
+    static constexpr uint32_t kSmem = 5 * kTile + 1024 < kOnePerSm ? kOnePerSm : 5 * kTile + 1024;
+    static_assert(2 * kCols <= 512 || 2 * (kSmem + 1024) > 228 * 1024, "CTAs that share an SM share its tensor memory");
 };
 
 // kind::f16 with f16 operands (formats 0), f32 accumulator; bit 16: B is MN-major

@@ -67,6 +67,25 @@ def test_causal_attention_tensor_core_tiles(ctx, oracle, hd, T, start, heads, kv
     assert worst <= 1.0, worst
 
 
+@pytest.mark.parametrize("hd", [128, 64])
+def test_causal_attention_calls_in_a_row(ctx, hd):
+    """Calls that follow one another without a wait, each with more blocks than SMs: a dependent call starts while the one before
+    it still holds tensor memory.  Every call gives the same bits."""
+    import runit_mac_b200 as R
+    T, heads = 1300, 16
+    rng = np.random.default_rng(hd)
+    q = ctx.buffer_from(rng.normal(0, 1, (T, heads * hd)).astype(np.float32))
+    kc, vc = (ctx.buffer_from(rng.normal(0, 1, (heads, T, hd)).astype(np.float16)) for _ in range(2))
+    outs = [ctx.new_buffer(T * heads * hd * 2) for _ in range(6)]
+    for ob in outs:
+        R.prefill_attention_f16kv(ctx, q, kc, vc, ob, T, heads, heads, hd, T, 0)
+    ctx.flush()
+    first = outs[0].download(np.uint16, T * heads * hd)
+    assert np.isfinite(bf16_bits_to_f32(first)).all()
+    for ob in outs[1:]:
+        assert np.array_equal(ob.download(np.uint16, T * heads * hd), first)
+
+
 def test_small_model_prefill_matches_restatement_and_decode(ctx, oracle):
     import runit_mac_b200 as R
     from oracle import prefill as OP
