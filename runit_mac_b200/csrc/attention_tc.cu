@@ -149,8 +149,9 @@ __global__ void __launch_bounds__(288, 1) attention_tc_kernel(const __grid_const
                 mbar_expect_tx(bar, S::kTile);
                 for (int p = 0; p < HD / 64; p++) tma_load_3d(dst + p * S::kPanel, m, 64 * p, (int32_t)(i * kKeys), kvh, bar);
             };
-            auto load_k = [&](uint32_t i) { load(&mk, ks + (i & 1) * S::kTile, k_full + 8 * (i & 1), i); };
-            auto load_v = [&](uint32_t i) { load(&mv, vs + (i & 1) * S::kTile, v_full + 8 * (i & 1), i); };
+            uint32_t n_k = 0, n_v = 0, n_s = 0, n_o = 0;         // started so far
+            auto load_k = [&](uint32_t i) { load(&mk, ks + (i & 1) * S::kTile, k_full + 8 * (i & 1), i); n_k++; };
+            auto load_v = [&](uint32_t i) { load(&mv, vs + (i & 1) * S::kTile, v_full + 8 * (i & 1), i); n_v++; };
             auto scores = [&](uint32_t i) {        // S of block i; its K has been waited for
                 const uint32_t kb = ks + (i & 1) * S::kTile;
 #pragma unroll
@@ -159,6 +160,7 @@ __global__ void __launch_bounds__(288, 1) attention_tc_kernel(const __grid_const
                     umma_bf16(tmem + 128 * (i & 1), umma_desc_sw128(qs + off), umma_desc_sw128(kb + off), idesc_f16(kRows, kKeys, 0), s > 0);
                 }
                 umma_commit(s_full + 8 * (i & 1));
+                n_s++;
             };
             load_k(0);
             load_v(0);
@@ -193,8 +195,15 @@ __global__ void __launch_bounds__(288, 1) attention_tc_kernel(const __grid_const
                 for (int s = 0; s < kKeys / 16; s++)
                     umma_f16_ts(tmem + 256, pb + 8 * s + (s >= 4 ? 32 : 0), desc_mn_sw128(vb + s * 2048, S::kPanel), idesc_f16(kRows, HD, 1), i > 0 || s > 0);
                 umma_commit(o_full);
+                n_o++;
             }
-            if (ok) ok = mbar_wait_timed(o_full, (n_blocks - 1) & 1, &abort_flag);      // nothing is in flight when the CTA leaves
+            if (ok) ok = mbar_wait_timed(o_full, (n_blocks - 1) & 1, &abort_flag);
+            if (!ok) {          // nothing is in flight when the CTA leaves, whatever it gave up on
+                mbar_drain(k_full, 2, n_k);
+                mbar_drain(v_full, 2, n_v);
+                mbar_drain(s_full, 2, n_s);
+                mbar_drain(o_full, 1, n_o);
+            }
         }
     } else {
         const uint32_t half = warp >> 2, row = (warp & 3) * 32 + lane, mine = tmem + (((warp & 3) * 32) << 16), qpos = a.start + q0 + row;

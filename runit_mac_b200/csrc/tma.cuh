@@ -40,6 +40,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     }
     return false;
 }
+// For the thread that starts copies (or MMAs) 0 .. issued - 1, in order, on a ring of `ring` barriers: waits (bounded) for those that can
+// still be in flight, so that nothing arrives after a block that gave up has handed back its shared and tensor memory.
+__device__ __forceinline__ void mbar_drain(uint32_t bars, uint32_t ring, uint32_t issued) {
+    for (uint32_t i = issued < ring ? 0 : issued - ring; i < issued; i++) mbar_wait(bars + 8 * (i % ring), (i / ring) & 1);
+}
 // 2-D tiled load: box (c0 = innermost coordinate in elements, c1 = row) -> dense shared tile.
 // c0 * element size must be a multiple of 16 bytes; dst must be 128-byte aligned.
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int32_t c0, int32_t c1, uint32_t bar) {

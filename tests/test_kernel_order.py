@@ -38,3 +38,16 @@ def test_dependents_are_released_after_tensor_memory_is_held():
             barrier = re.compile(r"__syncthreads\(\)|cluster_sync\(\)").search(body, alloc.end())
             assert barrier and trigger > barrier.end(), "%s (%s) releases its dependents before its allocation is known to be done" % (name, path.name)
     assert seen >= 3
+
+
+@pytest.mark.parametrize("source", ["attention_tc.cu"])
+def test_copies_in_flight_are_waited_for(source):
+    """A role that gives up a bounded wait must not leave with its bulk copies (or MMAs) in flight: they would arrive in shared (tensor)
+    memory that belongs to another block by then."""
+    seen = 0
+    for name, body in kernels(CSRC / source):
+        loads = [m.start() for m in re.finditer(r"\b(tma_load_\dd|bulk_load_1d)\(", body)]
+        if loads:
+            seen += 1
+            assert body.find("mbar_drain(", loads[-1]) > 0, "%s leaves copies in flight when it gives up" % name
+    assert seen
