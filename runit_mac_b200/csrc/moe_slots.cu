@@ -207,6 +207,7 @@ __global__ void __launch_bounds__(Shape<G>::kThreads, Shape<G>::kPerSm) slots_ge
                         bulk_load_1d(sb + S::kWBytes + j * kXBytes, a.frags + ((size_t)(t0 + j) * a.units + u) * kXBytes, kXBytes, bar);
                 }
             }
+            mbar_drain(full, kStages, c);          // the last loads; a warp that gave up its wait no longer waits for them
         }
     } else {
         const uint32_t row[2] = {DUAL ? warp * 8 + g : warp * 16 + g, DUAL ? S::kRows / 2 + warp * 8 + g : warp * 16 + 8 + g};

@@ -40,7 +40,7 @@ def test_dependents_are_released_after_tensor_memory_is_held():
     assert seen >= 3
 
 
-@pytest.mark.parametrize("source", ["attention_tc.cu"])
+@pytest.mark.parametrize("source", ["attention_tc.cu", "moe_slots.cu"])
 def test_copies_in_flight_are_waited_for(source):
     """A role that gives up a bounded wait must not leave with its bulk copies (or MMAs) in flight: they would arrive in shared (tensor)
     memory that belongs to another block by then."""
