@@ -83,6 +83,53 @@ __device__ __forceinline__ float exp2_approx(float v) {
     return r;
 }
 
+// O += P.V * scale of one block for this thread's row and half of the dimensions, over the n keys that the row sees and no others; P of
+// both halves is in tensor memory at p_cols, v is the block's V as TMA put it down.
+template <int HD>
+__device__ __forceinline__ void visible_products(uint32_t p_cols, uint32_t o_cols, const uint8_t* v, uint32_t half, uint32_t n, float scale, bool first) {
+#pragma unroll 1
+    for (uint32_t c = 0; c < HD / 64; c++) {
+        const uint32_t dim = HD / 2 * half + 32 * c;
+        const uint8_t* panel = v + (dim >> 6) * Shape<HD>::kPanel;
+        uint32_t r[32];
+        float o[32];
+        tmem_ld32(o_cols + 32 * c, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; j++) o[j] = first ? 0.f : __uint_as_float(r[j]);
+#pragma unroll 1
+        for (uint32_t k = 0; k < kKeys; k += 2) {
+            uint32_t two;
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(two) : "r"(p_cols + (k >> 1) + (k & 64 ? 32 : 0)) : "memory");
+            tmem_ld_wait();
+            const float2 w = __half22float2(*reinterpret_cast<const __half2*>(&two));
+#pragma unroll
+            for (uint32_t e = 0; e < 2; e++) {
+                if (k + e >= n) break;
+                const float we = (e ? w.y : w.x) * scale;
+#pragma unroll
+                for (uint32_t q = 0; q < 4; q++) {
+                    const uint4 x = *reinterpret_cast<const uint4*>(panel + (k + e) * 128 + (((((dim & 63) >> 3) + q) ^ ((k + e) & 7)) << 4));
+                    const __half2* h = reinterpret_cast<const __half2*>(&x);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const float2 f = __half22float2(h[j]);
+                        o[8 * q + 2 * j] = fmaf(we, f.x, o[8 * q + 2 * j]);
+                        o[8 * q + 2 * j + 1] = fmaf(we, f.y, o[8 * q + 2 * j + 1]);
+                    }
+                }
+            }
+            __syncwarp();
+        }
+#pragma unroll
+        for (int j = 0; j < 32; j++) r[j] = __float_as_uint(o[j]);
+        tmem_st32(o_cols + 32 * c, r);
+        tmem_st_wait();
+    }
+}
+// Not 0 where one of two bf16 values is an Inf or a NaN.
+__device__ __forceinline__ uint32_t not_finite(uint32_t b2) { return ((b2 & 0x7FFF7FFFu) + 0x00800080u) & 0x80008000u; }
+
 struct Args {
     const float* q;
     __nv_bfloat16* out;
@@ -140,181 +187,216 @@ __global__ void __launch_bounds__(288, 1) attention_tc_kernel(const __grid_const
     grid_launch_dependents();
     const uint32_t tmem = tmem_holder;
     const uint32_t last_q = min(a.T, q0 + kRows) - 1, n_blocks = (a.start + last_q) / kKeys + 1;
+    // blocks of which some row does not see all keys: the last two at most
+    const uint32_t first_masked = (a.start + q0 + 1) / kKeys;
     bool ok = true;
 
-    if (warp == 8) {
-        if (lane == 0) {
-            const int32_t kvh = (int32_t)(head / a.group);
-            auto load = [&](const CUtensorMap* m, uint32_t dst, uint32_t bar, uint32_t i) {
-                mbar_expect_tx(bar, S::kTile);
-                for (int p = 0; p < HD / 64; p++) tma_load_3d(dst + p * S::kPanel, m, 64 * p, (int32_t)(i * kKeys), kvh, bar);
-            };
-            uint32_t n_k = 0, n_v = 0, n_s = 0, n_o = 0;         // started so far
-            auto load_k = [&](uint32_t i) { load(&mk, ks + (i & 1) * S::kTile, k_full + 8 * (i & 1), i); n_k++; };
-            auto load_v = [&](uint32_t i) { load(&mv, vs + (i & 1) * S::kTile, v_full + 8 * (i & 1), i); n_v++; };
-            auto scores = [&](uint32_t i) {        // S of block i; its K has been waited for
-                const uint32_t kb = ks + (i & 1) * S::kTile;
+    // A hidden key's weight of 0 meets its V all the same, and 0 x Inf is NaN.  An output that is not finite is therefore taken again, with
+    // the products of the blocks that have hidden keys by visible_products; whatever is finite has met no such V.  (Looking at V
+    // first instead cost 2048 queries x 16 heads x 128 42.3 us in the softmax's warps and 42.6 in a warp of its own, against 39.8; the
+    // second look costs 33 queries behind 300 keys 0.2 of 9.0 us.)
+    for (bool careful = false;; careful = true) {
+        bool again = false;
+        if (warp == 8) {
+            if (lane == 0) {
+                const int32_t kvh = (int32_t)(head / a.group);
+                auto load = [&](const CUtensorMap* m, uint32_t dst, uint32_t bar, uint32_t i) {
+                    mbar_expect_tx(bar, S::kTile);
+                    for (int p = 0; p < HD / 64; p++) tma_load_3d(dst + p * S::kPanel, m, 64 * p, (int32_t)(i * kKeys), kvh, bar);
+                };
+                uint32_t n_k = 0, n_v = 0, n_s = 0, n_o = 0;         // started so far
+                auto load_k = [&](uint32_t i) { load(&mk, ks + (i & 1) * S::kTile, k_full + 8 * (i & 1), i); n_k++; };
+                auto load_v = [&](uint32_t i) { load(&mv, vs + (i & 1) * S::kTile, v_full + 8 * (i & 1), i); n_v++; };
+                auto scores = [&](uint32_t i) {        // S of block i; its K has been waited for
+                    const uint32_t kb = ks + (i & 1) * S::kTile;
 #pragma unroll
-                for (int s = 0; s < HD / 16; s++) {
-                    const uint32_t off = (s >> 2) * S::kPanel + (s & 3) * 32;
-                    umma_bf16(tmem + 128 * (i & 1), umma_desc_sw128(qs + off), umma_desc_sw128(kb + off), idesc_f16(kRows, kKeys, 0), s > 0);
+                    for (int s = 0; s < HD / 16; s++) {
+                        const uint32_t off = (s >> 2) * S::kPanel + (s & 3) * 32;
+                        umma_bf16(tmem + 128 * (i & 1), umma_desc_sw128(qs + off), umma_desc_sw128(kb + off), idesc_f16(kRows, kKeys, 0), s > 0);
+                    }
+                    umma_commit(s_full + 8 * (i & 1));
+                    n_s++;
+                };
+                load_k(0);
+                load_v(0);
+                if (n_blocks > 1) {
+                    load_k(1);
+                    load_v(1);
                 }
-                umma_commit(s_full + 8 * (i & 1));
-                n_s++;
-            };
-            load_k(0);
-            load_v(0);
-            if (n_blocks > 1) {
-                load_k(1);
-                load_v(1);
-            }
-            ok = mbar_wait_timed(k_full, 0, &abort_flag);
-            if (ok) {
-                tc_fence_after_sync();
-                scores(0);
-            }
-            for (uint32_t i = 0; i < n_blocks && ok; i++) {
-                const uint32_t ph = (i >> 1) & 1;
-                // block i + 1's columns hold P of block i - 1, whose product also frees V's buffer
-                if (i > 0) {
-                    if (!(ok = mbar_wait_timed(o_full, (i - 1) & 1, &abort_flag))) break;
-                    if (i + 1 < n_blocks) load_v(i + 1);
-                }
-                if (i + 1 < n_blocks) {
-                    if (!(ok = mbar_wait_timed(k_full + 8 * ((i + 1) & 1), ((i + 1) >> 1) & 1, &abort_flag))) break;
+                ok = mbar_wait_timed(k_full, 0, &abort_flag);
+                if (ok) {
                     tc_fence_after_sync();
-                    scores(i + 1);
+                    scores(0);
                 }
-                if (!(ok = mbar_wait_timed(s_full + 8 * (i & 1), ph, &abort_flag))) break;
-                if (i + 2 < n_blocks) load_k(i + 2);      // S of block i is there: its K buffer is free
-                if (!(ok = mbar_wait_timed(v_full + 8 * (i & 1), ph, &abort_flag))) break;
-                if (!(ok = mbar_wait_timed(p_full, i & 1, &abort_flag))) break;
-                tc_fence_after_sync();
-                const uint32_t vb = vs + (i & 1) * S::kTile, pb = tmem + 128 * (i & 1);
+                for (uint32_t i = 0; i < n_blocks && ok; i++) {
+                    const uint32_t ph = (i >> 1) & 1;
+                    // block i + 1's columns hold P of block i - 1, whose product also frees V's buffer
+                    if (i > 0) {
+                        if (!(ok = mbar_wait_timed(o_full, (i - 1) & 1, &abort_flag))) break;
+                        if (i + 1 < n_blocks) load_v(i + 1);
+                    }
+                    if (i + 1 < n_blocks) {
+                        if (!(ok = mbar_wait_timed(k_full + 8 * ((i + 1) & 1), ((i + 1) >> 1) & 1, &abort_flag))) break;
+                        tc_fence_after_sync();
+                        scores(i + 1);
+                    }
+                    if (!(ok = mbar_wait_timed(s_full + 8 * (i & 1), ph, &abort_flag))) break;
+                    if (i + 2 < n_blocks) load_k(i + 2);      // S of block i is there: its K buffer is free
+                    if (!(ok = mbar_wait_timed(v_full + 8 * (i & 1), ph, &abort_flag))) break;
+                    if (!(ok = mbar_wait_timed(p_full, i & 1, &abort_flag))) break;
+                    tc_fence_after_sync();
+                    const uint32_t vb = vs + (i & 1) * S::kTile, pb = tmem + 128 * (i & 1);
+                    if (!careful || i < first_masked) {
 #pragma unroll
-                for (int s = 0; s < kKeys / 16; s++)
-                    umma_f16_ts(tmem + 256, pb + 8 * s + (s >= 4 ? 32 : 0), desc_mn_sw128(vb + s * 2048, S::kPanel), idesc_f16(kRows, HD, 1), i > 0 || s > 0);
-                umma_commit(o_full);
-                n_o++;
+                        for (int s = 0; s < kKeys / 16; s++)
+                            umma_f16_ts(tmem + 256, pb + 8 * s + (s >= 4 ? 32 : 0), desc_mn_sw128(vb + s * 2048, S::kPanel), idesc_f16(kRows, HD, 1), i > 0 || s > 0);
+                    }
+                    umma_commit(o_full);
+                    n_o++;
+                }
+                if (ok) ok = mbar_wait_timed(o_full, (n_blocks - 1) & 1, &abort_flag);
+                if (!ok) {          // nothing is in flight when the CTA leaves, whatever it gave up on
+                    mbar_drain(k_full, 2, n_k);
+                    mbar_drain(v_full, 2, n_v);
+                    mbar_drain(s_full, 2, n_s);
+                    mbar_drain(o_full, 1, n_o);
+                }
+            }
+        } else {
+            const uint32_t half = warp >> 2, row = (warp & 3) * 32 + lane, mine = tmem + (((warp & 3) * 32) << 16), qpos = a.start + q0 + row;
+            const uint32_t o_cols = mine + 256 + HD / 2 * half;
+            float late = 1.f;                          // what the last block's rise scaled O by
+            float ref = -INFINITY, l = 0.f;            // reference in units of the scaled score times log2(e); l: this half's sum
+            // a thread whose wait gave up goes on without waiting: all 256 take the same barriers
+            for (uint32_t i = 0; i < n_blocks; i++) {
+                if (ok) ok = mbar_wait_timed(s_full + 8 * (i & 1), (i >> 1) & 1, &abort_flag);
+                __syncwarp();
+                tc_fence_after_sync();
+                const uint32_t s_cols = mine + 128 * (i & 1) + 64 * half, key0 = i * kKeys + 64 * half;
+                const bool masked = i >= first_masked;
+                float mx = -INFINITY;
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    uint32_t r[32];
+                    tmem_ld32(s_cols + 32 * c, r);
+                    tmem_ld_wait();
+                    if (masked) {
+#pragma unroll
+                        for (int j = 0; j < 32; j++)
+                            if (key0 + 32 * c + j <= qpos) mx = fmaxf(mx, __uint_as_float(r[j]));
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 32; j++) mx = fmaxf(mx, __uint_as_float(r[j]));
+                    }
+                }
+                part[i & 1][half][row] = mx;
+                asm volatile("bar.sync 1, 256;" ::: "memory");              // two blocks' slots: nobody is a whole block ahead of another
+                mx = fmaxf(mx, part[i & 1][half ^ 1][row]) * a.scale_log2;
+                const bool rise = mx > ref + kRise || (ref == -INFINITY && mx > ref);
+                late = 1.f;
+                if (__any_sync(0xffffffffu, rise)) {
+                    const float to = rise ? mx : ref, corr = rise ? exp2_approx(ref - to) : 1.f;
+                    l *= corr;
+                    late = corr;
+                    ref = to;
+                    if (i > 0) {
+                        if (ok) ok = mbar_wait_timed(o_full, (i - 1) & 1, &abort_flag);
+                        __syncwarp();
+                        tc_fence_after_sync();
+#pragma unroll
+                        for (int c = 0; c < HD / 64; c++) {
+                            uint32_t r[32];
+                            tmem_ld32(o_cols + 32 * c, r);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int j = 0; j < 32; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) * corr);
+                            tmem_st32(o_cols + 32 * c, r);
+                        }
+                    }
+                }
+                const float sub = ref == -INFINITY ? 0.f : ref;             // no finite score yet: every factor is 0
+                float sum = 0.f;
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    uint32_t r[32], p[16];
+                    tmem_ld32(s_cols + 32 * c, r);
+                    tmem_ld_wait();
+                    if (masked) {
+#pragma unroll
+                        for (int j = 0; j < 32; j++)
+                            if (key0 + 32 * c + j > qpos) r[j] = 0xFF800000u;
+                    }
+#pragma unroll
+                    for (int j = 0; j < 16; j++) {
+                        const float p0 = exp2_approx(fmaf(__uint_as_float(r[2 * j]), a.scale_log2, -sub)), p1 = exp2_approx(fmaf(__uint_as_float(r[2 * j + 1]), a.scale_log2, -sub));
+                        const __half2 h = __floats2half2_rn(p0, p1);
+                        const float2 hf = __half22float2(h);
+                        sum += hf.x + hf.y;            // of the rounded values: a row that one key decides comes out as that key's V
+                        p[j] = *reinterpret_cast<const uint32_t*>(&h);
+                    }
+                    tmem_st16(s_cols + 16 * c, p);     // behind what this thread has read: 16 columns for 32 keys
+                }
+                l += sum;
+                tmem_st_wait();
+                // every phase of o_full is waited for in turn (this one is long over), so that its parity says which
+                if (i > 0 && ok) ok = mbar_wait_timed(o_full, (i - 1) & 1, &abort_flag);
+                tc_fence_before_sync();
+                mbar_arrive(p_full);
             }
             if (ok) ok = mbar_wait_timed(o_full, (n_blocks - 1) & 1, &abort_flag);
-            if (!ok) {          // nothing is in flight when the CTA leaves, whatever it gave up on
-                mbar_drain(k_full, 2, n_k);
-                mbar_drain(v_full, 2, n_v);
-                mbar_drain(s_full, 2, n_s);
-                mbar_drain(o_full, 1, n_o);
-            }
-        }
-    } else {
-        const uint32_t half = warp >> 2, row = (warp & 3) * 32 + lane, mine = tmem + (((warp & 3) * 32) << 16), qpos = a.start + q0 + row;
-        const uint32_t o_cols = mine + 256 + HD / 2 * half;
-        float ref = -INFINITY, l = 0.f;            // reference in units of the scaled score times log2(e); l: this half's sum
-        // a thread whose wait gave up goes on without waiting: all 256 take the same barriers
-        for (uint32_t i = 0; i < n_blocks; i++) {
-            if (ok) ok = mbar_wait_timed(s_full + 8 * (i & 1), (i >> 1) & 1, &abort_flag);
             __syncwarp();
             tc_fence_after_sync();
-            const uint32_t s_cols = mine + 128 * (i & 1) + 64 * half, key0 = i * kKeys + 64 * half;
-            const bool masked = i * kKeys + kKeys - 1 > a.start + q0;      // some row of the CTA does not see the whole block
-            float mx = -INFINITY;
-#pragma unroll
-            for (int c = 0; c < 2; c++) {
-                uint32_t r[32];
-                tmem_ld32(s_cols + 32 * c, r);
-                tmem_ld_wait();
-                if (masked) {
-#pragma unroll
-                    for (int j = 0; j < 32; j++)
-                        if (key0 + 32 * c + j <= qpos) mx = fmaxf(mx, __uint_as_float(r[j]));
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 32; j++) mx = fmaxf(mx, __uint_as_float(r[j]));
+            // the slots of the block after the last one: its predecessor's readers have passed that block's barrier
+            part[n_blocks & 1][half][row] = l;
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            l += part[n_blocks & 1][half ^ 1][row];
+            if (careful) {
+                // P and V of the last two blocks are still there, P of the last but one relative to the reference before the last block's rise
+                tc_fence_after_sync();
+                for (uint32_t i = first_masked; i < n_blocks; i++) {
+                    if (ok) ok = mbar_wait_timed(v_full + 8 * (i & 1), (i >> 1) & 1, &abort_flag);
+                    __syncwarp();
+                    visible_products<HD>(mine + 128 * (i & 1), o_cols, smem_raw + (vs - smem_u32(smem_raw)) + (i & 1) * S::kTile, half,
+                                         qpos < i * kKeys ? 0 : min((uint32_t)kKeys, qpos - i * kKeys + 1), i + 1 < n_blocks ? late : 1.f, i == 0);
                 }
             }
-            part[i & 1][half][row] = mx;
-            asm volatile("bar.sync 1, 256;" ::: "memory");              // two blocks' slots: nobody is a whole block ahead of another
-            mx = fmaxf(mx, part[i & 1][half ^ 1][row]) * a.scale_log2;
-            const bool rise = mx > ref + kRise || (ref == -INFINITY && mx > ref);
-            if (__any_sync(0xffffffffu, rise)) {
-                const float to = rise ? mx : ref, corr = rise ? exp2_approx(ref - to) : 1.f;
-                l *= corr;
-                ref = to;
-                if (i > 0) {
-                    if (ok) ok = mbar_wait_timed(o_full, (i - 1) & 1, &abort_flag);
-                    __syncwarp();
-                    tc_fence_after_sync();
+            const float inv = l > 0.f || !(l == l) ? 1.0f / l : 0.f;
+            uint4* dst = reinterpret_cast<uint4*>(a.out + ((size_t)(q0 + row) * a.heads + head) * HD + HD / 2 * half);
 #pragma unroll
-                    for (int c = 0; c < HD / 64; c++) {
-                        uint32_t r[32];
-                        tmem_ld32(o_cols + 32 * c, r);
-                        tmem_ld_wait();
+            for (int c = 0; c < HD / 64; c++) {
+                uint32_t r[32];
+                tmem_ld32(o_cols + 32 * c, r);
+                tmem_ld_wait();
+                if (ok && q0 + row < a.T) {
 #pragma unroll
-                        for (int j = 0; j < 32; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) * corr);
-                        tmem_st32(o_cols + 32 * c, r);
+                    for (int k = 0; k < 4; k++) {
+                        __nv_bfloat162 h[4];
+#pragma unroll
+                        for (int j = 0; j < 4; j++)
+                            h[j] = __floats2bfloat162_rn(__uint_as_float(r[8 * k + 2 * j]) * inv, __uint_as_float(r[8 * k + 2 * j + 1]) * inv);
+                        const uint4 w = *reinterpret_cast<const uint4*>(h);
+                        dst[4 * c + k] = w;
+                        again |= ((not_finite(w.x) | not_finite(w.y)) | (not_finite(w.z) | not_finite(w.w))) != 0;
                     }
                 }
             }
-            const float sub = ref == -INFINITY ? 0.f : ref;             // no finite score yet: every factor is 0
-            float sum = 0.f;
-#pragma unroll
-            for (int c = 0; c < 2; c++) {
-                uint32_t r[32], p[16];
-                tmem_ld32(s_cols + 32 * c, r);
-                tmem_ld_wait();
-                if (masked) {
-#pragma unroll
-                    for (int j = 0; j < 32; j++)
-                        if (key0 + 32 * c + j > qpos) r[j] = 0xFF800000u;
-                }
-#pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    const float p0 = exp2_approx(fmaf(__uint_as_float(r[2 * j]), a.scale_log2, -sub)), p1 = exp2_approx(fmaf(__uint_as_float(r[2 * j + 1]), a.scale_log2, -sub));
-                    const __half2 h = __floats2half2_rn(p0, p1);
-                    const float2 hf = __half22float2(h);
-                    sum += hf.x + hf.y;            // of the rounded values: a row that one key decides comes out as that key's V
-                    p[j] = *reinterpret_cast<const uint32_t*>(&h);
-                }
-                tmem_st16(s_cols + 16 * c, p);     // behind what this thread has read: 16 columns for 32 keys
-            }
-            l += sum;
-            tmem_st_wait();
-            // every phase of o_full is waited for in turn (this one is long over), so that its parity says which
-            if (i > 0 && ok) ok = mbar_wait_timed(o_full, (i - 1) & 1, &abort_flag);
-            tc_fence_before_sync();
-            mbar_arrive(p_full);
         }
-        if (ok) ok = mbar_wait_timed(o_full, (n_blocks - 1) & 1, &abort_flag);
-        __syncwarp();
+        if (!ok) {
+            abort_flag = 1;
+            if (a.status) atomicExch(a.status, 1);
+        }
+        tc_fence_before_sync();
+        if (!__syncthreads_or(again) || careful || abort_flag) break;
+        if (tid == 0) {
+            for (int i = 0; i < 8; i++) {
+                mbar_inval(smem_u32(&bars[i]));
+                mbar_init(smem_u32(&bars[i]), i == 6 ? 256 : 1);
+            }
+            fence_mbar_init();
+        }
+        __syncthreads();
         tc_fence_after_sync();
-        // the slots of the block after the last one: its predecessor's readers have passed that block's barrier
-        part[n_blocks & 1][half][row] = l;
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        l += part[n_blocks & 1][half ^ 1][row];
-        const float inv = l > 0.f || !(l == l) ? 1.0f / l : 0.f;
-        uint4* dst = reinterpret_cast<uint4*>(a.out + ((size_t)(q0 + row) * a.heads + head) * HD + HD / 2 * half);
-#pragma unroll
-        for (int c = 0; c < HD / 64; c++) {
-            uint32_t r[32];
-            tmem_ld32(o_cols + 32 * c, r);
-            tmem_ld_wait();
-            if (ok && q0 + row < a.T) {
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    __nv_bfloat162 h[4];
-#pragma unroll
-                    for (int j = 0; j < 4; j++)
-                        h[j] = __floats2bfloat162_rn(__uint_as_float(r[8 * k + 2 * j]) * inv, __uint_as_float(r[8 * k + 2 * j + 1]) * inv);
-                    dst[4 * c + k] = *reinterpret_cast<const uint4*>(h);
-                }
-            }
-        }
     }
-    if (!ok) {
-        abort_flag = 1;
-        if (a.status) atomicExch(a.status, 1);
-    }
-    tc_fence_before_sync();
-    __syncthreads();
     if (warp == 0) {
         tc_fence_after_sync();
         tmem_dealloc(tmem, kCols);

@@ -67,6 +67,31 @@ def test_causal_attention_tensor_core_tiles(ctx, oracle, hd, T, start, heads, kv
     assert worst <= 1.0, worst
 
 
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+@pytest.mark.parametrize("hd", [128, 64])
+@pytest.mark.parametrize("T,start,key", [(200, 0, 70), (200, 37, 101), (127, 1, 127), (300, 100, 256), (40, 300, 339)])
+def test_causal_attention_hidden_value_does_not_show(ctx, oracle, hd, T, start, key, bad):
+    """One value of one position is not finite: the queries before that position do not see it, the others see it in its dimension
+    and nowhere else.  What stays finite is held to the bound of the kernel's other tests, against a cache with a 0 in its place."""
+    import runit_mac_b200 as R
+    from oracle import prefill as OP
+    heads, kvh, n, d = 4, 2, start + T, hd - 3
+    rng = np.random.default_rng(T + hd + key)
+    q = rng.normal(0, 1, (T, heads * hd)).astype(np.float32)
+    kc, vc = (rng.normal(0, 1, (kvh, n, hd)).astype(np.float16) for _ in range(2))
+    vc[1, key, d] = bad
+    ob = ctx.new_buffer(T * heads * hd * 2)
+    R.prefill_attention_f16kv(ctx, ctx.buffer_from(q), ctx.buffer_from(kc), ctx.buffer_from(vc), ob, T, heads, kvh, hd, n, start)
+    ctx.flush()
+    got = bf16_bits_to_f32(ob.download(np.uint16, T * heads * hd)).reshape(T, heads, hd)
+    vc[1, key, d] = 0
+    ref = OP.causal_attention_f16(q, kc, vc, heads, kvh, hd, start_pos=start).reshape(T, heads, hd)
+    sees = np.zeros(got.shape, bool)
+    sees[max(key - start, 0):, 2:, d] = True
+    assert not np.isfinite(got[sees]).any()
+    assert_close(oracle, ref[~sees], got[~sees], rel_tol=5e-3, what="value of position %d" % key)
+
+
 @pytest.mark.parametrize("hd", [128, 64])
 def test_causal_attention_calls_in_a_row(ctx, hd):
     """Calls that follow one another without a wait, each with more blocks than SMs: a dependent call starts while the one before
