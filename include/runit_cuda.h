@@ -278,9 +278,7 @@ int32_t runit_moe_route_topk(runit_ctx_t*, const void* logits, int32_t logits_f1
 enum { RUNIT_SCORE_SOFTMAX = 0, RUNIT_SCORE_SIGMOID = 1 };
 int32_t runit_moe_route_scored(runit_ctx_t*, const void* logits, uint32_t ld, uint32_t E, uint32_t k, int32_t score, int32_t renorm,
                                uint32_t T, void* out_idx, void* out_w);
-/* Scratch bytes runit_moe_layer_q4k uses for these shapes.  For 4 to 4096 tokens this includes the area in which the slots are
- * sorted by expert; a scratch that holds only the intermediates (T * (4 E + k (8 + 4 ff + 4 h)) bytes, every term rounded up to
- * 256) is accepted too and streams an expert for every slot. */
+/* Scratch bytes runit_moe_layer_q4k needs for these shapes. */
 size_t runit_moe_scratch_bytes(uint32_t T, uint32_t h, uint32_t ff, uint32_t E, uint32_t k);
 /* One MoE block over T tokens, all on the device:
  *   out[t] = (residual ? residual[t] : 0) + sum_i w_i * Wdown[e_i] . (silu(Wgate[e_i].x[t]) * (Wup[e_i].x[t]))
@@ -323,7 +321,7 @@ int32_t runit_moe_layer_q4k_ep(runit_ctx_t*, const void* router_w, const void* g
  * whole device.  This entry point allocates nothing (no cudaMalloc/cudaFree, no allocating library call);
  * its intermediates live in a fixed 4 MiB region (runit_moe_static_scratch_capacity()) built into the
  * library image, which every GPU that loads the library holds until the process exits.
- *   - Shapes whose intermediates do not fit (the smaller size named at runit_moe_scratch_bytes; e.g. OLMoE
+ *   - Shapes whose intermediates do not fit (runit_moe_scratch_bytes(T,h,ff,E,k) > capacity; e.g. OLMoE
  *     shapes beyond 32 tokens) are rejected with RUNIT_ERR_BUFFER_SIZE and nothing is launched.
  *   - The first call on a device looks up the region's device address (once per device, with that device
  *     made current for the lookup) and keeps it for the life of the process; make that first call before any

@@ -108,6 +108,9 @@ static int32_t ctx_init(int32_t device, cudaStream_t adopt, bool adopt_stream, r
     else { c->d_kq = nullptr; cudaGetLastError(); }
     if (cudaMalloc(&c->d_xq, 4u << 20) == cudaSuccess) c->xq_bytes = 4u << 20;
     else { c->d_xq = nullptr; cudaGetLastError(); }
+    // MoE layer with its slots sorted by expert: 1400 tokens of 8 of 64 experts at width 2048, 160 of 8 of 256 at width 7168
+    if (cudaMalloc(&c->d_slots, 96u << 20) == cudaSuccess) c->slots_bytes = 96u << 20;
+    else { c->d_slots = nullptr; cudaGetLastError(); }
     {
         cudaDriverEntryPointQueryResult qres;
         void* fn = nullptr;
@@ -167,6 +170,7 @@ int32_t runit_ctx_destroy(runit_ctx_t* ctx) {
     cudaStreamSynchronize(ctx->stream);   // Drop flushes, context.rs:299-304
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
     if (ctx->d_xq) cudaFree(ctx->d_xq);
+    if (ctx->d_slots) cudaFree(ctx->d_slots);
     if (ctx->d_am) cudaFree(ctx->d_am);
     if (ctx->d_xq_ctl) cudaFree(ctx->d_xq_ctl);
     if (ctx->d_kq) cudaFree(ctx->d_kq);
@@ -221,6 +225,7 @@ int32_t runit_set_tuning(runit_ctx_t* ctx, const char* key, int32_t value) {
     else if (!strcmp(key, "stream_ksl")) ctx->tune.stream_ksl = value;
     else if (!strcmp(key, "stream_dynamic")) ctx->tune.stream_dynamic = value;
     else if (!strcmp(key, "moe_slots")) ctx->tune.moe_slots = value;
+    else if (!strcmp(key, "moe_piece")) ctx->tune.moe_piece = value;
     else if (!strcmp(key, "router_variant")) ctx->tune.router_variant = value;
     else if (!strcmp(key, "ep_fused_exchange")) ctx->tune.ep_fused_exchange = value;
     else if (!strcmp(key, "imma_fold")) ctx->tune.imma_fold = value;

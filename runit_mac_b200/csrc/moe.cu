@@ -36,15 +36,21 @@ struct MoeScratch {
     size_t bytes;
 };
 
-// Tokens for which the scratch size includes the area in which the slots are sorted by expert (moe_slots.cu).
-static bool moe_has_staging(uint32_t T) { return T >= 4 && T <= 4096; }
+// Tokens that share a pass over the experts with their slots sorted by expert (moe_slots.cu), 0: launches per slot.  The sorted activations
+// lie in the context's staging area, so that neither the caller's scratch nor its size has a say; a call with more tokens than it holds is cut
+// into equal pieces.
 // Sorting by expert pays from 1.5 slots per expert on, where experts begin to be read for several slots at once (us with /
 // without, 64 experts of 2048 x 1024, top 8: 8 tokens 85 / 68, 12: 88 / 93, 24: 112 / 167; 128 experts of 2048 x 768, top 8: 12 tokens
 // 96 / 69, 24: 119 / 119; 60 of 2048 x 1024, top 4: 12 tokens 77 / 55, 24: 88 / 92), and where the products outweigh its four
 // more launches (8 experts of 1024 x 512, top 2: 48 tokens 38 / 34, 64: 39 / 41).
-static bool moe_by_expert(const runit_ctx* ctx, uint32_t T, uint32_t h, uint32_t ff, uint32_t E, uint32_t k) {
-    if (!moe_has_staging(T) || ctx->tune.moe_slots == 2) return false;
-    return ctx->tune.moe_slots == 1 || (2ull * T * k >= 3ull * E && (uint64_t)T * k * h * ff >= (1ull << 26));
+static uint32_t moe_piece(const runit_ctx* ctx, uint32_t T, uint32_t h, uint32_t ff, uint32_t E, uint32_t k) {
+    if (T < 4 || !ctx->d_slots || ctx->tune.moe_slots == 2) return 0;
+    uint32_t most = moe_slots_tokens(ctx->slots_bytes, h, ff, E, k);
+    if (ctx->tune.moe_piece > 0 && (uint32_t)ctx->tune.moe_piece < most) most = (uint32_t)ctx->tune.moe_piece;
+    if (most == 0) return 0;
+    const uint32_t n = (T + most - 1) / most, piece = (T + n - 1) / n;
+    const bool pays = 2ull * piece * k >= 3ull * E && (uint64_t)piece * k * h * ff >= (1ull << 26);
+    return pays || ctx->tune.moe_slots == 1 ? piece : 0;
 }
 
 // Expert-parallel decode block, replicated tokens.  This rank's weighted sum over the slots whose expert it owns
@@ -147,11 +153,15 @@ int32_t moe_layer_q4k_impl(runit_ctx* ctx, const void* router_w, const void* gat
         if (st != RUNIT_OK) return st;
     }
     const uint32_t slots = T * k;
-    // a scratch without the staging area (the built-in region at larger shapes) keeps the launches per slot
-    if (moe_by_expert(ctx, T, h, ff, E, k) && !fused_route && scratch_bytes >= s.bytes + moe_slots_bytes(T, h, ff, E, k) && ctx->encode_tiled && ctx->tune.gemv_math != 1 &&
-        ctx->tune.gemv_variant != 1 && runit_aligned(gate, 16) && runit_aligned(up, 16) && runit_aligned(down, 16)) {
-        st = moe_slots_experts(ctx, gate, up, down, (const float*)x, idx, s.act, s.y, (uint8_t*)scratch + s.bytes, T, h, ff, E, k);
-        if (st != RUNIT_OK) return st;
+    const uint32_t piece = moe_piece(ctx, T, h, ff, E, k);
+    if (piece > 0 && !fused_route && ctx->encode_tiled && ctx->tune.gemv_math != 1 && ctx->tune.gemv_variant != 1 && runit_aligned(gate, 16) &&
+        runit_aligned(up, 16) && runit_aligned(down, 16)) {
+        for (uint32_t t = 0; t < T; t += piece) {
+            const size_t slot = (size_t)t * k;
+            st = moe_slots_experts(ctx, gate, up, down, (const float*)x + (size_t)t * h, idx + slot, s.act + slot * ff, s.y + slot * h, ctx->d_slots,
+                                   T - t < piece ? T - t : piece, h, ff, E, k);
+            if (st != RUNIT_OK) return st;
+        }
         runit_launch_chain(ctx, moe_combine_kernel, dim3((h + 255) / 256, T), dim3(256), (const float*)s.y, (const float*)wts, (const float*)residual, (float*)out, T, h, k);
         st = runit_after_launch(ctx, "moe_combine");
         if (st != RUNIT_OK || !next_gamma) return st;
@@ -326,7 +336,7 @@ int32_t runit_moe_layer_q4k_static(runit_ctx_t* ctx, const void* router_w, const
 }
 
 size_t runit_moe_scratch_bytes(uint32_t T, uint32_t h, uint32_t ff, uint32_t E, uint32_t k) {
-    return moe_carve(nullptr, T, h, ff, E, k).bytes + (moe_has_staging(T) ? moe_slots_bytes(T, h, ff, E, k) : 0);
+    return moe_carve(nullptr, T, h, ff, E, k).bytes;
 }
 
 int32_t runit_moe_router_f32(runit_ctx_t* ctx, const void* router_w, const void* x, void* logits, uint32_t E, uint32_t h,

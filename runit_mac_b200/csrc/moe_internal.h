@@ -19,10 +19,10 @@ int32_t moe_route_gated(runit_ctx* ctx, const float* w, const float* x, float* l
                         float eps, float* xn_out);
 
 // moe_slots.cu: the expert products of T tokens with every expert read once for up to 32 slots; y[slot] f32 [T * k][h].
-// scratch: moe_slots_bytes, 256-byte aligned; matrices 16-byte aligned.
-size_t moe_slots_bytes(uint32_t T, uint32_t h, uint32_t ff, uint32_t E, uint32_t k);
+// T at most moe_slots_tokens(staging_bytes, ...); staging 256-byte aligned, matrices 16-byte aligned.
+uint32_t moe_slots_tokens(size_t staging_bytes, uint32_t h, uint32_t ff, uint32_t E, uint32_t k);
 int32_t moe_slots_experts(runit_ctx* ctx, const void* gate, const void* up, const void* down, const float* x, const int32_t* idx, float* act,
-                          float* y, void* scratch, uint32_t T, uint32_t h, uint32_t ff, uint32_t E, uint32_t k);
+                          float* y, void* staging, uint32_t T, uint32_t h, uint32_t ff, uint32_t E, uint32_t k);
 
 constexpr int kMoeRowAlign = 128;   // every expert's rows start at a multiple of this in the permuted order
 struct MoePermutation {

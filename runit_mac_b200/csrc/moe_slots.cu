@@ -323,14 +323,19 @@ static uint32_t slots_max_tiles(uint32_t n_slots, uint32_t E) {
     return (uint32_t)(t < n_slots ? t : n_slots);
 }
 
-size_t moe_slots_bytes(uint32_t T, uint32_t h, uint32_t ff, uint32_t E, uint32_t k) {
-    const uint32_t mt = slots_max_tiles(T * k, E), units = (h > ff ? h : ff) / 256;
-    return 256 + ((size_t)mt * (2 + slots::kCols) * 4 + 255) / 256 * 256 + (size_t)mt * units * slots::kXBytes;
+// staging: 256 bytes, table and order of the tiles (rounded up to 256), their activations
+uint32_t moe_slots_tokens(size_t staging_bytes, uint32_t h, uint32_t ff, uint32_t E, uint32_t k) {
+    const size_t per_tile = (2 + slots::kCols) * 4 + (size_t)((h > ff ? h : ff) / 256) * slots::kXBytes;
+    if (staging_bytes < 512 + per_tile) return 0;
+    const size_t tiles = (staging_bytes - 512) / per_tile;
+    // slots_max_tiles(n, E) <= tiles: n / 8 + E tiles at most, and never more than n
+    const size_t n = tiles > E ? (tiles - E) * slots::kCols : 0, slots = n > tiles ? n : tiles;
+    return (uint32_t)(slots / k < 65536 ? slots / k : 65536);
 }
 
 template <int G>
 static int32_t slots_run(runit_ctx* ctx, const void* gate, const void* up, const void* down, const float* x, const int32_t* idx, float* act, float* y,
-                         void* scratch, uint32_t n_slots, uint32_t h, uint32_t ff, uint32_t E, uint32_t k) {
+                         void* staging, uint32_t n_slots, uint32_t h, uint32_t ff, uint32_t E, uint32_t k) {
     using namespace slots;
     using S = Shape<G>;
     CUtensorMap mg, mu, md;
@@ -345,9 +350,9 @@ static int32_t slots_run(runit_ctx* ctx, const void* gate, const void* up, const
         if (ctx->device < 64) configured[ctx->device] = true;
     }
     const uint32_t mt = slots_max_tiles(n_slots, E), ctas = (uint32_t)ctx->sm_count * S::kPerSm;
-    int32_t* table = (int32_t*)scratch;
+    int32_t* table = (int32_t*)staging;
     int32_t* order = table + 64 + (size_t)mt * 2;
-    uint8_t* frags = (uint8_t*)scratch + 256 + ((size_t)mt * (2 + kCols) * 4 + 255) / 256 * 256;
+    uint8_t* frags = (uint8_t*)staging + 256 + ((size_t)mt * (2 + kCols) * 4 + 255) / 256 * 256;
     auto grid = [&](uint32_t tiles) { return dim3(mt * tiles < ctas ? mt * tiles : ctas); };
     runit_launch_chain(ctx, slots_table_kernel, dim3(1), dim3(1024), idx, n_slots, E, (uint32_t)G, table, order);
     if ((st = runit_after_launch(ctx, "moe_slots_table")) != RUNIT_OK) return st;
@@ -367,9 +372,9 @@ static int32_t slots_run(runit_ctx* ctx, const void* gate, const void* up, const
 }
 
 int32_t moe_slots_experts(runit_ctx* ctx, const void* gate, const void* up, const void* down, const float* x, const int32_t* idx, float* act,
-                          float* y, void* scratch, uint32_t T, uint32_t h, uint32_t ff, uint32_t E, uint32_t k) {
-    return T * k <= 8 * E ? slots_run<1>(ctx, gate, up, down, x, idx, act, y, scratch, T * k, h, ff, E, k)
-                          : slots_run<4>(ctx, gate, up, down, x, idx, act, y, scratch, T * k, h, ff, E, k);
+                          float* y, void* staging, uint32_t T, uint32_t h, uint32_t ff, uint32_t E, uint32_t k) {
+    return T * k <= 8 * E ? slots_run<1>(ctx, gate, up, down, x, idx, act, y, staging, T * k, h, ff, E, k)
+                          : slots_run<4>(ctx, gate, up, down, x, idx, act, y, staging, T * k, h, ff, E, k);
 }
 
 }  // namespace runit

@@ -52,6 +52,18 @@ def test_status_strings_and_null_context_are_rejected_without_a_gpu():
     assert lib.runit_gemv_q4k_f32in_f32out(None, None, None, None, 1, 256) == 2
 
 
+@pytest.mark.parametrize("T", [1, 4, 8, 16, 32, 4096, 4097])
+def test_moe_scratch_is_the_intermediates(T):
+    """The size that INTEGRATION.md compares with the built-in region: what the layer puts there and no more."""
+    from runit_mac_b200 import _lib
+    lib = _lib.load()
+    h, ff, E, k = 2048, 1024, 64, 8
+    up = lambda n: (n + 255) // 256 * 256  # noqa: E731
+    need = up(4 * T * E) + 2 * up(4 * T * k) + up(4 * T * k * ff) + up(4 * T * k * h)
+    assert lib.runit_moe_scratch_bytes(T, h, ff, E, k) == need
+    assert (need <= lib.runit_moe_static_scratch_capacity()) == (T <= 32)
+
+
 def test_no_product_file_touches_the_oracle():
     """The product path must not import, link or call anything under oracle/."""
     for p in list((ROOT / "runit_mac_b200").rglob("*.py")) + list((ROOT / "runit_mac_b200" / "csrc").glob("*")):

@@ -13,16 +13,19 @@ from helpers import assert_close
 pytestmark = pytest.mark.gpu
 
 
-def run(ctx, R, weights, x, res, h, ff, E, k, nbytes):
+def run(ctx, R, weights, x, res, h, ff, E, k, slots=1, piece=0):
     T = x.shape[0]
+    nbytes = R.moe_scratch_bytes(ctx, T, h, ff, E, k)
     out, idx, w = ctx.new_buffer(T * h * 4), ctx.new_buffer(T * k * 4), ctx.new_buffer(T * k * 4)
     scratch = ctx.new_buffer(nbytes)
-    ctx.set_tuning("moe_slots", 1)                  # small layers, too
+    ctx.set_tuning("moe_slots", slots)              # 1: small layers, too; 2: launches per slot
+    ctx.set_tuning("moe_piece", piece)
     try:
         R.moe_layer_q4k(ctx, *weights, ctx.buffer_from(x), ctx.buffer_from(res), out, idx, w, scratch, nbytes, T, h, ff, E, k, 0)
         ctx.flush()
     finally:
         ctx.set_tuning("moe_slots", 0)
+        ctx.set_tuning("moe_piece", 0)
     return out.download(np.float32, T * h).reshape(T, h), idx.download(np.int32, T * k).reshape(T, k)
 
 
@@ -42,15 +45,35 @@ def test_layer_matches_oracle(ctx, oracle, T, h, ff, E, k):
     res = rng.normal(0, 1, (T, h)).astype(np.float32)
     ref, ridx, _ = O.moe_layer_q4k(router, gate, up, down, x, h=h, ff=ff, E=E, top_k=k, renorm=False, residual=res)
     weights = [ctx.buffer_from(a) for a in (router, gate, up, down)]
-    full = R.moe_scratch_bytes(ctx, T, h, ff, E, k)
-    up256 = lambda n: (n + 255) // 256 * 256  # noqa: E731
-    small = up256(T * E * 4) + 2 * up256(T * k * 4) + up256(T * k * ff * 4) + up256(T * k * h * 4)
-    assert small < full
-    got, idx = run(ctx, R, weights, x, res, h, ff, E, k, full)
+    got, idx = run(ctx, R, weights, x, res, h, ff, E, k)
     same = (np.sort(idx, 1) == np.sort(ridx, 1)).all(1)
     assert same.sum() >= T - 1                      # at most one near tie
     assert_close(O, ref[same], got[same], rel_tol=2e-5, what="slots by expert")
-    again, _ = run(ctx, R, weights, x, res, h, ff, E, k, full)
+    again, _ = run(ctx, R, weights, x, res, h, ff, E, k)
     assert (again == got).all()                     # the order of the slots inside an expert does not show
-    per_slot, _ = run(ctx, R, weights, x, res, h, ff, E, k, small)
+    pieces, _ = run(ctx, R, weights, x, res, h, ff, E, k, piece=7)      # several passes over one staging area
+    assert_close(O, ref[same], pieces[same], rel_tol=2e-5, what="in pieces")
+    per_slot, _ = run(ctx, R, weights, x, res, h, ff, E, k, slots=2)
     assert_close(O, ref[same], per_slot[same], what="launches per slot")
+
+
+def test_built_in_scratch_gives_the_same_bits(ctx, oracle):
+    """A size at which the slots are sorted and the intermediates fill a good part of the built-in region."""
+    import runit_mac_b200 as R
+    O = oracle
+    T, h, ff, E, k = 48, 1024, 512, 16, 8
+    rng = np.random.default_rng(48)
+    weights = [ctx.buffer_from(a) for a in [rng.normal(0, 0.05, (E, h)).astype(np.float32)] + [O.rand_q4k(rng, E * r, c) for r, c in ((ff, h), (ff, h), (h, ff))]]
+    x = ctx.buffer_from(rng.normal(0, 1, (T, h)).astype(np.float32))
+    nbytes = R.moe_scratch_bytes(ctx, T, h, ff, E, k)
+    assert nbytes <= ctx.lib.runit_moe_static_scratch_capacity()
+    outs = [ctx.new_buffer(T * h * 4) for _ in range(2)]
+    count = [ctx.launches]
+    R.moe_layer_q4k(ctx, *weights, x, None, outs[0], None, None, ctx.new_buffer(nbytes), nbytes, T, h, ff, E, k, 0)
+    count.append(ctx.launches)
+    R.moe_layer_q4k_static(ctx, *weights, x, None, outs[1], None, None, T, h, ff, E, k, 0)
+    count.append(ctx.launches)
+    assert count[2] - count[1] == count[1] - count[0]
+    ctx.flush()
+    a, b = (o.download(np.float32, T * h) for o in outs)
+    assert np.isfinite(a).all() and np.array_equal(a, b)
