@@ -8,8 +8,9 @@
 //     multiply-add turn two nibbles into the operand (1024 + q) * sc - 1024 * sc without rounding; d and dmin meet the
 //     256-weight sums in f32.  The unpacked operand serves all the group's columns.
 //   * an activation is x = 2^e * (hi + lo) with f16 hi and lo and one power of two per 256 elements of a slot: 22 bits, error
-//     at most 2^-22 of the value or 2^-35 of the unit's largest (split_slots_kernel).
-//   * sum_j m_j * (sum of x over block j) is one more MMA per unit with the minimums as A and the split block sums as B.
+//     at most 2^-22 of the value or 2^-35 of the unit's largest (split_slots_kernel: the largest lies near the top of f16's range, because
+//     the halves of the high nibbles' activations, which are stored as x / 16, end at its smallest step).
+//   * sum_j m_j * (sum of x over block j) is one more MMA per unit with 32 * m as A and the split block sums / 32 as B.
 // Bound: at 2 slots per expert (16 tokens) the unpacking, 300 instructions per warp for 16 x 256 weights at 8 columns; at 32
 // slots (256 tokens) the MMA pipe (65 % active).  Measured for the layer of width 2048, 64 experts of 1024, top 8: 16 tokens 117 ->
 // 95 us, 256 tokens 1586 -> 291 us, error against 64 bits 4.2e-6 -> 1.2e-7 of the output.  One m16 tile per warp: with two
@@ -109,9 +110,9 @@ __global__ void __launch_bounds__(256) split_slots_kernel(const float* __restric
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     bad = __any_sync(0xffffffffu, bad);
-    // 2^e such that the largest |x| / 2^e lies in [512, 1024): a block sum stays below 2^15.  e is held above -116 so that both
-    // powers are normal numbers.
-    int e = (int)((__float_as_uint(amax) >> 23) & 255u) - 127 - 9;
+    // 2^e such that the largest |x| / 2^e lies in [2^14, 2^15): so does a 32nd of a block's sum.  e is held above -116 so that both powers
+    // are normal numbers.
+    int e = (int)((__float_as_uint(amax) >> 23) & 255u) - 127 - 14;
     e = e < -116 ? -116 : e;
     const float scale = bad ? __uint_as_float(0x7FC00000u) : __uint_as_float((uint32_t)(e + 127) << 23);
     const float inv = __uint_as_float((uint32_t)(127 - e) << 23);
@@ -129,6 +130,7 @@ __global__ void __launch_bounds__(256) split_slots_kernel(const float* __restric
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane == 0) {
+            s *= 0.03125f;
             const uint32_t si = (b >> 1) + 4 * (b & 1);
             const __half sh = __float2half_rn(s), sl = __float2half_rn(s - __half2float(sh));
             __half* q = reinterpret_cast<__half*>(out + 8192 + (n * 4 + (si >> 1)) * 8) + (si & 1);
@@ -277,7 +279,7 @@ __global__ void __launch_bounds__(Shape<G>::kThreads, Shape<G>::kPerSm) slots_ge
                 for (int r = 0; r < 2; r++) {
                     const uint32_t m = t < 2 ? sc[r].ml : sc[r].mh;
                     const uint32_t p = __byte_perm(m, 0x64646464u, (t & 1) ? 0x4342u : 0x4140u);
-                    am[r] = am[2 + r] = as_u32(__hsub2(as_half2(p), as_half2(0x64006400u)));
+                    am[r] = am[2 + r] = as_u32(__hfma2(as_half2(p), as_half2(0x50005000u), as_half2(0xF800F800u)));      // 32 * (p - 1024), exact
                 }
 #pragma unroll
                 for (int n = 0; n < G; n++)

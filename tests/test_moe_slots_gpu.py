@@ -1,6 +1,6 @@
 """Expert products with the slots sorted by expert (moe_slots.cu), through runit_moe_layer_q4k, against the oracle.
 
-Bound: an activation keeps 22 bits (two f16 halves of x / 2^e, error <= 2^-22 of it), products and the unpacked weights are
+Bound: an activation keeps 22 bits (two f16 halves of x / 2^e, error <= 2^-22 of it or 2^-35 of the largest of its 256), products and the unpacked weights are
 exact, sums are f32 over 256 weights and then over units.  With the 2^-24 of every f32 addition along h / 256 units and the
 rounding of silu, 2e-5 of max(|ref|, rms) holds with room.  The launches per slot have 16-bit activations: up to 2^-15 of the
 block's largest value in each of three products, 32 blocks' worth of which lie above the spread where a block holds an outlier;
@@ -55,6 +55,33 @@ def test_layer_matches_oracle(ctx, oracle, T, h, ff, E, k):
     assert_close(O, ref[same], pieces[same], rel_tol=2e-5, what="in pieces")
     per_slot, _ = run(ctx, R, weights, x, res, h, ff, E, k, slots=2)
     assert_close(O, ref[same], per_slot[same], what="launches per slot")
+
+
+def test_outlier_without_weight(ctx, oracle):
+    """An activation 2^18 times as large as the others of its unit, in a block whose weights are 0: what is left are the small ones, whose
+    halves are off by 2^-35 of the largest at most, 2^-17 of a small one, in the mean square over the 512 a quarter of 2^-17 / sqrt(3): 1e-6,
+    and five times that at the largest of the outputs."""
+    import runit_mac_b200 as R
+    O = oracle
+    T, h, ff, E, k = 16, 512, 256, 2, 2
+    rng = np.random.default_rng(16)
+
+    def matrix(rows, cols, hole):
+        nb = cols // 256
+        d, dmin = np.abs(rng.normal(0, 0.003, (rows, nb))) + 1e-3, np.abs(rng.normal(0, 0.003, (rows, nb)))
+        sc, mn = (rng.integers(0, 64, (rows, nb, 8), dtype=np.uint8) for _ in range(2))
+        if hole:
+            sc[:, 0, 0], mn[:, 0, 0] = 0, 0         # the unit's first block
+        return O.pack_q4k(d, dmin, sc, mn, rng.integers(0, 16, (rows, nb, 256), dtype=np.uint8))
+
+    router = rng.normal(0, 0.05, (E, h)).astype(np.float32)
+    router[:, :32] = 0
+    gate, up, down = (np.stack([matrix(r, c, c == h) for _ in range(E)]) for r, c in ((ff, h), (ff, h), (h, ff)))
+    x = rng.normal(0, 1, (T, h)).astype(np.float32)
+    x[:, 7] = 2.0 ** 18
+    ref, _, _ = O.moe_layer_q4k(router, gate, up, down, x, h=h, ff=ff, E=E, top_k=k, renorm=False)
+    got, _ = run(ctx, R, [ctx.buffer_from(a) for a in (router, gate, up, down)], x, np.zeros((T, h), np.float32), h, ff, E, k)
+    assert_close(O, ref, got, rel_tol=2e-5, what="outlier without weight")
 
 
 def test_built_in_scratch_gives_the_same_bits(ctx, oracle):
