@@ -176,6 +176,9 @@ pub fn moe_route_scored(ctx: &CudaContext, logits: &B, ld: u32, E: u32, k: u32, 
 pub fn moe_layer_q4k(ctx: &CudaContext, router_w: &B, gate: &B, up: &B, down: &B, x: &B, residual: &B, out: &B, idx_out: &B, w_out: &B, scratch: &B, scratch_bytes: usize, T: u32, h: u32, ff: u32, E: u32, k: u32, renorm: i32) -> Result<()> {
     ctx.check(unsafe { ffi::runit_moe_layer_q4k(ctx.raw, router_w.ptr as *const c_void, gate.ptr as *const c_void, up.ptr as *const c_void, down.ptr as *const c_void, x.ptr as *const c_void, residual.ptr as *const c_void, out.ptr, idx_out.ptr, w_out.ptr, scratch.ptr, scratch_bytes, T, h, ff, E, k, renorm) })
 }
+pub fn moe_layer_q4k_by_slot(ctx: &CudaContext, router_w: &B, gate: &B, up: &B, down: &B, x: &B, residual: &B, out: &B, idx_out: &B, w_out: &B, scratch: &B, scratch_bytes: usize, T: u32, h: u32, ff: u32, E: u32, k: u32, renorm: i32) -> Result<()> {
+    ctx.check(unsafe { ffi::runit_moe_layer_q4k_by_slot(ctx.raw, router_w.ptr as *const c_void, gate.ptr as *const c_void, up.ptr as *const c_void, down.ptr as *const c_void, x.ptr as *const c_void, residual.ptr as *const c_void, out.ptr, idx_out.ptr, w_out.ptr, scratch.ptr, scratch_bytes, T, h, ff, E, k, renorm) })
+}
 pub fn moe_experts_q4k(ctx: &CudaContext, gate: &B, up: &B, down: &B, x_slots: &B, slot_expert: &B, y_slots: &B, act_scratch: &B, n_slots: u32, h: u32, ff: u32, n_experts: u32) -> Result<()> {
     ctx.check(unsafe { ffi::runit_moe_experts_q4k(ctx.raw, gate.ptr as *const c_void, up.ptr as *const c_void, down.ptr as *const c_void, x_slots.ptr as *const c_void, slot_expert.ptr as *const c_void, y_slots.ptr, act_scratch.ptr, n_slots, h, ff, n_experts) })
 }

@@ -199,6 +199,7 @@ extern "C" {
     pub fn runit_moe_route_scored(a0: *mut runit_ctx_t, logits: *const c_void, ld: u32, E: u32, k: u32, score: i32, renorm: i32, T: u32, out_idx: *mut c_void, out_w: *mut c_void) -> i32;
     pub fn runit_moe_scratch_bytes(T: u32, h: u32, ff: u32, E: u32, k: u32) -> usize;
     pub fn runit_moe_layer_q4k(a0: *mut runit_ctx_t, router_w: *const c_void, gate: *const c_void, up: *const c_void, down: *const c_void, x: *const c_void, residual: *const c_void, out: *mut c_void, idx_out: *mut c_void, w_out: *mut c_void, scratch: *mut c_void, scratch_bytes: usize, T: u32, h: u32, ff: u32, E: u32, k: u32, renorm: i32) -> i32;
+    pub fn runit_moe_layer_q4k_by_slot(a0: *mut runit_ctx_t, router_w: *const c_void, gate: *const c_void, up: *const c_void, down: *const c_void, x: *const c_void, residual: *const c_void, out: *mut c_void, idx_out: *mut c_void, w_out: *mut c_void, scratch: *mut c_void, scratch_bytes: usize, T: u32, h: u32, ff: u32, E: u32, k: u32, renorm: i32) -> i32;
     pub fn runit_moe_experts_q4k(a0: *mut runit_ctx_t, gate: *const c_void, up: *const c_void, down: *const c_void, x_slots: *const c_void, slot_expert: *const c_void, y_slots: *mut c_void, act_scratch: *mut c_void, n_slots: u32, h: u32, ff: u32, n_experts: u32) -> i32;
     pub fn runit_moe_layer_q4k_ep(a0: *mut runit_ctx_t, router_w: *const c_void, gate_local: *const c_void, up_local: *const c_void, down_local: *const c_void, x: *const c_void, residual: *const c_void, out: *mut c_void, idx_out: *mut c_void, w_out: *mut c_void, scratch: *mut c_void, scratch_bytes: usize, partial_all: *const *mut c_void, signal_pads: *const *mut c_void, T: u32, h: u32, ff: u32, E: u32, k: u32, renorm: i32, world: u32, rank: u32, epoch: u32) -> i32;
     pub fn runit_moe_static_scratch_capacity() -> usize;

@@ -62,7 +62,8 @@ int32_t moe_layer_q4k_impl(runit_ctx* ctx, const void* router_w, const void* gat
                            // launch and the weighted sum of the experts runs inside the down-projection launch
                            uint32_t* route_counter,
                            // pre_gamma != nullptr: the block first writes RMSNorm(pre_x) into x (inside the routing launch when T == 1)
-                           const float* pre_x, const float* pre_gamma, float pre_eps);
+                           const float* pre_x, const float* pre_gamma, float pre_eps,
+                           bool by_slot = false);      // launches per slot at every T: the bits of a token do not depend on T
 size_t moe_scratch_bytes_impl(uint32_t T, uint32_t h, uint32_t ff, uint32_t E, uint32_t k);
 
 }  // namespace runit

@@ -115,7 +115,7 @@ int32_t moe_layer_q4k_impl(runit_ctx* ctx, const void* router_w, const void* gat
                            const void* x, const void* residual, void* out, int32_t* idx_out, float* w_out, void* scratch,
                            size_t scratch_bytes, uint32_t T, uint32_t h, uint32_t ff, uint32_t E, uint32_t k, int32_t renorm,
                            const float* next_gamma, float* next_xn, float next_eps, uint32_t* route_counter,
-                           const float* pre_x, const float* pre_gamma, float pre_eps) {
+                           const float* pre_x, const float* pre_gamma, float pre_eps, bool by_slot) {
     RUNIT_REQUIRE(ctx, router_w && gate && up && down && x && out && scratch, "moe_layer_q4k: null pointer");
     RUNIT_REQUIRE(ctx, T > 0 && T <= 65536, "moe_layer_q4k: T=%u out of range", T);
     RUNIT_REQUIRE(ctx, h % 256 == 0 && ff % 256 == 0 && h > 0 && ff > 0, "moe_layer_q4k: h=%u, ff=%u must be multiples of 256", h, ff);
@@ -153,7 +153,7 @@ int32_t moe_layer_q4k_impl(runit_ctx* ctx, const void* router_w, const void* gat
         if (st != RUNIT_OK) return st;
     }
     const uint32_t slots = T * k;
-    const uint32_t piece = moe_piece(ctx, T, h, ff, E, k);
+    const uint32_t piece = by_slot ? 0 : moe_piece(ctx, T, h, ff, E, k);
     if (piece > 0 && !fused_route && ctx->encode_tiled && ctx->tune.gemv_math != 1 && ctx->tune.gemv_variant != 1 && runit_aligned(gate, 16) &&
         runit_aligned(up, 16) && runit_aligned(down, 16)) {
         for (uint32_t t = 0; t < T; t += piece) {
@@ -393,6 +393,14 @@ int32_t runit_moe_layer_q4k(runit_ctx_t* ctx, const void* router_w, const void* 
     if (!ctx) return RUNIT_ERR_BAD_ARG;
     return moe_layer_q4k_impl(ctx, router_w, gate, up, down, x, residual, out, (int32_t*)idx_out, (float*)w_out, scratch,
                               scratch_bytes, T, h, ff, E, k, renorm, nullptr, nullptr, 0.f, nullptr, nullptr, nullptr, 0.f);
+}
+
+int32_t runit_moe_layer_q4k_by_slot(runit_ctx_t* ctx, const void* router_w, const void* gate, const void* up, const void* down,
+                                    const void* x, const void* residual, void* out, void* idx_out, void* w_out, void* scratch,
+                                    size_t scratch_bytes, uint32_t T, uint32_t h, uint32_t ff, uint32_t E, uint32_t k, int32_t renorm) {
+    if (!ctx) return RUNIT_ERR_BAD_ARG;
+    return moe_layer_q4k_impl(ctx, router_w, gate, up, down, x, residual, out, (int32_t*)idx_out, (float*)w_out, scratch,
+                              scratch_bytes, T, h, ff, E, k, renorm, nullptr, nullptr, 0.f, nullptr, nullptr, nullptr, 0.f, true);
 }
 
 }  // extern "C"

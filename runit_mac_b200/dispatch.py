@@ -268,6 +268,7 @@ _TWINS = [
     ("moe_route_scored", "no twin: (logits, ld, E, k, score, renorm, T, out_idx, out_w), score = SCORE_SOFTMAX / SCORE_SIGMOID"),
     ("moe_layer_q4k", "forward.rs:1644-1679 as one call: (router_w, gate, up, down, x, residual, out, idx_out, w_out, "
                       "scratch, scratch_bytes, T, h, ff, E, k, renorm)"),
+    ("moe_layer_q4k_by_slot", "the same with the decoding step's arithmetic at every T: a token's bits do not depend on T"),
     ("moe_experts_q4k", "no twin: (gate, up, down, x_slots, slot_expert, y_slots, act_scratch, n_slots, h, ff, n_experts)"),
     ("moe_layer_q4k_static", "no twin: moe_layer_q4k without the scratch arguments (built-in 4 MiB region)"),
     ("moe_layer_q4k_bf16", "no twin (prefill.rs:156-215 batched): same arguments as moe_layer_q4k, scratch from "

@@ -57,6 +57,28 @@ def test_layer_matches_oracle(ctx, oracle, T, h, ff, E, k):
     assert_close(O, ref[same], per_slot[same], what="launches per slot")
 
 
+@pytest.mark.parametrize("T", [2, 12, 65])
+def test_by_slot_gives_a_token_the_same_bits_at_every_size(ctx, oracle, T):
+    """What INTEGRATION.md promises for prefill against decode; the sizes are those at which runit_moe_layer_q4k sorts, too."""
+    import runit_mac_b200 as R
+    O = oracle
+    h, ff, E, k = 2048, 1024, 16, 4
+    rng = np.random.default_rng(T)
+    weights = [ctx.buffer_from(a) for a in [rng.normal(0, 0.05, (E, h)).astype(np.float32)] + [O.rand_q4k(rng, E * r, c) for r, c in ((ff, h), (ff, h), (h, ff))]]
+    x, res = rng.normal(0, 1, (T, h)).astype(np.float32), rng.normal(0, 1, (T, h)).astype(np.float32)
+
+    def layer(op, lo, hi):
+        n = hi - lo
+        out, nbytes = ctx.new_buffer(n * h * 4), R.moe_scratch_bytes(ctx, n, h, ff, E, k)
+        op(ctx, *weights, ctx.buffer_from(x[lo:hi]), ctx.buffer_from(res[lo:hi]), out, None, None, ctx.new_buffer(nbytes), nbytes, n, h, ff, E, k, 0)
+        ctx.flush()
+        return out.download(np.float32, n * h).reshape(n, h)
+
+    alone = np.concatenate([layer(R.moe_layer_q4k, t, t + 1) for t in range(T)])       # the decoding step's size
+    assert np.array_equal(layer(R.moe_layer_q4k_by_slot, 0, T), alone)
+    assert_close(O, alone, layer(R.moe_layer_q4k, 0, T), rel_tol=3e-4, what="sorted")
+
+
 def test_outlier_without_weight(ctx, oracle):
     """An activation 2^18 times as large as the others of its unit, in a block whose weights are 0: what is left are the small ones, whose
     halves are off by 2^-35 of the largest at most, 2^-17 of a small one, in the mean square over the 512 a quarter of 2^-17 / sqrt(3): 1e-6,
