@@ -74,6 +74,7 @@ static int32_t ctx_init(int32_t device, cudaStream_t adopt, bool adopt_stream, r
     if (adopt_stream) {
         c->stream = adopt;
         c->owns_stream = false;
+        c->foreign_kernels = true;
     } else {
         if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
             delete c;
@@ -181,7 +182,11 @@ int32_t runit_ctx_destroy(runit_ctx_t* ctx) {
     return RUNIT_OK;
 }
 
-void* runit_ctx_stream(runit_ctx_t* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
+void* runit_ctx_stream(runit_ctx_t* ctx) {
+    if (!ctx) return nullptr;
+    ctx->foreign_kernels = true;
+    return (void*)ctx->stream;
+}
 
 int32_t runit_flush(runit_ctx_t* ctx) {
     if (!ctx) return RUNIT_ERR_BAD_ARG;

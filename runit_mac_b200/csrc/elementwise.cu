@@ -236,6 +236,7 @@ int32_t runit_fill_weights(runit_ctx_t* ctx, int32_t fmt, void* dst, uint64_t n_
     RUNIT_REQUIRE(ctx, fmt >= 0 && fmt <= 2 && dst && n_blocks > 0, "fill_weights: bad argument");
     RUNIT_REQUIRE(ctx, n_blocks < (1ull << 38), "fill_weights: too many blocks");
     const uint64_t grid = (n_blocks + 255) / 256;
+    ctx->weights_written = true;
     fill_weights_kernel<<<(unsigned)grid, 256, 0, ctx->stream>>>(fmt, (uint8_t*)dst, n_blocks, seed, sigma, 0);
     return runit_after_launch(ctx, "fill_weights");
 }
@@ -244,6 +245,7 @@ int32_t runit_fill_weights_q4k_zero_mean(runit_ctx_t* ctx, void* dst, uint64_t n
     if (!ctx) return RUNIT_ERR_BAD_ARG;
     RUNIT_REQUIRE(ctx, dst && n_blocks > 0 && n_blocks < (1ull << 38), "fill_weights_q4k_zero_mean: bad argument");
     const uint64_t grid = (n_blocks + 255) / 256;
+    ctx->weights_written = true;
     fill_weights_kernel<<<(unsigned)grid, 256, 0, ctx->stream>>>(RUNIT_FMT_Q4K, (uint8_t*)dst, n_blocks, seed, sigma, 1);
     return runit_after_launch(ctx, "fill_weights_q4k_zero_mean");
 }

@@ -98,6 +98,8 @@ struct GemvArgs {
     // returned, i.e. once everything older than itself has completed.  grp_early: the predecessor was launched with
     // late_trigger, so the expert ids are final when this kernel starts: it requests its first weight stages before
     // its own wait (the activations come from the predecessor and follow the wait).
+    // grp_early == 2 (without groups, cp.async, set by launch_staged): the predecessor may be a kernel that writes the weights, so they
+    // are requested behind the wait as well.
     int32_t late_trigger, grp_early;
     const float* cmb_w;
     const float* cmb_res;
@@ -382,7 +384,7 @@ __global__ void __launch_bounds__(kNT, S <= 2 ? 4 : 3) gemv_staged_kernel(const 
     const uint32_t bar0 = smem_u32(&mbar[warp][0]);
 
     if (!a.late_trigger) grid_launch_dependents();   // let the next kernel of the stream begin its own prologue
-    const bool early_weights = a.grp_expert == nullptr || (LD == 1 && a.grp_early);
+    const bool early_weights = a.grp_expert == nullptr ? LD == 1 || a.grp_early != 2 : LD == 1 && a.grp_early;
     if (!early_weights) {
         grid_dependency_wait();
         if (a.late_trigger) grid_launch_dependents();

@@ -189,6 +189,7 @@ struct Args {
     float* part;
     uint32_t* tickets;       // one word per tile, zero at rest
     const uint8_t* xq;       // PRE: the prepared activations, kXq bytes per unit
+    uint32_t wait_first;     // the predecessor may be a kernel that writes the weights
 };
 constexpr int kXq = IntX<8>::BYTES;                  // 832: a multiple of 16
 
@@ -346,7 +347,8 @@ __global__ void __launch_bounds__(128) gemv_kquant_tile_kernel(const Args a) {
         }
         cp_async_commit();
     };
-    // the weights do not depend on the kernel before; its output may be x or the residual
+    // the weights do not depend on the kernel before, unless it is the caller's own; its output may be x or the residual
+    if (a.wait_first) grid_dependency_wait();
 #pragma unroll
     for (int s = 0; s < kS; s++) issue_w(s);
     grid_dependency_wait();
@@ -620,6 +622,7 @@ static int32_t launch(runit_ctx* ctx, const char* name, const void* w, const voi
         // 72 MB, 33 us without and 35 with it)
         const bool pre = FMT != RUNIT_FMT_Q5_0 && split == 0 && ctx->d_xq && (size_t)t.nb * kt::kXq <= ctx->xq_bytes && (uint64_t)m * t.row_bytes >= 150000000ull;
         t.xq = (const uint8_t*)ctx->d_xq;
+        t.wait_first = ctx->foreign_kernels ? 1u : 0u;
         int smem;
         void (*kern)(const kt::Args);
         if constexpr (FMT == RUNIT_FMT_Q5_0) {

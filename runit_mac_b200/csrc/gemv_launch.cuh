@@ -43,7 +43,11 @@ static inline int32_t launch_staged(runit_ctx* ctx, const GemvArgs& a, const Gem
     // (the early CTAs of the next grid double up on busy SMs instead of spreading out).  The cp.async kernels (Q8_0), whose copies
     // take a CTA longer to issue, gain at every size: decoding step of a 0.5B model 467 us with that exception, 451 without.
     const uint32_t sms = (uint32_t)ctx->sm_count;
-    const bool pdl = ctx->tune.pdl == 1 || (ctx->tune.pdl == 2 && (LD == 0 || grid < (2 * sms) / 3 || grid > (4 * sms) / 3));
+    const bool wait_first = LD == 0 && ctx->foreign_kernels;
+    if (wait_first && !a.grp_expert) args.grp_early = 2;
+    // behind an op that has written weights: an ordinary launch, which starts when all of it can be seen
+    const bool pdl = !ctx->weights_written && (ctx->tune.pdl == 1 || (ctx->tune.pdl == 2 && ((LD == 0 && !wait_first) || grid < (2 * sms) / 3 || grid > (4 * sms) / 3)));
+    ctx->weights_written = false;
     if (pdl) {
         attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[na].val.programmaticStreamSerializationAllowed = 1;

@@ -49,6 +49,9 @@ struct runit_ctx {
     int32_t device = 0;
     cudaStream_t stream = nullptr;
     bool owns_stream = false;
+    // The caller can put kernels of its own on the stream (adopted, or handed out): a launch that requests weights before it waits for its
+    // predecessor could read what such a kernel is about to write.  weights_written: an op of this library has just written weights.
+    bool foreign_kernels = false, weights_written = false;
     int32_t sm_count = 0;
     int32_t max_smem_optin = 0;
     uint64_t launches = 0;

@@ -1,0 +1,60 @@
+"""Weights that the kernel directly before a GEMV writes: ops of a context are in order on its stream, the caller's own kernels on an
+adopted stream and the library's fills included, although a dependent launch requests its first weights early elsewhere."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("tag,m,k,block,at", [("q8_0", 896, 896, 34, (0,)), ("q8_0", 4864, 896, 34, (0,)), ("q6k", 2048, 2048, 210, (208,)), ("q6k", 100, 256, 210, (208,)),
+                                              ("q5k", 3584, 1792, 176, (0, 2))])
+def test_callers_kernel_on_an_adopted_stream(tag, m, k, block, at):
+    import torch
+    import runit_mac_b200 as R
+    stream = torch.cuda.Stream()
+    ctx = R.Context(0, stream=stream.cuda_stream)
+    op = getattr(R, "gemv_%s_f32in_f32out" % tag)
+    try:
+        with torch.cuda.stream(stream):
+            n = m * k // (32 if block == 34 else 256)
+            g = torch.Generator(device="cuda").manual_seed(m)
+            sets = torch.randint(0, 256, (2, n, block), generator=g, device="cuda", dtype=torch.uint8)
+            scale = (torch.rand((2, n, 1), generator=g, device="cuda") + 0.5).half().view(torch.uint8)
+            for a in at:
+                sets[:, :, a:a + 2] = scale
+            w, x = torch.zeros_like(sets[0]), torch.randn(k, generator=g, device="cuda")
+            y = torch.zeros(50, m, device="cuda")
+            ref = torch.zeros(2, m, device="cuda")
+            for i in range(2):
+                torch.bitwise_xor(sets[i], 0, out=w)
+                torch.cuda.synchronize()
+                op(ctx, w, x, ref[i], m, k)
+                ctx.flush()
+            for i in range(50):
+                torch.bitwise_xor(sets[i % 2], 0, out=w)          # a kernel, not a copy
+                op(ctx, w, x, y[i], m, k)
+            ctx.flush()
+            assert torch.isfinite(ref).all() and not torch.equal(ref[0], ref[1])
+            for i in range(50):
+                assert torch.equal(y[i], ref[i % 2]), i
+    finally:
+        ctx.close()
+
+
+def test_fill_before_a_gemv(ctx):
+    import runit_mac_b200 as R
+    m = k = 896
+    w, x = ctx.new_buffer(m * k // 32 * 34), ctx.buffer_from(np.random.default_rng(0).normal(0, 1, k).astype(np.float32))
+    outs = []
+    for wait in (True, False):
+        ys = [ctx.new_buffer(m * 4) for _ in range(20)]
+        for i, y in enumerate(ys):
+            R.fill_weights(ctx, R.FMT_Q8_0, w, m * k // 32, i % 3, 0.02)
+            if wait:
+                ctx.flush()
+            R.gemv_q8_0_f32in_f32out(ctx, w, x, y, m, k)
+        ctx.flush()
+        outs.append([y.download(np.float32, m) for y in ys])
+    assert not np.array_equal(outs[0][0], outs[0][1])
+    for a, b in zip(*outs):
+        assert np.array_equal(a, b)
