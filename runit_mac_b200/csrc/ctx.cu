@@ -238,6 +238,7 @@ int32_t runit_set_tuning(runit_ctx_t* ctx, const char* key, int32_t value) {
     else if (!strcmp(key, "imma_csplit")) ctx->tune.imma_csplit = value;
     else if (!strcmp(key, "imma_stages")) ctx->tune.imma_stages = value;
     else if (!strcmp(key, "kquant_variant")) ctx->tune.kquant_variant = value;
+    else if (!strcmp(key, "kquant_prepare")) ctx->tune.kquant_prepare = value;
     else if (!strcmp(key, "kquant_split")) ctx->tune.kquant_split = value;
     else return runit_fail(ctx, RUNIT_ERR_BAD_ARG, "unknown tuning key '%s'", key);
     return RUNIT_OK;

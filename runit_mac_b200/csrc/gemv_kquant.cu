@@ -618,9 +618,13 @@ static int32_t launch(runit_ctx* ctx, const char* name, const void* w, const voi
         t.m = m;
         t.nb = k / 256;
         t.row_bytes = (k / 256) * (FMT == RUNIT_FMT_Q6K ? 210u : 176u);
-        // the preparing launch costs 2 us: from 150 MB of weights on it pays (Q6_K 152064 x 3584 147 -> 127 us; Q5_K 50304 x 2048,
-        // 72 MB, 33 us without and 35 with it)
-        const bool pre = FMT != RUNIT_FMT_Q5_0 && split == 0 && ctx->d_xq && (size_t)t.nb * kt::kXq <= ctx->xq_bytes && (uint64_t)m * t.row_bytes >= 150000000ull;
+        // The preparing launch costs 2 us, and rows of few units gain nothing from it (us without / with it).  K = 1024, Q6_K 300 MB 94 / 105;
+        // 2048, Q6_K 110 MB 47 / 44, 300 MB 91 / 97; 2560, Q6_K 260 MB 80 / 88, Q5_K 350 MB 100 / 103; 3072, 160 to 450 MB, -3 to +8 % in turn;
+        // 3584, Q6_K 160 MB 59 / 59, 220 MB 80 / 74, 450 MB 127 / 125, Q5_K 130 MB 46 / 48, 350 MB 100 / 95; 4096 to 12288, 160 MB and
+        // more: 1 to 10 % faster with it.
+        const bool pays = k >= 3584 && (uint64_t)m * t.row_bytes >= 150000000ull;
+        const bool pre = FMT != RUNIT_FMT_Q5_0 && split == 0 && ctx->d_xq && (size_t)t.nb * kt::kXq <= ctx->xq_bytes &&
+                         (ctx->tune.kquant_prepare == 0 ? pays : ctx->tune.kquant_prepare == 1);
         t.xq = (const uint8_t*)ctx->d_xq;
         t.wait_first = ctx->foreign_kernels ? 1u : 0u;
         int smem;

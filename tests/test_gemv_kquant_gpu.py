@@ -124,10 +124,12 @@ def test_kquant_tile_kernel(ctx, oracle, fmt, tag):
         ctx.set_tuning("kquant_variant", 0)
 
 
-@pytest.mark.parametrize("fmt,tag,m,k", [(5, "q6k", 100003, 2048), (5, "q6k", 100001, 1792), (4, "q5k", 110010, 2048)])
+@pytest.mark.parametrize("fmt,tag,m,k", [(5, "q6k", 101, 1792), (5, "q6k", 37901, 3584), (5, "q6k", 37895, 2304), (4, "q5k", 77, 1280), (4, "q5k", 37890, 2048),
+                                         (5, "q6k", 55811, 3584)])
 def test_kquant_prepared_activations(ctx, oracle, fmt, tag, m, k):
-    """Matrices large enough for the launch that prepares the activations: last rows of a partial tile, rows of odd half-word
-    offsets (1792 = 7 superblocks), next to the oracle on a sample of rows.  Same integers as without it: the bar above."""
+    """Activations prepared by a launch of their own: last rows of a partial tile, rows whose offset differs from row to row (odd counts of
+    210-byte superblocks), the size from which on the rule takes it (the last case).  The same integers and sums as without that
+    launch: the same bits, and the bar above on a sample of rows."""
     import torch
     import runit_mac_b200 as R
     O = oracle
@@ -139,11 +141,23 @@ def test_kquant_prepared_activations(ctx, oracle, fmt, tag, m, k):
         w[:, at:at + 2] = scale
     x = torch.randn(k, generator=g, device="cuda")
     x[5] = 500.0
-    y = torch.zeros(m, device="cuda")
+    y = torch.zeros(3, m, device="cuda")
     torch.cuda.synchronize()
-    getattr(R, "gemv_%s_f32in_f32out" % tag)(ctx, w, x, y, m, k)
+    launches = []
+    ctx.set_tuning("kquant_variant", 2)             # the tile kernel for few rows, too
+    try:
+        for i, how in enumerate((1, 2, 0)):
+            ctx.set_tuning("kquant_prepare", how)
+            before = ctx.launches
+            getattr(R, "gemv_%s_f32in_f32out" % tag)(ctx, w, x, y[i], m, k)
+            launches.append(ctx.launches - before)
+    finally:
+        ctx.set_tuning("kquant_variant", 0)
+        ctx.set_tuning("kquant_prepare", 0)
     ctx.flush()
-    rows = torch.cat([torch.arange(64), torch.arange(m - 70, m), torch.randint(0, m, (100,))])
+    assert launches == [2, 1, 2 if m * nb >= 150e6 and k >= 3584 else 1]
+    assert torch.equal(y[0], y[1]) and torch.equal(y[0], y[2])
+    rows = torch.cat([torch.arange(min(64, m)), torch.arange(max(0, m - 70), m), torch.randint(0, m, (100,))])
     ref = O.gemv(fmt, w.reshape(m, nb)[rows.cuda()].cpu().numpy(), x.cpu().numpy(), len(rows), k, O.TIER_F64)
-    st = assert_close(O, ref, y[rows.cuda()].cpu().numpy(), what=tag + " prepared activations")
+    st = assert_close(O, ref, y[0][rows.cuda()].cpu().numpy(), what=tag + " prepared activations")
     assert st.max_rel < 2e-5, st
