@@ -8,16 +8,16 @@
 //                 block i + 1 runs under the softmax of block i
 //   P             row maximum, exp2 and sum from tensor memory, two passes over S; P is rounded to f16 into the columns of S that the
 //                 thread has already read, which makes it the A operand of the second product
-//   O += P.V      V by TMA as it lies in the cache (hd contiguous: B is MN-major), accumulated in tensor memory.  P, the sum and O are
-//                 relative to a reference score, which follows the row maximum only when that has risen by more than 2^8 (P
-//                 then stays below 256, and f16 keeps its 11 bits); O and the sum are scaled by then, by the row's own threads.
-//                 The sum is that of the rounded P, because the largest P is no longer exactly 1.
+//   O += P.V      V by TMA as it lies in the cache (hd contiguous: B is MN-major), accumulated in tensor memory.  P, the sum (of the
+//                 unrounded P, f32) and O are relative to the row maximum so far; O is scaled by the row's own threads when that has risen, behind
+//                 P, where the product that it waits for is long over.
 // One CTA per SM: 161 KB (two buffers of K and V; 116 asked for at head dim 64) and all 512 tensor-memory columns.  Query blocks go from the most keys to the fewest.
-// Bound: a block's softmax (two passes, 1024 clocks of exponentials at 16 a clock and SM, the maximum's exchange).
+// Bound: one dependent chain per SM, about 5000 clocks per block, of which the exponentials are 1024 (16 a clock) and the products 512.
 // Measured, 2048 queries x 16 heads x 128: 102 us (mma.sync, 64 queries of 4 warps, 167 TFLOP/s of useful products), 58 with one
-// thread per query, one buffer of S and the block's output added in registers, 51 with two threads per query, 41 as it is (424
-// TFLOP/s); 1024 queries 45 -> 19 us, 2000 behind 1000 cached ones 156 -> 64.  The error against 64 bits is the bf16 output's, 1.7e-3,
-// on all of them.
+// thread per query, one buffer of S and the block's output added in registers, 51 with two threads per query, 41 as it is (421 TFLOP/s; 30
+// at head dim 64); 1024 queries 45 -> 19 us, 2000 behind 1000 cached ones 156 -> 62, 33 behind 300 17 -> 9.
+// The error against 64 bits is the bf16 output's, 1.677e-3, as it was.  A reference that follows the maximum only when that has risen by
+// 2^8 saves the scaling of O (40 us) but rounds the largest weights, which then are not 1: 1.678e-3, and up to twice the error before bf16.
 // Rows of the tensor maps end at start + T, so that what the cache holds behind the data (NaN included) reads as zeros.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -33,7 +33,6 @@ namespace atc {
 constexpr int kRows = 128, kKeys = 128;
 constexpr uint32_t kCols = 512;                    // tensor memory: S | P in columns 0..127 and 128..255, O from 256
 constexpr uint32_t kOnePerSm = 116 * 1024;         // shared memory that only one CTA of an SM can have
-constexpr float kRise = 8.f;                       // log2 of how far the maximum may rise above the reference
 
 template <int HD> struct Shape {
     static constexpr uint32_t kPanel = 128 * 128;  // 64 elements of 128 rows
@@ -292,28 +291,12 @@ __global__ void __launch_bounds__(288, 1) attention_tc_kernel(const __grid_const
                 part[i & 1][half][row] = mx;
                 asm volatile("bar.sync 1, 256;" ::: "memory");              // two blocks' slots: nobody is a whole block ahead of another
                 mx = fmaxf(mx, part[i & 1][half ^ 1][row]) * a.scale_log2;
-                const bool rise = mx > ref + kRise || (ref == -INFINITY && mx > ref);
-                late = 1.f;
-                if (__any_sync(0xffffffffu, rise)) {
-                    const float to = rise ? mx : ref, corr = rise ? exp2_approx(ref - to) : 1.f;
-                    l *= corr;
-                    late = corr;
-                    ref = to;
-                    if (i > 0) {
-                        if (ok) ok = mbar_wait_timed(o_full, (i - 1) & 1, &abort_flag);
-                        __syncwarp();
-                        tc_fence_after_sync();
-#pragma unroll
-                        for (int c = 0; c < HD / 64; c++) {
-                            uint32_t r[32];
-                            tmem_ld32(o_cols + 32 * c, r);
-                            tmem_ld_wait();
-#pragma unroll
-                            for (int j = 0; j < 32; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) * corr);
-                            tmem_st32(o_cols + 32 * c, r);
-                        }
-                    }
-                }
+                const bool rise = mx > ref;
+                const bool any = __any_sync(0xffffffffu, rise);
+                const float corr = rise ? exp2_approx(ref - mx) : 1.f;
+                late = corr;
+                l *= corr;
+                ref = rise ? mx : ref;
                 const float sub = ref == -INFINITY ? 0.f : ref;             // no finite score yet: every factor is 0
                 float sum = 0.f;
 #pragma unroll
@@ -328,18 +311,35 @@ __global__ void __launch_bounds__(288, 1) attention_tc_kernel(const __grid_const
                     }
 #pragma unroll
                     for (int j = 0; j < 16; j++) {
-                        const float p0 = exp2_approx(fmaf(__uint_as_float(r[2 * j]), a.scale_log2, -sub)), p1 = exp2_approx(fmaf(__uint_as_float(r[2 * j + 1]), a.scale_log2, -sub));
+                        // not one multiply-add: the maximum itself must come out as exactly 1, so that a row of one key is that key's V
+                        const float p0 = exp2_approx(__fsub_rn(__fmul_rn(__uint_as_float(r[2 * j]), a.scale_log2), sub));
+                        const float p1 = exp2_approx(__fsub_rn(__fmul_rn(__uint_as_float(r[2 * j + 1]), a.scale_log2), sub));
                         const __half2 h = __floats2half2_rn(p0, p1);
-                        const float2 hf = __half22float2(h);
-                        sum += hf.x + hf.y;            // of the rounded values: a row that one key decides comes out as that key's V
+                        sum += p0 + p1;
                         p[j] = *reinterpret_cast<const uint32_t*>(&h);
                     }
                     tmem_st16(s_cols + 16 * c, p);     // behind what this thread has read: 16 columns for 32 keys
                 }
                 l += sum;
                 tmem_st_wait();
-                // every phase of o_full is waited for in turn (this one is long over), so that its parity says which
-                if (i > 0 && ok) ok = mbar_wait_timed(o_full, (i - 1) & 1, &abort_flag);
+                // every phase of o_full is waited for in turn, so that its parity says which
+                if (i > 0) {
+                    if (ok) ok = mbar_wait_timed(o_full, (i - 1) & 1, &abort_flag);
+                    __syncwarp();
+                    if (any) {
+                        tc_fence_after_sync();
+#pragma unroll
+                        for (int c = 0; c < HD / 64; c++) {
+                            uint32_t r[32];
+                            tmem_ld32(o_cols + 32 * c, r);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int j = 0; j < 32; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) * corr);
+                            tmem_st32(o_cols + 32 * c, r);
+                        }
+                        tmem_st_wait();
+                    }
+                }
                 tc_fence_before_sync();
                 mbar_arrive(p_full);
             }

@@ -42,8 +42,8 @@ def test_causal_attention_kernel(ctx, oracle, hd, T, start):
 @pytest.mark.parametrize("T,start,heads,kvh", [(65, 63, 2, 2), (127, 1, 4, 1), (128, 0, 2, 1), (129, 127, 2, 2), (257, 300, 6, 3)])
 def test_causal_attention_tensor_core_tiles(ctx, oracle, hd, T, start, heads, kvh):
     """Edges of the 128-query tiles and 128-key blocks; NaN in the cache behind the data must not show; a large score decides its
-    row.  Bound: q is rounded alike on both sides; P is rounded to f16 relative to another reference score than the restatement's
-    running maximum, so either side's weights are off by 2^-11, which is d = 2 * 2^-11 * (P . |V|) of an output (f32 sums are far
+    row.  Bound: q is rounded alike on both sides; P is rounded to f16 relative to the maximum over blocks of other lengths than the
+    restatement's, so either side's weights are off by 2^-11, which is d = 2 * 2^-11 * (P . |V|) of an output (f32 sums are far
     below), and the output's rounding to bf16 is half an ulp, 2^-8 of it."""
     import runit_mac_b200 as R
     from oracle import prefill as OP
@@ -65,6 +65,30 @@ def test_causal_attention_tensor_core_tiles(ctx, oracle, hd, T, start, heads, kv
     assert np.isfinite(got).all()
     worst = (np.abs(got - ref) / (d + 2.0 ** -8 * (np.abs(ref) + d))).max()
     assert worst <= 1.0, worst
+
+
+def test_causal_attention_weights_are_relative_to_the_maximum(ctx, oracle):
+    """Two keys of the second block decide the row, 5.3 bits above the first block's largest score, and their values cancel to a few
+    thousandths: what is left shows how their weights were rounded to f16.  Relative to the row maximum the largest is 1 and exact, as in the
+    restatement, and the outputs agree to the rounding to bf16; relative to another reference both weights are off by up to 2^-12, which
+    would be 2e-4 here."""
+    import runit_mac_b200 as R
+    from oracle import prefill as OP
+    hd, n = 64, 256
+    q = np.zeros((1, hd), np.float32)
+    q[0, 0] = 8.0                                   # score = the first element of the key
+    kc, vc = np.zeros((1, n, hd), np.float16), np.zeros((1, n, hd), np.float16)
+    kc[0, :, 0] = -14
+    kc[0, 5, 0], kc[0, 200, 0], kc[0, 201, 0] = 0, 3.7, 2.8
+    vc[0, 200] = 1
+    vc[0, 201] = -np.exp(0.9) * (1 + np.linspace(-0.004, 0.004, hd))
+    ob = ctx.new_buffer(hd * 2)
+    R.prefill_attention_f16kv(ctx, ctx.buffer_from(q), ctx.buffer_from(kc), ctx.buffer_from(vc), ob, 1, 1, 1, hd, n, n - 1)
+    ctx.flush()
+    got = bf16_bits_to_f32(ob.download(np.uint16, hd))
+    ref = OP.causal_attention_f16(q, kc, vc, 1, 1, hd, start_pos=n - 1).reshape(-1)
+    assert np.abs(ref).max() < 0.01
+    assert (np.abs(got - ref) <= 2.0 ** -8 * np.abs(ref) + 1e-6).all(), np.abs(got - ref).max()
 
 
 @pytest.mark.parametrize("bad", [np.inf, np.nan])
