@@ -11,9 +11,10 @@
 //     at most 2^-22 of the value or 2^-35 of the unit's largest (split_slots_kernel: the largest lies near the top of f16's range, because
 //     the halves of the high nibbles' activations, which are stored as x / 16, end at its smallest step).
 //   * sum_j m_j * (sum of x over block j) is one more MMA per unit with 32 * m as A and the split block sums / 32 as B.
-// Bound: at 2 slots per expert (16 tokens) the unpacking, 300 instructions per warp for 16 x 256 weights at 8 columns; at 32
+// An Inf or a NaN among a unit's activations makes its scale, and with it the token's products, NaN (as the launches per slot do).
+// Bound: at 2 slots per expert (16 tokens) the unpacking, about 470 instructions per warp for 16 x 256 weights at 8 columns; at 32
 // slots (256 tokens) the MMA pipe (65 % active).  Measured for the layer of width 2048, 64 experts of 1024, top 8: 16 tokens 117 ->
-// 95 us, 256 tokens 1586 -> 291 us, error against 64 bits 4.2e-6 -> 1.2e-7 of the output.  One m16 tile per warp: with two
+// 88 to 101 us (by the number of experts hit), 256 tokens 1590 -> 275 to 300 us, error against 64 bits 4.2e-6 -> 1.2e-7 of the output.  One m16 tile per warp: with two
 // (half the reads of the activations' fragments, half as many warps) 256 tokens took 302 us, and 16 tokens 107 us with 256 rows per CTA.
 #include <cuda_fp16.h>
 
@@ -375,7 +376,9 @@ static int32_t slots_run(runit_ctx* ctx, const void* gate, const void* up, const
 
 int32_t moe_slots_experts(runit_ctx* ctx, const void* gate, const void* up, const void* down, const float* x, const int32_t* idx, float* act,
                           float* y, void* staging, uint32_t T, uint32_t h, uint32_t ff, uint32_t E, uint32_t k) {
-    return T * k <= 8 * E ? slots_run<1>(ctx, gate, up, down, x, idx, act, y, staging, T * k, h, ff, E, k)
+    // one tile per group up to 12 slots per expert (us with one / with four: 64 experts of 2048 x 1024: 8 slots 146 / 182, 12 177 / 190, 16
+    // 209 / 201, 24 283 / 225; 128 of 2048 x 768: 8 194 / 260, 12 257 / 279, 16 323 / 300; 16 of 1024 x 512: 8 32 / 38, 24 40 / 45)
+    return T * k <= 12 * E ? slots_run<1>(ctx, gate, up, down, x, idx, act, y, staging, T * k, h, ff, E, k)
                           : slots_run<4>(ctx, gate, up, down, x, idx, act, y, staging, T * k, h, ff, E, k);
 }
 
