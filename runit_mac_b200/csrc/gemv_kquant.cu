@@ -163,8 +163,8 @@ __global__ void __launch_bounds__(kWarps * 32) gemv_kquant_kernel(const Args a) 
 //     (g, t) ends up with every limb's exact sums of blocks t and t + 4 of its rows g and g + 8.
 // 16 MMAs for 16 rows x 256 weights; integers, combination and error against 64 bits are those of dp4a on the same limbs.
 // Bound: instruction issue (unpacking, the activations' limbs where they are not prepared) at 11 warps per SM, which the stages'
-// shared memory allows.  Measured, lane = row with dp4a before: Q6_K 152064 x 3584 164 -> 127 us (3.5 TB/s), 3584 x 18944 25.6 ->
-// 22.4, 32000 x 2048 26.1 -> 23.5; Q5_K 152064 x 3584 106 -> 100, 3584 x 3584 8.4 -> 7.8.
+// shared memory allows.  Measured, lane = row with dp4a before: Q6_K 152064 x 3584 164 -> 133 us (125 in a stream over three matrices,
+// 3.6 TB/s), 3584 x 18944 25.6 -> 22.4, 32000 x 2048 26.1 -> 23.5; Q5_K 152064 x 3584 106 -> 100, 3584 x 3584 8.4 -> 7.8.
 namespace kt {
 
 template <int FMT> struct Tile {

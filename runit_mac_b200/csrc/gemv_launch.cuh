@@ -40,8 +40,11 @@ static inline int32_t launch_staged(runit_ctx* ctx, const GemvArgs& a, const Gem
     cudaLaunchAttribute attr[2];
     int na = 0;
     // Dependent launch pays except for grids of about one CTA per SM, which were measured 15-25% slower with it
-    // (the early CTAs of the next grid double up on busy SMs instead of spreading out).  The cp.async kernels (Q8_0), whose copies
-    // take a CTA longer to issue, gain at every size: decoding step of a 0.5B model 467 us with that exception, 451 without.
+    // (the early CTAs of the next grid double up on busy SMs instead of spreading out).  The cp.async kernels, whose copies take a CTA
+    // longer to issue, gain at every size: decoding step of a 0.5B model in Q8_0 467 us with that exception, 451 without.  With the weights
+    // requested before the wait (both, before -> now): Q8_0 steps of width 896 / 2048 / 3584 at batch 1 510 -> 431, 257 -> 224, 332 -> 310 us,
+    // at batch 2 868 -> 737, 435 -> 390, 578 -> 541, at batch 8 1974 -> 1793, 1181 -> 1129, 1706 -> 1668; f16 input 896 x 896 3.2 -> 2.4 us a
+    // launch, 4864 x 4864 14.5 -> 12.7; Q4_K without bulk loads 1024 x 1024 2.8 -> 2.2, 3584 x 3584 6.6 -> 4.8.
     const uint32_t sms = (uint32_t)ctx->sm_count;
     const bool wait_first = LD == 0 && ctx->foreign_kernels;
     if (wait_first && !a.grp_expert) args.grp_early = 2;
