@@ -106,6 +106,24 @@ def test_outlier_without_weight(ctx, oracle):
     assert_close(O, ref, got, rel_tol=2e-5, what="outlier without weight")
 
 
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("T", [8, 40])
+def test_activation_that_is_not_finite_stays_with_its_token(ctx, oracle, T, bad):
+    """One and several tiles per expert: the other columns of the token's tiles keep their bits, the token's output is not finite."""
+    import runit_mac_b200 as R
+    O = oracle
+    h, ff, E, k = 512, 256, 2, 2                    # k = E: every expert has every token, whatever the router makes of the bad one
+    rng = np.random.default_rng(T)
+    weights = [ctx.buffer_from(a) for a in [rng.normal(0, 0.05, (E, h)).astype(np.float32)] + [O.rand_q4k(rng, E * r, c) for r, c in ((ff, h), (ff, h), (h, ff))]]
+    x, res = rng.normal(0, 1, (T, h)).astype(np.float32), rng.normal(0, 1, (T, h)).astype(np.float32)
+    clean, _ = run(ctx, R, weights, x, res, h, ff, E, k)
+    x[3, 300] = bad
+    got, _ = run(ctx, R, weights, x, res, h, ff, E, k)
+    others = np.arange(T) != 3
+    assert np.array_equal(got[others], clean[others]) and np.isfinite(clean).all()
+    assert not np.isfinite(got[3]).any()
+
+
 def test_built_in_scratch_gives_the_same_bits(ctx, oracle):
     """A size at which the slots are sorted and the intermediates fill a good part of the built-in region."""
     import runit_mac_b200 as R
