@@ -67,6 +67,13 @@ def test_causal_attention_tensor_core_tiles(ctx, oracle, hd, T, start, heads, kv
     assert worst <= 1.0, worst
 
 
+@pytest.mark.parametrize("hd", [128, 64])
+@pytest.mark.parametrize("T,start", [(1, 127), (1, 128), (2, 254), (129, 128), (3, 509), (256, 129), (1, 640)])
+def test_causal_attention_chains_of_even_and_odd_blocks(ctx, oracle, hd, T, start):
+    """One to six blocks of keys: a chain without a block, chains of one and of several, a last block with a single visible key.  Same bound."""
+    test_causal_attention_tensor_core_tiles(ctx, oracle, hd, T, start, 2, 1)
+
+
 def test_causal_attention_weights_are_relative_to_the_maximum(ctx, oracle):
     """Two keys of the second block decide the row, 5.3 bits above the first block's largest score, and their values cancel to a few
     thousandths: what is left shows how their weights were rounded to f16.  Relative to the row maximum the largest is 1 and exact, as in the
