@@ -107,9 +107,9 @@ __device__ __forceinline__ void dequant_half(const uint32_t* q, float sc, float 
 // Two CTAs of one cluster share a work item of 256 weight rows x up to 256 token slots.  Each CTA dequantises 128
 // of the rows and loads half of the token tile; the leader CTA issues M = 256 MMAs that write 128 accumulator rows
 // into each CTA's tensor memory.  What shaped it (all measured on B200):
-//   * one thread can issue a tcgen05.mma about every 110-130 cycles, whatever its size: only M = 256, N = 256 MMAs
-//     (128 cycles of tensor work) keep the pipe busy, and barrier waits, the fence and the commits are all paid by
-//     that same thread, so a pipeline step covers 128 K (8 MMAs) rather than 64;
+//   * the issuing warp walks its loop as a whole and one lane issues (elect_one: a loop that only lane 0 entered took 110-130 cycles
+//     per MMA whatever its size, so that tiles of a few slots cost as much as full ones; 4096 tokens x 8 of 128 experts 638 -> 609 us, 300 tokens
+//     275 -> 227); barrier waits, the fence and the commits are all paid by that same warp, so a pipeline step covers 128 K (8 MMAs) rather than 64;
 //   * with the weight operand in shared memory the dequantisers' stores, the TMA writes and the MMAs' operand reads
 //     need more than the 128 B/clk an SM's shared memory delivers: the dequantiser warps write their bf16 rows
 //     straight into tensor memory (tcgen05.st) and the MMA takes A from there; shared memory carries the token
@@ -160,7 +160,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_b, const __grid
     volatile int* abort_flag = reinterpret_cast<volatile int*>(base_p + kOffCtrl + (holder - ctrl) + 4);
     float* xchg = reinterpret_cast<float*>(base_p + kOffXchg);
 
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const uint32_t rank = cluster_ctarank();
     const uint32_t pair_id = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     if (tid == 0) {
@@ -237,28 +237,32 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_b, const __grid
             }
         }
     } else if (warp == 1) {
-        // ───────── MMA issuer (leader CTA only) ─────────
-        if (lane == 0 && rank == 0) {
+        // ───────── MMA issuer (leader CTA only): the whole warp walks the loop, one lane issues ─────────
+        if (rank == 0) {
             uint32_t it = 0, n = 0;
             bool ok = true;
-            for (uint32_t item = pair_id; item < n_items && ok && !*abort_flag; item += n_pairs, n++) {
+            for (uint32_t item = pair_id; item < n_items && ok && !__any_sync(0xffffffffu, *abort_flag); item += n_pairs, n++) {
                 const uint32_t idesc = umma_idesc_bf16(256, tile_cols(a.tile_nvalid[item / nb]));
-                if (!mbar_wait_timed_cluster(bar_acce, (n & 1) ^ 1, abort_flag)) break;   // the epilogue has drained the accumulator
+                // the epilogue has drained the accumulator
+                if (!__all_sync(0xffffffffu, mbar_wait_timed_cluster(bar_acce, (n & 1) ^ 1, abort_flag))) break;
                 for (uint32_t st = 0; st < units * 2; st++, it++) {
                     const uint32_t sa = it % kNS, sb = sa, pa = (it / kNS) & 1;
-                    if (!mbar_wait_timed_cluster(bar_full + 8 * sa, pa, abort_flag)) { ok = false; break; }
+                    if (!(ok = __all_sync(0xffffffffu, mbar_wait_timed_cluster(bar_full + 8 * sa, pa, abort_flag)))) break;
                     tc_fence_after_sync();
-                    const uint32_t at = tmem_base + kACol0 + 64 * sa;
+                    if (elect_one()) {
+                        const uint32_t at = tmem_base + kACol0 + 64 * sa;
 #pragma unroll
-                    for (uint32_t c = 0; c < 2; c++) {
-                        const uint64_t db = umma_desc_sw128(base + sb * kStageB + c * kTileBytes);
+                        for (uint32_t c = 0; c < 2; c++) {
+                            const uint64_t db = umma_desc_sw128(base + sb * kStageB + c * kTileBytes);
 #pragma unroll
-                        for (uint32_t k4 = 0; k4 < 4; k4++)
-                            umma_bf16_pair_ts(tmem_base, at + 32 * c + 8 * k4, db + 2 * k4, idesc, (st | c | k4) != 0);
+                            for (uint32_t k4 = 0; k4 < 4; k4++)
+                                umma_bf16_pair_ts(tmem_base, at + 32 * c + 8 * k4, db + 2 * k4, idesc, (st | c | k4) != 0);
+                        }
+                        umma_commit_pair(bar_empty + 8 * sa, 3);
+                        if (st + 1 == units * 2) umma_commit_pair(bar_accf, 3);
                     }
-                    umma_commit_pair(bar_empty + 8 * sa, 3);
+                    __syncwarp();
                 }
-                if (ok) umma_commit_pair(bar_accf, 3);
             }
         }
     } else if (warp < kDeqWarp0) {
