@@ -39,17 +39,17 @@ struct MoeScratch {
 // Tokens that share a pass over the experts with their slots sorted by expert (moe_slots.cu), 0: launches per slot.  The sorted activations
 // lie in the context's staging area, so that neither the caller's scratch nor its size has a say; a call with more tokens than it holds is cut
 // into equal pieces.
-// Sorting by expert pays from 1.5 slots per expert on, where experts begin to be read for several slots at once (us with /
-// without, 64 experts of 2048 x 1024, top 8: 8 tokens 85 / 68, 12: 88 / 93, 24: 112 / 167; 128 experts of 2048 x 768, top 8: 12 tokens
-// 96 / 69, 24: 119 / 119; 60 of 2048 x 1024, top 4: 12 tokens 77 / 55, 24: 88 / 92), and where the products outweigh its four
-// more launches (8 experts of 1024 x 512, top 2: 48 tokens 38 / 34, 64: 39 / 41).
+// Sorting by expert pays from 1.25 slots per expert on, where experts begin to be read for several slots at once (us with /
+// without, 64 experts of 2048 x 1024, top 8: 6 tokens 56 / 55, 8: 66 / 68, 12: 68 / 93, 24: 80 / 167; 60 of 2048 x 768, top 4: 16 tokens 54 / 51,
+// 24: 59 / 67), and where the products outweigh its four more launches (16 experts of 1024 x 512, top 4: 16 tokens 28 / 26, 24: 29 / 34; 8 of
+// 2048 x 512, top 2: 24 tokens 32 / 31).
 static uint32_t moe_piece(const runit_ctx* ctx, uint32_t T, uint32_t h, uint32_t ff, uint32_t E, uint32_t k) {
     if (T < 4 || !ctx->d_slots || ctx->tune.moe_slots == 2) return 0;
     uint32_t most = moe_slots_tokens(ctx->slots_bytes, h, ff, E, k);
     if (ctx->tune.moe_piece > 0 && (uint32_t)ctx->tune.moe_piece < most) most = (uint32_t)ctx->tune.moe_piece;
     if (most == 0) return 0;
     const uint32_t n = (T + most - 1) / most, piece = (T + n - 1) / n;
-    const bool pays = 2ull * piece * k >= 3ull * E && (uint64_t)piece * k * h * ff >= (1ull << 26);
+    const bool pays = 4ull * piece * k >= 5ull * E && (uint64_t)piece * k * h * ff >= (1ull << 26);
     return pays || ctx->tune.moe_slots == 1 ? piece : 0;
 }
 

@@ -18,7 +18,7 @@ int32_t moe_route_gated(runit_ctx* ctx, const float* w, const float* x, float* l
                         int32_t score, int32_t renorm, int32_t* idx, float* wts, float* gates, uint32_t* counter, const float* gain,
                         float eps, float* xn_out);
 
-// moe_slots.cu: the expert products of T tokens with every expert read once for up to 32 slots; y[slot] f32 [T * k][h].
+// moe_slots.cu: the expert products of T tokens with every expert read once for up to 48 slots; y[slot] f32 [T * k][h].
 // T at most moe_slots_tokens(staging_bytes, ...); staging 256-byte aligned, matrices 16-byte aligned.
 uint32_t moe_slots_tokens(size_t staging_bytes, uint32_t h, uint32_t ff, uint32_t E, uint32_t k);
 int32_t moe_slots_experts(runit_ctx* ctx, const void* gate, const void* up, const void* down, const float* x, const int32_t* idx, float* act,
