@@ -109,6 +109,8 @@ static int32_t ctx_init(int32_t device, cudaStream_t adopt, bool adopt_stream, r
     else { c->d_kq = nullptr; cudaGetLastError(); }
     if (cudaMalloc(&c->d_xq, 4u << 20) == cudaSuccess) c->xq_bytes = 4u << 20;
     else { c->d_xq = nullptr; cudaGetLastError(); }
+    if (cudaMalloc(&c->d_tc, runit::gemv_tc_bytes()) == cudaSuccess) cudaMemset(c->d_tc, 0, runit::gemv_tc_bytes());
+    else { c->d_tc = nullptr; cudaGetLastError(); }
     // MoE layer with its slots sorted by expert: 1400 tokens of 8 of 64 experts at width 2048, 160 of 8 of 256 at width 7168
     if (cudaMalloc(&c->d_slots, 96u << 20) == cudaSuccess) c->slots_bytes = 96u << 20;
     else { c->d_slots = nullptr; cudaGetLastError(); }
@@ -142,12 +144,14 @@ int32_t runit_get_tmap(runit_ctx* ctx, const void* ptr, uint64_t rows, uint64_t 
                                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill)>(
         ctx->encode_tiled);
-    const cuuint64_t gdim[2] = {row_bytes, rows};
+    // a box has at most 256 elements a side: wider ones count in elements of two bytes
+    const uint32_t elem = box_bytes > 256 ? 2 : 1;
+    const cuuint64_t gdim[2] = {row_bytes / elem, rows};
     const cuuint64_t gstride[1] = {row_bytes};
-    const cuuint32_t box[2] = {box_bytes, box_rows};
+    const cuuint32_t box[2] = {box_bytes / elem, box_rows};
     const cuuint32_t estr[2] = {1, 1};
     CUtensorMap m;
-    CUresult r = encode(&m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), gdim, gstride, box, estr,
+    CUresult r = encode(&m, elem == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), gdim, gstride, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -171,6 +175,7 @@ int32_t runit_ctx_destroy(runit_ctx_t* ctx) {
     cudaStreamSynchronize(ctx->stream);   // Drop flushes, context.rs:299-304
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
     if (ctx->d_xq) cudaFree(ctx->d_xq);
+    if (ctx->d_tc) cudaFree(ctx->d_tc);
     if (ctx->d_slots) cudaFree(ctx->d_slots);
     if (ctx->d_am) cudaFree(ctx->d_am);
     if (ctx->d_xq_ctl) cudaFree(ctx->d_xq_ctl);
@@ -196,6 +201,7 @@ int32_t runit_flush(runit_ctx_t* ctx) {
         const int32_t why = ctx->h_status[0];
         ctx->h_status[0] = 0;
         if (ctx->d_abort) cudaMemset(ctx->d_abort, 0, 4);   // the stream is idle: barriers wait again after this report
+        if (ctx->d_tc) cudaMemset(ctx->d_tc, 0, runit::gemv_tc_bytes());      // tickets of a launch that gave up
         if (why == 4) {
             runit_fail(ctx, RUNIT_ERR_UNSUPPORTED, "sampler: top-k is off and the nucleus is wider than the 1024 most probable tokens (code %d)", why);
             if (ctx->sticky_status == RUNIT_OK) ctx->sticky_status = RUNIT_ERR_UNSUPPORTED;   // reported by this flush

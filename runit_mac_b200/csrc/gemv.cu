@@ -497,12 +497,15 @@ int32_t runit_gemv_batched_multi_f32(runit_ctx_t* ctx, int32_t fmt, uint32_t n_m
     if (!ctx) return RUNIT_ERR_BAD_ARG;
     RUNIT_REQUIRE(ctx, n_mats >= 1 && n_mats <= 3 && weights && outputs && rows && input, "gemv_batched_multi_f32: 1..3 matrices, no null table");
     RUNIT_REQUIRE(ctx, batch >= 1 && batch <= 8, "gemv_batched_multi_f32: batch=%u not in 1..8", batch);
-    bool ok = gemv_imma_applies(ctx, fmt, k, batch) && runit_aligned(input, 16) && (k / 256 * 144) % 16 == 0 && ctx->tune.gemv_variant != 1;
+    bool ok = runit_aligned(input, 16) && ctx->tune.gemv_variant != 1;
     for (uint32_t i = 0; i < n_mats; i++) {
         RUNIT_REQUIRE(ctx, weights[i] && outputs[i] && rows[i] > 0, "gemv_batched_multi_f32: null matrix or output %u", i);
         ok = ok && runit_aligned(weights[i], 16) && runit_aligned(outputs[i], 4);
     }
-    if (ok) return gemv_imma_multi(ctx, fmt, n_mats, weights, (const float*)input, (float* const*)outputs, nullptr, rows, k, batch);
+    if (ok && gemv_tc_applies(ctx, fmt, k, batch))
+        return gemv_tc_multi(ctx, n_mats, weights, (const float*)input, (float* const*)outputs, nullptr, rows, k, batch);
+    if (ok && gemv_imma_applies(ctx, fmt, k, batch) && (k / 256 * 144) % 16 == 0)
+        return gemv_imma_multi(ctx, fmt, n_mats, weights, (const float*)input, (float* const*)outputs, nullptr, rows, k, batch);
     for (uint32_t i = 0; i < n_mats; i++) {      // other formats and batch 1: one launch per matrix
         const int32_t st = runit_gemv_batched_f32(ctx, fmt, weights[i], input, outputs[i], nullptr, rows[i], k, batch);
         if (st != RUNIT_OK) return st;
@@ -515,9 +518,15 @@ int32_t runit_gemv_batched_f32(runit_ctx_t* ctx, int32_t fmt, const void* weight
     if (!ctx) return RUNIT_ERR_BAD_ARG;
     RUNIT_REQUIRE(ctx, batch >= 1 && batch <= 8, "gemv_batched_f32: batch=%u not in 1..8", batch);
     RUNIT_REQUIRE(ctx, m > 0, "gemv_batched_f32: m == 0");
-    // 4-bit formats, batch 2..8: integer tensor-core path (activations quantised once, weights streamed once).
-    if (gemv_imma_applies(ctx, fmt, k, batch) && weight && input && output && runit_aligned(weight, 16) && runit_aligned(input, 16) &&
-        runit_aligned(output, 4) && (k / 256 * 144) % 16 == 0 && ctx->tune.gemv_variant != 1)
+    // batch 2..8: Q8_0 on tcgen05, the 4-bit formats on the integer tensor-core path (activations prepared once, weights streamed once)
+    const bool aligned = weight && input && output && runit_aligned(weight, 16) && runit_aligned(input, 16) && runit_aligned(output, 4) &&
+                         runit_aligned(residual, 4) && ctx->tune.gemv_variant != 1;
+    if (aligned && gemv_tc_applies(ctx, fmt, k, batch)) {
+        const float* res = (const float*)residual;
+        float* y = (float*)output;
+        return gemv_tc_multi(ctx, 1, &weight, (const float*)input, &y, &res, &m, k, batch);
+    }
+    if (aligned && gemv_imma_applies(ctx, fmt, k, batch) && (k / 256 * 144) % 16 == 0)
         return gemv_imma(ctx, fmt, weight, (const float*)input, (float*)output, (const float*)residual, m, k, batch);
     // Kernels exist for batch 1, 2, 4, 8; other sizes run as a sum of those.
     uint32_t done = 0;

@@ -1,0 +1,282 @@
+// Batched (2..8 activation rows) Q8_0 GEMV on tcgen05 (tc_rows.cuh): the weights stream once and are unpacked into tensor memory, the two halves
+// of the activations are the 16 columns of one product.
+//
+// A pre-pass splits the activations once per call.  Work is cut into items of (128 rows, share of K); the shares of a row depend on K alone
+// and are added in order, so an output's bits depend neither on the other matrices of a launch nor on how the items fall on the CTAs.  Each
+// CTA takes a stretch of consecutive items: the tiles that it has whole it stores itself, those that it shares with its neighbours are filed share by share and
+// added by the warp that files last.
+//
+// Bound: the unpacking warps, about 1000 clocks per 128 x 256 weights and SM (2.1 TB/s), and some 4 us between dependent calls (the pre-pass and
+// its hand-over).  The packed f32 kernel that it replaces multiplies every weight 8 times on the CUDA cores.  Decoding steps, us, f32 -> now: width 3584, two layers
+// and a head of 30000 rows, 2 / 4 / 8 sequences 294 / 421 / 915 -> 173 / 175 / 183; width 2048, four layers, 274 / 365 / 693 -> 208 / 209 / 221.
+// Error against 64 bits 2.0e-7 (f32 sums: 2.0e-7).  The 4-bit formats stay with gemv_imma.cu: the same kernel for them took 362 us where that one
+// takes 350 (Q4_K, 7B, four layers and head, 8 sequences), 332 against 353 (Q4_0, 4 sequences) and 198 against 187 (width 2048).
+#include <cuda_fp16.h>
+
+#include "runit_internal.h"
+#include "tc_rows.cuh"
+
+namespace runit {
+namespace tcg {
+
+constexpr tcr::Kind kKind = tcr::Q8_0_8;
+using C = tcr::Cfg<kKind>;
+constexpr uint32_t kMaxShares = 10, kMaxCtas = 160, kTickets = kMaxCtas * 8, kPartBytes = 4096;      // a share's sums of a tile
+
+// One CTA per 256 activations, one warp per activation row (rows behind the batch are zeros).
+__global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x, uint8_t* __restrict__ images, float* __restrict__ scales, uint32_t k, uint32_t batch) {
+    __shared__ __align__(16) uint8_t out[C::kBStage];
+    const uint32_t u = blockIdx.x, n = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    grid_launch_dependents();      // the product may start requesting its weights; it waits for this grid before it reads anything else
+    grid_dependency_wait();
+    float v[8];
+#pragma unroll
+    for (int b = 0; b < 8; b++) v[b] = n < batch ? x[(size_t)n * k + (size_t)u * 256 + b * 32 + lane] : 0.f;
+    const float scale = tcr::split_column<kKind>(
+        v, 2 * n, 2 * n + 1, 0, lane,
+        [&](uint32_t panel, uint32_t hi_off, __half hi, uint32_t lo_off, __half lo) {
+            *reinterpret_cast<__half*>(out + panel * 2048 + hi_off) = hi;
+            *reinterpret_cast<__half*>(out + panel * 2048 + lo_off) = lo;
+        },
+        [](uint32_t, __half) {});
+    if (lane == 0) scales[u * 8 + n] = scale;
+    __syncthreads();
+    uint4* dst = reinterpret_cast<uint4*>(images + (size_t)u * C::kBStage);
+    for (uint32_t i = threadIdx.x; i < C::kBStage / 16; i += 256) dst[i] = reinterpret_cast<const uint4*>(out)[i];
+}
+
+// Up to three matrices that share the activations (q | k | v, gate | up) ride one launch: segment i owns the row tiles from tile0[i] on.
+struct Args {
+    const uint8_t* images;
+    const float* scales;
+    float* y[3];
+    const float* res[3];
+    uint32_t m[3], tile0[3];
+    uint32_t nseg, units, shares, items, batch;
+    uint32_t inverse;            // 2^32 / shares, rounded up (0: one share): the quotient's high word, exact below 2^32 / shares
+    float* part;                 // [tile's place][share][sum of a thread][thread]
+    uint32_t* tickets;           // [tile's place][warp], zero at rest
+    int32_t* status;
+};
+struct Maps {
+    CUtensorMap m[3];
+};
+
+struct Policy {
+    static constexpr int kAcc = C::kAcc;
+    const Args& a;
+    const Maps& maps;
+    const uint32_t i0, i1;       // items of this CTA
+    float total[kAcc];
+
+    __device__ __forceinline__ Policy(const Args& args, const Maps& m)
+        : a(args), maps(m), i0((uint32_t)((uint64_t)blockIdx.x * args.items / gridDim.x)), i1((uint32_t)((uint64_t)(blockIdx.x + 1) * args.items / gridDim.x)) {}
+
+    __device__ __forceinline__ bool few() const { return a.batch <= 4; }
+
+    __device__ __forceinline__ uint32_t begin() const { return i0; }
+    __device__ __forceinline__ uint32_t end() const { return i1; }
+    // 32-bit divisions cost the sums' warps more than a step's sums
+    __device__ __forceinline__ uint32_t by_shares(uint32_t v) const { return a.inverse ? __umulhi(v, a.inverse) : v; }
+    __device__ __forceinline__ uint32_t unit(uint32_t i) const {
+        const uint32_t tile = by_shares(i);
+        return tile * a.units + by_shares((i - tile * a.shares) * a.units);
+    }
+    __device__ __forceinline__ uint32_t steps() const { return unit(i1) - unit(i0); }
+    __device__ __forceinline__ int segment(uint32_t tile) const { return a.nseg > 2 && tile >= a.tile0[2] ? 2 : a.nseg > 1 && tile >= a.tile0[1] ? 1 : 0; }
+    __device__ __forceinline__ tcr::Run run(uint32_t i) const {
+        const uint32_t tile = by_shares(i), share = i - tile * a.shares;
+        const int s = segment(tile);
+        tcr::Run r;
+        r.map[0] = &maps.m[s];
+        r.row[0] = (int32_t)((tile - a.tile0[s]) * 128);
+        r.u0 = by_shares(share * a.units);
+        r.u1 = by_shares((share + 1) * a.units);
+        r.b = a.images + (size_t)r.u0 * C::kBStage;
+        r.xs = a.scales + r.u0 * 8;
+        r.n = 8;
+        return r;
+    }
+    __device__ __forceinline__ void store(uint32_t tile, uint32_t warp, uint32_t lane) const {
+        const int s = segment(tile);
+        const uint32_t row = (tile - a.tile0[s]) * 128 + (warp & 3) * 32 + lane, m = a.m[s];
+        if (row >= m) return;
+#pragma unroll
+        for (uint32_t j = 0; j < kAcc; j++) {
+            const uint32_t users = few() ? 2 : 4, c = users * (warp >> 2) + j;
+            if (j >= users) break;
+            if (c < a.batch) {
+                const size_t o = (size_t)c * m + row;
+                a.y[s][o] = a.res[s] ? total[j] + a.res[s][o] : total[j];
+            }
+        }
+    }
+    __device__ __forceinline__ void finish(uint32_t i, float (&acc)[1][kAcc], uint32_t warp, uint32_t lane) {
+        const uint32_t tile = by_shares(i), share = i - tile * a.shares, t0 = tile * a.shares;
+        if (t0 >= i0 && t0 + a.shares <= i1) {
+#pragma unroll
+            for (int j = 0; j < kAcc; j++) total[j] = share ? total[j] + acc[0][j] : acc[0][j];
+            if (share + 1 == a.shares) store(tile, warp, lane);
+        } else {
+            // the place of a tile that several CTAs share: the first CTA that starts inside it
+            const uint32_t place = (uint32_t)(((uint64_t)(t0 + 1) * gridDim.x + a.items - 1) / a.items);
+            constexpr uint32_t kT = 32 * C::kSumWarps;
+            static_assert(kAcc * kT * 4 <= kPartBytes, "a share's place");
+            float* p = a.part + (size_t)place * kMaxShares * (kPartBytes / 4) + warp * 32 + lane;
+#pragma unroll
+            for (int j = 0; j < kAcc; j++) __stcg(p + (share * kAcc + j) * kT, acc[0][j]);
+            if (share + 1 == a.shares || i + 1 == i1) {
+                const uint32_t mine = i - (t0 > i0 ? t0 : i0) + 1;
+                uint32_t before = 0;
+                __threadfence();
+                __syncwarp();
+                if (lane == 0) before = atomicAdd(&a.tickets[place * 8 + warp], mine);
+                before = __shfl_sync(0xffffffffu, before, 0);
+                if (before + mine == a.shares) {
+                    __threadfence();
+#pragma unroll
+                    for (int j = 0; j < kAcc; j++) total[j] = __ldcg(p + j * kT);
+                    for (uint32_t q = 1; q < a.shares; q++)
+#pragma unroll
+                        for (int j = 0; j < kAcc; j++) total[j] += __ldcg(p + (q * kAcc + j) * kT);
+                    store(tile, warp, lane);
+                    if (lane == 0) a.tickets[place * 8 + warp] = 0;
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kAcc; j++) acc[0][j] = 0.f;
+    }
+};
+
+__global__ void __launch_bounds__(C::kThreads, 1) gemv_tc_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Args a) {
+    extern __shared__ uint8_t smem_raw[];
+    tcr::Block<kKind, 1> blk(smem_raw);
+    Policy p(a, maps);
+    if (blk.warp == C::kCopyW) {
+        // raw blocks: the first steps' ahead of the dependency wait; the columns' scales behind it
+        uint32_t s = 0, early = 0;
+        auto load = [&](const tcr::Run& r, uint32_t u, uint32_t step) {
+            if (elect_one()) {
+                mbar_expect_tx(blk.raw_bar(step), C::kWBytes + r.n * 4);
+                tma_load_2d(blk.raw(step), r.map[0], (int32_t)(u * 136), r.row[0], blk.raw_bar(step));       // elements of two bytes
+            }
+            __syncwarp();
+        };
+        for (uint32_t i = p.begin(); i < p.end() && early < C::kW; i++) {
+            const tcr::Run r = p.run(i);
+            for (uint32_t u = r.u0; u < r.u1 && early < C::kW; u++) load(r, u, early++);
+        }
+        grid_dependency_wait();
+        for (uint32_t i = p.begin(); i < p.end() && blk.ok; i++) {
+            const tcr::Run r = p.run(i);
+            for (uint32_t u = r.u0; u < r.u1; u++, s++) {
+                if (s >= early) {
+                    if (!blk.raw_free(s)) break;
+                    load(r, u, s);
+                }
+                if (elect_one()) bulk_load_1d(blk.scales(s), r.xs + (size_t)(u - r.u0) * r.n, r.n * 4, blk.raw_bar(s));
+                __syncwarp();
+            }
+        }
+        // whatever was requested arrives before the CTA leaves (weights whose step's scales were never requested can only be waited for until
+        // the limit)
+        if (blk.given_up()) mbar_drain(blk.w_full, C::kW, s > early ? s : early);
+    } else if (blk.warp == C::kCopyB) {
+        uint32_t c = 0;
+        grid_dependency_wait();
+        for (uint32_t i = p.begin(); i < p.end() && blk.ok; i++) {
+            const tcr::Run r = p.run(i);
+            for (uint32_t u = r.u0; u < r.u1; u++, c++) {
+                if (!blk.image_free(c)) break;
+                if (elect_one()) {
+                    mbar_expect_tx(blk.image_bar(c), C::kBStage);
+                    bulk_load_1d(blk.image(c), r.b + (size_t)(u - r.u0) * C::kBStage, C::kBStage, blk.image_bar(c));
+                }
+                __syncwarp();
+            }
+        }
+        if (blk.given_up()) mbar_drain(blk.b_full, C::kB, c);
+    } else {
+        blk.work(p);
+    }
+    blk.leave(a.status);
+}
+
+}  // namespace tcg
+
+// Bytes that the context keeps for this path: tickets, then partial sums.
+size_t gemv_tc_bytes() { return tcg::kTickets * 4 + (size_t)tcg::kMaxCtas * tcg::kMaxShares * tcg::kPartBytes; }
+
+bool gemv_tc_applies(const runit_ctx* ctx, int fmt, uint32_t k, uint32_t batch) {
+    if (fmt != RUNIT_FMT_Q8_0 || batch < 2 || batch > 8 || k % 256 != 0 || ctx->tune.gemv_math == 1 || !ctx->encode_tiled || !ctx->d_xq || !ctx->d_tc) return false;
+    return (size_t)(k / 256) * (tcg::C::kBStage + 32) <= ctx->xq_bytes;
+}
+
+// n_mats (1..3) matrices over the same activations in one launch.
+int32_t gemv_tc_multi(runit_ctx* ctx, uint32_t n_mats, const void* const* w, const float* x, float* const* y, const float* const* res, const uint32_t* m,
+                      uint32_t k, uint32_t batch) {
+    using namespace tcg;
+    Args a{};
+    Maps maps{};
+    a.units = k / 256;
+    a.batch = batch;
+    a.nseg = n_mats;
+    uint64_t tiles = 0;
+    for (uint32_t i = 0; i < 3; i++) {
+        const uint32_t s = i < n_mats ? i : 0;      // unused entries repeat segment 0 (never selected)
+        a.y[i] = y[s];
+        a.res[i] = res ? res[s] : nullptr;
+        a.m[i] = m[s];
+        a.tile0[i] = i < n_mats ? (uint32_t)tiles : 0xFFFFFFFFu;
+        if (i < n_mats) {
+            const int32_t st = runit_get_tmap(ctx, w[i], m[i], (uint64_t)a.units * 272, 128, 272, &maps.m[i]);
+            if (st != RUNIT_OK) return st;
+            tiles += ((uint64_t)m[i] + 127) / 128;
+        } else {
+            maps.m[i] = maps.m[0];
+        }
+    }
+    // two units per share, ten shares at most: enough items for every SM at the sizes where a tile per CTA would leave most of them idle
+    a.shares = (a.units + 1) / 2 < kMaxShares ? (a.units + 1) / 2 : kMaxShares;
+    a.items = (uint32_t)(tiles * a.shares);         // at most 3 * 2^25 tiles
+    a.inverse = a.shares > 1 ? (uint32_t)((0x100000000ull + a.shares - 1) / a.shares) : 0;
+    uint32_t grid = (uint32_t)ctx->sm_count;
+    grid = grid < kMaxCtas ? grid : kMaxCtas;
+    grid = grid < a.items ? grid : a.items;
+    a.images = (const uint8_t*)ctx->d_xq;
+    a.scales = (const float*)(a.images + (size_t)a.units * C::kBStage);
+    a.tickets = (uint32_t*)ctx->d_tc;
+    a.part = (float*)((uint8_t*)ctx->d_tc + kTickets * 4);
+    a.status = ctx->d_status;
+    static bool configured[64] = {false};
+    if (ctx->device >= 64 || !configured[ctx->device]) {
+        RUNIT_CUDA_TRY(ctx, cudaFuncSetAttribute(gemv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem));
+        if (ctx->device < 64) configured[ctx->device] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.stream = ctx->stream;
+    cfg.attrs = attr;
+    // The product requests weights as soon as the pre-pass lets it start.  Where a kernel before the pre-pass may have written them, the
+    // pre-pass is an ordinary launch, which starts when all of it can be seen.
+    cfg.numAttrs = !ctx->foreign_kernels && !ctx->weights_written && ctx->tune.pdl != 0 ? 1 : 0;
+    ctx->weights_written = false;
+    cfg.gridDim = dim3(a.units);
+    cfg.blockDim = dim3(256);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, split_kernel, x, (uint8_t*)ctx->d_xq, (float*)a.scales, k, batch);
+    if (e != cudaSuccess) return runit_fail(ctx, RUNIT_ERR_LAUNCH, "launch of gemv_batched (split of the activations) failed: %s", cudaGetErrorString(e));
+    const int32_t st = runit_after_launch(ctx, "gemv_batched_split_x");
+    if (st != RUNIT_OK) return st;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(C::kThreads);
+    cfg.dynamicSmemBytes = C::kSmem;
+    e = cudaLaunchKernelEx(&cfg, gemv_tc_kernel, maps, a);
+    if (e != cudaSuccess) return runit_fail(ctx, RUNIT_ERR_LAUNCH, "launch of gemv_batched (tcgen05) failed: %s", cudaGetErrorString(e));
+    return runit_after_launch(ctx, "gemv_batched_tc");
+}
+
+}  // namespace runit

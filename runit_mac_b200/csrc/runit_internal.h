@@ -69,6 +69,7 @@ struct runit_ctx {
     void* d_kq = nullptr;               // Q6_K GEMV with K split over CTAs: 2048 tile tickets (zero at rest), then 1 MiB of partial sums
     void* d_xq = nullptr;               // staging area of the batched GEMV's quantised activations
     size_t xq_bytes = 0;
+    void* d_tc = nullptr;               // batched Q8_0 GEMV: tickets (zero at rest) and partial sums of row tiles that CTAs share
     void* d_slots = nullptr;            // staging area of the MoE layer's slots sorted by expert
     size_t slots_bytes = 0;
     void* encode_tiled = nullptr;       // cuTensorMapEncodeTiled, resolved at context creation
@@ -184,6 +185,11 @@ int32_t gemv_imma(runit_ctx* ctx, int fmt, const void* w, const float* x, float*
                   uint32_t batch);
 int32_t gemv_imma_multi(runit_ctx* ctx, int fmt, uint32_t n_mats, const void* const* w, const float* x, float* const* y,
                         const float* const* res, const uint32_t* m, uint32_t k, uint32_t batch);
+// gemv_tc.cu: batched Q8_0 GEMV on the tcgen05 tensor cores.
+size_t gemv_tc_bytes();
+bool gemv_tc_applies(const runit_ctx* ctx, int fmt, uint32_t k, uint32_t batch);
+int32_t gemv_tc_multi(runit_ctx* ctx, uint32_t n_mats, const void* const* w, const float* x, float* const* y, const float* const* res, const uint32_t* m,
+                      uint32_t k, uint32_t batch);
 // gemv.cu: grouped GEMVs over stacked expert matrices (MoE block).  Slot s uses expert slot_expert[s] - expert_lo of the
 // n_experts stacked ones; an id outside that range marks an unused slot.
 int32_t gemv_grouped(runit_ctx* ctx, const char* name, int fmt, const void* w, const void* w2, uint32_t n_experts,

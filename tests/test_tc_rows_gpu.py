@@ -1,4 +1,5 @@
-"""Packed rows times a few columns on tcgen05 (tc_rows.cuh): the MoE layer with its slots sorted by expert, at the edges of its tiles.
+"""Packed rows times a few columns on tcgen05 (tc_rows.cuh): the batched Q8_0 GEMV and the MoE layer with its slots sorted by expert, at the edges of their
+tiles and rings.
 
 Bound: an activation keeps 22 bits (two f16 halves of x / 2^e, error <= 2^-22 of it or 2^-35 of the largest of its 256), products are exact, sums
 are f32: 2^-24 of the running sum per addition along 32 products, 8 blocks and K / 256 units.  2e-5 of max(|ref|, rms) holds with room."""
@@ -9,6 +10,80 @@ from helpers import assert_close
 from test_moe_slots_gpu import run
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,k,batch", [(1, 256, 2), (127, 512, 8), (128, 256, 3), (129, 1280, 4), (1000, 2560, 5), (300, 18944, 8), (19100, 768, 7), (40, 5376, 6)])
+def test_batched_q8_0(ctx, oracle, m, k, batch):
+    import runit_mac_b200 as R
+    O = oracle
+    rng = np.random.default_rng(m + k + batch)
+    w = O.rand_weights(0, rng, m, k)
+    x = (rng.normal(0, 1, (batch, k)) * 10.0 ** rng.uniform(-2, 2, (batch, 1))).astype(np.float32)
+    x[0, 3] = 4000.0
+    x[1, :256] = 0
+    res = rng.normal(0, 1, (batch, m)).astype(np.float32)
+    ref = O.gemv(0, w, x, m, k, O.TIER_F64)
+    wb, xb, yb = ctx.buffer_from(w), ctx.buffer_from(x), ctx.new_buffer(batch * m * 4)
+    outs = []
+    for r in (None, res, None):
+        R.gemv_batched_f32(ctx, 0, wb, xb, yb, None if r is None else ctx.buffer_from(r), m, k, batch)
+        ctx.flush()
+        outs.append(yb.download(np.float32, batch * m))
+    for n in range(batch):
+        at = slice(n * m, (n + 1) * m)
+        assert_close(O, ref.reshape(-1)[at], outs[0][at], rel_tol=2e-5, what="row %d" % n)
+        assert_close(O, ref.reshape(-1)[at] + res[n], outs[1][at], rel_tol=2e-5, what="row %d with residual" % n)
+    assert np.array_equal(outs[0], outs[2])
+    ctx.set_tuning("gemv_math", 1)                  # the packed f32 kernel
+    try:
+        R.gemv_batched_f32(ctx, 0, wb, xb, yb, None, m, k, batch)
+        ctx.flush()
+    finally:
+        ctx.set_tuning("gemv_math", 0)
+    for n in range(batch):
+        assert_close(O, yb.download(np.float32, batch * m)[n * m:(n + 1) * m], outs[0][n * m:(n + 1) * m], rel_tol=2e-5, what="against packed f32")
+
+
+@pytest.mark.parametrize("k", [256, 1536, 3584])
+def test_batched_q8_0_bits_do_not_depend_on_the_launch(ctx, oracle, k):
+    """A matrix alone, in one launch with two others, and as the first rows of a larger one: the same bits."""
+    import runit_mac_b200 as R
+    O = oracle
+    rows, batch = (700, 128, 2000), 6
+    rng = np.random.default_rng(k)
+    ws = [O.rand_weights(0, rng, m, k) for m in rows]
+    xb = ctx.buffer_from(rng.normal(0, 1, (batch, k)).astype(np.float32))
+    wb = [ctx.buffer_from(w) for w in ws]
+    outs = [ctx.new_buffer(batch * m * 4) for m in rows]
+    R.gemv_batched_multi_f32(ctx, 0, wb, xb, outs, rows, k, batch)
+    both = ctx.buffer_from(np.concatenate([ws[0].reshape(rows[0], -1)[:640], ws[2].reshape(rows[2], -1)]))
+    large, single = ctx.new_buffer(batch * 2640 * 4), ctx.new_buffer(batch * 2000 * 4)
+    R.gemv_batched_f32(ctx, 0, both, xb, large, None, 2640, k, batch)
+    ctx.flush()
+    for b1, m, o in zip(wb, rows, outs):
+        R.gemv_batched_f32(ctx, 0, b1, xb, single, None, m, k, batch)
+        ctx.flush()
+        assert np.array_equal(single.download(np.float32, batch * m), o.download(np.float32, batch * m))
+    large = large.download(np.float32, batch * 2640).reshape(batch, 2640)
+    assert np.array_equal(large[:, :640], outs[0].download(np.float32, batch * 700).reshape(batch, 700)[:, :640])
+    assert np.array_equal(large[:, 640:], outs[2].download(np.float32, batch * 2000).reshape(batch, 2000))
+
+
+def test_batched_q8_0_value_that_is_not_finite_stays_with_its_row(ctx, oracle):
+    import runit_mac_b200 as R
+    O = oracle
+    m, k, batch = 200, 1024, 5
+    rng = np.random.default_rng(5)
+    w = O.rand_weights(0, rng, m, k)
+    x = rng.normal(0, 1, (batch, k)).astype(np.float32)
+    x[1, 700], x[3, 0] = np.inf, np.nan
+    yb = ctx.new_buffer(batch * m * 4)
+    R.gemv_batched_f32(ctx, 0, ctx.buffer_from(w), ctx.buffer_from(x), yb, None, m, k, batch)
+    ctx.flush()
+    got = yb.download(np.float32, batch * m).reshape(batch, m)
+    assert not np.isfinite(got[[1, 3]]).any()
+    for n in (0, 2, 4):
+        assert_close(O, O.gemv(0, w, x[n], m, k, O.TIER_F64), got[n], rel_tol=2e-5, what="row %d" % n)
 
 
 @pytest.mark.parametrize("counts", [(0, 1, 7, 8, 9, 16, 17, 30),            # groups of 8 columns
