@@ -17,7 +17,7 @@
 //   * per 128-wide K step: the weight operand is dequantised by 16 warps from raw Q4_K superblocks (TMA ring in shared
 //     memory) straight into tensor memory (tcgen05.st), the token tile arrives by TMA into 128-byte-swizzled shared
 //     memory, and the leader CTA issues 8 MMAs of M = 256, N <= 256, K = 16;
-//   * 23 warps per CTA: 0 = token-tile producer (+ tensor-memory allocation), 1 = MMA issuer (leader CTA), 2-5 =
+//   * 27 warps per CTA: 0 = token-tile producer (+ tensor-memory allocation), 1 = MMA issuer (leader CTA), 2-5 and 23-26 =
 //     epilogue (tensor memory -> registers -> global), 6-21 = dequantisers, 22 = raw-superblock producer.
 // The reasons for each of these choices, with the measurements behind them, are in the comment above the kernel.
 // Every wait is bounded in time; a wait that gives up raises the CTA's abort flag, all roles leave their loops,
@@ -55,6 +55,8 @@ struct Args {
     // pointers may lie in another GPU's memory (plain stores): the expert outputs of an expert-parallel block go straight
     // back to the ranks that sent the tokens while the GEMM is still running.
     float* const* row_ptr;
+    uint32_t plain;               // f32 output by plain stores: to row_ptr, or where `out` is not 16-byte aligned
+    uint32_t tile;                // token slots of a tile at most: 128 (two accumulators) or 256 (one)
     int32_t* status;
 };
 
@@ -118,20 +120,24 @@ __device__ __forceinline__ void dequant_half(const uint32_t* q, float sc, float 
 //     weight stages (64 tensor-memory columns each) and 5 token-tile stages (32 KiB each) cover it;
 //   * Q4_K rows arrive by TMA (box 128 rows x 144 bytes = one superblock per row) into a 3-deep raw ring, issued
 //     by a warp of their own so that they never queue behind the token-tile loads;
-//   * 16 dequantiser warps in two groups, each taking one of the two 64-wide chunks of a step;
+//   * 16 dequantiser warps, four for each of a unit's four 64-wide chunks: a thread waits, reads the row's header and stores once per 64
+//     weights (with 32 per thread and step the waits and the unpacking of the scales cost as much as the weights);
 //   * fused gate/up: the CTA's 128 tile rows are 64 gate rows followed by the 64 up rows of the same
 //     intermediate indices; gate and up warps of the epilogue swap half of their columns through shared memory, so
 //     all four warps compute, and the bf16 results leave through a shared-memory transpose as 16-byte stores
 //     (two-byte stores cost 60 cycles each);
-//   * one 256-column accumulator (the other 256 columns hold the weight stages): the epilogue of an item is not
-//     overlapped with the MMAs of the next, but both rings refill during it.
+//   * 256 columns of accumulators (the other 256 hold the weight stages): tiles of up to 128 slots take two in turn, so that the epilogue of an
+//     item runs under the MMAs of the next; tiles of up to 256 take them all, and only the rings refill during it (the rule is in experts_impl);
+//   * the f32 output of the down product leaves by TMA from a shared-memory tile of 32 slots x 128 rows, and two groups of four epilogue warps
+//     take the column groups in turn (stores of 128 bytes by four warps were the longest part of its items: 230 -> 158 us at 4096 tokens).
+// The block of 4096 tokens, 128 experts of 2048 x 768, top 8 (Zipf): 609 -> 469 us; 1024 tokens 297 -> 220, 64 tokens 171 -> 138.
 // Barriers: a_full[s], b_full[s] and acc_empty live in the leader and also take arrivals from the peer;
 // a_empty[s], b_empty[s] and acc_full are signalled in both CTAs at once by the leader's tcgen05.commit.
 namespace pair {
 
-constexpr int kThreads = 736;              // 23 warps: token-tile producer, MMA, 4 epilogue, 16 dequantisers, raw producer
-constexpr int kRawWarp = 22;
-constexpr int kDeqWarp0 = 6, kGroupWarps = 8;
+constexpr int kThreads = 864;              // 27 warps: token-tile producer, MMA, 4 epilogue, 16 dequantisers, raw producer, 4 epilogue
+constexpr int kRawWarp = 22, kEpiWarp1 = 23;
+constexpr int kDeqWarp0 = 6;
 constexpr int kNS = 4;                     // pipeline stages: token tile (shared memory, two 64-wide K chunks = 32 KiB) +
                                            // weight tile (tensor memory, 64 columns); one full / one empty barrier each, so
                                            // the MMA thread pays one wait and one commit per step
@@ -141,40 +147,45 @@ constexpr int kRawBytes = 128 * 144;
 constexpr int kXchgBytes = 2 * 2 * 32 * 17 * 4;
 constexpr int kOffRaw = kNS * kStageB;
 constexpr int kOffXchg = kOffRaw + kNR * kRawBytes;
-constexpr int kOffCtrl = kOffXchg + kXchgBytes;
+constexpr int kOutBytes = 32 * 128 * 4;                // f32 output of 32 slots x this CTA's 128 rows, on its way out
+constexpr int kOffOut = kOffXchg + kXchgBytes;         // one of each epilogue group
+static_assert(kXchgBytes <= kOutBytes, "the second group's exchange");
+constexpr int kOffCtrl = kOffOut + 2 * kOutBytes;
 constexpr int kSmem = kOffCtrl + 512 + 1024;
 constexpr int kTmemCols = 512, kACol0 = 256;
-constexpr int kTokPair = 256;
+constexpr int kTokPair = 256, kTokSmall = 128;
+static_assert(kOffOut % 128 == 0 && kSmem <= 227 * 1024, "shared memory");
 
 template <bool DUAL>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_w0,
-                         const __grid_constant__ CUtensorMap map_w1, const Args a) {
+                         const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUtensorMap map_out, const Args a) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* base_p = smem_raw + (base - smem_u32(smem_raw));
     const uint32_t ctrl = base + kOffCtrl;
     const uint32_t bar_full = ctrl, bar_empty = bar_full + 8 * kNS, bar_rawf = bar_empty + 8 * kNS, bar_rawe = bar_rawf + 8 * kNR,
-                   bar_accf = bar_rawe + 8 * kNR, bar_acce = bar_accf + 8, holder = bar_acce + 8;
+                   bar_accf = bar_rawe + 8 * kNR, bar_acce = bar_accf + 16, holder = bar_acce + 16;
     volatile uint32_t* holder_p = reinterpret_cast<volatile uint32_t*>(base_p + kOffCtrl + (holder - ctrl));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(base_p + kOffCtrl + (holder - ctrl) + 4);
-    float* xchg = reinterpret_cast<float*>(base_p + kOffXchg);
 
     const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const uint32_t rank = cluster_ctarank();
     const uint32_t pair_id = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     if (tid == 0) {
         for (int s = 0; s < kNS; s++) {
-            // full: both dequantiser groups of each CTA (one K chunk each) + the leader's expect_tx (bytes from both CTAs' loads)
-            mbar_init(bar_full + 8 * s, 4 * kGroupWarps + 1);
+            // full: the eight warps of a step's two chunks in each CTA + the leader's expect_tx (bytes from both CTAs' loads)
+            mbar_init(bar_full + 8 * s, 17);
             mbar_init(bar_empty + 8 * s, 1);
         }
         for (int u = 0; u < kNR; u++) {
             mbar_init(bar_rawf + 8 * u, 1);
-            mbar_init(bar_rawe + 8 * u, 2 * kGroupWarps);
+            mbar_init(bar_rawe + 8 * u, 16);
         }
-        mbar_init(bar_accf, 1);
-        mbar_init(bar_acce, 8);                                 // 4 epilogue warps of each CTA
+        for (int i = 0; i < 2; i++) {
+            mbar_init(bar_accf + 8 * i, 1);
+            mbar_init(bar_acce + 8 * i, 16);                    // 8 epilogue warps of each CTA
+        }
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -193,6 +204,9 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_b, const __grid
     const uint32_t units = a.K / 256;
     const uint32_t leader_full = cluster_map(bar_full, 0), leader_acce = cluster_map(bar_acce, 0);
 
+    // accumulators: item n of the pair uses number n % accs, for the (n / accs)-th time
+    const uint32_t acc_shift = a.tile <= 128 ? 1 : 0, acc_mask = acc_shift, load_bytes = a.tile * 2 * 128;
+
     auto tile_cols = [&](int32_t nvalid) -> uint32_t { return nvalid <= 32 ? 32u : (uint32_t)((nvalid + 31) & ~31); };
 
     if (warp == 0) {
@@ -207,7 +221,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_b, const __grid
                 for (uint32_t st = 0; st < units * 2; st++, it++) {
                     const uint32_t s = it % kNS, ph = (it / kNS) & 1;
                     if (!mbar_wait_timed(bar_empty + 8 * s, ph ^ 1, abort_flag)) { ok = false; break; }
-                    if (rank == 0) mbar_expect_tx(bar_full + 8 * s, 2 * kStageB);
+                    if (rank == 0) mbar_expect_tx(bar_full + 8 * s, load_bytes);
                     tma_load_2d_pair(base + s * kStageB, &map_b, (int32_t)(st * 256), row_b, leader_full + 8 * s);
                     tma_load_2d_pair(base + s * kStageB + kTileBytes, &map_b, (int32_t)(st * 256 + 128), row_b, leader_full + 8 * s);
                 }
@@ -244,7 +258,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_b, const __grid
             for (uint32_t item = pair_id; item < n_items && ok && !__any_sync(0xffffffffu, *abort_flag); item += n_pairs, n++) {
                 const uint32_t idesc = umma_idesc_bf16(256, tile_cols(a.tile_nvalid[item / nb]));
                 // the epilogue has drained the accumulator
-                if (!__all_sync(0xffffffffu, mbar_wait_timed_cluster(bar_acce, (n & 1) ^ 1, abort_flag))) break;
+                const uint32_t buf = n & acc_mask, acc = tmem_base + 128 * buf;
+                if (!__all_sync(0xffffffffu, mbar_wait_timed_cluster(bar_acce + 8 * buf, ((n >> acc_shift) & 1) ^ 1, abort_flag))) break;
                 for (uint32_t st = 0; st < units * 2; st++, it++) {
                     const uint32_t sa = it % kNS, sb = sa, pa = (it / kNS) & 1;
                     if (!(ok = __all_sync(0xffffffffu, mbar_wait_timed_cluster(bar_full + 8 * sa, pa, abort_flag)))) break;
@@ -256,36 +271,44 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_b, const __grid
                             const uint64_t db = umma_desc_sw128(base + sb * kStageB + c * kTileBytes);
 #pragma unroll
                             for (uint32_t k4 = 0; k4 < 4; k4++)
-                                umma_bf16_pair_ts(tmem_base, at + 32 * c + 8 * k4, db + 2 * k4, idesc, (st | c | k4) != 0);
+                                umma_bf16_pair_ts(acc, at + 32 * c + 8 * k4, db + 2 * k4, idesc, (st | c | k4) != 0);
                         }
                         umma_commit_pair(bar_empty + 8 * sa, 3);
-                        if (st + 1 == units * 2) umma_commit_pair(bar_accf, 3);
+                        if (st + 1 == units * 2) umma_commit_pair(bar_accf + 8 * buf, 3);
                     }
                     __syncwarp();
                 }
             }
         }
-    } else if (warp < kDeqWarp0) {
-        // ───────── epilogue ─────────
-        // The four warps meet on a named barrier inside the loop, so they must leave it together: one thread waits
+    } else if (warp < kDeqWarp0 || warp >= kEpiWarp1) {
+        // ───────── epilogue: two groups of four warps take the groups of 32 columns in turn ─────────
+        // The warps of a group meet on a named barrier inside the loop, so they must leave it together: one thread waits
         // for the accumulator and publishes the outcome (also on abort) to the other 127.
+        const uint32_t group = warp >= kEpiWarp1;
+        auto meet = [&]() {
+            if (group) asm volatile("bar.sync 2, 128;" ::: "memory");
+            else asm volatile("bar.sync 1, 128;" ::: "memory");
+        };
         const uint32_t quarter = warp & 3;
-        volatile int* go = reinterpret_cast<volatile int*>(base_p + kOffCtrl + (holder - ctrl) + 8);
+        volatile int* go = reinterpret_cast<volatile int*>(base_p + kOffCtrl + (holder - ctrl) + 8 + 4 * group);
         uint32_t n = 0;
+        const bool storer = (warp == kEpiWarp0 || warp == kEpiWarp1) && lane == 0;
+        const uint32_t out_place = kOffOut + group * kOutBytes;
+        float* const xchg = reinterpret_cast<float*>(base_p + (group ? kOffOut : kOffXchg));       // gate and up have no f32 output
         for (uint32_t item = pair_id; item < n_items; item += n_pairs, n++) {
-            const uint32_t tt = item / nb, rb = item % nb;
+            const uint32_t tt = item / nb, rb = item % nb, buf = n & acc_mask;
             const int32_t nvalid = a.tile_nvalid[tt];
             const size_t row0 = (size_t)a.tile_row0[tt];
-            if (warp == kEpiWarp0 && lane == 0)
-                *go = (mbar_wait_timed(bar_accf, n & 1, abort_flag) && !*abort_flag) ? 1 : 0;
-            asm volatile("bar.sync 1, 128;" ::: "memory");
+            if (storer)
+                *go = (mbar_wait_timed(bar_accf + 8 * buf, (n >> acc_shift) & 1, abort_flag) && !*abort_flag) ? 1 : 0;
+            meet();
             const int ready = *go;
-            asm volatile("bar.sync 1, 128;" ::: "memory");   // everyone has read it before the next item overwrites it
+            meet();   // everyone has read it before the next item overwrites it
             if (!ready) break;
             tc_fence_after_sync();
-            const uint32_t taddr0 = tmem_base + ((quarter * 32) << 16);
+            const uint32_t taddr0 = tmem_base + 128 * buf + ((quarter * 32) << 16);
 #pragma unroll 1
-            for (int cg = 0; cg * 32 < nvalid; cg++) {
+            for (int cg = group; cg * 32 < nvalid; cg += 2) {
                 uint32_t v[32];
                 tmem_ld32(taddr0 + cg * 32, v);
                 tmem_ld_wait();
@@ -303,14 +326,14 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_b, const __grid
 #pragma unroll
                         for (int i = 0; i < 16; i++) xu[i] = __uint_as_float(v[i]);
                     }
-                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                    meet();
                     float gv[16], uv[16];
 #pragma unroll
                     for (int i = 0; i < 16; i++) {
                         gv[i] = is_gate ? __uint_as_float(v[i]) : xg[i];
                         uv[i] = is_gate ? xu[i] : __uint_as_float(v[16 + i]);
                     }
-                    asm volatile("bar.sync 1, 128;" ::: "memory");   // the exchange area may be rewritten
+                    meet();   // the exchange area may be rewritten
                     // 16 tokens x 32 intermediate indices of bf16 go through the warp's own (now idle) exchange array so
                     // that every lane stores 16 bytes: 2 stores per lane instead of 16 two-byte ones.
                     __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(a.out);
@@ -329,72 +352,73 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_b, const __grid
                     }
                     __syncwarp();
                 } else {
-                    float* out = reinterpret_cast<float*>(a.out);
-                    const uint32_t col = rb * 256 + rank * 128 + quarter * 32 + lane;
-                    if (a.row_ptr != nullptr) {
+                    if (a.plain) {
+                        const uint32_t col = rb * 256 + rank * 128 + quarter * 32 + lane;
 #pragma unroll
                         for (int i = 0; i < 32; i++)
-                            if (cg * 32 + i < nvalid) a.row_ptr[row0 + cg * 32 + i][col] = __uint_as_float(v[i]);
+                            if (cg * 32 + i < nvalid)
+                                (a.row_ptr ? a.row_ptr[row0 + cg * 32 + i] : reinterpret_cast<float*>(a.out) + (row0 + cg * 32 + i) * a.ld)[col] = __uint_as_float(v[i]);
                     } else {
+                        // 32 slots x 128 rows through shared memory and out by TMA (256 stores of 128 bytes per warp and item were the longest part
+                        // of the down product); rows behind the last valid slot are padding of the same expert
+                        if (storer) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");       // the last store has left this place
+                        meet();
+                        float* o = reinterpret_cast<float*>(base_p + out_place) + quarter * 32 + lane;
 #pragma unroll
-                        for (int i = 0; i < 32; i++)
-                            if (cg * 32 + i < nvalid) out[(row0 + cg * 32 + i) * a.ld + col] = __uint_as_float(v[i]);
+                        for (int i = 0; i < 32; i++) o[i * 128] = __uint_as_float(v[i]);
+                        fence_proxy_async();
+                        meet();
+                        if (storer) {
+                            tma_store_2d(&map_out, base + out_place, (int32_t)((rb * 256 + rank * 128) * 2), (int32_t)row0 + cg * 32);    // elements of two bytes
+                            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                        }
                     }
                 }
             }
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) {
-                if (rank == 0) mbar_arrive(bar_acce);
-                else mbar_arrive_cluster(leader_acce);
+                if (rank == 0) mbar_arrive(bar_acce + 8 * buf);
+                else mbar_arrive_cluster(leader_acce + 8 * buf);
             }
         }
+        if (storer) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     } else if (warp < kRawWarp) {
-        // ───────── dequantisers: raw ring -> bf16 rows in tensor memory.  Group g takes chunk g of every step (the
-        //            chunks j of a unit with j % 2 == g).  A warp may only write the tensor-memory lanes
+        // ───────── dequantisers: raw ring -> bf16 rows in tensor memory.  Four warps take one of a unit's four 64-wide chunks, for a row each thread:
+        //            chunks 0, 1 make the unit's first step, 2, 3 its second.  A warp may only write the tensor-memory lanes
         //            32 * (warp % 4) .. + 31: those are its rows. ─────────
-        const uint32_t dw = warp - kDeqWarp0;
-        const uint32_t g = dw / kGroupWarps, part = (dw % kGroupWarps) / 4;   // part 0: low nibbles (K 0..31 of the chunk), 1: high
-        const uint32_t quarter = warp & 3, r = quarter * 32 + lane;
+        const uint32_t j = (warp - kDeqWarp0) / 4, g = j & 1, jj = j >> 1;
+        const uint32_t quarter = warp & 3, r = quarter * 32 + lane, sh = 8 * j;
         uint32_t uc = 0;
         bool ok = true;
         for (uint32_t item = pair_id; item < n_items && ok && !*abort_flag; item += n_pairs) {
-            for (uint32_t u = 0; u < units && ok; u++, uc++) {
+            for (uint32_t u = 0; u < units; u++, uc++) {
                 const uint32_t ur = uc % kNR;
-                if (!mbar_wait_timed(bar_rawf + 8 * ur, (uc / kNR) & 1, abort_flag)) { ok = false; break; }
+                if (!(ok = __all_sync(0xffffffffu, mbar_wait_timed(bar_rawf + 8 * ur, (uc / kNR) & 1, abort_flag)))) break;
                 const uint32_t raw_row = base + kOffRaw + ur * kRawBytes + r * 144;
-                uint32_t h0, h1, h2, h3;
+                uint32_t h0, h1, h2, h3, q[8];
                 asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(h0), "=r"(h1), "=r"(h2), "=r"(h3) : "r"(raw_row) : "memory");
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]) : "r"(raw_row + 16 + 32 * j) : "memory");
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7]) : "r"(raw_row + 32 + 32 * j) : "memory");
                 const float dd = half_bits_to_float(h0), dmin = half_bits_to_float(h0 >> 16);
                 const Q4KScales sc = q4k_unpack_scales(h1, h2, h3);
-#pragma unroll
-                for (int jj = 0; jj < 2; jj++) {
-                    const uint32_t j = 2 * jj + g;               // chunk of the unit; step 2 * unit + jj holds chunks 2jj, 2jj + 1
-                    const uint32_t it = uc * 2 + jj;
-                    const uint32_t s = it % kNS, ph = (it / kNS) & 1;
-                    uint32_t q[8];
-                    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]) : "r"(raw_row + 16 + 32 * j) : "memory");
-                    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7]) : "r"(raw_row + 32 + 32 * j) : "memory");
-                    const uint32_t sh = 8 * j;
-                    uint32_t out[16];
-                    if (part == 0) dequant_half<false>(q, dd * (float)((sc.sl >> sh) & 0xFFu), dmin * (float)((sc.ml >> sh) & 0xFFu), out);
-                    else dequant_half<true>(q, dd * (float)((sc.sh >> sh) & 0xFFu), dmin * (float)((sc.mh >> sh) & 0xFFu), out);
-                    uint32_t got = 1;
-                    if (lane == 0) got = mbar_wait_timed(bar_empty + 8 * s, ph ^ 1, abort_flag);
-                    got = __shfl_sync(0xffffffffu, got, 0);
-                    if (!got) { ok = false; break; }
-                    tc_fence_after_sync();
-                    tmem_st16(tmem_base + ((quarter * 32) << 16) + kACol0 + 64 * s + 32 * g + 16 * part, out);
-                    tmem_st_wait();
-                    tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) {
-                        if (rank == 0) mbar_arrive(bar_full + 8 * s);
-                        else mbar_arrive_cluster(leader_full + 8 * s);
-                    }
-                }
+                uint32_t out[16];
+                dequant_half<false>(q, dd * (float)((sc.sl >> sh) & 0xFFu), dmin * (float)((sc.ml >> sh) & 0xFFu), out);
+                const uint32_t it = uc * 2 + jj, s = it % kNS, ph = (it / kNS) & 1;
+                if (!(ok = __all_sync(0xffffffffu, mbar_wait_timed(bar_empty + 8 * s, ph ^ 1, abort_flag)))) break;
+                tc_fence_after_sync();
+                const uint32_t at = tmem_base + ((quarter * 32) << 16) + kACol0 + 64 * s + 32 * g;
+                tmem_st16(at, out);
+                dequant_half<true>(q, dd * (float)((sc.sh >> sh) & 0xFFu), dmin * (float)((sc.mh >> sh) & 0xFFu), out);
+                tmem_st16(at + 16, out);
+                if (lane == 0) mbar_arrive(bar_rawe + 8 * ur);
+                tmem_st_wait();
+                tc_fence_before_sync();
                 __syncwarp();
-                if (lane == 0 && ok) mbar_arrive(bar_rawe + 8 * ur);
+                if (lane == 0) {
+                    if (rank == 0) mbar_arrive(bar_full + 8 * s);
+                    else mbar_arrive_cluster(leader_full + 8 * s);
+                }
             }
         }
     }
@@ -485,25 +509,28 @@ static Scratch carve(void* base, uint32_t T, uint32_t h, uint32_t ff, uint32_t E
 }
 
 template <bool DUAL>
-static int32_t launch_pair(runit_ctx* ctx, const char* name, const Args& a, const void* b_ptr, uint32_t b_rows, uint32_t n_experts,
-                           uint32_t max_items) {
+static int32_t launch_pair(runit_ctx* ctx, const char* name, Args a, const void* b_ptr, uint32_t b_rows, uint32_t n_experts,
+                           uint32_t max_items, uint64_t out_rows) {
     static bool attr_set[64] = {false};
     if (ctx->device >= 0 && ctx->device < 64 && !attr_set[ctx->device]) {
         RUNIT_CUDA_TRY(ctx, cudaFuncSetAttribute(pair::grouped_gemm_pair_kernel<DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::kSmem));
         attr_set[ctx->device] = true;
     }
-    CUtensorMap map_b, map_w0, map_w1;
-    int32_t st = runit_get_tmap(ctx, b_ptr, b_rows, (uint64_t)a.K * 2, kTok, 128, &map_b, 1);
+    CUtensorMap map_b, map_w0, map_w1, map_out;
+    int32_t st = runit_get_tmap(ctx, b_ptr, b_rows, (uint64_t)a.K * 2, a.tile / 2, 128, &map_b, 1);
     if (st != RUNIT_OK) return st;
     const uint64_t w_rows = (uint64_t)n_experts * a.rows, row_bytes = (uint64_t)a.K / 256 * 144;
     st = runit_get_tmap(ctx, a.w0, w_rows, row_bytes, DUAL ? 64 : 128, 144, &map_w0);
     if (st != RUNIT_OK) return st;
     map_w1 = map_w0;
     if (DUAL && (st = runit_get_tmap(ctx, a.w1, w_rows, row_bytes, 64, 144, &map_w1)) != RUNIT_OK) return st;
+    map_out = map_w0;                               // unused where the output is bf16 or goes to peers
+    a.plain = a.row_ptr != nullptr || !runit_aligned(a.out, 16);
+    if (!DUAL && !a.plain && (st = runit_get_tmap(ctx, a.out, out_rows, (uint64_t)a.ld * 4, 32, 512, &map_out)) != RUNIT_OK) return st;
     uint32_t pairs = (uint32_t)ctx->sm_count / 2;
     if (pairs > max_items) pairs = max_items;
     if (pairs == 0) pairs = 1;
-    pair::grouped_gemm_pair_kernel<DUAL><<<2 * pairs, pair::kThreads, pair::kSmem, ctx->stream>>>(map_b, map_w0, map_w1, a);
+    pair::grouped_gemm_pair_kernel<DUAL><<<2 * pairs, pair::kThreads, pair::kSmem, ctx->stream>>>(map_b, map_w0, map_w1, map_out, a);
     return runit_after_launch(ctx, name);
 }
 
@@ -518,7 +545,11 @@ static int32_t experts_impl(runit_ctx* ctx, const Scratch& s, const void* gate, 
                             uint32_t cap_src = 0) {
     const uint32_t S = T * k;
     MoePermutation p{s.counts, s.n_tok_tiles, s.tile_expert, s.tile_nvalid, s.tile_row0, s.pos_of_slot};
-    int32_t st = moe_permute(ctx, idx, S, E, pair::kTokPair, p);
+    // Tiles of 128 slots, whose epilogue runs under the next tile's products, up to 256 slots per expert; behind that of 256, because a tile costs the
+    // dequantisation of its weights whatever it holds (us with 128 / 256: 128 experts of 2048 x 768, top 8: 300 tokens 175 / 188, 4096 469 / 478; 64
+    // experts: 1024 tokens 170 / 178, 4096 443 / 424; 8 of 1024 x 512, top 2: 300 tokens 44 / 47, 1024 59 / 58).
+    const uint32_t tile = (uint64_t)S <= 256ull * E ? pair::kTokSmall : pair::kTokPair;
+    int32_t st = moe_permute(ctx, idx, S, E, tile, p);
     if (st != RUNIT_OK) return st;
     if (x_bf16) {
         if ((st = moe_gather_rows(ctx, x_bf16, s.pos_of_slot, s.xperm, S, (size_t)h * 2, 1)) != RUNIT_OK) return st;
@@ -529,11 +560,11 @@ static int32_t experts_impl(runit_ctx* ctx, const Scratch& s, const void* gate, 
     Args a1{};
     a1.w0 = (const uint8_t*)gate; a1.w1 = (const uint8_t*)up; a1.rows = ff; a1.K = h; a1.nb = ff / kRows;
     a1.tile_expert = s.tile_expert; a1.tile_nvalid = s.tile_nvalid; a1.tile_row0 = s.tile_row0; a1.n_tok_tiles = s.n_tok_tiles;
-    a1.out = s.act; a1.ld = ff; a1.status = ctx->d_status;
+    a1.out = s.act; a1.ld = ff; a1.tile = tile; a1.status = ctx->d_status;
     Args a2{};
     a2.w0 = (const uint8_t*)down; a2.w1 = nullptr; a2.rows = h; a2.K = ff; a2.nb = h / kRows;
     a2.tile_expert = s.tile_expert; a2.tile_nvalid = s.tile_nvalid; a2.tile_row0 = s.tile_row0; a2.n_tok_tiles = s.n_tok_tiles;
-    a2.out = s.y; a2.ld = h; a2.status = ctx->d_status;
+    a2.out = s.y; a2.ld = h; a2.tile = tile; a2.status = ctx->d_status;
     if (cap_src > 0) {
         // the table of row destinations lives in the output area the GEMM no longer writes (8 bytes per row of 4*h)
         float** table = reinterpret_cast<float**>(s.y);
@@ -541,8 +572,8 @@ static int32_t experts_impl(runit_ctx* ctx, const Scratch& s, const void* gate, 
         if ((st = runit_after_launch(ctx, "moe_grouped_row_ptr")) != RUNIT_OK) return st;
         a2.row_ptr = table;
     }
-    if ((st = launch_pair<true>(ctx, "moe_grouped_gate_up", a1, s.xperm, rows, E, s.max_tiles * (ff / 128))) != RUNIT_OK) return st;
-    if ((st = launch_pair<false>(ctx, "moe_grouped_down", a2, s.act, rows, E, s.max_tiles * (h / 256))) != RUNIT_OK) return st;
+    if ((st = launch_pair<true>(ctx, "moe_grouped_gate_up", a1, s.xperm, rows, E, s.max_tiles * (ff / 128), rows)) != RUNIT_OK) return st;
+    if ((st = launch_pair<false>(ctx, "moe_grouped_down", a2, s.act, rows, E, s.max_tiles * (h / 256), rows)) != RUNIT_OK) return st;
     if (!out) return RUNIT_OK;
     return moe_grouped_combine(ctx, s.y, s.pos_of_slot, w, residual, out, T, h, k);
 }
@@ -611,9 +642,10 @@ int32_t dense_gemm_q4k_bf16(runit_ctx* ctx, const char* name, const void* w, con
     a.n_tok_tiles = tables;
     a.out = out;
     a.ld = ld;
+    a.tile = gg::pair::kTokPair;
     a.status = ctx->d_status;
-    if (w_up) return gg::launch_pair<true>(ctx, name, a, x_bf16, x_rows, 1, n * (rows / 128));
-    return gg::launch_pair<false>(ctx, name, a, x_bf16, x_rows, 1, n * (rows / 256));
+    if (w_up) return gg::launch_pair<true>(ctx, name, a, x_bf16, x_rows, 1, n * (rows / 128), T);
+    return gg::launch_pair<false>(ctx, name, a, x_bf16, x_rows, 1, n * (rows / 256), T);
 }
 
 }  // namespace runit

@@ -6,13 +6,15 @@
 
 namespace runit {
 
+constexpr uint32_t kCountSlots = 1024;              // of a CTA
+
 // counts[e] = slots routed to expert e; slots with an id outside [0, E) get position -1.
 __global__ void __launch_bounds__(256) count_kernel(const int32_t* __restrict__ idx, uint32_t S, uint32_t E,
                                                      int32_t* __restrict__ counts, int32_t* __restrict__ pos_of_slot) {
     __shared__ int hist[256];
     hist[threadIdx.x] = 0;
     __syncthreads();
-    for (uint32_t s = blockIdx.x * 4096 + threadIdx.x, i = 0; i < 16 && s < S; i++, s += 256) {
+    for (uint32_t s = blockIdx.x * kCountSlots + threadIdx.x, i = 0; i < kCountSlots / 256 && s < S; i++, s += 256) {
         const int32_t e = idx[s];
         if (e >= 0 && (uint32_t)e < E) atomicAdd(&hist[e], 1);
         else pos_of_slot[s] = -1;
@@ -29,46 +31,42 @@ __global__ void __launch_bounds__(1024) place_kernel(const int32_t* __restrict__
                                                       int32_t* __restrict__ pos_of_slot, int32_t* __restrict__ tile_expert,
                                                       int32_t* __restrict__ tile_nvalid, int32_t* __restrict__ tile_row0,
                                                       int32_t* __restrict__ n_tok_tiles) {
-    __shared__ int s_cnt[256];
-    __shared__ int s_warp[32];
-    __shared__ int s_off, s_tile0, s_chunk;
+    __shared__ int s_warp[32], s_red[8][3];
+    __shared__ int s_cnt, s_chunk;
     const uint32_t e = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (tid < 256) s_cnt[tid] = tid < E ? counts[tid] : 0;
-    __syncthreads();
-    if (tid == 0) {
-        int off = 0, tiles = 0;
-        for (uint32_t i = 0; i < E; i++) {
-            if (i == e) { s_off = off; s_tile0 = tiles; }
-            off += ((s_cnt[i] + kMoeRowAlign - 1) / kMoeRowAlign) * kMoeRowAlign;
-            tiles += (s_cnt[i] + tile_tok - 1) / tile_tok;
-        }
-        if (e == 0) n_tok_tiles[0] = tiles;
+    // rows and tiles of the experts before this one, all tiles (one thread that adds them up in order takes 15 us at 128 experts)
+    if (tid < 256) {
+        const int c = tid < E ? counts[tid] : 0, tiles = (c + tile_tok - 1) / tile_tok;
+        const int off = __reduce_add_sync(0xffffffffu, tid < e ? (c + kMoeRowAlign - 1) / kMoeRowAlign * kMoeRowAlign : 0);
+        const int before = __reduce_add_sync(0xffffffffu, tid < e ? tiles : 0), all = __reduce_add_sync(0xffffffffu, tiles);
+        if (lane == 0) s_red[warp][0] = off, s_red[warp][1] = before, s_red[warp][2] = all;
+        if (tid == e) s_cnt = c;
     }
     __syncthreads();
-    const int cnt = s_cnt[e], off = s_off, tile0 = s_tile0;
+    int off = 0, tile0 = 0, all = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) off += s_red[i][0], tile0 += s_red[i][1], all += s_red[i][2];
+    if (e == 0 && tid == 0) n_tok_tiles[0] = all;
+    const int cnt = s_cnt;
     for (int i = tid; i * tile_tok < cnt; i += 1024) {
         tile_expert[tile0 + i] = (int32_t)e;
         tile_nvalid[tile0 + i] = min(tile_tok, cnt - i * tile_tok);
         tile_row0[tile0 + i] = off + i * tile_tok;
     }
-    // every thread takes 4 consecutive slots per round, so a round covers 4096 slots in slot order
+    // A round covers 16384 slots in slot order: every warp takes 512 consecutive ones, 32 at a time, and counts its hits by ballots.  (With 4 slots
+    // a thread and three barriers for every 4096, 32768 slots took 20 us.)
+    constexpr int kRows = 16;
     int running = 0;
-    for (uint32_t s0 = 0; s0 < S; s0 += 4096) {
-        const uint32_t s = s0 + 4 * tid;
-        bool hit[4];
+    for (uint32_t s0 = 0; s0 < S; s0 += 1024 * kRows) {
+        const uint32_t s = s0 + warp * 32 * kRows + lane;
+        uint32_t hits[kRows];
         int mine = 0;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            hit[i] = s + i < S && idx[s + i] == (int32_t)e;
-            mine += hit[i];
+        for (int i = 0; i < kRows; i++) {
+            hits[i] = __ballot_sync(0xffffffffu, s + 32 * i < S && idx[s + 32 * i] == (int32_t)e);
+            mine += __popc(hits[i]);
         }
-        int incl = mine;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, incl, o);
-            if ((int)lane >= o) incl += t;
-        }
-        if (lane == 31) s_warp[warp] = incl;
+        if (lane == 0) s_warp[warp] = mine;
         __syncthreads();
         if (warp == 0) {
             int v = s_warp[lane], wi = v;
@@ -81,10 +79,12 @@ __global__ void __launch_bounds__(1024) place_kernel(const int32_t* __restrict__
             if (lane == 31) s_chunk = wi;
         }
         __syncthreads();
-        int p = off + running + s_warp[warp] + incl - mine;
+        int p = off + running + s_warp[warp];
 #pragma unroll
-        for (int i = 0; i < 4; i++)
-            if (hit[i]) pos_of_slot[s + i] = p++;
+        for (int i = 0; i < kRows; i++) {
+            if (hits[i] >> lane & 1) pos_of_slot[s + 32 * i] = p + __popc(hits[i] & ((1u << lane) - 1));
+            p += __popc(hits[i]);
+        }
         running += s_chunk;
         __syncthreads();
     }
@@ -158,7 +158,7 @@ __global__ void dense_tiles_kernel(uint32_t T, uint32_t tile_tok, int32_t* tile_
 
 int32_t moe_permute(runit_ctx* ctx, const int32_t* idx, uint32_t S, uint32_t E, uint32_t tile_tok, const MoePermutation& p) {
     RUNIT_CUDA_TRY(ctx, cudaMemsetAsync(p.counts, 0, 4 * 256, ctx->stream));
-    count_kernel<<<(S + 4095) / 4096, 256, 0, ctx->stream>>>(idx, S, E, p.counts, p.pos_of_slot);
+    count_kernel<<<(S + kCountSlots - 1) / kCountSlots, 256, 0, ctx->stream>>>(idx, S, E, p.counts, p.pos_of_slot);
     int32_t st = runit_after_launch(ctx, "moe_grouped_count");
     if (st != RUNIT_OK) return st;
     place_kernel<<<E, 1024, 0, ctx->stream>>>(idx, S, E, p.counts, (int)tile_tok, p.pos_of_slot, p.tile_expert, p.tile_nvalid, p.tile_row0,
