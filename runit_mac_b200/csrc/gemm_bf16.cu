@@ -106,6 +106,77 @@ struct Cfg {
     static constexpr int tmem_cols = 2 * NT;
 };
 
+// The accumulator at taddr (this warp's 32 lanes: row r of the weight matrix) into the output of the tile's tokens.
+template <int EPI>
+__device__ __forceinline__ void drain(const Args& a, const Tile& t, uint32_t taddr, uint32_t r, uint32_t lane) {
+    const bool live = r < a.rows;
+#pragma unroll 1
+    for (uint32_t cg = 0; cg * 32 < t.nvalid; cg++) {
+        uint32_t v[32];
+        tmem_ld32(taddr + cg * 32, v);
+        tmem_ld_wait();
+        const uint32_t tok0 = t.row0 + cg * 32, cnt = min(32u, t.nvalid - cg * 32);
+        if constexpr (EPI == EPI_SILU_GLU || EPI == EPI_RELU2 || EPI == EPI_CAST) {
+            // Four lanes exchange their values of four tokens, so that each holds four neighbouring rows of one token: one
+            // wide store and one pair of factors instead of four.
+            __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(a.out);
+            const bool odd = lane & 1, high = lane & 2;
+            const uint32_t r4 = r & ~3u;
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+                float y[4];
+                quad_transpose(v + j, y, odd, high);
+                const uint32_t jj = j + (lane & 3);
+                if (jj >= cnt || r4 >= a.rows) continue;
+                const uint32_t tok = tok0 + jj;
+                __nv_bfloat16* o = out + (size_t)tok * a.ldo;
+                if constexpr (EPI == EPI_CAST) {
+                    if (r4 + 4 <= a.tail_from) {
+                        store_rows<4>(o + r4, y, a.rows - r4, a.ldo);
+                    } else {
+                        for (uint32_t i = 0; i < 4 && r4 + i < a.rows; i++) {
+                            if (r4 + i < a.tail_from) o[r4 + i] = __float2bfloat16_rn(y[i]);
+                            else a.tail[(size_t)tok * a.ldt + r4 + i - a.tail_from] = y[i];
+                        }
+                    }
+                } else {
+                    const float pre = a.pre ? a.pre[tok] : 1.f, post = a.post ? a.post[tok] : 1.f;
+                    if constexpr (EPI == EPI_SILU_GLU) {      // rows 2i, 2i+1: gate and up of output i
+#pragma unroll
+                        for (int i = 0; i < 2; i++) {
+                            const float g = y[2 * i] * pre, u = y[2 * i + 1] * pre;
+                            y[i] = __fdividef(g, 1.0f + __expf(-g)) * u * post;
+                        }
+                        store_rows<2>(o + r4 / 2, y, (a.rows - r4) / 2, a.ldo);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 4; i++) y[i] = relu2(y[i] * pre) * post;
+                        store_rows<4>(o + r4, y, a.rows - r4, a.ldo);
+                    }
+                }
+            }
+        } else if constexpr (EPI == EPI_ADD) {
+            // all loads of the group before its first store (the compiler may not reorder them across one)
+            float* out = reinterpret_cast<float*>(a.out) + (size_t)tok0 * a.ldo + r;
+            float old[32];
+#pragma unroll
+            for (int j = 0; j < 32; j++) old[j] = (live && (uint32_t)j < cnt) ? out[(size_t)j * a.ldo] : 0.f;
+#pragma unroll
+            for (int j = 0; j < 32; j++)
+                if (live && (uint32_t)j < cnt) out[(size_t)j * a.ldo] = old[j] + __uint_as_float(v[j]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 32; j++) {
+                if (!live || (uint32_t)j >= cnt) continue;
+                float f = __uint_as_float(v[j]);
+                if (a.cap != 0.f) f = a.cap * tanhf(f / a.cap);
+                const size_t o = (size_t)(tok0 + j) * a.ldo + r;
+                reinterpret_cast<float*>(a.out)[o] = f;
+            }
+        }
+    }
+}
+
 template <int EPI, int NT>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Args a) {
@@ -197,72 +268,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             tc_fence_after_sync();
             const uint32_t taddr = tmem + ((quarter * 32) << 16) + acc * NT;
             const uint32_t r = t.rb * kRowsTile + quarter * 32 + lane;     // row of the weight matrix
-            const bool live = r < a.rows;
-#pragma unroll 1
-            for (uint32_t cg = 0; cg * 32 < t.nvalid; cg++) {
-                uint32_t v[32];
-                tmem_ld32(taddr + cg * 32, v);
-                tmem_ld_wait();
-                const uint32_t tok0 = t.row0 + cg * 32, cnt = min(32u, t.nvalid - cg * 32);
-                if constexpr (EPI == EPI_SILU_GLU || EPI == EPI_RELU2 || EPI == EPI_CAST) {
-                    // Four lanes exchange their values of four tokens, so that each holds four neighbouring rows of one token: one
-                    // wide store and one pair of factors instead of four.
-                    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(a.out);
-                    const bool odd = lane & 1, high = lane & 2;
-                    const uint32_t r4 = r & ~3u;
-#pragma unroll
-                    for (int j = 0; j < 32; j += 4) {
-                        float y[4];
-                        quad_transpose(v + j, y, odd, high);
-                        const uint32_t jj = j + (lane & 3);
-                        if (jj >= cnt || r4 >= a.rows) continue;
-                        const uint32_t tok = tok0 + jj;
-                        __nv_bfloat16* o = out + (size_t)tok * a.ldo;
-                        if constexpr (EPI == EPI_CAST) {
-                            if (r4 + 4 <= a.tail_from) {
-                                store_rows<4>(o + r4, y, a.rows - r4, a.ldo);
-                            } else {
-                                for (uint32_t i = 0; i < 4 && r4 + i < a.rows; i++) {
-                                    if (r4 + i < a.tail_from) o[r4 + i] = __float2bfloat16_rn(y[i]);
-                                    else a.tail[(size_t)tok * a.ldt + r4 + i - a.tail_from] = y[i];
-                                }
-                            }
-                        } else {
-                            const float pre = a.pre ? a.pre[tok] : 1.f, post = a.post ? a.post[tok] : 1.f;
-                            if constexpr (EPI == EPI_SILU_GLU) {      // rows 2i, 2i+1: gate and up of output i
-#pragma unroll
-                                for (int i = 0; i < 2; i++) {
-                                    const float g = y[2 * i] * pre, u = y[2 * i + 1] * pre;
-                                    y[i] = __fdividef(g, 1.0f + __expf(-g)) * u * post;
-                                }
-                                store_rows<2>(o + r4 / 2, y, (a.rows - r4) / 2, a.ldo);
-                            } else {
-#pragma unroll
-                                for (int i = 0; i < 4; i++) y[i] = relu2(y[i] * pre) * post;
-                                store_rows<4>(o + r4, y, a.rows - r4, a.ldo);
-                            }
-                        }
-                    }
-                } else if constexpr (EPI == EPI_ADD) {
-                    // all loads of the group before its first store (the compiler may not reorder them across one)
-                    float* out = reinterpret_cast<float*>(a.out) + (size_t)tok0 * a.ldo + r;
-                    float old[32];
-#pragma unroll
-                    for (int j = 0; j < 32; j++) old[j] = (live && (uint32_t)j < cnt) ? out[(size_t)j * a.ldo] : 0.f;
-#pragma unroll
-                    for (int j = 0; j < 32; j++)
-                        if (live && (uint32_t)j < cnt) out[(size_t)j * a.ldo] = old[j] + __uint_as_float(v[j]);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        if (!live || (uint32_t)j >= cnt) continue;
-                        float f = __uint_as_float(v[j]);
-                        if (a.cap != 0.f) f = a.cap * tanhf(f / a.cap);
-                        const size_t o = (size_t)(tok0 + j) * a.ldo + r;
-                        reinterpret_cast<float*>(a.out)[o] = f;
-                    }
-                }
-            }
+            drain<EPI>(a, t, taddr, r, lane);
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_acce + 8 * acc);
@@ -274,6 +280,121 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     if (warp == 1) {
         tc_fence_after_sync();
         tmem_dealloc(tmem, Cfg<NT>::tmem_cols);
+    }
+    if (tid == 0 && *abort_flag && a.status) atomicExch(a.status, 2);
+}
+
+// ───────────────────────── CTA pairs (cta_group::2), tiles of 256 rows x 256 tokens ─────────────────────────
+// Each CTA of a pair holds 128 rows and half of the tokens of every stage; the leader issues M = 256 MMAs that leave 128 accumulator rows in
+// either CTA's tensor memory.  A 128 x 256 tile of one CTA fetches 48 KB per 512 clocks of MMAs, and 148 of them ask the L2 for 11.5 TB/s, which is what it
+// gives: the products took twice their time.  A pair's CTAs fetch 32 KB each for as many products.
+// Barriers: full and acc_empty live in the leader (loads and epilogues of both CTAs arrive there); empty and acc_full are signalled in both at once.
+constexpr int kPairStage = 2 * kABytes, kPairNs = 6, kPairSmem = kPairNs * kPairStage + 1024 + 512;
+
+template <int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Args a) {
+    constexpr int NS = kPairNs, NT = 256;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* base_p = smem_raw + (base - smem_u32(smem_raw));
+    const uint32_t ctrl = base + NS * kPairStage;
+    const uint32_t bar_full = ctrl, bar_empty = bar_full + 8 * NS, bar_accf = bar_empty + 8 * NS, bar_acce = bar_accf + 16, holder = bar_acce + 16;
+    volatile uint32_t* holder_p = reinterpret_cast<volatile uint32_t*>(base_p + (holder - base));
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(base_p + (holder - base) + 4);
+    const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const uint32_t rank = cluster_ctarank(), pair_id = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+    if (tid == 0) {
+        for (int s = 0; s < NS; s++) {
+            mbar_init(bar_full + 8 * s, 1);
+            mbar_init(bar_empty + 8 * s, 1);
+        }
+        for (int s = 0; s < 2; s++) {
+            mbar_init(bar_accf + 8 * s, 1);
+            mbar_init(bar_acce + 8 * s, 8);
+        }
+        *abort_flag = 0;
+        fence_mbar_init();
+    }
+    if (warp == 1) {
+        tmem_alloc_pair(holder, 2 * NT);
+        tmem_relinquish_pair();
+    }
+    __syncwarp();
+    tc_fence_before_sync();
+    cluster_sync();
+    tc_fence_after_sync();
+    const uint32_t tmem = *holder_p;
+    const uint32_t ntt = tok_tiles(a), n_items = ntt * a.nb, ksteps = (a.K + 63) / 64;
+    const uint32_t leader_full = cluster_map(bar_full, 0), leader_acce = cluster_map(bar_acce, 0);
+    auto cols = [](const Tile& t) { return (t.nvalid + 31) & ~31u; };
+
+    if (warp == 0) {
+        if (lane == 0) {
+            uint32_t it = 0;
+            bool ok = true;
+            for (uint32_t item = pair_id; item < n_items && ok && !*abort_flag; item += n_pairs) {
+                const Tile t = tile_of(a, item, ntt);
+                const int32_t wrow = (int32_t)(t.expert * a.rows + t.rb * 256 + rank * kRowsTile), xrow = (int32_t)(t.row0 + rank * (cols(t) / 2));
+                for (uint32_t k = 0; k < ksteps; k++, it++) {
+                    const uint32_t s = it % NS, ph = (it / NS) & 1;
+                    if (!mbar_wait_timed(bar_empty + 8 * s, ph ^ 1, abort_flag)) { ok = false; break; }
+                    const uint32_t dst = base + s * kPairStage;
+                    if (rank == 0) mbar_expect_tx(bar_full + 8 * s, 2 * kPairStage);
+                    tma_load_2d_pair(dst, &map_w, (int32_t)(k * 128), wrow, leader_full + 8 * s);
+                    tma_load_2d_pair(dst + kABytes, &map_x, (int32_t)(k * 128), xrow, leader_full + 8 * s);
+                }
+            }
+            // nobody consumes them any more: wait (bounded) for the loads in flight.  Those of both CTAs count on the leader's barriers; the other
+            // CTA leaves behind the cluster barrier at the end, when the leader has waited.
+            if (rank == 0 && (!ok || *abort_flag)) mbar_drain(bar_full, NS, it);
+        }
+    } else if (warp == 1) {
+        if (rank == 0) {
+            uint32_t it = 0, n = 0;
+            bool ok = true;
+            for (uint32_t item = pair_id; item < n_items && ok && !__any_sync(0xffffffffu, *abort_flag); item += n_pairs, n++) {
+                const Tile t = tile_of(a, item, ntt);
+                const uint32_t idesc = umma_idesc_bf16(256, cols(t)), acc = n & 1, d = tmem + acc * NT;
+                if (!__all_sync(0xffffffffu, mbar_wait_timed_cluster(bar_acce + 8 * acc, ((n >> 1) & 1) ^ 1, abort_flag))) break;
+                for (uint32_t k = 0; k < ksteps; k++, it++) {
+                    const uint32_t s = it % NS, ph = (it / NS) & 1;
+                    if (!(ok = __all_sync(0xffffffffu, mbar_wait_timed_cluster(bar_full + 8 * s, ph, abort_flag)))) break;
+                    tc_fence_after_sync();
+                    if (elect_one()) {
+                        const uint64_t da = umma_desc_sw128(base + s * kPairStage), db = umma_desc_sw128(base + s * kPairStage + kABytes);
+#pragma unroll
+                        for (uint32_t k4 = 0; k4 < 4; k4++) umma_bf16_pair(d, da + 2 * k4, db + 2 * k4, idesc, (k | k4) != 0);
+                        umma_commit_pair(bar_empty + 8 * s, 3);
+                        if (k + 1 == ksteps) umma_commit_pair(bar_accf + 8 * acc, 3);
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+    } else {
+        const uint32_t quarter = warp & 3;
+        uint32_t n = 0;
+        for (uint32_t item = pair_id; item < n_items; item += n_pairs, n++) {
+            const Tile t = tile_of(a, item, ntt);
+            const uint32_t acc = n & 1;
+            if (!__all_sync(0xffffffffu, mbar_wait_timed(bar_accf + 8 * acc, (n >> 1) & 1, abort_flag))) break;
+            tc_fence_after_sync();
+            drain<EPI>(a, t, tmem + ((quarter * 32) << 16) + acc * NT, t.rb * 256 + rank * kRowsTile + quarter * 32 + lane, lane);
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) {
+                if (rank == 0) mbar_arrive(bar_acce + 8 * acc);
+                else mbar_arrive_cluster(leader_acce + 8 * acc);
+            }
+        }
+    }
+    __syncwarp();
+    tc_fence_before_sync();
+    cluster_sync();
+    if (warp == 1) {
+        tc_fence_after_sync();
+        tmem_dealloc_pair(tmem, 2 * NT);
     }
     if (tid == 0 && *abort_flag && a.status) atomicExch(a.status, 2);
 }
@@ -353,6 +474,32 @@ static int32_t launch_tc(runit_ctx* ctx, const char* name, const GemmDesc& d, Ar
     return runit_after_launch(ctx, name);
 }
 
+template <int EPI>
+static int32_t launch_pair(runit_ctx* ctx, const char* name, const GemmDesc& d, Args a, uint32_t items) {
+    static bool attr_set[64] = {false};
+    if (ctx->device >= 64 || !attr_set[ctx->device]) {
+        RUNIT_CUDA_TRY(ctx, cudaFuncSetAttribute(gemm_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
+        if (ctx->device < 64) attr_set[ctx->device] = true;
+    }
+    CUtensorMap map_w, map_x;
+    int32_t st = runit_get_tmap(ctx, d.w, (uint64_t)d.n_experts * d.rows, (uint64_t)d.ldw * 2, kRowsTile, 128, &map_w, 1);
+    if (st != RUNIT_OK) return st;
+    if ((st = runit_get_tmap(ctx, d.x, d.x_rows, (uint64_t)d.ldx * 2, 128, 128, &map_x, 1)) != RUNIT_OK) return st;
+    const uint32_t pairs = items < (uint32_t)ctx->sm_count / 2 ? items : (uint32_t)ctx->sm_count / 2;
+    gemm_pair_kernel<EPI><<<2 * pairs, kThreads, kPairSmem, ctx->stream>>>(map_w, map_x, a);
+    return runit_after_launch(ctx, name);
+}
+
+static int32_t dispatch_pair(runit_ctx* ctx, const char* name, const GemmDesc& d, const Args& a, uint32_t items) {
+    switch (d.epi) {
+        case EPI_F32: return launch_pair<EPI_F32>(ctx, name, d, a, items);
+        case EPI_ADD: return launch_pair<EPI_ADD>(ctx, name, d, a, items);
+        case EPI_CAST: return launch_pair<EPI_CAST>(ctx, name, d, a, items);
+        case EPI_SILU_GLU: return launch_pair<EPI_SILU_GLU>(ctx, name, d, a, items);
+        default: return launch_pair<EPI_RELU2>(ctx, name, d, a, items);
+    }
+}
+
 template <int NT>
 static int32_t dispatch_tc(runit_ctx* ctx, const char* name, const GemmDesc& d, const Args& a, uint32_t items) {
     switch (d.epi) {
@@ -412,6 +559,13 @@ int32_t gemm_bf16(runit_ctx* ctx, const char* name, const GemmDesc& d, bool exac
     a.tile_tok = grouped ? d.tile_tok : gm::dense_tile_tok(ctx, a.nb, d.T);
     const uint64_t items64 = (uint64_t)a.nb * (grouped ? d.max_tiles : (d.T + a.tile_tok - 1) / a.tile_tok);
     const uint32_t items = items64 < 0x7fffffffull ? (uint32_t)items64 : 0x7fffffffu;
+    // pairs where the tiles take several waves or K is long: the cluster's launch and meeting cost a single wave of short ones 1.3 us (512 tokens x
+    // 8192 x 1024: 19.3 us without, 20.6 with; 2048 x 2048 x 4096 43.3 and 41.1, 2048 x 8192 x 2048 69.8 and 65)
+    if (a.tile_tok == 256 && d.rows > gm::kRowsTile && (items > (uint32_t)ctx->sm_count || d.K >= 2048)) {
+        a.nb = (d.rows + 255) / 256;
+        const uint64_t n = (uint64_t)a.nb * (grouped ? d.max_tiles : (d.T + 255) / 256);
+        return gm::dispatch_pair(ctx, name, d, a, n < 0x7fffffffull ? (uint32_t)n : 0x7fffffffu);
+    }
     if (a.tile_tok == 256) return gm::dispatch_tc<256>(ctx, name, d, a, items);
     if (a.tile_tok == 128) return gm::dispatch_tc<128>(ctx, name, d, a, items);
     RUNIT_REQUIRE(ctx, a.tile_tok == 64, "%s: token tiles of 64, 128 or 256 only", name);
