@@ -11,13 +11,14 @@
 //   O += P.V      V by TMA as it lies in the cache (hd contiguous: B is MN-major), accumulated in tensor memory.  P, the sum (of the
 //                 unrounded P, f32) and O are relative to the chain's row maximum so far; O is scaled by the row's own threads when that has risen,
 //                 ahead of P.  The next S takes P's columns: its MMAs come behind those that read them.
-// The odd chain starts half a period late, so that the products of one chain run under the exponentials of the other.
+// The chains take their exponentials in turn, so that the products of one run under the exponentials of the other.
 // One CTA per SM: 161 KB (one buffer of K and V a chain; 116 asked for at head dim 64) and all 512 tensor-memory columns.  Query blocks go from the
 // most keys to the fewest.
-// Bound: two dependent chains per SM, about 4500 clocks per pair of blocks, of which the exponentials are 2048 (16 a clock) and the products
-// 2048.  Measured, 2048 queries x 16 heads x 128: 102 us (mma.sync, 64 queries of 4 warps), 41 with one chain and two buffers of S, 37 with two chains in
-// step, 34.5 as it is (498 TFLOP/s of useful products; 26 at head dim 64, before 31); 1024 queries 17.8 -> 16.8 us, 2000 behind 1000 cached ones 61 -> 52, 64
-// behind 1900 27.6 -> 25.2, a single block (launch and hand-overs) 6.7 -> 6.9.  O scaled between the exponentials instead: 35.7 (register spills).
+// Bound: two dependent chains per SM: a block's maximum, scaling of O, exponentials (1024 clocks at 16 a clock), hand-over and products (1024).
+// Measured, 2048 queries x 16 heads x 128: 102 us (mma.sync, 64 queries of 4 warps), 41 with one chain and two buffers of S, 37 with two chains in
+// step, 34.5 with the odd one started half a period late (they drift into step again), 32.8 in turn (524 TFLOP/s of useful products; 24.6 at head dim 64, 29 with one
+// chain); 1024 queries 17.8 -> 15.3 us, 2000 behind 1000 cached ones 62 -> 48, 64 behind 1900 27.6 -> 22.5, a single block 6.8 -> 6.5.  O scaled between the
+// exponentials instead: slower (register spills).
 // The error against 64 bits is the bf16 output's, 1.677e-3, as it was.  A reference that follows the maximum only when that has risen by
 // 2^8 saves the scaling of O but rounds the largest weights, which then are not 1: 1.678e-3, and up to twice the error before bf16.
 // Rows of the tensor maps end at start + T, so that what the cache holds behind the data (NaN included) reads as zeros.
@@ -34,7 +35,7 @@ namespace atc {
 
 constexpr int kRows = 128, kKeys = 128;
 constexpr uint32_t kSoftWarps = 16, kThreads = 32 * (kSoftWarps + 2);
-constexpr int kBars = 6;                           // of a chain: k_full, v_full, s_full, p_full, o_full, done
+constexpr int kBars = 7;                           // of a chain: k_full, v_full, s_full, p_full, o_full, done, turn
 constexpr uint32_t kCols = 512;                    // tensor memory: S | P of the chains in columns 0..127 and 128..255, their O from 256 and 384
 constexpr uint32_t kOnePerSm = 116 * 1024;         // shared memory that only one CTA of an SM can have
 
@@ -149,7 +150,7 @@ template <int HD>
 __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mv, const Args a) {
     using S = Shape<HD>;
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t bars[2 * kBars + 1];
+    __shared__ __align__(8) uint64_t bars[2 * kBars];
     __shared__ uint32_t tmem_holder;
     __shared__ volatile int abort_flag;
     __shared__ float part[2][2][2][kRows];         // [block parity][chain][half]: row maximum of a half
@@ -161,10 +162,11 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const __grid_
     // this chain's K, V and barriers; k_full, v_full, s_full, p_full, o_full: one phase per block of the chain; done: one
     const uint32_t kb = base + S::kTile + chain * 2 * S::kTile, vb = kb + S::kTile;
     const uint32_t bar0 = smem_u32(&bars[chain * kBars]);
-    const uint32_t k_full = bar0, v_full = bar0 + 8, s_full = bar0 + 16, p_full = bar0 + 24, o_full = bar0 + 32, done = bar0 + 40, go = smem_u32(&bars[2 * kBars]);
+    const uint32_t k_full = bar0, v_full = bar0 + 8, s_full = bar0 + 16, p_full = bar0 + 24, o_full = bar0 + 32, done = bar0 + 40, turn = bar0 + 48;
+    const uint32_t other_turn = smem_u32(&bars[(chain ^ 1) * kBars + 6]);
     const uint32_t head = blockIdx.x, q0 = (gridDim.y - 1 - blockIdx.y) * kRows;
     auto init_bars = [&]() {
-        for (int i = 0; i <= 2 * kBars; i++) mbar_init(smem_u32(&bars[i]), i < 2 * kBars && i % kBars == 3 ? 256 : 1);
+        for (int i = 0; i < 2 * kBars; i++) mbar_init(smem_u32(&bars[i]), i % kBars == 3 ? 256 : i % kBars == 6 ? 8 : 1);
         fence_mbar_init();
     };
     if (tid == 0) {
@@ -222,17 +224,17 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const __grid_
             };
             auto load_k = [&](uint32_t j) { load(&mk, kb, k_full, j); n_k++; };
             auto load_v = [&](uint32_t j) { load(&mv, vb, v_full, j); n_v++; };
-            auto scores = [&](bool report) {       // S of the block whose K has been waited for; behind the product that reads P from these columns
+            auto scores = [&]() {                  // S of the block whose K has been waited for; behind the product that reads P from these columns
                 if (elect_one()) {
 #pragma unroll
                     for (int s = 0; s < HD / 16; s++) {
                         const uint32_t off = (s >> 2) * S::kPanel + (s & 3) * 32;
                         umma_bf16(s_cols, umma_desc_sw128(qs + off), umma_desc_sw128(kb + off), idesc_f16(kRows, kKeys, 0), s > 0);
                     }
-                    if (report) umma_commit(s_full);
+                    umma_commit(s_full);
                 }
                 __syncwarp();
-                n_s += report;
+                n_s++;
             };
             if (mine > 0) {
                 load_k(0);
@@ -240,15 +242,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const __grid_
                 ok = mbar_wait_timed(k_full, 0, &abort_flag);
                 if (__all_sync(0xffffffffu, ok)) {
                     tc_fence_after_sync();
-                    // half a period behind the other chain, whose P is done: the products of one run under the exponentials of the other
-                    const bool hold = chain == 1 && mine > 1;
-                    scores(!hold);
-                    if (hold) {
-                        ok = __all_sync(0xffffffffu, mbar_wait_timed(go, 0, &abort_flag));
-                        if (elect_one()) umma_commit(s_full);
-                        __syncwarp();
-                        n_s++;
-                    }
+                    scores();
                 } else ok = false;
             }
             for (uint32_t j = 0; j < mine && ok; j++) {
@@ -261,7 +255,6 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const __grid_
                 if (!(ok = __all_sync(0xffffffffu, ok))) break;
                 tc_fence_after_sync();
                 if (elect_one()) {
-                    if (chain == 0 && j == 0) mbar_arrive(go);
                     if (!careful || 2 * j + chain < first_masked) {
 #pragma unroll
                         for (int s = 0; s < kKeys / 16; s++)
@@ -278,7 +271,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const __grid_
                 ok = mbar_wait_timed(k_full, ph ^ 1, &abort_flag);
                 if (!(ok = __all_sync(0xffffffffu, ok))) break;
                 tc_fence_after_sync();
-                scores(true);
+                scores();
                 ok = mbar_wait_timed(o_full, ph, &abort_flag);
                 if (!(ok = __all_sync(0xffffffffu, ok))) break;
                 load_v(j + 1);
@@ -339,6 +332,10 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const __grid_
                         tmem_st16(my_o + 16 * c, o);
                     }
                 }
+                // The chains take their exponentials in turn (block j of the odd one behind block j of the even one, and that behind block j - 1 of the
+                // odd one): the products of one run under the exponentials of the other.  Left alone they fall into step.
+                if (ok && (chain == 1 || j > 0)) ok = mbar_wait_timed(turn, (chain == 1 ? j : j - 1) & 1, &abort_flag);
+                __syncwarp();
 #pragma unroll
                 for (int c = 0; c < 2; c++) {
                     uint32_t r[32], p[16];
@@ -361,6 +358,8 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const __grid_
                     tmem_st16(my_s + 16 * c, p);       // behind what this thread has read: 16 columns for 32 keys
                 }
                 l += sum2(both);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(other_turn);
                 tmem_st_wait();
                 tc_fence_before_sync();
                 mbar_arrive(p_full);
@@ -418,7 +417,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const __grid_
         tc_fence_before_sync();
         if (!__syncthreads_or(again) || careful || abort_flag) break;
         if (tid == 0) {
-            for (int i = 0; i <= 2 * kBars; i++) mbar_inval(smem_u32(&bars[i]));
+            for (int i = 0; i < 2 * kBars; i++) mbar_inval(smem_u32(&bars[i]));
             init_bars();
         }
         __syncthreads();
