@@ -30,15 +30,8 @@ __global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x,
     grid_launch_dependents();      // the product may start requesting its weights; it waits for this grid before it reads anything else
     grid_dependency_wait();
     float v[8];
-#pragma unroll
-    for (int b = 0; b < 8; b++) v[b] = n < batch ? x[(size_t)n * k + (size_t)u * 256 + b * 32 + lane] : 0.f;
-    const float scale = tcr::split_column<kKind>(
-        v, 2 * n, 2 * n + 1, 0, lane,
-        [&](uint32_t panel, uint32_t hi_off, __half hi, uint32_t lo_off, __half lo) {
-            *reinterpret_cast<__half*>(out + panel * 2048 + hi_off) = hi;
-            *reinterpret_cast<__half*>(out + panel * 2048 + lo_off) = lo;
-        },
-        [](uint32_t, __half) {});
+    tcr::load8(x + (size_t)n * k + (size_t)u * 256 + 8 * lane, n < batch, v);
+    const float scale = tcr::split_column<kKind>(v, lane, out, 2 * n, out, 2 * n + 1, 2048, nullptr, 0);
     if (lane == 0) scales[u * 8 + n] = scale;
     __syncthreads();
     uint4* dst = reinterpret_cast<uint4*>(images + (size_t)u * C::kBStage);

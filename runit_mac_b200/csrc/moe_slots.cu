@@ -96,15 +96,8 @@ __global__ void __launch_bounds__(32 * Shape<COLS>::kTile) split_slots_kernel(co
     if (tile >= (uint32_t)table[1]) return;
     const int32_t slot = order[tile * S::kTile + n];
     float v[8];
-#pragma unroll
-    for (int b = 0; b < 8; b++) v[b] = slot >= 0 ? x[(size_t)((uint32_t)slot / xdiv) * k + u * 256 + b * 32 + lane] : 0.f;
-    const float scale = tcr::split_column<S::kKind>(
-        v, n, COLS == 8 ? 8 + n : n, n, lane,
-        [&](uint32_t panel, uint32_t ho, __half hi, uint32_t lo_off, __half lo) {
-            *reinterpret_cast<__half*>(out + panel * S::kPanel + ho) = hi;
-            *reinterpret_cast<__half*>(out + (COLS == 8 ? panel : 4 + panel) * S::kPanel + lo_off) = lo;
-        },
-        [&](uint32_t off, __half s) { *reinterpret_cast<__half*>(out + kSums + off) = s; });
+    tcr::load8(x + (size_t)((uint32_t)(slot < 0 ? 0 : slot) / xdiv) * k + u * 256 + 8 * lane, slot >= 0, v);
+    const float scale = tcr::split_column<S::kKind>(v, lane, out, n, out + (COLS == 8 ? 0 : 4 * S::kPanel), COLS == 8 ? 8 + n : n, S::kPanel, out + kSums, n);
     const uint32_t at = (uint32_t)place[tile], first = at >> 3, nt = at & 7, mine = tile - first;
     const size_t unit = (size_t)first * units + (size_t)u * nt;        // in tiles
     if (lane == 0) scales[unit * S::kTile + mine * S::kTile + n] = scale;

@@ -35,7 +35,7 @@ namespace tcr {
 //   Q4K_48  up to 48 columns in multiples of 16, the halves in turn into the same sums
 //   Q8_0_8  up to 8 columns, both halves of a column side by side; a sum for each of the eight blocks, because their scales are f16 values that
 //           no integer factor expresses
-// Image of 256 activations of N columns (128-byte swizzled rows of 64 elements, in the order of b_offset):
+// Image of 256 activations of N columns (128-byte swizzled rows of 64 elements, in the order of split_column):
 //   Q4K_8   4 panels of 16 rows (8 hi, 8 lo), then a panel whose row n holds the block sums of column n
 //   Q4K_48  4 panels of N rows of hi, 4 of lo, one of block sums
 //   else    4 panels of 16 rows (hi and lo of a column in neighbouring rows)
@@ -87,26 +87,35 @@ __device__ __forceinline__ __half2 scale_pair(uint32_t p, uint32_t j) {
     return __hsub2(as_half2(__byte_perm(p, 0x64646464u, 0x4040u + 0x0101u * j)), as_half2(0x64006400u));
 }
 
-// An activation's place: element i (0..3) of weight word w of a 64-element chunk, half 1 = high nibbles.  A word's eight elements are
-// consecutive in K: low 0, 2, 1, 3, high 0, 2, 1, 3.
-__device__ __forceinline__ uint32_t b_offset(uint32_t row, uint32_t w, uint32_t half, uint32_t i) {
-    return row * 128 + ((w ^ (row & 7)) << 4) + (2 * (2 * half + (i & 1)) + (i >> 1)) * 2;
-}
-// The same for Q8_0, element e of block b of a pair: in order.
-__device__ __forceinline__ uint32_t b_offset_block(uint32_t row, uint32_t b, uint32_t e) { return row * 128 + (((4 * b + (e >> 3)) ^ (row & 7)) << 4) + (e & 7) * 2; }
-// 16 bytes c of a row of the block sums' panel: 0 = the eight blocks' hi halves, 1 = lo
-__device__ __forceinline__ uint32_t sums_offset(uint32_t row, uint32_t c) { return row * 128 + ((c ^ (row & 7)) << 4); }
+// Where activations lie in a row of a 128-byte swizzled panel of 64 K.  Q4_K: a weight word's eight elements are consecutive in K, low nibbles
+// 0, 2, 1, 3, high nibbles 0, 2, 1, 3; 8 bytes per word w and half.  Q8_0: in order; 16 bytes per 8 elements.
+__device__ __forceinline__ uint32_t chunk_offset(uint32_t row, uint32_t chunk) { return row * 128 + ((chunk ^ (row & 7)) << 4); }
 
-// One column's 256 activations by a warp: lane has element `lane` of each of the eight blocks in v.  Writes both halves and, for Q4_K, the block
-// sums through `put(panel, hi offset, hi, lo offset, lo)` and `sum(offset, value)`, and returns the column's scale.
-template <Kind K, class Put, class Sum>
-__device__ __forceinline__ float split_column(const float (&v)[8], uint32_t hi_row, uint32_t lo_row, uint32_t sum_row, uint32_t lane, Put put, Sum sum) {
+// Eight consecutive activations by a lane: element 8 * lane and on of a column's 256.
+__device__ __forceinline__ void load8(const float* x, bool live, float (&v)[8]) {
+    if (!live) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = 0.f;
+    } else if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+        const float4 a = *reinterpret_cast<const float4*>(x), b = *reinterpret_cast<const float4*>(x + 4);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = x[i];
+    }
+}
+// One column's 256 activations by a warp (load8) into the panels of an image: panels of hi from `hi` on, of lo from `lo`, `panel` bytes apart, and for
+// Q4_K the block sums' panel `sums`, in the rows given.  Returns the column's scale.
+template <Kind K>
+__device__ __forceinline__ float split_column(const float (&v)[8], uint32_t lane, uint8_t* hi, uint32_t hi_row, uint8_t* lo, uint32_t lo_row, uint32_t panel,
+                                              uint8_t* sums, uint32_t sum_row) {
     float amax = 0.f;
     bool bad = false;
 #pragma unroll
-    for (int b = 0; b < 8; b++) {
-        amax = fmaxf(amax, fabsf(v[b]));
-        bad |= !(fabsf(v[b]) <= 3.4028235e38f);
+    for (int i = 0; i < 8; i++) {
+        amax = fmaxf(amax, fabsf(v[i]));
+        bad |= !(fabsf(v[i]) <= 3.4028235e38f);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
@@ -116,25 +125,40 @@ __device__ __forceinline__ float split_column(const float (&v)[8], uint32_t hi_r
     int e = (int)((__float_as_uint(amax) >> 23) & 255u) - 127 - 14;
     e = e < -116 ? -116 : e;
     const float inv = __uint_as_float((uint32_t)(127 - e) << 23);
+    const uint32_t block = lane >> 2, half = block & 1;
+    __half h[8], l[8];
+    float sum = 0.f;
 #pragma unroll
-    for (int b = 0; b < 8; b++) {
-        const float w = bad ? 0.f : v[b] * inv;
-        const float ws = K != Q8_0_8 && (b & 1) ? w * 0.0625f : w;       // meets 16 q
-        const __half hi = __float2half_rn(ws), lo = __float2half_rn(ws - __half2float(hi));
-        if (Cfg<K>::kBlocks) {
-            put(b >> 1, b_offset_block(hi_row, b & 1, lane), hi, b_offset_block(lo_row, b & 1, lane), lo);
-            continue;
+    for (int i = 0; i < 8; i++) {
+        const float w = bad ? 0.f : v[i] * inv;
+        const float ws = K != Q8_0_8 && half ? w * 0.0625f : w;       // meets 16 q
+        h[i] = __float2half_rn(ws);
+        l[i] = __float2half_rn(ws - __half2float(h[i]));
+        sum += w;
+    }
+    hi += (block >> 1) * panel;
+    lo += (block >> 1) * panel;
+    if constexpr (K == Q8_0_8) {
+        const uint32_t c = 4 * half + (lane & 3);
+        *reinterpret_cast<uint4*>(hi + chunk_offset(hi_row, c)) = *reinterpret_cast<const uint4*>(h);
+        *reinterpret_cast<uint4*>(lo + chunk_offset(lo_row, c)) = *reinterpret_cast<const uint4*>(l);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const uint32_t w = 2 * (lane & 3) + i;
+            const __half2 ph[2] = {__halves2half2(h[4 * i], h[4 * i + 2]), __halves2half2(h[4 * i + 1], h[4 * i + 3])};
+            const __half2 pl[2] = {__halves2half2(l[4 * i], l[4 * i + 2]), __halves2half2(l[4 * i + 1], l[4 * i + 3])};
+            *reinterpret_cast<uint2*>(hi + chunk_offset(hi_row, w) + 8 * half) = *reinterpret_cast<const uint2*>(ph);
+            *reinterpret_cast<uint2*>(lo + chunk_offset(lo_row, w) + 8 * half) = *reinterpret_cast<const uint2*>(pl);
         }
-        put(b >> 1, b_offset(hi_row, lane >> 2, b & 1, lane & 3), hi, b_offset(lo_row, lane >> 2, b & 1, lane & 3), lo);
-        float s = w;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) {
-            s *= 0.03125f;
-            const uint32_t si = (b >> 1) + 4 * (b & 1);            // the order of the unpacked minimums
-            const __half sh = __float2half_rn(s), sl = __float2half_rn(s - __half2float(sh));
-            sum(sums_offset(sum_row, 0) + 2 * si, sh);
-            sum(sums_offset(sum_row, 1) + 2 * si, sl);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        if ((lane & 3) == 0) {
+            sum *= 0.03125f;
+            const uint32_t si = (block >> 1) + 4 * half;              // the order of the unpacked minimums
+            const __half sh = __float2half_rn(sum), sl = __float2half_rn(sum - __half2float(sh));
+            *reinterpret_cast<__half*>(sums + chunk_offset(sum_row, 0) + 2 * si) = sh;
+            *reinterpret_cast<__half*>(sums + chunk_offset(sum_row, 1) + 2 * si) = sl;
         }
     }
     return bad ? __uint_as_float(0x7FC00000u) : __uint_as_float((uint32_t)(e + 127) << 23);
@@ -160,7 +184,7 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
                  ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 
-// Half H (128 weights) of a row, as f16 pairs in the order of b_offset, into 64 columns of tensor memory at `at`, 16 at a time.
+// Half H (128 weights) of a row, as f16 pairs in the order of split_column, into 64 columns of tensor memory at `at`, 16 at a time.
 template <int H> __device__ __forceinline__ void unpack_q4k(const uint8_t* raw, const Q4KScales& sc, uint32_t at) {
 #pragma unroll
     for (int jj = 0; jj < 2; jj++) {
