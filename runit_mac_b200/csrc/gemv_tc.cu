@@ -6,6 +6,12 @@
 // CTA takes a stretch of consecutive items: the tiles that it has whole it stores itself, those that it shares with its neighbours are filed share by share and
 // added by the warp that files last.
 //
+// The same kernel takes one activation row of Q6_K (gemv_kquant.cu has the line).  Its rows start on even bytes, which no tiled load takes: rows
+// eight apart start alike modulo 16, so a step comes as eight boxes of 16 rows, each from the last multiple of 16 before its unit.  152064 x 3584:
+// 127 -> 90 us (4.9 TB/s).  Bound now by the unpacking warps' instructions and the copies together (without the arithmetic 79, with an eighth of
+// the copies 78).  Copying words with cp.async instead, 322; six teams 112, unpacking ahead of the wait for the place 96.
+// Error against 64 bits 1.0e-7 (before 2.8e-7).
+//
 // Bound: the unpacking warps, about 1000 clocks per 128 x 256 weights and SM (2.1 TB/s), and some 4 us between dependent calls (the pre-pass and
 // its hand-over).  The packed f32 kernel that it replaces multiplies every weight 8 times on the CUDA cores.  Decoding steps, us, f32 -> now: width 3584, two layers
 // and a head of 30000 rows, 2 / 4 / 8 sequences 294 / 421 / 915 -> 173 / 175 / 183; width 2048, four layers, 274 / 365 / 693 -> 208 / 209 / 221.
@@ -23,16 +29,25 @@ constexpr tcr::Kind kKind = tcr::Q8_0_8;
 using C = tcr::Cfg<kKind>;
 constexpr uint32_t kMaxShares = 10, kMaxCtas = 160, kTickets = kMaxCtas * 8, kPartBytes = 4096;      // a share's sums of a tile
 
-// One CTA per 256 activations, one warp per activation row (rows behind the batch are zeros).
+// One CTA per 256 activations, one warp per activation row (rows behind the batch are zeros).  Q6_K: one activation row, block b of it in rows
+// 2 b and 2 b + 1 of the image.
+template <tcr::Kind K>
 __global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x, uint8_t* __restrict__ images, float* __restrict__ scales, uint32_t k, uint32_t batch) {
     __shared__ __align__(16) uint8_t out[C::kBStage];
     const uint32_t u = blockIdx.x, n = threadIdx.x >> 5, lane = threadIdx.x & 31;
     grid_launch_dependents();      // the product may start requesting its weights; it waits for this grid before it reads anything else
     grid_dependency_wait();
     float v[8];
+    if (K == tcr::Q6K_8) {
+        for (uint32_t i = threadIdx.x; i < C::kBStage / 16; i += 256) reinterpret_cast<uint4*>(out)[i] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
+    }
     tcr::load8(x + (size_t)n * k + (size_t)u * 256 + 8 * lane, n < batch, v);
-    const float scale = tcr::split_column<kKind>(v, lane, out, 2 * n, out, 2 * n + 1, 2048, nullptr, 0);
-    if (lane == 0) scales[u * 8 + n] = scale;
+    if (K != tcr::Q6K_8 || n == 0) {
+        const uint32_t at = K == tcr::Q6K_8 ? lane >> 2 : n;
+        const float scale = tcr::split_column<K>(v, lane, out, 2 * at, out, 2 * at + 1, 2048, nullptr, 0);
+        if (lane == 0) scales[u * 8 + n] = scale;
+    }
     __syncthreads();
     uint4* dst = reinterpret_cast<uint4*>(images + (size_t)u * C::kBStage);
     for (uint32_t i = threadIdx.x; i < C::kBStage / 16; i += 256) dst[i] = reinterpret_cast<const uint4*>(out)[i];
@@ -55,7 +70,8 @@ struct Maps {
     CUtensorMap m[3];
 };
 
-struct Policy {
+template <tcr::Kind K> struct Policy {
+    using C = tcr::Cfg<K>;
     static constexpr int kAcc = C::kAcc;
     const Args& a;
     const Maps& maps;
@@ -92,11 +108,11 @@ struct Policy {
     }
     __device__ __forceinline__ void store(uint32_t tile, uint32_t warp, uint32_t lane) const {
         const int s = segment(tile);
-        const uint32_t row = (tile - a.tile0[s]) * 128 + (warp & 3) * 32 + lane, m = a.m[s];
+        const uint32_t t = (warp & 3) * 32 + lane, row = (tile - a.tile0[s]) * 128 + (K == tcr::Q6K_8 ? tcr::q6k_row(t) : t), m = a.m[s];
         if (row >= m) return;
 #pragma unroll
         for (uint32_t j = 0; j < kAcc; j++) {
-            const uint32_t users = few() ? 2 : 4, c = users * (warp >> 2) + j;
+            const uint32_t users = kAcc == 1 ? 1 : few() ? 2 : 4, c = users * (warp >> 2) + j;
             if (j >= users) break;
             if (c < a.batch) {
                 const size_t o = (size_t)c * m + row;
@@ -142,15 +158,26 @@ struct Policy {
     }
 };
 
-__global__ void __launch_bounds__(C::kThreads, 1) gemv_tc_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Args a) {
+template <tcr::Kind K>
+__global__ void __launch_bounds__(tcr::Cfg<K>::kThreads, 1) gemv_tc_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Args a) {
+    using C = tcr::Cfg<K>;
     extern __shared__ uint8_t smem_raw[];
-    tcr::Block<kKind, 1> blk(smem_raw);
-    Policy p(a, maps);
+    tcr::Block<K, 1> blk(smem_raw);
+    Policy<K> p(a, maps);
     if (blk.warp == C::kCopyW) {
         // raw blocks: the first steps' ahead of the dependency wait; the columns' scales behind it
         uint32_t s = 0, early = 0;
         auto load = [&](const tcr::Run& r, uint32_t u, uint32_t step) {
-            if (elect_one()) {
+            if (K == tcr::Q6K_8) {
+                const uint32_t row_bytes = a.units * 210;
+                if (blk.lane == 0) {
+                    *reinterpret_cast<volatile uint32_t*>(blk.base_p + C::kOffAt + 4 * (step % C::kW)) = (u * 210 & 15) | (row_bytes & 15) << 8;
+                    mbar_expect_tx(blk.raw_bar(step), C::kWBytes + r.n * 4);
+                }
+                __syncwarp();
+                if (blk.lane < 8)
+                    tma_load_2d(blk.raw(step) + blk.lane * (C::kWBytes / 8), r.map[0], (int32_t)((blk.lane * row_bytes + u * 210) & ~15u), r.row[0] / 8, blk.raw_bar(step));
+            } else if (elect_one()) {
                 mbar_expect_tx(blk.raw_bar(step), C::kWBytes + r.n * 4);
                 tma_load_2d(blk.raw(step), r.map[0], (int32_t)(u * 136), r.row[0], blk.raw_bar(step));       // elements of two bytes
             }
@@ -196,6 +223,50 @@ __global__ void __launch_bounds__(C::kThreads, 1) gemv_tc_kernel(const __grid_co
     blk.leave(a.status);
 }
 
+// Shares, grid and the context's places; the pre-pass and the product as dependent launches.
+template <tcr::Kind K> static int32_t launch(runit_ctx* ctx, const char* name, Args& a, const Maps& maps, const float* x, uint32_t k, uint32_t batch) {
+    static bool configured[64] = {false};
+    if (ctx->device >= 64 || !configured[ctx->device]) {
+        RUNIT_CUDA_TRY(ctx, cudaFuncSetAttribute(gemv_tc_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, tcr::Cfg<K>::kSmem));
+        if (ctx->device < 64) configured[ctx->device] = true;
+    }
+    // two units per share, ten shares at most: enough items for every SM at the sizes where a tile per CTA would leave most of them idle
+    a.shares = (a.units + 1) / 2 < kMaxShares ? (a.units + 1) / 2 : kMaxShares;
+    a.items *= a.shares;
+    a.inverse = a.shares > 1 ? (uint32_t)((0x100000000ull + a.shares - 1) / a.shares) : 0;
+    uint32_t grid = (uint32_t)ctx->sm_count;
+    grid = grid < kMaxCtas ? grid : kMaxCtas;
+    grid = grid < a.items ? grid : a.items;
+    a.images = (const uint8_t*)ctx->d_xq;
+    a.scales = (const float*)(a.images + (size_t)a.units * C::kBStage);
+    a.tickets = (uint32_t*)ctx->d_tc;
+    a.part = (float*)((uint8_t*)ctx->d_tc + kTickets * 4);
+    a.status = ctx->d_status;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.stream = ctx->stream;
+    cfg.attrs = attr;
+    // The product requests weights as soon as the pre-pass lets it start.  Where a kernel before the pre-pass may have written them, the
+    // pre-pass is an ordinary launch, which starts when all of it can be seen.
+    cfg.numAttrs = !ctx->foreign_kernels && !ctx->weights_written && ctx->tune.pdl != 0 ? 1 : 0;
+    ctx->weights_written = false;
+    cfg.gridDim = dim3(a.units);
+    cfg.blockDim = dim3(256);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, split_kernel<K>, x, (uint8_t*)ctx->d_xq, (float*)a.scales, k, batch);
+    if (e != cudaSuccess) return runit_fail(ctx, RUNIT_ERR_LAUNCH, "launch of %s (split of the activations) failed: %s", name, cudaGetErrorString(e));
+    const int32_t st = runit_after_launch(ctx, "gemv_split_x");
+    if (st != RUNIT_OK) return st;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(tcr::Cfg<K>::kThreads);
+    cfg.dynamicSmemBytes = tcr::Cfg<K>::kSmem;
+    e = cudaLaunchKernelEx(&cfg, gemv_tc_kernel<K>, maps, a);
+    if (e != cudaSuccess) return runit_fail(ctx, RUNIT_ERR_LAUNCH, "launch of %s (tcgen05) failed: %s", name, cudaGetErrorString(e));
+    return runit_after_launch(ctx, name);
+}
+
 }  // namespace tcg
 
 // Bytes that the context keeps for this path: tickets, then partial sums.
@@ -230,46 +301,28 @@ int32_t gemv_tc_multi(runit_ctx* ctx, uint32_t n_mats, const void* const* w, con
             maps.m[i] = maps.m[0];
         }
     }
-    // two units per share, ten shares at most: enough items for every SM at the sizes where a tile per CTA would leave most of them idle
-    a.shares = (a.units + 1) / 2 < kMaxShares ? (a.units + 1) / 2 : kMaxShares;
-    a.items = (uint32_t)(tiles * a.shares);         // at most 3 * 2^25 tiles
-    a.inverse = a.shares > 1 ? (uint32_t)((0x100000000ull + a.shares - 1) / a.shares) : 0;
-    uint32_t grid = (uint32_t)ctx->sm_count;
-    grid = grid < kMaxCtas ? grid : kMaxCtas;
-    grid = grid < a.items ? grid : a.items;
-    a.images = (const uint8_t*)ctx->d_xq;
-    a.scales = (const float*)(a.images + (size_t)a.units * C::kBStage);
-    a.tickets = (uint32_t*)ctx->d_tc;
-    a.part = (float*)((uint8_t*)ctx->d_tc + kTickets * 4);
-    a.status = ctx->d_status;
-    static bool configured[64] = {false};
-    if (ctx->device >= 64 || !configured[ctx->device]) {
-        RUNIT_CUDA_TRY(ctx, cudaFuncSetAttribute(gemv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem));
-        if (ctx->device < 64) configured[ctx->device] = true;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.stream = ctx->stream;
-    cfg.attrs = attr;
-    // The product requests weights as soon as the pre-pass lets it start.  Where a kernel before the pre-pass may have written them, the
-    // pre-pass is an ordinary launch, which starts when all of it can be seen.
-    cfg.numAttrs = !ctx->foreign_kernels && !ctx->weights_written && ctx->tune.pdl != 0 ? 1 : 0;
-    ctx->weights_written = false;
-    cfg.gridDim = dim3(a.units);
-    cfg.blockDim = dim3(256);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, split_kernel, x, (uint8_t*)ctx->d_xq, (float*)a.scales, k, batch);
-    if (e != cudaSuccess) return runit_fail(ctx, RUNIT_ERR_LAUNCH, "launch of gemv_batched (split of the activations) failed: %s", cudaGetErrorString(e));
-    const int32_t st = runit_after_launch(ctx, "gemv_batched_split_x");
+    a.items = (uint32_t)tiles;         // at most 3 * 2^25, times ten shares
+    return launch<kKind>(ctx, "gemv_batched_tc", a, maps, x, k, batch);
+}
+
+// Q6_K, one activation row.  w 16-byte aligned; whole groups of eight rows, which the boxes are made of.
+bool gemv_q6k_tc_applies(const runit_ctx* ctx, const void* w, uint32_t m, uint32_t k) {
+    return m % 8 == 0 && k % 256 == 0 && runit_aligned(w, 16) && ctx->d_xq && ctx->d_tc && ctx->encode_tiled && (size_t)(k / 256) * (tcg::C::kBStage + 32) <= ctx->xq_bytes;
+}
+int32_t gemv_q6k_tc(runit_ctx* ctx, const char* name, const void* w, const float* x, float* y, const float* res, uint32_t m, uint32_t k) {
+    using namespace tcg;
+    Args a{};
+    Maps maps{};
+    a.units = k / 256;
+    a.batch = 1;
+    a.nseg = 1;
+    a.y[0] = y;
+    a.res[0] = res;
+    a.m[0] = m;
+    a.items = (m + 127) / 128;
+    const int32_t st = runit_get_tmap(ctx, w, m / 8, (uint64_t)a.units * 1680, 16, 240, &maps.m[0]);
     if (st != RUNIT_OK) return st;
-    cfg.numAttrs = 1;
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(C::kThreads);
-    cfg.dynamicSmemBytes = C::kSmem;
-    e = cudaLaunchKernelEx(&cfg, gemv_tc_kernel, maps, a);
-    if (e != cudaSuccess) return runit_fail(ctx, RUNIT_ERR_LAUNCH, "launch of gemv_batched (tcgen05) failed: %s", cudaGetErrorString(e));
-    return runit_after_launch(ctx, "gemv_batched_tc");
+    return launch<tcr::Q6K_8>(ctx, name, a, maps, x, k, 1);
 }
 
 }  // namespace runit

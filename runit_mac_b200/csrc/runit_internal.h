@@ -190,6 +190,9 @@ size_t gemv_tc_bytes();
 bool gemv_tc_applies(const runit_ctx* ctx, int fmt, uint32_t k, uint32_t batch);
 int32_t gemv_tc_multi(runit_ctx* ctx, uint32_t n_mats, const void* const* w, const float* x, float* const* y, const float* const* res, const uint32_t* m,
                       uint32_t k, uint32_t batch);
+// the same for Q6_K and one activation row
+bool gemv_q6k_tc_applies(const runit_ctx* ctx, const void* w, uint32_t m, uint32_t k);
+int32_t gemv_q6k_tc(runit_ctx* ctx, const char* name, const void* w, const float* x, float* y, const float* res, uint32_t m, uint32_t k);
 // gemv.cu: grouped GEMVs over stacked expert matrices (MoE block).  Slot s uses expert slot_expert[s] - expert_lo of the
 // n_experts stacked ones; an id outside that range marks an unused slot.
 int32_t gemv_grouped(runit_ctx* ctx, const char* name, int fmt, const void* w, const void* w2, uint32_t n_experts,

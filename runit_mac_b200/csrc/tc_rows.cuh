@@ -35,31 +35,34 @@ namespace tcr {
 //   Q4K_48  up to 48 columns in multiples of 16, the halves in turn into the same sums
 //   Q8_0_8  up to 8 columns, both halves of a column side by side; a sum for each of the eight blocks, because their scales are f16 values that
 //           no integer factor expresses
+//   Q6K_8   one column; block b of it has columns 2 b (hi) and 2 b + 1 (lo) of one product to itself, with zeros in the others' rows: one
+//           load of sixteen sums and not eight
 // Image of 256 activations of N columns (128-byte swizzled rows of 64 elements, in the order of split_column):
 //   Q4K_8   4 panels of 16 rows (8 hi, 8 lo), then a panel whose row n holds the block sums of column n
 //   Q4K_48  4 panels of N rows of hi, 4 of lo, one of block sums
 //   else    4 panels of 16 rows (hi and lo of a column in neighbouring rows)
-enum Kind { Q4K_8, Q4K_48, Q8_0_8 };
+enum Kind { Q4K_8, Q4K_48, Q8_0_8, Q6K_8 };
 
 template <Kind K> struct Cfg {
-    static constexpr bool kBlocks = K == Q8_0_8;                  // sums per block
+    static constexpr bool kBlocks = K == Q8_0_8 || K == Q6K_8;                  // sums per block
     static constexpr uint32_t kCols = K == Q4K_48 ? 48 : 8;
     // kParts: a step is unpacked in one piece, or in halves (an empty tensor memory holds two steps, not three)
-    static constexpr uint32_t kParts = K == Q4K_48 ? 2 : 1, kTeams = K == Q4K_8 ? 3 : 2, kSumWarps = K == Q4K_48 ? 12 : kBlocks ? 8 : 4;
+    static constexpr uint32_t kParts = K == Q4K_48 || K == Q6K_8 ? 2 : 1, kTeams = K == Q4K_8 ? 3 : K == Q6K_8 ? 4 : 2, kSumWarps = K == Q4K_48 ? 12 : K == Q8_0_8 ? 8 : 4;
     static constexpr uint32_t kSum0 = 4 * kTeams, kMma = kSum0 + kSumWarps, kMmaWarps = K == Q4K_8 ? 3 : 2, kCopyW = kMma + kMmaWarps, kCopyB = kCopyW + 1, kThreads = 32 * (kCopyB + 1);      // warps by role
-    static constexpr uint32_t kUnit = K == Q8_0_8 ? 272 : 144, kWBytes = 128 * kUnit;      // bytes of 256 weights; raw superblocks of a step
+    static constexpr uint32_t kUnit = K == Q8_0_8 ? 272 : K == Q6K_8 ? 240 : 144, kWBytes = 128 * kUnit;      // bytes of 256 weights; raw superblocks of a step
     // rings: raw steps, activations' images, unpacked pieces (kSteps steps) in tensor memory, sums; columns' scales and rows' scales (see the bounds below)
     static constexpr uint32_t kW = K == Q4K_8 ? 6 : 4, kB = K == Q4K_48 ? 2 : 4, kSteps = K == Q4K_8 ? 3 : 2, kA = kSteps * kParts, kD = kSteps;
-    static constexpr uint32_t kXs = K == Q4K_48 ? 8 : 16, kRows = 8, kMins = K == Q4K_8 ? 3 : 2;
+    static constexpr uint32_t kXs = K == Q4K_48 ? 8 : 16, kRows = 8, kMins = kSteps;
     static constexpr uint32_t kBRow = K == Q4K_8 ? 1280 : K == Q4K_48 ? 1152 : 1024;       // bytes of an image per column
     static constexpr uint32_t kBStage = kCols * kBRow;
     static constexpr uint32_t kMinCol = 128 * kSteps, kDCol = kMinCol + (kBlocks ? 0 : 32);
-    static constexpr uint32_t kDCols = K == Q4K_8 ? 32 : K == Q4K_48 ? 96 : 128, kMOff = kDCols / 2;          // sums of a step: products, then minimums; or of its blocks
+    static constexpr uint32_t kDCols = K == Q4K_8 ? 32 : K == Q4K_48 ? 96 : K == Q6K_8 ? 16 : 128, kMOff = kDCols / 2;          // sums of a step: products, then minimums; or of its blocks
     static constexpr uint32_t kRowScale = kBlocks ? 16 : 4;                                // bytes of a row's scales: eight d; d and dmin
     static constexpr uint32_t kOffW = kB * kBStage, kOffXs = kOffW + kW * kWBytes, kOffRows = kOffXs + kXs * kCols * 4, kOffBar = kOffRows + kRows * 128 * kRowScale;
     static constexpr uint32_t kBars = 2 * (kA + kW + kB + kD) + kMmaWarps;
-    static constexpr uint32_t kSmem = kOffBar + kBars * 8 + 16 + 1024;
-    static constexpr int kAcc = K == Q4K_8 ? 8 : K == Q4K_48 ? 16 : 4;           // sums of a thread and tile
+    static constexpr uint32_t kOffAt = kOffBar + kBars * 8 + 16;                 // Q6_K: where a raw step's rows start (row_start)
+    static constexpr uint32_t kSmem = kOffAt + 4 * kW + 1024;
+    static constexpr int kAcc = K == Q4K_8 ? 8 : K == Q4K_48 ? 16 : K == Q6K_8 ? 1 : 4;           // sums of a thread and tile
     static_assert(kBStage % 1024 == 0 && kWBytes % 128 == 0 && kOffRows % 16 == 0 && kOffBar % 8 == 0 && kSmem <= 227 * 1024, "shared memory");
     static_assert((kBlocks || kMinCol + 8 * kMins <= kDCol) && kMinCol <= kDCol && kDCol + kD * kDCols <= 512, "tensor memory");
     // A piece is unpacked once that of the step kSteps before has been multiplied, the minimums of that step with it.  Its sums had a place then, so
@@ -131,14 +134,14 @@ __device__ __forceinline__ float split_column(const float (&v)[8], uint32_t lane
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const float w = bad ? 0.f : v[i] * inv;
-        const float ws = K != Q8_0_8 && half ? w * 0.0625f : w;       // meets 16 q
+        const float ws = !Cfg<K>::kBlocks && half ? w * 0.0625f : w;       // meets 16 q
         h[i] = __float2half_rn(ws);
         l[i] = __float2half_rn(ws - __half2float(h[i]));
         sum += w;
     }
     hi += (block >> 1) * panel;
     lo += (block >> 1) * panel;
-    if constexpr (K == Q8_0_8) {
+    if constexpr (Cfg<K>::kBlocks) {
         const uint32_t c = 4 * half + (lane & 3);
         *reinterpret_cast<uint4*>(hi + chunk_offset(hi_row, c)) = *reinterpret_cast<const uint4*>(h);
         *reinterpret_cast<uint4*>(lo + chunk_offset(lo_row, c)) = *reinterpret_cast<const uint4*>(l);
@@ -232,6 +235,44 @@ template <int H> __device__ __forceinline__ uint2 unpack_q8_0(const uint8_t* raw
         sc[p] = __byte_perm(w[w0], w[w0 + 8], 0x7610);
     }
     return make_uint2(sc[0], sc[1]);
+}
+
+// Q6_K: rows start on even bytes, and a copy on a multiple of 16.  Rows eight apart start alike, so a step comes as eight boxes, box r with rows
+// r, r + 8, ..., each from the last multiple of 16 before its unit.  at: (2 unit | bytes of a row << 8), both mod 16: a row's first byte in its box.
+__device__ __forceinline__ uint32_t row_start(uint32_t at, uint32_t r) { return (at + r * (at >> 8)) & 14; }
+// The tile's row of a lane of tensor memory: a warp reads eight rows of each of four boxes (240-byte pitch: eight banks apart by 4; where the boxes
+// start differently, K / 256 = 2 mod 4, all 32 banks).
+__device__ __forceinline__ uint32_t q6k_row(uint32_t t) { return 8 * ((t & 7) + 8 * (t >> 6)) + ((t >> 3) & 7); }
+
+// Q6_K, half h of a row that starts `shift` bits (0 or 16) behind its first word: 16 words of low nibbles for every two of four blocks, 8 of high
+// bits; a byte becomes 1024 + 32 + q without arithmetic.  Returns the four blocks' scales.
+__device__ __forceinline__ uint32_t unpack_q6k(const uint8_t* raw, uint32_t h, uint32_t shift, uint32_t at) {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(raw);
+    auto word = [&](uint32_t i) { return __funnelshift_r(w[i], w[i + 1], shift); };
+#pragma unroll
+    for (int g = 0; g < 2; g++) {                  // words 4 g .. of the blocks: 16 of their 32 elements
+        uint32_t a0[4], a1[4], hb[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            a0[i] = word(16 * h + 4 * g + i);
+            a1[i] = word(16 * h + 8 + 4 * g + i);
+            hb[i] = word(32 + 8 * h + 4 * g + i);
+        }
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            uint32_t o[8];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const uint32_t a = b & 1 ? a1[i] : a0[i], top = b == 0 ? hb[i] << 4 : b == 1 ? hb[i] << 2 : b == 2 ? hb[i] : hb[i] >> 2;
+                const uint32_t q = ((b & 2 ? a >> 4 : a) & 0x0F0F0F0Fu) | (top & 0x30303030u);
+                o[2 * i + 0] = as_u32(__hsub2(as_half2(__byte_perm(q, 0x64646464u, 0x4140u)), as_half2(0x64206420u)));
+                o[2 * i + 1] = as_u32(__hsub2(as_half2(__byte_perm(q, 0x64646464u, 0x4342u)), as_half2(0x64206420u)));
+            }
+            tmem_st8(at + 16 * b + 8 * g, o);
+        }
+    }
+    // the first of a block's two scales serves all of it: bytes 0, 2, 4, 6 of the half's eight
+    return __byte_perm(word(48 + 2 * h), word(49 + 2 * h), 0x6420u);
 }
 
 // A stretch of units of K over SUBS row tiles, with one image of activations per unit.
@@ -341,7 +382,7 @@ template <Kind K, int SUBS> struct Block {
                     for (uint32_t j = 0; j < kK; j++) {
                         const uint32_t k = h * kK + j;
                         const uint64_t b = img + (((k >> 2) * panel + (k & 3) * 32) >> 4);
-                        if (C::kBlocks) umma_f16_ts(d + 16 * (k >> 1), at + 8 * j, b, idesc, k & 1);
+                        if (K == Q8_0_8) umma_f16_ts(d + 16 * (k >> 1), at + 8 * j, b, idesc, k & 1);
                         else umma_f16_ts(d, at + 8 * j, b, idesc, k);
                         if (K == Q4K_48) umma_f16_ts(d, at + 8 * j, b + (4 * panel >> 4), idesc, 1);
                     }
@@ -380,7 +421,7 @@ template <Kind K, int SUBS> struct Block {
         for (uint32_t e = warp >> 2; e < pieces; e += C::kTeams) {
             const uint32_t s = e / C::kParts, h = e % C::kParts, ws = s % C::kW;
             if (!wait(w_full + 8 * ws, (s / C::kW) & 1)) break;
-            const uint8_t* raw = base_p + C::kOffW + ws * C::kWBytes + row * C::kUnit;
+            const uint8_t* raw = base_p + C::kOffW + ws * C::kWBytes + (K == Q6K_8 ? 0 : row * C::kUnit);
             uint8_t* const scales = base_p + C::kOffRows + ((s % C::kRows) * 128 + row) * C::kRowScale;
             const uint32_t as = e % C::kA, at = tmem + lanes + 128 / C::kParts * as;
             uint4 head = make_uint4(0, 0, 0, 0);
@@ -388,7 +429,12 @@ template <Kind K, int SUBS> struct Block {
             const Q4KScales sc = q4k_unpack_scales(head.y, head.z, head.w);
             if (e >= C::kA && !wait(a_empty + 8 * as, (e / C::kA - 1) & 1)) break;
             tc_fence_after_sync();
-            if constexpr (C::kBlocks) {
+            if constexpr (K == Q6K_8) {
+                const uint32_t r = q6k_row(row) & 7, start = row_start(*reinterpret_cast<volatile uint32_t*>(base_p + C::kOffAt + 4 * ws), r), shift = 8 * (start & 2);
+                raw += (16 * r + (q6k_row(row) >> 3)) * C::kUnit + (start & ~3u);
+                *reinterpret_cast<uint32_t*>(scales + 4 * h) = unpack_q6k(raw, h, shift, at);
+                if (h == 0) *reinterpret_cast<uint32_t*>(scales + 8) = __funnelshift_r(reinterpret_cast<const uint32_t*>(raw)[52], 0u, shift);
+            } else if constexpr (C::kBlocks) {
                 const uint2 lo = unpack_q8_0<0>(raw, at), hi = unpack_q8_0<1>(raw, at + 64);
                 *reinterpret_cast<uint4*>(scales) = make_uint4(lo.x, lo.y, hi.x, hi.y);
             } else {
@@ -431,7 +477,17 @@ template <Kind K, int SUBS> struct Block {
                     float* to = acc[sub];
                     if (!wait(d_full + 8 * ds, (s / C::kD) & 1)) break;
                     tc_fence_after_sync();
-                    if constexpr (C::kBlocks) {
+                    if constexpr (K == Q6K_8) {
+                        const uint4 d4 = *reinterpret_cast<const uint4*>(scales);
+                        const float d = half_bits_to_float(d4.z);
+                        uint32_t v[16];
+                        float t = 0.f;
+                        tmem_ld16(dt, v);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int b = 0; b < 8; b++) t = fmaf(d * (float)(int8_t)((b < 4 ? d4.x : d4.y) >> (8 * (b & 3))), __uint_as_float(v[2 * b]) + __uint_as_float(v[2 * b + 1]), t);
+                        to[0] = fmaf(xs[0], t, to[0]);
+                    } else if constexpr (C::kBlocks) {
                         const uint4 d4 = *reinterpret_cast<const uint4*>(scales);
                         const uint32_t dw[4] = {d4.x, d4.y, d4.z, d4.w};
                         // columns (hi, lo) of four users, or of two

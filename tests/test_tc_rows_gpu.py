@@ -109,3 +109,38 @@ def test_moe_slots_per_expert(ctx, oracle, counts, h, ff):
     got, idx = run(ctx, R, [ctx.buffer_from(a) for a in (router, *weights)], x, res, h, ff, E, 1)
     assert (idx[:, 0] == expert).all() and (ridx[:, 0] == expert).all()
     assert_close(O, ref, got, rel_tol=2e-5, what="slots per expert")
+
+
+@pytest.mark.parametrize("m,k", [(18944, 256), (37888, 256), (18952, 512), (38008, 768), (37960, 1792), (38000, 2560), (40016, 3584), (37904, 8192)])
+def test_q6k(ctx, oracle, m, k):
+    """Rows of odd and even counts of 210-byte superblocks (a row's first byte modulo 16 takes every even value, or a few), a last tile of 8 to 120
+    rows; with and without a residual, in place."""
+    import torch
+    import runit_mac_b200 as R
+    O = oracle
+    nb = k // 256
+    g = torch.Generator(device="cuda").manual_seed(m)
+    w = torch.randint(0, 256, (m * nb, 210), generator=g, device="cuda", dtype=torch.uint8)
+    w[:, 208:210] = (torch.rand(m * nb, generator=g, device="cuda") + 0.5).half().view(torch.uint8).reshape(-1, 2)
+    x = torch.randn(k, generator=g, device="cuda")
+    x[5] = 500.0
+    res = torch.randn(m, generator=g, device="cuda") * 100
+    y = torch.zeros(2, m, device="cuda")
+    old = torch.zeros(m, device="cuda")
+    z = res.clone()
+    torch.cuda.synchronize()
+    R.gemv_q6k_f32in_f32out(ctx, w, x, y[0], m, k)
+    R.gemv_q6k_f32in_f32out(ctx, w, x, y[1], m, k)
+    R.gemv_q6k_add_f32_f32in(ctx, w, x, z, z, m, k)
+    ctx.set_tuning("kquant_variant", 2)             # the tile kernel, with f32 products
+    try:
+        R.gemv_q6k_f32in_f32out(ctx, w, x, old, m, k)
+    finally:
+        ctx.set_tuning("kquant_variant", 0)
+    ctx.flush()
+    assert torch.equal(y[0], y[1])
+    assert_close(O, old.cpu().numpy(), y[0].cpu().numpy(), rel_tol=2e-5, what="against packed f32")
+    rows = torch.cat([torch.arange(200), torch.arange(m - 200, m), torch.randint(0, m, (100,))])
+    ref = O.gemv(5, w.reshape(m, -1)[rows.cuda()].cpu().numpy(), x.cpu().numpy(), len(rows), k, O.TIER_F64)
+    assert_close(O, ref, y[0][rows.cuda()].cpu().numpy(), rel_tol=2e-5, what="q6k")
+    assert_close(O, ref + res[rows.cuda()].double().cpu().numpy(), z[rows.cuda()].cpu().numpy(), rel_tol=2e-5, what="q6k with residual")
