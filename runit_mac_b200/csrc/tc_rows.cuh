@@ -9,7 +9,7 @@
 //     2^-22 of the value or 2^-35 of the largest of the 256 (which is brought near the top of f16's range, because the halves that meet high
 //     nibbles are stored as x / 16 and end at its smallest step).
 //   * sum_j m_j * (sum of x over block j) is one more product of K = 16 per 256: A = 32 m twice, B = both halves of the block sums / 32.
-// An Inf or a NaN among a column's 256 activations makes its scale, and with it the column, NaN.
+// Q4_K: an Inf or a NaN among a column's 256 activations makes its scale, and with it the column, NaN.  Sums per block: it is a half like others.
 //
 // A CTA walks steps of 128 rows x 256 K.  Teams of four warps take the steps, or the halves of steps, in turn: a thread owns a row (tensor-memory
 // lane), unpacks its weights from the raw superblocks (TMA ring) and stores them to tensor memory.  The sums' warps read a step's sums
@@ -117,8 +117,9 @@ __device__ __forceinline__ float split_column(const float (&v)[8], uint32_t lane
     bool bad = false;
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-        amax = fmaxf(amax, fabsf(v[i]));
-        bad |= !(fabsf(v[i]) <= 3.4028235e38f);
+        const bool finite = fabsf(v[i]) <= 3.4028235e38f;
+        if (finite || !Cfg<K>::kBlocks) amax = fmaxf(amax, fabsf(v[i]));
+        if (!Cfg<K>::kBlocks) bad |= !finite;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
@@ -133,10 +134,12 @@ __device__ __forceinline__ float split_column(const float (&v)[8], uint32_t lane
     float sum = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-        const float w = bad ? 0.f : v[i] * inv;
+        // with sums per block an Inf or a NaN goes through the products like any value
+        const bool finite = !Cfg<K>::kBlocks || fabsf(v[i]) <= 3.4028235e38f;
+        const float w = bad ? 0.f : finite ? v[i] * inv : v[i];
         const float ws = !Cfg<K>::kBlocks && half ? w * 0.0625f : w;       // meets 16 q
         h[i] = __float2half_rn(ws);
-        l[i] = __float2half_rn(ws - __half2float(h[i]));
+        l[i] = __float2half_rn(finite ? ws - __half2float(h[i]) : 0.f);
         sum += w;
     }
     hi += (block >> 1) * panel;

@@ -144,3 +144,35 @@ def test_q6k(ctx, oracle, m, k):
     ref = O.gemv(5, w.reshape(m, -1)[rows.cuda()].cpu().numpy(), x.cpu().numpy(), len(rows), k, O.TIER_F64)
     assert_close(O, ref, y[0][rows.cuda()].cpu().numpy(), rel_tol=2e-5, what="q6k")
     assert_close(O, ref + res[rows.cuda()].double().cpu().numpy(), z[rows.cuda()].cpu().numpy(), rel_tol=2e-5, what="q6k with residual")
+
+
+@pytest.mark.parametrize("fmt", [0, 5])
+def test_infinities_and_nan(ctx, oracle, fmt):
+    """An infinite activation gives infinities of the weights' signs (NaN where the weight is 0), a NaN gives NaN, in its own row of activations."""
+    import torch
+    import runit_mac_b200 as R
+    O = oracle
+    m, k, batch = (19200, 768, 1) if fmt == 5 else (300, 768, 3)
+    g = torch.Generator(device="cuda").manual_seed(fmt)
+    if fmt == 5:
+        w = torch.randint(0, 256, (m * k // 256, 210), generator=g, device="cuda", dtype=torch.uint8)
+        w[:, 208:210] = (torch.rand(len(w), generator=g, device="cuda") + 0.5).half().view(torch.uint8).reshape(-1, 2)
+    else:
+        w = torch.randint(0, 256, (m * k // 32, 34), generator=g, device="cuda", dtype=torch.uint8)
+        w[:, :2] = (torch.rand(len(w), generator=g, device="cuda") + 0.5).half().view(torch.uint8).reshape(-1, 2)
+    for at, value in (([300], float("inf")), ([300], float("-inf")), ([10], float("nan")), ([0, 700], float("inf"))):
+        x = torch.randn(batch, k, generator=g, device="cuda")
+        x[batch - 1, at] = value
+        y = torch.zeros(batch, m, device="cuda")
+        torch.cuda.synchronize()
+        if fmt == 5:
+            R.gemv_q6k_f32in_f32out(ctx, w, x, y, m, k)
+        else:
+            R.gemv_batched_f32(ctx, 0, w, x, y, None, m, k, batch)
+        ctx.flush()
+        assert torch.isfinite(y[:batch - 1]).all()
+        got = y[batch - 1].cpu().numpy()
+        assert not np.isfinite(got).any()
+        with np.errstate(invalid="ignore"):
+            ref = O.gemv(fmt, w.reshape(m, -1)[:300].cpu().numpy(), x[batch - 1].cpu().numpy(), 300, k, O.TIER_F64).reshape(-1)
+        assert np.array_equal(got[:300], ref.astype(np.float32), equal_nan=True)
