@@ -147,7 +147,7 @@ int32_t runit_get_tmap(runit_ctx* ctx, const void* ptr, uint64_t rows, uint64_t 
     // a box has at most 256 elements a side: wider ones count in elements of two bytes
     const uint32_t elem = box_bytes > 256 ? 2 : 1;
     const cuuint64_t gdim[2] = {row_bytes / elem, rows};
-    const cuuint64_t gstride[1] = {row_bytes};
+    const cuuint64_t gstride[1] = {rows == 1 ? (row_bytes + 15) & ~15ull : row_bytes};      // a lone row has no next one
     const cuuint32_t box[2] = {box_bytes / elem, box_rows};
     const cuuint32_t estr[2] = {1, 1};
     CUtensorMap m;

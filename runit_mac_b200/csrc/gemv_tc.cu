@@ -305,9 +305,9 @@ int32_t gemv_tc_multi(runit_ctx* ctx, uint32_t n_mats, const void* const* w, con
     return launch<kKind>(ctx, "gemv_batched_tc", a, maps, x, k, batch);
 }
 
-// Q6_K, one activation row.  w 16-byte aligned; whole groups of eight rows, which the boxes are made of.
+// Q6_K, one activation row; w 16-byte aligned.
 bool gemv_q6k_tc_applies(const runit_ctx* ctx, const void* w, uint32_t m, uint32_t k) {
-    return m % 8 == 0 && k % 256 == 0 && runit_aligned(w, 16) && ctx->d_xq && ctx->d_tc && ctx->encode_tiled && (size_t)(k / 256) * (tcg::C::kBStage + 32) <= ctx->xq_bytes;
+    return m >= 8 && k % 256 == 0 && runit_aligned(w, 16) && ctx->d_xq && ctx->d_tc && ctx->encode_tiled && (size_t)(k / 256) * (tcg::C::kBStage + 32) <= ctx->xq_bytes;
 }
 int32_t gemv_q6k_tc(runit_ctx* ctx, const char* name, const void* w, const float* x, float* y, const float* res, uint32_t m, uint32_t k) {
     using namespace tcg;
@@ -315,13 +315,20 @@ int32_t gemv_q6k_tc(runit_ctx* ctx, const char* name, const void* w, const float
     Maps maps{};
     a.units = k / 256;
     a.batch = 1;
-    a.nseg = 1;
-    a.y[0] = y;
-    a.res[0] = res;
-    a.m[0] = m;
-    a.items = (m + 127) / 128;
-    const int32_t st = runit_get_tmap(ctx, w, m / 8, (uint64_t)a.units * 1680, 16, 240, &maps.m[0]);
+    // The boxes are made of groups of eight rows; the rows behind the last whole group are a tile of their own, whose map ends where the matrix does.
+    const uint32_t whole = m & ~7u, row_bytes = a.units * 210;
+    int32_t st = runit_get_tmap(ctx, w, whole / 8, (uint64_t)row_bytes * 8, 16, 240, &maps.m[0]);
+    if (st == RUNIT_OK && whole < m) st = runit_get_tmap(ctx, (const uint8_t*)w + (size_t)whole * row_bytes, 1, (uint64_t)row_bytes * (m - whole), 16, 240, &maps.m[1]);
     if (st != RUNIT_OK) return st;
+    a.nseg = whole < m ? 2 : 1;
+    a.y[0] = y;
+    a.y[1] = y + whole;
+    a.res[0] = res;
+    a.res[1] = res ? res + whole : nullptr;
+    a.m[0] = whole;
+    a.m[1] = m - whole;
+    a.tile0[1] = (whole + 127) / 128;
+    a.items = a.tile0[1] + a.nseg - 1;
     return launch<tcr::Q6K_8>(ctx, name, a, maps, x, k, 1);
 }
 
