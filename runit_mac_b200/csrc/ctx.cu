@@ -111,8 +111,8 @@ static int32_t ctx_init(int32_t device, cudaStream_t adopt, bool adopt_stream, r
     else { c->d_xq = nullptr; cudaGetLastError(); }
     if (cudaMalloc(&c->d_tc, runit::gemv_tc_bytes()) == cudaSuccess) cudaMemset(c->d_tc, 0, runit::gemv_tc_bytes());
     else { c->d_tc = nullptr; cudaGetLastError(); }
-    // MoE layer with its slots sorted by expert: 1400 tokens of 8 of 64 experts at width 2048, 160 of 8 of 256 at width 7168
-    if (cudaMalloc(&c->d_slots, 96u << 20) == cudaSuccess) c->slots_bytes = 96u << 20;
+    // MoE layer with its slots sorted by expert: 1460 tokens of 8 of 64 experts at width 2048, 180 of 8 of 256 at width 7168
+    if (cudaMalloc(&c->d_slots, 112u << 20) == cudaSuccess) c->slots_bytes = 112u << 20;
     else { c->d_slots = nullptr; cudaGetLastError(); }
     {
         cudaDriverEntryPointQueryResult qres;

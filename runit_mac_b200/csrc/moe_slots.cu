@@ -5,8 +5,8 @@
 // which most serve an expert that another slot has just streamed.  Here the slots are sorted by expert (slots_table_kernel),
 // their activations are split into two f16 halves (split_slots_kernel), and a group of slots of one expert meets its matrices on tcgen05
 // (tc_rows.cuh): up to 8 slots per group where an expert has a few, up to 48 where it has many.
-// The layer of width 2048, 64 experts of 1024, top 8 (us; mma.sync with tiles of 8 columns -> now): 16 tokens 95 -> 71, 32 114 -> 80, 64 146 -> 96, 128
-// 200 -> 119, 256 285 -> 147; 60 experts of 768, top 4, 256 tokens 171 -> 110; 8 of 512, top 2, 64 tokens 53 -> 39.  Error against 64 bits 1.2e-7, as before.
+// The layer of width 2048, 64 experts of 1024, top 8 (us; mma.sync with tiles of 8 columns -> now): 16 tokens 95 -> 68, 32 114 -> 77, 64 146 -> 93, 128
+// 200 -> 116, 256 285 -> 142; 60 experts of 768, top 4, 256 tokens 171 -> 106; 8 of 512, top 2, 64 tokens 53 -> 37.  Error against 64 bits 1.2e-7, as before.
 #include <cuda_fp16.h>
 
 #include "moe_internal.h"
@@ -217,10 +217,9 @@ __global__ void __launch_bounds__(Shape<COLS>::C::kThreads, 1) slots_gemm_kernel
 
 }  // namespace slots
 
-// Tiles that n_slots slots of E experts can fill.
+// Tiles that n_slots slots of E experts can fill: an expert of c slots takes at most (c + tile - 1) / tile.
 static uint32_t slots_max_tiles(uint32_t n_slots, uint32_t E, uint32_t tile) {
-    const uint32_t full = n_slots / tile, open = E < n_slots ? E : n_slots;
-    const uint64_t t = (uint64_t)full + open;
+    const uint64_t experts = E < n_slots ? E : n_slots, t = (n_slots + (tile - 1) * experts) / tile;
     return (uint32_t)(t < n_slots ? t : n_slots);
 }
 
@@ -234,8 +233,8 @@ template <int COLS> static size_t slots_most(size_t staging_bytes, uint32_t h, u
     const size_t per_tile = S::kTableBytes + (size_t)((h > ff ? h : ff) / 256) * (S::kImage + S::kTile * 4);
     if (staging_bytes < 512 + per_tile) return 0;
     const size_t tiles = (staging_bytes - 512) / per_tile;
-    // slots_max_tiles(n, E) <= tiles: n / tile + E tiles at most, and never more than n
-    const size_t n = tiles > E ? (tiles - E) * S::kTile : 0;
+    // slots_max_tiles(n, E) <= tiles: (n + (tile - 1) E) / tile at most, and never more than n
+    const size_t room = tiles * S::kTile, open = (size_t)(S::kTile - 1) * E, n = room > open ? room - open : 0;
     return n > tiles ? n : tiles;
 }
 uint32_t moe_slots_tokens(size_t staging_bytes, uint32_t h, uint32_t ff, uint32_t E, uint32_t k) {
