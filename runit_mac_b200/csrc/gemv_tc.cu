@@ -8,7 +8,8 @@
 //
 // The same kernel takes one activation row of Q6_K (gemv_kquant.cu has the line).  Its rows start on even bytes, which no tiled load takes: rows
 // eight apart start alike modulo 16, so a step comes as eight boxes of 16 rows, each from the last multiple of 16 before its unit.  152064 x 3584:
-// 127 -> 90 us (4.9 TB/s).  Bound now by the unpacking warps' instructions and the copies together (without the arithmetic 79, with an eighth of
+// 127 -> 87 us (5.1 TB/s).  There the warp that would copy images splits the one activation row itself, a unit per step, into images
+// whose other values stay zeros: a pre-pass cost 1.5 to 3.5 us a call (152064 x 3584 90 us, 18944 x 512 6.0 against 4.5).  Bound now by the unpacking warps' instructions and the copies together (without the arithmetic 79, with an eighth of
 // the copies 78).  Copying words with cp.async instead, 322; six teams 112, unpacking ahead of the wait for the place 96.
 // Error against 64 bits 1.0e-7 (before 2.8e-7).
 //
@@ -29,25 +30,16 @@ constexpr tcr::Kind kKind = tcr::Q8_0_8;
 using C = tcr::Cfg<kKind>;
 constexpr uint32_t kMaxShares = 10, kMaxCtas = 160, kTickets = kMaxCtas * 8, kPartBytes = 4096;      // a share's sums of a tile
 
-// One CTA per 256 activations, one warp per activation row (rows behind the batch are zeros).  Q6_K: one activation row, block b of it in rows
-// 2 b and 2 b + 1 of the image.
-template <tcr::Kind K>
+// One CTA per 256 activations, one warp per activation row (rows behind the batch are zeros).
 __global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x, uint8_t* __restrict__ images, float* __restrict__ scales, uint32_t k, uint32_t batch) {
     __shared__ __align__(16) uint8_t out[C::kBStage];
     const uint32_t u = blockIdx.x, n = threadIdx.x >> 5, lane = threadIdx.x & 31;
     grid_launch_dependents();      // the product may start requesting its weights; it waits for this grid before it reads anything else
     grid_dependency_wait();
     float v[8];
-    if (K == tcr::Q6K_8) {
-        for (uint32_t i = threadIdx.x; i < C::kBStage / 16; i += 256) reinterpret_cast<uint4*>(out)[i] = make_uint4(0, 0, 0, 0);
-        __syncthreads();
-    }
     tcr::load8(x + (size_t)n * k + (size_t)u * 256 + 8 * lane, n < batch, v);
-    if (K != tcr::Q6K_8 || n == 0) {
-        const uint32_t at = K == tcr::Q6K_8 ? lane >> 2 : n;
-        const float scale = tcr::split_column<K>(v, lane, out, 2 * at, out, 2 * at + 1, 2048, nullptr, 0);
-        if (lane == 0) scales[u * 8 + n] = scale;
-    }
+    const float scale = tcr::split_column<kKind>(v, lane, out, 2 * n, out, 2 * n + 1, 2048, nullptr, 0);
+    if (lane == 0) scales[u * 8 + n] = scale;
     __syncthreads();
     uint4* dst = reinterpret_cast<uint4*>(images + (size_t)u * C::kBStage);
     for (uint32_t i = threadIdx.x; i < C::kBStage / 16; i += 256) dst[i] = reinterpret_cast<const uint4*>(out)[i];
@@ -55,7 +47,8 @@ __global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x,
 
 // Up to three matrices that share the activations (q | k | v, gate | up) ride one launch: segment i owns the row tiles from tile0[i] on.
 struct Args {
-    const uint8_t* images;
+    const float* x;              // Q6_K
+    const uint8_t* images;       // else
     const float* scales;
     float* y[3];
     const float* res[3];
@@ -172,7 +165,7 @@ __global__ void __launch_bounds__(tcr::Cfg<K>::kThreads, 1) gemv_tc_kernel(const
                 const uint32_t row_bytes = a.units * 210;
                 if (blk.lane == 0) {
                     *reinterpret_cast<volatile uint32_t*>(blk.base_p + C::kOffAt + 4 * (step % C::kW)) = (u * 210 & 15) | (row_bytes & 15) << 8;
-                    mbar_expect_tx(blk.raw_bar(step), C::kWBytes + r.n * 4);
+                    mbar_expect_tx(blk.raw_bar(step), C::kWBytes);
                 }
                 __syncwarp();
                 if (blk.lane < 8)
@@ -195,13 +188,37 @@ __global__ void __launch_bounds__(tcr::Cfg<K>::kThreads, 1) gemv_tc_kernel(const
                     if (!blk.raw_free(s)) break;
                     load(r, u, s);
                 }
-                if (elect_one()) bulk_load_1d(blk.scales(s), r.xs + (size_t)(u - r.u0) * r.n, r.n * 4, blk.raw_bar(s));
+                if (K != tcr::Q6K_8 && elect_one()) bulk_load_1d(blk.scales(s), r.xs + (size_t)(u - r.u0) * r.n, r.n * 4, blk.raw_bar(s));
                 __syncwarp();
             }
         }
         // whatever was requested arrives before the CTA leaves (weights whose step's scales were never requested can only be waited for until
         // the limit)
         if (blk.given_up()) mbar_drain(blk.w_full, C::kW, s > early ? s : early);
+    } else if (blk.warp == C::kCopyB && K == tcr::Q6K_8) {
+        // One activation row is split here, a unit per step: block b into rows 2 b and 2 b + 1 of an image whose other values stay zeros.
+        uint4* const images = reinterpret_cast<uint4*>(blk.base_p);
+        for (uint32_t i = blk.lane; i < C::kB * C::kBStage / 16; i += 32) images[i] = make_uint4(0, 0, 0, 0);
+        __syncwarp();
+        const uint32_t steps = p.steps(), row = 2 * (blk.lane >> 2);
+        uint32_t unit = p.run(p.begin()).u0;
+        float next[8];
+        grid_dependency_wait();
+        tcr::load8(a.x + (size_t)unit * 256 + 8 * blk.lane, true, next);
+        for (uint32_t c = 0; c < steps; c++) {
+            float v[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = next[i];
+            if (++unit == a.units) unit = 0;
+            tcr::load8(a.x + (size_t)unit * 256 + 8 * blk.lane, true, next);
+            if (!blk.image_free(c)) break;
+            uint8_t* const image = blk.base_p + c % C::kB * C::kBStage;
+            const float scale = tcr::split_column<K>(v, blk.lane, image, row, image, row + 1, 2048, nullptr, 0);
+            if (blk.lane == 0) reinterpret_cast<float*>(blk.base_p + C::kOffXs)[c % C::kXs * C::kCols] = scale;
+            fence_proxy_async();
+            __syncwarp();
+            if (blk.lane == 0) mbar_arrive(blk.image_bar(c));
+        }
     } else if (blk.warp == C::kCopyB) {
         uint32_t c = 0;
         grid_dependency_wait();
@@ -237,6 +254,7 @@ template <tcr::Kind K> static int32_t launch(runit_ctx* ctx, const char* name, A
     uint32_t grid = (uint32_t)ctx->sm_count;
     grid = grid < kMaxCtas ? grid : kMaxCtas;
     grid = grid < a.items ? grid : a.items;
+    a.x = x;
     a.images = (const uint8_t*)ctx->d_xq;
     a.scales = (const float*)(a.images + (size_t)a.units * C::kBStage);
     a.tickets = (uint32_t*)ctx->d_tc;
@@ -248,17 +266,20 @@ template <tcr::Kind K> static int32_t launch(runit_ctx* ctx, const char* name, A
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.stream = ctx->stream;
     cfg.attrs = attr;
-    // The product requests weights as soon as the pre-pass lets it start.  Where a kernel before the pre-pass may have written them, the
-    // pre-pass is an ordinary launch, which starts when all of it can be seen.
+    // The product requests weights as soon as the launch before it lets it start.  Where a kernel before the call may have written them, the call's
+    // first launch is an ordinary one, which starts when all of it can be seen.
     cfg.numAttrs = !ctx->foreign_kernels && !ctx->weights_written && ctx->tune.pdl != 0 ? 1 : 0;
     ctx->weights_written = false;
-    cfg.gridDim = dim3(a.units);
-    cfg.blockDim = dim3(256);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, split_kernel<K>, x, (uint8_t*)ctx->d_xq, (float*)a.scales, k, batch);
-    if (e != cudaSuccess) return runit_fail(ctx, RUNIT_ERR_LAUNCH, "launch of %s (split of the activations) failed: %s", name, cudaGetErrorString(e));
-    const int32_t st = runit_after_launch(ctx, "gemv_split_x");
-    if (st != RUNIT_OK) return st;
-    cfg.numAttrs = 1;
+    cudaError_t e;
+    if (K != tcr::Q6K_8) {
+        cfg.gridDim = dim3(a.units);
+        cfg.blockDim = dim3(256);
+        e = cudaLaunchKernelEx(&cfg, split_kernel, x, (uint8_t*)ctx->d_xq, (float*)a.scales, k, batch);
+        if (e != cudaSuccess) return runit_fail(ctx, RUNIT_ERR_LAUNCH, "launch of %s (split of the activations) failed: %s", name, cudaGetErrorString(e));
+        const int32_t st = runit_after_launch(ctx, "gemv_split_x");
+        if (st != RUNIT_OK) return st;
+        cfg.numAttrs = 1;
+    }
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(tcr::Cfg<K>::kThreads);
     cfg.dynamicSmemBytes = tcr::Cfg<K>::kSmem;
@@ -307,7 +328,7 @@ int32_t gemv_tc_multi(runit_ctx* ctx, uint32_t n_mats, const void* const* w, con
 
 // Q6_K, one activation row; w 16-byte aligned.
 bool gemv_q6k_tc_applies(const runit_ctx* ctx, const void* w, uint32_t m, uint32_t k) {
-    return m >= 8 && k % 256 == 0 && runit_aligned(w, 16) && ctx->d_xq && ctx->d_tc && ctx->encode_tiled && (size_t)(k / 256) * (tcg::C::kBStage + 32) <= ctx->xq_bytes;
+    return m >= 8 && k % 256 == 0 && runit_aligned(w, 16) && ctx->d_tc && ctx->encode_tiled;
 }
 int32_t gemv_q6k_tc(runit_ctx* ctx, const char* name, const void* w, const float* x, float* y, const float* res, uint32_t m, uint32_t k) {
     using namespace tcg;
