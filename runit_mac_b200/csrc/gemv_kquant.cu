@@ -593,10 +593,10 @@ static int32_t launch(runit_ctx* ctx, const char* name, const void* w, const voi
     RUNIT_REQUIRE(ctx, k > 0 && k % be == 0 && k <= (1u << 24), "%s: k=%u is not a positive multiple of %u", name, k, be);
     RUNIT_REQUIRE(ctx, runit_aligned(w, 16) && runit_aligned(x, 16) && runit_aligned(y, 4) && (!res || runit_aligned(res, 4)),
                   "%s: weights and input 16-byte aligned, output 4-byte aligned", name);
-    // Q6_K on the tensor cores: from a tile of 128 rows per SM on (us, the kernels below / tensor cores: 18944 rows of K = 512 9.5 / 4.5, 1024 13.5 / 5.9,
-    // 3584 24 / 14; 40000 x 3584 50 / 28, 152064 x 3584 127 / 87, 128256 x 4096 120 / 95; with a pre-pass 12000 x 2048 12.0 / 13.3, 4096 x 14336 20 / 25;
-    // K = 256 later: a tile more than SMs costs a whole round there: 24003 rows 8.7 / 7.0)
-    if (FMT == RUNIT_FMT_Q6K && m >= (k == 256 ? 160u : 128u) * (uint32_t)ctx->sm_count && ctx->tune.kquant_variant == 0 && ctx->tune.kquant_prepare == 0 && ctx->tune.kquant_split == 0 &&
+    // Q6_K on the tensor cores, from 64 tiles of 128 rows on (us, the kernels below / tensor cores: 8192 rows of K = 256 5.7 / 4.8, 2048 9.5 / 8.6, 3584 13.6 / 10.4,
+    // 14336 34 / 30; 12000 x 1024 10.9 / 7.9, 18944 x 3584 24 / 14, 40000 x 3584 50 / 28, 152064 x 3584 127 / 87, 128256 x 4096 120 / 95; 4096 rows of
+    // K = 512 5.7 / 6.9, 3584 8.7 / 8.1, 14336 20.4 / 20.2; 2560 x 14336 13.4 / 15.2)
+    if (FMT == RUNIT_FMT_Q6K && m >= 8192 && ctx->tune.kquant_variant == 0 && ctx->tune.kquant_prepare == 0 && ctx->tune.kquant_split == 0 &&
         gemv_q6k_tc_applies(ctx, w, m, k))
         return gemv_q6k_tc(ctx, name, w, (const float*)x, (float*)y, (const float*)res, m, k);
     // the tile kernel needs a tile of 32 rows per warp: with fewer than two warps' worth of tiles per scheduler the first

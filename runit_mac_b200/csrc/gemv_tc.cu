@@ -9,8 +9,8 @@
 // The same kernel takes one activation row of Q6_K (gemv_kquant.cu has the line).  Its rows start on even bytes, which no tiled load takes: rows
 // eight apart start alike modulo 16, so a step comes as eight boxes of 16 rows, each from the last multiple of 16 before its unit.  152064 x 3584:
 // 127 -> 87 us (5.1 TB/s).  There the warp that would copy images splits the one activation row itself, a unit per step, into images
-// whose other values stay zeros: a pre-pass cost 1.5 to 3.5 us a call (152064 x 3584 90 us, 18944 x 512 6.0 against 4.5).  Bound now by the unpacking warps' instructions and the copies together (without the arithmetic 79, with an eighth of
-// the copies 78).  Copying words with cp.async instead, 322; six teams 112, unpacking ahead of the wait for the place 96.
+// whose other values stay zeros: a pre-pass cost 1.5 to 3.5 us a call (152064 x 3584 90 us, 18944 x 512 6.0 against 4.5).  Bound now by the
+// unpacking warps' instructions and the copies together (with the pre-pass, without the arithmetic 79, with an eighth of the copies 78).  Copying words with cp.async instead, 322; six teams 112, unpacking ahead of the wait for the place 96.
 // Error against 64 bits 1.0e-7 (before 2.8e-7).
 //
 // Bound: the unpacking warps, about 1000 clocks per 128 x 256 weights and SM (2.1 TB/s), and some 4 us between dependent calls (the pre-pass and

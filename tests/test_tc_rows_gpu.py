@@ -111,7 +111,7 @@ def test_moe_slots_per_expert(ctx, oracle, counts, h, ff):
     assert_close(O, ref, got, rel_tol=2e-5, what="slots per expert")
 
 
-@pytest.mark.parametrize("m,k", [(23680, 256), (37889, 256), (18944, 512), (18945, 512), (18951, 768), (38008, 768), (40001, 3584), (38023, 1280), (37960, 1792), (38000, 2560), (40016, 3584), (37904, 8192)])
+@pytest.mark.parametrize("m,k", [(8192, 256), (8193, 512), (8199, 14336), (37889, 256), (18944, 512), (18945, 512), (18951, 768), (38008, 768), (40001, 3584), (38023, 1280), (37960, 1792), (38000, 2560), (40016, 3584), (37904, 8192)])
 def test_q6k(ctx, oracle, m, k):
     """Rows of odd and even counts of 210-byte superblocks (a row's first byte modulo 16 takes every even value, or a few), a last tile of 8 to 120
     rows, 1 to 7 rows behind the last group of eight, a matrix that ends in the middle of a word; with and without a residual, in place."""
