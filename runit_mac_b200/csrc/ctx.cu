@@ -92,25 +92,28 @@ static int32_t ctx_init(int32_t device, cudaStream_t adopt, bool adopt_stream, r
         return RUNIT_ERR_ALLOC;
     }
     memset(c->h_status, 0, 64);
-    if (cudaMalloc((void**)&c->d_abort, 64) != cudaSuccess || cudaMemset(c->d_abort, 0, 64) != cudaSuccess) {
-        cudaGetLastError();
+    // Memory with its first `zeros` bytes cleared, on the context's stream: it does not wait for the legacy one, on which cudaMemset would run.
+    auto cleared = [&](size_t bytes, size_t zeros) -> void* {
+        void* p = nullptr;
+        if (cudaMalloc(&p, bytes) != cudaSuccess) p = nullptr;
+        else if (cudaMemsetAsync(p, 0, zeros, c->stream) != cudaSuccess) { cudaFree(p); p = nullptr; }
+        if (!p) cudaGetLastError();
+        return p;
+    };
+    if (!(c->d_abort = (uint32_t*)cleared(64, 64))) {
         cudaFreeHost(c->h_status);
         if (c->owns_stream) cudaStreamDestroy(c->stream);
         delete c;
         return RUNIT_ERR_ALLOC;
     }
-    // Staging area of the batched GEMV (its activations, quantised once per call): 4 MiB = K up to 232,960.
     // Greedy epilogue of the GEMV: 65536 tile pairs (2,097,152 rows) behind a zeroed ticket word.
-    if (cudaMalloc(&c->d_am, 256 + 65536 * 8) == cudaSuccess) cudaMemset(c->d_am, 0, 256);
-    else { c->d_am = nullptr; cudaGetLastError(); }
-    if (cudaMalloc((void**)&c->d_xq_ctl, 4096) == cudaSuccess) cudaMemset(c->d_xq_ctl, 0, 4096);
-    else { c->d_xq_ctl = nullptr; cudaGetLastError(); }
-    if (cudaMalloc(&c->d_kq, 8192 + (1u << 20)) == cudaSuccess) cudaMemset(c->d_kq, 0, 8192);
-    else { c->d_kq = nullptr; cudaGetLastError(); }
+    c->d_am = cleared(256 + 65536 * 8, 256);
+    c->d_xq_ctl = (uint32_t*)cleared(4096, 4096);
+    c->d_kq = cleared(8192 + (1u << 20), 8192);
+    c->d_tc = cleared(runit::gemv_tc_bytes(), runit::gemv_tc_ticket_bytes());
+    // Staging area of the batched GEMV (its activations, quantised once per call): 4 MiB = K up to 232,960.
     if (cudaMalloc(&c->d_xq, 4u << 20) == cudaSuccess) c->xq_bytes = 4u << 20;
     else { c->d_xq = nullptr; cudaGetLastError(); }
-    if (cudaMalloc(&c->d_tc, runit::gemv_tc_bytes()) == cudaSuccess) cudaMemset(c->d_tc, 0, runit::gemv_tc_bytes());
-    else { c->d_tc = nullptr; cudaGetLastError(); }
     // MoE layer with its slots sorted by expert: 1460 tokens of 8 of 64 experts at width 2048, 180 of 8 of 256 at width 7168
     if (cudaMalloc(&c->d_slots, 112u << 20) == cudaSuccess) c->slots_bytes = 112u << 20;
     else { c->d_slots = nullptr; cudaGetLastError(); }
@@ -200,8 +203,10 @@ int32_t runit_flush(runit_ctx_t* ctx) {
     if (ctx->h_status && ctx->h_status[0] != 0) {
         const int32_t why = ctx->h_status[0];
         ctx->h_status[0] = 0;
-        if (ctx->d_abort) cudaMemset(ctx->d_abort, 0, 4);   // the stream is idle: barriers wait again after this report
-        if (ctx->d_tc) cudaMemset(ctx->d_tc, 0, runit::gemv_tc_bytes());      // tickets of a launch that gave up
+        // barriers wait again after this report; the tickets of a launch that gave up are cleared ahead of whatever the stream gets next
+        cudaError_t c = ctx->d_abort ? cudaMemsetAsync(ctx->d_abort, 0, 4, ctx->stream) : cudaSuccess;
+        if (c == cudaSuccess && ctx->d_tc) c = cudaMemsetAsync(ctx->d_tc, 0, runit::gemv_tc_ticket_bytes(), ctx->stream);
+        if (c != cudaSuccess) runit_fail(ctx, RUNIT_ERR_LAUNCH, "clearing after a wait that gave up: %s", cudaGetErrorString(c));
         if (why == 4) {
             runit_fail(ctx, RUNIT_ERR_UNSUPPORTED, "sampler: top-k is off and the nucleus is wider than the 1024 most probable tokens (code %d)", why);
             if (ctx->sticky_status == RUNIT_OK) ctx->sticky_status = RUNIT_ERR_UNSUPPORTED;   // reported by this flush

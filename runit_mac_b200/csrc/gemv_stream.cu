@@ -180,9 +180,10 @@ static int32_t program_emit(runit_ctx* ctx, const Program& P, int fmt, const Ker
         return runit_fail(ctx, RUNIT_ERR_ALLOC, "fused GEMV stream: allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
     }
     allocs->push_back(d);
-    RUNIT_CUDA_TRY(ctx, cudaMemset(d, 0, bytes));   // counters at rest
-    RUNIT_CUDA_TRY(ctx, cudaMemcpy(d + off_full, P.full.data(), n * sizeof(OpFull), cudaMemcpyHostToDevice));
-    RUNIT_CUDA_TRY(ctx, cudaMemcpy(d + off_lite, P.lite.data(), n * sizeof(OpLite), cudaMemcpyHostToDevice));
+    // counters at rest; all three on the stream that the program runs on (the copies leave pageable memory before they return)
+    RUNIT_CUDA_TRY(ctx, cudaMemsetAsync(d, 0, bytes, ctx->stream));
+    RUNIT_CUDA_TRY(ctx, cudaMemcpyAsync(d + off_full, P.full.data(), n * sizeof(OpFull), cudaMemcpyHostToDevice, ctx->stream));
+    RUNIT_CUDA_TRY(ctx, cudaMemcpyAsync(d + off_lite, P.lite.data(), n * sizeof(OpLite), cudaMemcpyHostToDevice, ctx->stream));
     Params prm;
     memset(&prm, 0, sizeof(prm));
     prm.full = reinterpret_cast<const OpFull*>(d + off_full);

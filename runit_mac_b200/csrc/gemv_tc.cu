@@ -291,7 +291,8 @@ template <tcr::Kind K> static int32_t launch(runit_ctx* ctx, const char* name, A
 }  // namespace tcg
 
 // Bytes that the context keeps for this path: tickets, then partial sums.
-size_t gemv_tc_bytes() { return tcg::kTickets * 4 + (size_t)tcg::kMaxCtas * tcg::kMaxShares * tcg::kPartBytes; }
+size_t gemv_tc_ticket_bytes() { return tcg::kTickets * 4; }
+size_t gemv_tc_bytes() { return gemv_tc_ticket_bytes() + (size_t)tcg::kMaxCtas * tcg::kMaxShares * tcg::kPartBytes; }
 
 bool gemv_tc_applies(const runit_ctx* ctx, int fmt, uint32_t k, uint32_t batch) {
     if (fmt != RUNIT_FMT_Q8_0 || batch < 2 || batch > 8 || k % 256 != 0 || ctx->tune.gemv_math == 1 || !ctx->encode_tiled || !ctx->d_xq || !ctx->d_tc) return false;

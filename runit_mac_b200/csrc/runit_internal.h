@@ -186,7 +186,8 @@ int32_t gemv_imma(runit_ctx* ctx, int fmt, const void* w, const float* x, float*
 int32_t gemv_imma_multi(runit_ctx* ctx, int fmt, uint32_t n_mats, const void* const* w, const float* x, float* const* y,
                         const float* const* res, const uint32_t* m, uint32_t k, uint32_t batch);
 // gemv_tc.cu: batched Q8_0 GEMV on the tcgen05 tensor cores.
-size_t gemv_tc_bytes();
+size_t gemv_tc_bytes();              // tickets, which are zero at rest, then partial sums
+size_t gemv_tc_ticket_bytes();
 bool gemv_tc_applies(const runit_ctx* ctx, int fmt, uint32_t k, uint32_t batch);
 int32_t gemv_tc_multi(runit_ctx* ctx, uint32_t n_mats, const void* const* w, const float* x, float* const* y, const float* const* res, const uint32_t* m,
                       uint32_t k, uint32_t batch);

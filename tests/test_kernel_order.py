@@ -51,3 +51,10 @@ def test_copies_in_flight_are_waited_for(source):
             seen += 1
             assert body.find("mbar_drain(", loads[-1]) > 0, "%s leaves copies in flight when it gives up" % name
     assert seen
+
+
+def test_clears_are_ordered_with_the_stream():
+    """cudaMemset runs on the legacy stream, for which a context's non-blocking stream does not wait: a launch could find tickets or partial
+    sums while they are being cleared."""
+    for path in sorted(CSRC.glob("*.cu*")):
+        assert not re.search(r"\bcudaMemset\(", re.sub(r"//[^\n]*", "", path.read_text())), path.name
