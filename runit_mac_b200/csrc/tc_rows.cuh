@@ -70,6 +70,7 @@ template <Kind K> struct Cfg {
     // replaces.  The copies of a step's columns' scales wait for the raw steps kW before to have been unpacked.
     // A team and an issuing warp have their own places in the rings that they wait on: a parity tells two phases of a place apart and not three.
     static_assert(kA % kTeams == 0 && kW * kParts % kTeams == 0 && kMmaWarps == kSteps, "places of a team, of an issuing warp");
+    static_assert(K != Q6K_8 || (kTeams <= kA && kTeams <= kW * kParts), "a team's first piece waits for weights alone");
     static_assert(kRows > kSteps + kD && kMins == kSteps && kXs * (K == Q4K_48 ? 2 : 1) > kW + kSteps + kD, "rings of scales");
 };
 
@@ -369,6 +370,7 @@ template <Kind K, int SUBS> struct Block {
     // takes 1440 clocks a step).
     template <class P> __device__ __forceinline__ void products(P& p) {
         const uint32_t w = warp - C::kMma;
+        grid_dependency_wait();                    // bounded waits begin behind it: the grid before may take as long as it likes
         auto step = [&](uint32_t s, uint32_t c, uint32_t n) {
             const uint32_t panel = n * 128, idesc = idesc_f16(n), bs = c % C::kB, ds = s % C::kD, d = tmem + C::kDCol + ds * C::kDCols;
             const uint64_t img = umma_desc_sw128(base + bs * C::kBStage);
@@ -421,8 +423,12 @@ template <Kind K, int SUBS> struct Block {
     // A team takes every kTeams-th piece, whichever rows and columns it is of.
     __device__ __forceinline__ void unpack(uint32_t steps) {
         const uint32_t row = (warp & 3) * 32 + lane, lanes = ((warp & 3) * 32) << 16, pieces = steps * C::kParts;
+        // Q6_K: a team's first piece needs nothing but weights, which come ahead of the dependency wait; a raw step of the others waits for its
+        // columns' scales as well.  Every bounded wait for something else begins behind it.
+        if (K != Q6K_8) grid_dependency_wait();
         for (uint32_t e = warp >> 2; e < pieces; e += C::kTeams) {
             const uint32_t s = e / C::kParts, h = e % C::kParts, ws = s % C::kW;
+            if (K == Q6K_8 && e >= C::kTeams && e < 2 * C::kTeams) grid_dependency_wait();
             if (!wait(w_full + 8 * ws, (s / C::kW) & 1)) break;
             const uint8_t* raw = base_p + C::kOffW + ws * C::kWBytes + (K == Q6K_8 ? 0 : row * C::kUnit);
             uint8_t* const scales = base_p + C::kOffRows + ((s % C::kRows) * 128 + row) * C::kRowScale;
@@ -460,7 +466,7 @@ template <Kind K, int SUBS> struct Block {
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(a_full + 8 * as);
-    }
+        }
     }
     template <class P> __device__ __forceinline__ void sums(P& p) {
         const uint32_t sw = warp - C::kSum0, part = sw >> 2, row = (sw & 3) * 32 + lane, lanes = ((sw & 3) * 32) << 16, i0 = p.begin(), i1 = p.end();
@@ -544,7 +550,7 @@ template <Kind K, int SUBS> struct Block {
                 }
             }
             if (ok) p.finish(i, acc, sw, lane);
-    }
+        }
     }
     template <class P> __device__ __forceinline__ void work(P& p) {
         if (warp >= C::kMma) products(p);

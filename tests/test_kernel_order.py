@@ -58,3 +58,28 @@ def test_clears_are_ordered_with_the_stream():
     sums while they are being cleared."""
     for path in sorted(CSRC.glob("*.cu*")):
         assert not re.search(r"\bcudaMemset\(", re.sub(r"//[^\n]*", "", path.read_text())), path.name
+
+
+def body_after(text, pattern):
+    """The braces that follow the first match of a pattern."""
+    m = re.search(pattern, text)
+    at = i = text.index("{", m.end())
+    depth = 0
+    while True:
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        i += 1
+        if depth == 0:
+            return text[at:i]
+
+
+@pytest.mark.parametrize("role", ["products", "unpack", "sums"])
+def test_bounded_waits_begin_behind_the_dependency_wait(role):
+    """A dependent grid may be resident while its predecessors still run, for any time: a role that counts that time towards its limit gives up
+    on work that is in order.  (A first piece of Q6_K weights is waited for ahead of it: its copies depend on nothing.)"""
+    text = re.sub(r"//[^\n]*", "", (CSRC / "tc_rows.cuh").read_text())
+    body = body_after(text, r"__device__ __forceinline__ void %s\(" % role)
+    assert 0 <= body.find("grid_dependency_wait()") < body.find("wait(", body.find("grid_dependency_wait()") + 22)
+    assert not re.search(r"!wait\(", body[:body.index("grid_dependency_wait()")])
+    if role == "unpack":
+        loop = body[body.index("for (uint32_t e"):]
+        assert re.search(r"K == Q6K_8 && e >= C::kTeams && e < 2 \* C::kTeams\) grid_dependency_wait\(\)", loop[:loop.index("!wait(")])
