@@ -8,8 +8,8 @@
 //   * gemm_f32_kernel: f32 activations and f32 multiply-adds (the weights are bf16 values, exact in f32), for passes that
 //     run in 32-bit throughout.
 // A tile never mixes experts: token tiles come from a table (moe_permute), or are cut from the token index when dense.
-// Every wait is bounded; a wait that gives up raises the CTA's abort flag, all roles leave their loops, the loads in flight
-// are waited for, tensor memory is freed and the host sees RUNIT_ERR_TIMEOUT at the next flush.
+// Every wait is bounded; a wait that gives up raises the CTA's abort flag, all roles leave their loops, the loads and products in
+// flight are waited for, tensor memory is freed and the host sees RUNIT_ERR_TIMEOUT at the next flush.
 #include "bf16_ops.cuh"
 #include "gemv_common.cuh"
 #include "tcgen05.cuh"
@@ -185,7 +185,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* base_p = smem_raw + (base - smem_u32(smem_raw));
     const uint32_t ctrl = base + NS * Cfg<NT>::stage;
-    const uint32_t bar_full = ctrl, bar_empty = bar_full + 8 * NS, bar_accf = bar_empty + 8 * NS, bar_acce = bar_accf + 16, holder = bar_acce + 16;
+    const uint32_t bar_full = ctrl, bar_empty = bar_full + 8 * NS, bar_accf = bar_empty + 8 * NS, bar_acce = bar_accf + 16, bar_mma = bar_acce + 16, holder = bar_mma + 8;
     volatile uint32_t* holder_p = reinterpret_cast<volatile uint32_t*>(base_p + (holder - base));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(base_p + (holder - base) + 4);
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -198,6 +198,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             mbar_init(bar_accf + 8 * s, 1);
             mbar_init(bar_acce + 8 * s, 4);
         }
+        mbar_init(bar_mma, 1);
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -228,10 +229,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     tma_load_2d(dst + kABytes, &map_x, (int32_t)(k * 128), (int32_t)t.row0, bar_full + 8 * s);
                 }
             }
-            if (!ok || *abort_flag) {       // nobody consumes them any more: wait (bounded) for the loads in flight
-                const uint32_t n = it < (uint32_t)NS ? it : (uint32_t)NS;
-                for (uint32_t i = it - n; i < it; i++) mbar_wait(bar_full + 8 * (i % NS), (i / NS) & 1);
-            }
+            mbar_drain(bar_full, NS, it);       // whoever gives up, and when: no load is in flight when the CTA leaves
         }
     } else if (warp == 1) {
         if (lane == 0) {
@@ -254,6 +252,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 }
                 if (ok) umma_commit(bar_accf + 8 * acc);
             }
+            umma_commit(bar_mma);           // nor a product when the tensor memory goes back
+            mbar_wait(bar_mma, 0);
         }
     } else {
         const uint32_t quarter = warp & 3;
@@ -299,7 +299,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* base_p = smem_raw + (base - smem_u32(smem_raw));
     const uint32_t ctrl = base + NS * kPairStage;
-    const uint32_t bar_full = ctrl, bar_empty = bar_full + 8 * NS, bar_accf = bar_empty + 8 * NS, bar_acce = bar_accf + 16, holder = bar_acce + 16;
+    const uint32_t bar_full = ctrl, bar_empty = bar_full + 8 * NS, bar_accf = bar_empty + 8 * NS, bar_acce = bar_accf + 16, bar_mma = bar_acce + 16, holder = bar_mma + 8;
     volatile uint32_t* holder_p = reinterpret_cast<volatile uint32_t*>(base_p + (holder - base));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(base_p + (holder - base) + 4);
     const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -313,6 +313,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             mbar_init(bar_accf + 8 * s, 1);
             mbar_init(bar_acce + 8 * s, 8);
         }
+        mbar_init(bar_mma, 1);
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -345,9 +346,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                     tma_load_2d_pair(dst + kABytes, &map_x, (int32_t)(k * 128), xrow, leader_full + 8 * s);
                 }
             }
-            // nobody consumes them any more: wait (bounded) for the loads in flight.  Those of both CTAs count on the leader's barriers; the other
-            // CTA leaves behind the cluster barrier at the end, when the leader has waited.
-            if (rank == 0 && (!ok || *abort_flag)) mbar_drain(bar_full, NS, it);
+            // No load is in flight when the CTAs leave, whoever gives up, and when.  Those of both count on the leader's barriers, where the leader waits
+            // for as many steps as it has requested itself.
+            if (rank == 0) mbar_drain(bar_full, NS, it);
+            else if (!ok || *abort_flag) copies_settle();
         }
     } else if (warp == 1) {
         if (rank == 0) {
@@ -371,6 +373,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                     __syncwarp();
                 }
             }
+            if (elect_one()) umma_commit_pair(bar_mma, 1);      // nor a product in either CTA when the tensor memory goes back
+            __syncwarp();
+            mbar_wait(bar_mma, 0);
         }
     } else {
         const uint32_t quarter = warp & 3;

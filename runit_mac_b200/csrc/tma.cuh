@@ -45,6 +45,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
 __device__ __forceinline__ void mbar_drain(uint32_t bars, uint32_t ring, uint32_t issued) {
     for (uint32_t i = issued < ring ? 0 : issued - ring; i < issued; i++) mbar_wait(bars + 8 * (i % ring), (i / ring) & 1);
 }
+// The same for copies that are counted on no barrier that the thread could wait on (a peer CTA's): some two milliseconds, a thousand times what a
+// copy takes.
+__device__ __forceinline__ void copies_settle() {
+    const long long t0 = clock64();
+    while (clock64() - t0 < (1ll << 22)) __nanosleep(1000);
+}
 // 2-D tiled load: box (c0 = innermost coordinate in elements, c1 = row) -> dense shared tile.
 // c0 * element size must be a multiple of 16 bytes; dst must be 128-byte aligned.
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int32_t c0, int32_t c1, uint32_t bar) {

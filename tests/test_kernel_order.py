@@ -40,17 +40,29 @@ def test_dependents_are_released_after_tensor_memory_is_held():
     assert seen >= 3
 
 
-@pytest.mark.parametrize("source", ["attention_tc.cu", "moe_slots.cu"])
+@pytest.mark.parametrize("source", ["attention_tc.cu", "moe_slots.cu", "gemv_tc.cu", "gemm_bf16.cu"])
 def test_copies_in_flight_are_waited_for(source):
     """A role that gives up a bounded wait must not leave with its bulk copies (or MMAs) in flight: they would arrive in shared (tensor)
     memory that belongs to another block by then."""
     seen = 0
     for name, body in kernels(CSRC / source):
         loads = [m.start() for m in re.finditer(r"\b(tma_load_\dd|bulk_load_1d)\(", body)]
+        loads = loads or [m.start() for m in re.finditer(r"\btma_load_2d_pair\(", body)]
         if loads:
             seen += 1
             assert body.find("mbar_drain(", loads[-1]) > 0, "%s leaves copies in flight when it gives up" % name
     assert seen
+
+
+@pytest.mark.parametrize("source,count", [("attention_tc.cu", 1), ("tc_rows.cuh", 1), ("gemm_bf16.cu", 2)])
+def test_products_in_flight_are_waited_for(source, count):
+    """Likewise for MMAs: tensor memory goes back when every one that was issued is over."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / source).read_text())
+    commits = [m.end() for m in re.finditer(r"umma_commit(_pair)?\((last \? done : o_full|drain \+ 8 \* w|bar_mma)", text)]
+    assert len(commits) == count
+    for at in commits:
+        wait = re.compile(r"mbar_wait(_timed)?\((done|drain \+ 8 \* w|bar_mma), 0").search(text, at)
+        assert wait and "umma_commit" not in text[at:wait.start()] and "tmem_dealloc" not in text[at:wait.start()]
 
 
 def test_clears_are_ordered_with_the_stream():
