@@ -20,8 +20,8 @@
 //   * 27 warps per CTA: 0 = token-tile producer (+ tensor-memory allocation), 1 = MMA issuer (leader CTA), 2-5 and 23-26 =
 //     epilogue (tensor memory -> registers -> global), 6-21 = dequantisers, 22 = raw-superblock producer.
 // The reasons for each of these choices, with the measurements behind them, are in the comment above the kernel.
-// Every wait is bounded in time; a wait that gives up raises the CTA's abort flag, all roles leave their loops,
-// tensor memory is freed and the host sees RUNIT_ERR_TIMEOUT at the next flush.
+// Every wait is bounded in time; a wait that gives up raises the CTA's abort flag, all roles leave their loops, the loads
+// and products in flight are waited for, tensor memory is freed and the host sees RUNIT_ERR_TIMEOUT at the next flush.
 #include <cuda_bf16.h>
 
 #include "gemv_common.cuh"
@@ -165,7 +165,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_b, const __grid
     uint8_t* base_p = smem_raw + (base - smem_u32(smem_raw));
     const uint32_t ctrl = base + kOffCtrl;
     const uint32_t bar_full = ctrl, bar_empty = bar_full + 8 * kNS, bar_rawf = bar_empty + 8 * kNS, bar_rawe = bar_rawf + 8 * kNR,
-                   bar_accf = bar_rawe + 8 * kNR, bar_acce = bar_accf + 16, holder = bar_acce + 16;
+                   bar_accf = bar_rawe + 8 * kNR, bar_acce = bar_accf + 16, bar_mma = bar_acce + 16, holder = bar_mma + 8;
     volatile uint32_t* holder_p = reinterpret_cast<volatile uint32_t*>(base_p + kOffCtrl + (holder - ctrl));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(base_p + kOffCtrl + (holder - ctrl) + 4);
 
@@ -186,6 +186,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_b, const __grid
             mbar_init(bar_accf + 8 * i, 1);
             mbar_init(bar_acce + 8 * i, 16);                    // 8 epilogue warps of each CTA
         }
+        mbar_init(bar_mma, 1);
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -226,6 +227,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_b, const __grid
                     tma_load_2d_pair(base + s * kStageB + kTileBytes, &map_b, (int32_t)(st * 256 + 128), row_b, leader_full + 8 * s);
                 }
             }
+            // No load is in flight when the CTAs leave, whoever gives up, and when.  The barriers of both CTAs' loads are the leader's and count the
+            // dequantisers as well, which may have left: then there is nothing to wait on.
+            if (!ok || *abort_flag) copies_settle();
+            else if (rank == 0) mbar_drain(bar_full, kNS, it);
         }
     } else if (warp == kRawWarp) {
         // ───────── TMA producer: raw Q4_K superblocks, one unit (256 K) of the CTA's 128 rows per ring slot ─────────
@@ -249,6 +254,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_b, const __grid
                     }
                 }
             }
+            mbar_drain(bar_rawf, kNR, uc);
         }
     } else if (warp == 1) {
         // ───────── MMA issuer (leader CTA only): the whole warp walks the loop, one lane issues ─────────
@@ -279,6 +285,9 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_b, const __grid
                     __syncwarp();
                 }
             }
+            if (elect_one()) umma_commit_pair(bar_mma, 1);      // nor a product in either CTA when the tensor memory goes back
+            __syncwarp();
+            mbar_wait(bar_mma, 0);
         }
     } else if (warp < kDeqWarp0 || warp >= kEpiWarp1) {
         // ───────── epilogue: two groups of four warps take the groups of 32 columns in turn ─────────

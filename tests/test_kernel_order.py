@@ -40,7 +40,7 @@ def test_dependents_are_released_after_tensor_memory_is_held():
     assert seen >= 3
 
 
-@pytest.mark.parametrize("source", ["attention_tc.cu", "moe_slots.cu", "gemv_tc.cu", "gemm_bf16.cu"])
+@pytest.mark.parametrize("source", ["attention_tc.cu", "moe_slots.cu", "gemv_tc.cu", "gemm_bf16.cu", "moe_grouped.cu"])
 def test_copies_in_flight_are_waited_for(source):
     """A role that gives up a bounded wait must not leave with its bulk copies (or MMAs) in flight: they would arrive in shared (tensor)
     memory that belongs to another block by then."""
@@ -54,7 +54,7 @@ def test_copies_in_flight_are_waited_for(source):
     assert seen
 
 
-@pytest.mark.parametrize("source,count", [("attention_tc.cu", 1), ("tc_rows.cuh", 1), ("gemm_bf16.cu", 2)])
+@pytest.mark.parametrize("source,count", [("attention_tc.cu", 1), ("tc_rows.cuh", 1), ("gemm_bf16.cu", 2), ("moe_grouped.cu", 1)])
 def test_products_in_flight_are_waited_for(source, count):
     """Likewise for MMAs: tensor memory goes back when every one that was issued is over."""
     text = re.sub(r"//[^\n]*", "", (CSRC / source).read_text())
