@@ -192,9 +192,9 @@ __global__ void __launch_bounds__(tcr::Cfg<K>::kThreads, 1) gemv_tc_kernel(const
                 __syncwarp();
             }
         }
-        // whatever was requested arrives before the CTA leaves (weights whose step's scales were never requested can only be waited for until
-        // the limit)
-        if (blk.given_up()) mbar_drain(blk.w_full, C::kW, s > early ? s : early);
+        // whatever was requested arrives before the CTA leaves, whichever role gives up, and when (weights whose step's scales were never requested can only
+        // be waited for until the limit)
+        mbar_drain(blk.w_full, C::kW, s > early ? s : early);
     } else if (blk.warp == C::kCopyB && K == tcr::Q6K_8) {
         // One activation row is split here, a unit per step: block b into rows 2 b and 2 b + 1 of an image whose other values stay zeros.
         uint4* const images = reinterpret_cast<uint4*>(blk.base_p);
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(tcr::Cfg<K>::kThreads, 1) gemv_tc_kernel(const
                 __syncwarp();
             }
         }
-        if (blk.given_up()) mbar_drain(blk.b_full, C::kB, c);
+        mbar_drain(blk.b_full, C::kB, c);
     } else {
         blk.work(p);
     }

@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(Shape<COLS>::C::kThreads, 1) slots_gemm_kernel
                     __syncwarp();
                 }
         }
-        if (blk.given_up()) mbar_drain(blk.w_full, C::kW, s);        // whatever was requested arrives before the CTA leaves
+        mbar_drain(blk.w_full, C::kW, s);        // whatever was requested arrives before the CTA leaves, whichever role gives up, and when
     } else if (blk.warp == C::kCopyB) {
         uint32_t c = 0;
         for (uint32_t i = 0; i < p.end() && blk.ok; i++) {
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(Shape<COLS>::C::kThreads, 1) slots_gemm_kernel
                 __syncwarp();
             }
         }
-        if (blk.given_up()) mbar_drain(blk.b_full, C::kB, c);
+        mbar_drain(blk.b_full, C::kB, c);
     } else {
         blk.work(p);
     }

@@ -364,7 +364,6 @@ template <Kind K, int SUBS> struct Block {
     __device__ __forceinline__ uint32_t image(uint32_t c) const { return base + c % C::kB * C::kBStage; }
     __device__ __forceinline__ uint32_t image_bar(uint32_t c) const { return b_full + 8 * (c % C::kB); }
     __device__ __forceinline__ bool image_free(uint32_t c) { return c < C::kB || wait(b_empty + 8 * (c % C::kB), (c / C::kB - 1) & 1); }
-    __device__ __forceinline__ bool given_up() const { return !ok || *abort_flag; }
 
     // A step's sums have a place of their own, so the issuing warps take the steps in turn (one warp alone, with a wait for every barrier,
     // takes 1440 clocks a step).
@@ -414,11 +413,10 @@ template <Kind K, int SUBS> struct Block {
             const uint32_t steps = p.steps();
             for (uint32_t s = w; s < steps && ok; s += C::kMmaWarps) step(s, s / SUBS, 16);
         }
-        if (!ok) {                  // nothing is in flight when the tensor memory goes back
-            if (elect_one()) umma_commit(drain + 8 * w);
-            __syncwarp();
-            mbar_wait(drain + 8 * w, 0);
-        }
+        // whoever gives up, and when: no product is in flight when the tensor memory goes back
+        if (elect_one()) umma_commit(drain + 8 * w);
+        __syncwarp();
+        mbar_wait(drain + 8 * w, 0);
     }
     // A team takes every kTeams-th piece, whichever rows and columns it is of.
     __device__ __forceinline__ void unpack(uint32_t steps) {

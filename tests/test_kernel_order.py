@@ -51,6 +51,8 @@ def test_copies_in_flight_are_waited_for(source):
         if loads:
             seen += 1
             assert body.find("mbar_drain(", loads[-1]) > 0, "%s leaves copies in flight when it gives up" % name
+            # whether anyone has given up is known when all roles have ended, and not when the copying one has
+            assert "given_up" not in body, name
     assert seen
 
 
@@ -63,6 +65,8 @@ def test_products_in_flight_are_waited_for(source, count):
     for at in commits:
         wait = re.compile(r"mbar_wait(_timed)?\((done|drain \+ 8 \* w|bar_mma), 0").search(text, at)
         assert wait and "umma_commit" not in text[at:wait.start()] and "tmem_dealloc" not in text[at:wait.start()]
+        if "drain" in wait.group():
+            assert not re.search(r"if \(!ok\) \{[^}]*$", text[:at])
 
 
 def test_clears_are_ordered_with_the_stream():
