@@ -22,22 +22,39 @@ def kernels(path):
         yield m.group(1), text[at:i]
 
 
+def device_functions(path):
+    """(name, body) of every kernel, device function and constructor of a source file or header, comments removed."""
+    text = re.sub(r"//[^\n]*", "", path.read_text())
+    for m in re.finditer(r"__(?:global|device)__[^;{}]*?\b(\w+)\s*\([^(){};]*\)\s*(?=\{)", text):
+        depth, i = 0, m.end()
+        while True:
+            depth += {"{": 1, "}": -1}.get(text[i], 0)
+            i += 1
+            if depth == 0:
+                break
+        yield m.group(1), text[m.end():i]
+
+
 def test_dependents_are_released_after_tensor_memory_is_held():
     """tcgen05.alloc waits without a limit.  A kernel that allocates may let a dependent grid start only when all of its own blocks
     hold their columns: else a block of the dependent grid, which allocates before it waits for its predecessor, can take the columns
     that the predecessor still waits for."""
-    seen = 0
-    for path in sorted(CSRC.glob("*.cu")):
-        for name, body in kernels(path):
+    seen = set()
+    for path in sorted(CSRC.glob("*.cu*")):
+        for name, body in device_functions(path):
             alloc, trigger = re.search(r"\btmem_alloc(_pair)?\(", body), body.find("grid_launch_dependents(")
             if not alloc:
                 continue
-            seen += 1
+            seen.add(name)
             if trigger < 0:
                 continue
             barrier = re.compile(r"__syncthreads\(\)|cluster_sync\(\)").search(body, alloc.end())
             assert barrier and trigger > barrier.end(), "%s (%s) releases its dependents before its allocation is known to be done" % (name, path.name)
-    assert seen >= 3
+    # Block: the constructor that the kernels over tc_rows.cuh begin with; nothing else of theirs may release dependents
+    assert seen == {"attention_tc_kernel", "gemm_tc_kernel", "gemm_pair_kernel", "grouped_gemm_pair_kernel", "Block"}
+    for source, users in (("gemv_tc.cu", 1), ("moe_slots.cu", 1)):
+        bodies = [body for _, body in kernels(CSRC / source) if "tcr::Block<" in body]
+        assert len(bodies) == users and not any("grid_launch_dependents(" in b for b in bodies)
 
 
 @pytest.mark.parametrize("source", ["attention_tc.cu", "moe_slots.cu", "gemv_tc.cu", "gemm_bf16.cu", "moe_grouped.cu"])
