@@ -12,6 +12,8 @@ nothing is computed in Python.
 from __future__ import annotations
 
 import ctypes as C
+import inspect
+import types
 
 import numpy as np
 
@@ -98,13 +100,23 @@ _CONVERT = {DeviceBuffer: lambda b: b.ptr, float: float, type(None): lambda n: N
 
 
 def _convert(a):
-    t = type(a)
     if isinstance(a, DeviceBuffer):
         return a.ptr
-    if hasattr(t, "data_ptr"):
-        _CONVERT[t] = t.data_ptr
-        return a.data_ptr()
+    method = inspect.getattr_static(type(a), "data_ptr", None)
+    if method is not None:         # torch's is a method of C: called as it is, 0.03 us less a buffer; anything else is looked up on its object each time
+        _CONVERT[type(a)] = method if type(method) is types.MethodDescriptorType else lambda b: b.data_ptr()
     return a.data_ptr() if hasattr(a, "data_ptr") else a
+
+
+def _caller(name: str):
+    """The function that calls ``runit_<name>(ctx, *args)``."""
+    symbol, known = "runit_" + name, _CONVERT.get
+
+    def f(ctx, *args):
+        status = getattr(ctx.lib, symbol)(ctx.handle, *[a if type(a) is int else known(type(a), _convert)(a) for a in args])
+        if status:
+            ctx._check(status)
+    return f
 
 
 class Context:
@@ -172,10 +184,7 @@ class Context:
 
     def call(self, name: str, *args):
         """Call ``runit_<name>(ctx, *args)``; buffers may be DeviceBuffers, ints or torch tensors."""
-        known = _CONVERT.get
-        status = getattr(self.lib, "runit_" + name)(self.handle, *[a if type(a) is int else known(type(a), _convert)(a) for a in args])
-        if status:
-            self._check(status)
+        _caller(name)(self, *args)
 
 
 class Graph:
@@ -204,12 +213,7 @@ class Graph:
 
 
 def _twin(name: str, doc: str):
-    symbol, known = "runit_" + name, _CONVERT.get
-
-    def f(ctx: Context, *args):
-        status = getattr(ctx.lib, symbol)(ctx.handle, *[a if type(a) is int else known(type(a), _convert)(a) for a in args])
-        if status:
-            ctx._check(status)
+    f = _caller(name)
     f.__name__ = name
     f.__doc__ = doc
     return f

@@ -98,3 +98,64 @@ def test_rust_shim_covers_the_whole_boundary(tmp_path):
     for variant in ("NoDevice,", "LibraryLoad { path: String, reason: String }", "PipelineNotFound(String)",
                     "PipelineCreate { name: String, reason: String }", "Dispatch(String)", "BufferSize { expected: usize, actual: usize }"):
         assert variant in err, variant
+
+
+class _Recorder:
+    """Stands for a context whose library writes down what a call would pass."""
+
+    def __init__(self):
+        self.handle, self.lib, self.got = 7, self, []
+
+    def __getattr__(self, symbol):
+        def call(*args):
+            self.got.append((symbol, args))
+            return 0
+        return call
+
+
+class _PropertyBuffer:
+    """data_ptr is a property that returns a callable, another one for every buffer."""
+
+    def __init__(self, at):
+        self.at = at
+
+    @property
+    def data_ptr(self):
+        return lambda: self.at
+
+
+class _StaticBuffer:
+    @staticmethod
+    def data_ptr():
+        return 11
+
+
+def test_arguments_are_converted_by_what_each_one_is():
+    import torch
+    from runit_mac_b200 import dispatch
+
+    class Tensor(torch.Tensor):
+        pass
+
+    class Buffer(dispatch.DeviceBuffer):
+        def __init__(self, ptr):
+            self.ctx, self.ptr, self.nbytes = None, ptr, 0
+
+    class Plain:
+        pass
+
+    t = torch.zeros(4)
+    sub = t.as_subclass(Tensor)
+    late = Plain()
+    late.data_ptr = lambda: 13
+    own = _StaticBuffer()
+    own.data_ptr = lambda: 17
+    args = [t, sub, torch.nn.Parameter(t), _PropertyBuffer(3), _PropertyBuffer(4), _StaticBuffer(), own, late, Buffer(19), None, 5, True, 2.5, np.float32(1.5), np.uint32(6)]
+    want = [t.data_ptr()] * 3 + [3, 4, 11, 17, 13, 19, None, 5, True, 2.5, np.float32(1.5), np.uint32(6)]
+    for _ in range(2):             # the second time by the table
+        ctx = _Recorder()
+        dispatch.silu_mul_f32(ctx, *args)
+        dispatch.Context.call(ctx, "anything", *args)
+        for symbol, got in ctx.got:
+            assert got[0] == 7 and list(got[1:]) == want and [type(a) for a in got[1:]] == [type(a) for a in want]
+        assert [symbol for symbol, _ in ctx.got] == ["runit_silu_mul_f32", "runit_anything"]
