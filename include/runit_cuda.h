@@ -285,7 +285,7 @@ size_t runit_moe_scratch_bytes(uint32_t T, uint32_t h, uint32_t ff, uint32_t E, 
  * router_w: f32 [E][h]; gate, up: Q4_K [E][ff][h]; down: Q4_K [E][h][ff] (experts stacked contiguously, as
  * the reference slices merged expert tensors, forward.rs:1339-1408); x, residual, out: f32 [T][h] (out may
  * alias residual); idx_out (int32 [T][k]) and w_out (f32 [T][k]) may be NULL; scratch: caller-owned device
- * memory of at least runit_moe_scratch_bytes(), 256-byte aligned.  h, ff multiples of 256.  From T >= 4 and about 1.5 slots
+ * memory of at least runit_moe_scratch_bytes(), 256-byte aligned.  h, ff multiples of 256.  From T >= 4 and 1.25 slots
  * (T * k / E) per expert on, in layers of some size, the slots are sorted by expert, in a staging area of the context: products with 22-bit
  * instead of 16-bit activations, so that a token's bits differ (by about 5e-6 of the output) from those of the same token alone. */
 int32_t runit_moe_layer_q4k(runit_ctx_t*, const void* router_w, const void* gate, const void* up, const void* down,
@@ -294,7 +294,7 @@ int32_t runit_moe_layer_q4k(runit_ctx_t*, const void* router_w, const void* gate
 
 /* The same block with an expert streamed for every slot at every T, which is the arithmetic of the decoding step: a token's bits do not
  * depend on the tokens that share its call (h and ff 1024 or 2048 and T * E < 49152; at other widths the split of K can change with T, which
- * moves last bits).  Slower from the sizes named above on: 16 tokens of an OLMoE layer 117 instead of 100 us, 256 tokens 1590 instead of 285. */
+ * moves last bits).  Slower from the sizes named above on: 16 tokens of an OLMoE layer 117 instead of 68 us, 256 tokens 1590 instead of 142. */
 int32_t runit_moe_layer_q4k_by_slot(runit_ctx_t*, const void* router_w, const void* gate, const void* up, const void* down,
                                     const void* x, const void* residual, void* out, void* idx_out, void* w_out, void* scratch,
                                     size_t scratch_bytes, uint32_t T, uint32_t h, uint32_t ff, uint32_t E, uint32_t k, int32_t renorm);

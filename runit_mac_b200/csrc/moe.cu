@@ -40,9 +40,10 @@ struct MoeScratch {
 // lie in the context's staging area, so that neither the caller's scratch nor its size has a say; a call with more tokens than it holds is cut
 // into equal pieces.
 // Sorting by expert pays from 1.25 slots per expert on, where experts begin to be read for several slots at once (us with /
-// without, 64 experts of 2048 x 1024, top 8: 6 tokens 56 / 55, 8: 66 / 68, 12: 68 / 93, 24: 80 / 167; 60 of 2048 x 768, top 4: 16 tokens 54 / 51,
-// 24: 59 / 67), and where the products outweigh its four more launches (16 experts of 1024 x 512, top 4: 16 tokens 28 / 26, 24: 29 / 34; 8 of
-// 2048 x 512, top 2: 24 tokens 32 / 31).
+// without, 64 experts of 2048 x 1024, top 8: 6 tokens 56 / 55, 12: 68 / 93, 24: 80 / 167; 60 of 2048 x 768, top 4: 16 tokens 54 / 51, 24: 59 / 67; at one slot
+// per expert either side wins by 3 %: 8 tokens of the first layer 66 / 68), and where the products outweigh its four more launches: from 2^26
+// multiply-adds a matrix on no layer loses; at 3/4 of that some do and some gain (24 tokens: 8 experts of 2048 x 512, top 2, 32 / 31; 16 of 1024 x 512, top 4,
+// 29 / 34), at 1/2 all lose (16 tokens of the latter 28 / 26).
 static uint32_t moe_piece(const runit_ctx* ctx, uint32_t T, uint32_t h, uint32_t ff, uint32_t E, uint32_t k) {
     if (T < 4 || !ctx->d_slots || ctx->tune.moe_slots == 2) return 0;
     uint32_t most = moe_slots_tokens(ctx->slots_bytes, h, ff, E, k);

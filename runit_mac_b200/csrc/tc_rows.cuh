@@ -1,14 +1,14 @@
-// Products of packed Q4_K rows with a few columns of activations on tcgen05, in 32-bit grade: the body that the batched GEMV
-// (gemv_tc.cu) and the sorted MoE layer (moe_slots.cu) share.
+// Products of packed rows (Q4_K, Q8_0, Q6_K) with a few columns of activations on tcgen05, in 32-bit grade: the body that the batched Q8_0 GEMV, the Q6_K
+// GEMV of many rows (both gemv_tc.cu) and the sorted MoE layer (Q4_K, moe_slots.cu) share.
 //
 // The weights are A and come from tensor memory, where the warps that unpack them put them:
-//   * a weight is d * (sc * q) - dmin * m.  sc * q is an integer of at most 945, exact in f16, so one AND-OR and one f16x2 multiply-add turn
+//   * Q4_K: a weight is d * (sc * q) - dmin * m.  sc * q is an integer of at most 945, exact in f16, so one AND-OR and one f16x2 multiply-add turn
 //     two nibbles into the operand (1024 + q) * sc - 1024 * sc without rounding (a high nibble stays in place as 16 q).  d and dmin
-//     meet the 256-weight sums in f32.
+//     meet the 256-weight sums in f32.  Q8_0, Q6_K: the integers themselves; the scales meet the sums of 32 in f32.
 //   * an activation is x = 2^e * (hi + lo) with f16 hi and lo and one power of two per 256 elements of a column: 22 bits, error at most
 //     2^-22 of the value or 2^-35 of the largest of the 256 (which is brought near the top of f16's range, because the halves that meet high
 //     nibbles are stored as x / 16 and end at its smallest step).
-//   * sum_j m_j * (sum of x over block j) is one more product of K = 16 per 256: A = 32 m twice, B = both halves of the block sums / 32.
+//   * Q4_K: sum_j m_j * (sum of x over block j) is one more product of K = 16 per 256: A = 32 m twice, B = both halves of the block sums / 32.
 // Q4_K: an Inf or a NaN among a column's 256 activations makes its scale, and with it the column, NaN.  Sums per block: it is a half like others.
 //
 // A CTA walks steps of 128 rows x 256 K.  Teams of four warps take the steps, or the halves of steps, in turn: a thread owns a row (tensor-memory
@@ -18,9 +18,10 @@
 // Every wait is bounded; a wait that gives up sets the CTA's abort flag and all roles leave.
 //
 // Bound: the unpacking warps and the hand-overs between roles, 850 to 1000 clocks per step of 8 columns (2.8 warp instructions per
-// weight and 32 rows; a step's bytes arrive in 800), the products from about 40 columns on.  Why the roles are split like this (Q4_K, 152064 x 3584, 8 columns): the
-// unpacking warps also reading the sums, two CTAs of 8 warps per SM 114 us; sums in warps of their own but one issuing warp, which pays a wait of
-// about 150 clocks per barrier, 102; an issuing warp per place of the sums 83; no integer divisions in the sums' warps 75; one piece per step 73.
+// weight and 32 rows; a step's bytes arrive in 800), the products from about 40 columns on.  Why the roles are split like this, measured on one Q4_K matrix of
+// 152064 x 3584 with 8 columns (a product that gemv_imma.cu serves, faster over a whole step): the unpacking warps also reading the sums, two CTAs of 8
+// warps per SM, 114 us; sums in warps of their own but one issuing warp, which pays a wait of about 150 clocks per barrier, 102; an issuing warp per
+// place of the sums 83; no integer divisions in the sums' warps 75; one piece per step 73.
 #pragma once
 
 #include "gemv_common.cuh"
