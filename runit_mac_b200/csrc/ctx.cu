@@ -110,7 +110,7 @@ static int32_t ctx_init(int32_t device, cudaStream_t adopt, bool adopt_stream, r
     c->d_am = cleared(256 + 65536 * 8, 256);
     c->d_xq_ctl = (uint32_t*)cleared(4096, 4096);
     c->d_kq = cleared(8192 + (1u << 20), 8192);
-    c->d_tc = cleared(runit::gemv_tc_bytes(), runit::gemv_tc_ticket_bytes());
+    c->d_tc = cleared(runit::tcg::kContextBytes, runit::tcg::kTicketBytes);
     // Staging area of the batched GEMV (its activations, quantised once per call): 4 MiB = K up to 232,960.
     if (cudaMalloc(&c->d_xq, 4u << 20) == cudaSuccess) c->xq_bytes = 4u << 20;
     else { c->d_xq = nullptr; cudaGetLastError(); }
@@ -205,7 +205,7 @@ int32_t runit_flush(runit_ctx_t* ctx) {
         ctx->h_status[0] = 0;
         // barriers wait again after this report; the tickets of a launch that gave up are cleared ahead of whatever the stream gets next
         cudaError_t c = ctx->d_abort ? cudaMemsetAsync(ctx->d_abort, 0, 4, ctx->stream) : cudaSuccess;
-        if (c == cudaSuccess && ctx->d_tc) c = cudaMemsetAsync(ctx->d_tc, 0, runit::gemv_tc_ticket_bytes(), ctx->stream);
+        if (c == cudaSuccess && ctx->d_tc) c = cudaMemsetAsync(ctx->d_tc, 0, runit::tcg::kTicketBytes, ctx->stream);
         if (c != cudaSuccess) runit_fail(ctx, RUNIT_ERR_LAUNCH, "clearing after a wait that gave up: %s", cudaGetErrorString(c));
         if (why == 4) {
             runit_fail(ctx, RUNIT_ERR_UNSUPPORTED, "sampler: top-k is off and the nucleus is wider than the 1024 most probable tokens (code %d)", why);

@@ -28,7 +28,6 @@ namespace tcg {
 
 constexpr tcr::Kind kKind = tcr::Q8_0_8;
 using C = tcr::Cfg<kKind>;
-constexpr uint32_t kMaxShares = 10, kMaxCtas = 160, kTickets = kMaxCtas * 8, kPartBytes = 4096;      // a share's sums of a tile
 
 // One CTA per 256 activations, one warp per activation row (rows behind the batch are zeros).
 __global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x, uint8_t* __restrict__ images, float* __restrict__ scales, uint32_t k, uint32_t batch) {
@@ -258,7 +257,7 @@ template <tcr::Kind K> static int32_t launch(runit_ctx* ctx, const char* name, A
     a.images = (const uint8_t*)ctx->d_xq;
     a.scales = (const float*)(a.images + (size_t)a.units * C::kBStage);
     a.tickets = (uint32_t*)ctx->d_tc;
-    a.part = (float*)((uint8_t*)ctx->d_tc + kTickets * 4);
+    a.part = (float*)((uint8_t*)ctx->d_tc + kTicketBytes);
     a.status = ctx->d_status;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
@@ -289,10 +288,6 @@ template <tcr::Kind K> static int32_t launch(runit_ctx* ctx, const char* name, A
 }
 
 }  // namespace tcg
-
-// Bytes that the context keeps for this path: tickets, then partial sums.
-size_t gemv_tc_ticket_bytes() { return tcg::kTickets * 4; }
-size_t gemv_tc_bytes() { return gemv_tc_ticket_bytes() + (size_t)tcg::kMaxCtas * tcg::kMaxShares * tcg::kPartBytes; }
 
 bool gemv_tc_applies(const runit_ctx* ctx, int fmt, uint32_t k, uint32_t batch) {
     if (fmt != RUNIT_FMT_Q8_0 || batch < 2 || batch > 8 || k % 256 != 0 || ctx->tune.gemv_math == 1 || !ctx->encode_tiled || !ctx->d_xq || !ctx->d_tc) return false;

@@ -185,9 +185,12 @@ int32_t gemv_imma(runit_ctx* ctx, int fmt, const void* w, const float* x, float*
                   uint32_t batch);
 int32_t gemv_imma_multi(runit_ctx* ctx, int fmt, uint32_t n_mats, const void* const* w, const float* x, float* const* y,
                         const float* const* res, const uint32_t* m, uint32_t k, uint32_t batch);
-// gemv_tc.cu: batched Q8_0 GEMV on the tcgen05 tensor cores.
-size_t gemv_tc_bytes();              // tickets, which are zero at rest, then partial sums
-size_t gemv_tc_ticket_bytes();
+// gemv_tc.cu: batched Q8_0 GEMV on the tcgen05 tensor cores.  The context keeps tickets, zero at rest, for every CTA and warp, and behind them a place
+// per CTA for the partial sums of a row tile's shares of K.  (Here, because a library without the quantised GEMVs has contexts too.)
+namespace tcg {
+constexpr uint32_t kMaxShares = 10, kMaxCtas = 160, kTickets = kMaxCtas * 8, kPartBytes = 4096;      // a share's sums of a tile
+constexpr size_t kTicketBytes = kTickets * 4, kContextBytes = kTicketBytes + (size_t)kMaxCtas * kMaxShares * kPartBytes;
+}  // namespace tcg
 bool gemv_tc_applies(const runit_ctx* ctx, int fmt, uint32_t k, uint32_t batch);
 int32_t gemv_tc_multi(runit_ctx* ctx, uint32_t n_mats, const void* const* w, const float* x, float* const* y, const float* const* res, const uint32_t* m,
                       uint32_t k, uint32_t batch);

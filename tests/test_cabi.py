@@ -159,3 +159,11 @@ def test_arguments_are_converted_by_what_each_one_is():
         for symbol, got in ctx.got:
             assert got[0] == 7 and list(got[1:]) == want and [type(a) for a in got[1:]] == [type(a) for a in want]
         assert [symbol for symbol, _ in ctx.got] == ["runit_silu_mul_f32", "runit_anything"]
+
+
+def test_every_part_of_the_library_links_alone(tmp_path, monkeypatch):
+    """A part takes the objects of the full build; what its sources call has to be among them."""
+    from runit_mac_b200 import build
+    for name, (lib, sources) in build.PARTS.items():
+        monkeypatch.setitem(build.PARTS, name, (tmp_path / lib.name, sources))
+        assert build.build(part=name).exists()
