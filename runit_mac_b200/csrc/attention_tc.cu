@@ -49,22 +49,10 @@ template <int HD> struct Shape {
     static_assert(2 * kCols <= 512 || 2 * (kSmem + 1024) > 228 * 1024, "CTAs that share an SM share its tensor memory");
 };
 
-// kind::f16 with f16 operands (formats 0), f32 accumulator; bit 16: B is MN-major
-__host__ __device__ constexpr uint32_t idesc_f16(uint32_t m, uint32_t n, uint32_t b_mn) {
-    return (1u << 4) | (b_mn << 16) | ((n >> 3) << 17) | ((m >> 4) << 24);
-}
 // MN-major tile in the 128-byte swizzled layout: 64 elements (128 bytes) per row of K, groups of 8 K rows 1024 bytes apart (stride
 // byte offset), the next 64 elements a panel further (leading byte offset)
 __device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t addr, uint32_t panel) {
     return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)(panel >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-// A in tensor memory: 128 lanes, 32-bit column c = K elements 2c, 2c + 1
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
 }
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int32_t c0, int32_t c1, int32_t c2, uint32_t bar) {
     asm volatile(
@@ -229,7 +217,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const __grid_
 #pragma unroll
                     for (int s = 0; s < HD / 16; s++) {
                         const uint32_t off = (s >> 2) * S::kPanel + (s & 3) * 32;
-                        umma_bf16(s_cols, umma_desc_sw128(qs + off), umma_desc_sw128(kb + off), idesc_f16(kRows, kKeys, 0), s > 0);
+                        umma_bf16(s_cols, umma_desc_sw128(qs + off), umma_desc_sw128(kb + off), umma_idesc_f16(kRows, kKeys, 0), s > 0);
                     }
                     umma_commit(s_full);
                 }
@@ -258,7 +246,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const __grid_
                     if (!careful || 2 * j + chain < first_masked) {
 #pragma unroll
                         for (int s = 0; s < kKeys / 16; s++)
-                            umma_f16_ts(o_cols, s_cols + 8 * s + (s >= 4 ? 32 : 0), desc_mn_sw128(vb + s * 2048, S::kPanel), idesc_f16(kRows, HD, 1), j > 0 || s > 0);
+                            umma_f16_ts(o_cols, s_cols + 8 * s + (s >= 4 ? 32 : 0), desc_mn_sw128(vb + s * 2048, S::kPanel), umma_idesc_f16(kRows, HD, 1), j > 0 || s > 0);
                     }
                     umma_commit(last ? done : o_full);
                 }

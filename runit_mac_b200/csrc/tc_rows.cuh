@@ -172,14 +172,6 @@ __device__ __forceinline__ float split_column(const float (&v)[8], uint32_t lane
     return bad ? __uint_as_float(0x7FC00000u) : __uint_as_float((uint32_t)(e + 127) << 23);
 }
 
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__host__ __device__ constexpr uint32_t idesc_f16(uint32_t n) { return (1u << 4) | ((n >> 3) << 17) | (8u << 24); }      // f16 x f16 -> f32, M = 128
 __device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&r)[4]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]) : "r"(taddr) : "memory");
 }
@@ -372,7 +364,7 @@ template <Kind K, int SUBS> struct Block {
         const uint32_t w = warp - C::kMma;
         grid_dependency_wait();                    // bounded waits begin behind it: the grid before may take as long as it likes
         auto step = [&](uint32_t s, uint32_t c, uint32_t n) {
-            const uint32_t panel = n * 128, idesc = idesc_f16(n), bs = c % C::kB, ds = s % C::kD, d = tmem + C::kDCol + ds * C::kDCols;
+            const uint32_t panel = n * 128, idesc = umma_idesc_f16(128, n, 0), bs = c % C::kB, ds = s % C::kD, d = tmem + C::kDCol + ds * C::kDCols;
             const uint64_t img = umma_desc_sw128(base + bs * C::kBStage);
             if (!wait(b_full + 8 * bs, (c / C::kB) & 1)) return;
             if (s >= C::kD && !wait(d_empty + 8 * ds, (s / C::kD - 1) & 1)) return;

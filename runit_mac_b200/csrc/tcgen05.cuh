@@ -43,6 +43,10 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t addr) {
 __host__ __device__ constexpr uint32_t umma_idesc_bf16(uint32_t m, uint32_t n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
+// kind::f16 with f16 operands (formats 0), f32 accumulator; bit 16: B is MN-major
+__host__ __device__ constexpr uint32_t umma_idesc_f16(uint32_t m, uint32_t n, uint32_t b_mn) {
+    return (1u << 4) | (b_mn << 16) | ((n >> 3) << 17) | ((m >> 4) << 24);
+}
 
 // One lane of a converged warp, the same one each time.  An issuing loop that the whole warp walks, with the tcgen05 instructions of one lane
 // under this, keeps descriptors in uniform registers: 128 x N x 16 products with A in tensor memory issue every 12 clocks at N = 16 and 16 at
@@ -59,6 +63,14 @@ __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t desc_a, uint
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
         " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
         ::"r"(d_tmem), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// A in tensor memory: 128 lanes, 32-bit column c = K elements 2c, 2c + 1
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(desc_b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 // The mbarrier receives one arrival when every MMA issued so far by this thread has completed
