@@ -7,6 +7,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("tag,m,k,block,at", [("q8_0", 896, 896, 34, (0,)), ("q8_0", 4864, 896, 34, (0,)), ("q6k", 2048, 2048, 210, (208,)), ("q6k", 100, 256, 210, (208,)),
+                                              ("q6k", 8192, 768, 210, (208,)), ("q6k", 8199, 512, 210, (208,)),
                                               ("q5k", 3584, 1792, 176, (0, 2))])
 def test_callers_kernel_on_an_adopted_stream(tag, m, k, block, at):
     import torch
@@ -41,20 +42,62 @@ def test_callers_kernel_on_an_adopted_stream(tag, m, k, block, at):
         ctx.close()
 
 
-def test_fill_before_a_gemv(ctx):
+@pytest.mark.parametrize("rows,k,batch", [((896,), 1024, 2), ((4864, 300, 128), 768, 7)])
+def test_callers_kernel_before_a_batched_gemv(rows, k, batch):
+    """One matrix, or three in one launch."""
+    import torch
     import runit_mac_b200 as R
-    m = k = 896
-    w, x = ctx.new_buffer(m * k // 32 * 34), ctx.buffer_from(np.random.default_rng(0).normal(0, 1, k).astype(np.float32))
+    stream = torch.cuda.Stream()
+    ctx = R.Context(0, stream=stream.cuda_stream)
+    try:
+        with torch.cuda.stream(stream):
+            g = torch.Generator(device="cuda").manual_seed(k)
+            sets = [torch.randint(0, 256, (2, m * k // 32, 34), generator=g, device="cuda", dtype=torch.uint8) for m in rows]
+            for s in sets:
+                s[:, :, :2] = (torch.rand(s.shape[:2] + (1,), generator=g, device="cuda") + 0.5).half().view(torch.uint8)
+            ws, x = [torch.zeros_like(s[0]) for s in sets], torch.randn(batch, k, generator=g, device="cuda")
+            ys = [torch.zeros(52, batch, m, device="cuda") for m in rows]
+
+            def call(i, which):
+                for s, w in zip(sets, ws):
+                    torch.bitwise_xor(s[which], 0, out=w)             # a kernel, not a copy
+                if i < 2:
+                    torch.cuda.synchronize()
+                if len(rows) == 1:
+                    R.gemv_batched_f32(ctx, 0, ws[0], x, ys[0][i], None, rows[0], k, batch)
+                else:
+                    R.gemv_batched_multi_f32(ctx, 0, ws, x, [y[i] for y in ys], rows, k, batch)
+                if i < 2:
+                    ctx.flush()
+            for i in range(52):
+                call(i, i % 2)
+            ctx.flush()
+            for y in ys:
+                assert torch.isfinite(y).all() and not torch.equal(y[0], y[1])
+                for i in range(2, 52):
+                    assert torch.equal(y[i], y[i % 2]), i
+    finally:
+        ctx.close()
+
+
+@pytest.mark.parametrize("batch", [1, 4])
+def test_fill_before_a_gemv(ctx, batch):
+    import runit_mac_b200 as R
+    m, k = 896, 896 if batch == 1 else 1024
+    w, x = ctx.new_buffer(m * k // 32 * 34), ctx.buffer_from(np.random.default_rng(0).normal(0, 1, batch * k).astype(np.float32))
     outs = []
     for wait in (True, False):
-        ys = [ctx.new_buffer(m * 4) for _ in range(20)]
+        ys = [ctx.new_buffer(batch * m * 4) for _ in range(20)]
         for i, y in enumerate(ys):
             R.fill_weights(ctx, R.FMT_Q8_0, w, m * k // 32, i % 3, 0.02)
             if wait:
                 ctx.flush()
-            R.gemv_q8_0_f32in_f32out(ctx, w, x, y, m, k)
+            if batch == 1:
+                R.gemv_q8_0_f32in_f32out(ctx, w, x, y, m, k)
+            else:
+                R.gemv_batched_f32(ctx, R.FMT_Q8_0, w, x, y, None, m, k, batch)
         ctx.flush()
-        outs.append([y.download(np.float32, m) for y in ys])
+        outs.append([y.download(np.float32, batch * m) for y in ys])
     assert not np.array_equal(outs[0][0], outs[0][1])
     for a, b in zip(*outs):
         assert np.array_equal(a, b)
