@@ -167,3 +167,55 @@ def test_grouped_experts_one_slot_per_row_and_command_list(ctx, oracle):
     ctx.flush()
     assert np.array_equal(got, out.download(np.float32, n * h).reshape(n, h))
     g.destroy()
+
+
+def values(O, w, E, rows, k):
+    """bf16 values of packed matrices, on the device in 64 bits: [E][rows][k]."""
+    import torch
+    return torch.from_numpy(O.dequant_rows(2, w, E * rows, k)).cuda().bfloat16().double().reshape(E, rows, k)
+
+
+def expert_outputs(x, gate, up, down):
+    """What one expert's matrices (64 bits) make of x (f32), with the block's bf16 operands."""
+    import torch
+    xd = x.bfloat16().double()
+    g, u = (xd @ gate.T).float(), (xd @ up.T).float()
+    return (torch.nn.functional.silu(g) * u).bfloat16().double() @ down.T
+
+
+@pytest.mark.parametrize("E,k,h,ff,T,counts", [
+    (9, 1, 1024, 512, 20000, (1, 129, 255, 256, 257, 0, 513, 31, None)),       # tiles of 256 slots; some 320 items of either product on 74 pairs
+    (8, 2, 512, 256, 1024, None), (8, 2, 512, 256, 1025, None),                # 256 slots per expert on average, and one token more: either side of the rule
+    (3, 1, 768, 256, 20001, (6667, 6667, 6667)),                               # every expert ends in the same place of a tile
+])
+def test_grouped_block_of_many_slots_per_expert(ctx, oracle, E, k, h, ff, T, counts):
+    import torch
+    import runit_mac_b200 as R
+    O = oracle
+    rng = np.random.default_rng(T)
+    _, gate, up, down = make_layer(O, rng, E, h, ff)
+    if counts:
+        counts = [T - sum(c for c in counts if c) if c is None else c for c in counts]
+        idx = np.repeat(np.arange(E), counts).astype(np.int32)
+        rng.shuffle(idx)
+        idx = idx.reshape(T, 1)
+    else:
+        idx = np.argsort(rng.random((T, E)) - 0.1 * np.arange(E), axis=1)[:, :k].astype(np.int32)
+    w = rng.random((T, k)).astype(np.float32)
+    x, res = (torch.from_numpy(rng.normal(0, 1, (T, h)).astype(np.float32)).cuda() for _ in range(2))
+    ib, wb = torch.from_numpy(idx).cuda(), torch.from_numpy(w).cuda()
+    bufs = [ctx.buffer_from(a) for a in (gate, up, down)]
+    nbytes = R.moe_grouped_scratch_bytes(ctx, T, h, ff, E, k)
+    scratch = ctx.new_buffer(nbytes)
+    outs = [torch.zeros(T, h, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    for out in outs:
+        R.moe_experts_grouped_q4k_bf16(ctx, *bufs, x, ib, wb, res, out, scratch, nbytes, T, h, ff, E, k)
+    ctx.flush()
+    assert torch.equal(*outs)
+    mats = [values(O, a, E, r, c) for a, r, c in ((gate, ff, h), (up, ff, h), (down, h, ff))]
+    ref = torch.zeros(T, h, device="cuda", dtype=torch.float64)
+    for e in range(E):
+        t, i = torch.nonzero(ib == e, as_tuple=True)
+        ref.index_add_(0, t, wb[t, i, None].double() * expert_outputs(x[t], *(m[e] for m in mats)))
+    assert_close_bf16_chain(O, ref.cpu().numpy(), (outs[0] - res).cpu().numpy(), what="%d tokens of %d experts" % (T, E))

@@ -247,3 +247,25 @@ def test_dense_ffn_block(ctx, oracle, T):
         scale = np.maximum(np.abs(ref), np.sqrt(np.mean(ref.astype(np.float64) ** 2)))
         rel = float((np.abs(got - ref) / scale).max())
         assert rel <= 4e-3, (T, use_gamma, use_res, rel)
+
+
+def test_dense_ffn_block_of_many_tokens(ctx, oracle):
+    """Several items per pair of CTAs, a last token tile of 139; nothing behind the last token is written."""
+    import torch
+    import runit_mac_b200 as R
+    from test_moe_grouped_gpu import expert_outputs, values
+    O = oracle
+    T, h, ff = 19851, 512, 768
+    rng = np.random.default_rng(4)
+    ws = [O.rand_q4k(rng, r, c) for r, c in ((ff, h), (ff, h), (h, ff))]
+    x = torch.from_numpy(rng.normal(0, 1, (T, h)).astype(np.float32)).cuda()
+    nb = ctx.lib.runit_ffn_q4k_bf16_scratch_bytes(T, h, ff)
+    scratch, out = ctx.new_buffer(nb), torch.full((T + 64, h), 7.5, device="cuda")
+    torch.cuda.synchronize()
+    wb = [ctx.buffer_from(w) for w in ws]
+    R.ffn_q4k_bf16(ctx, *wb, x, None, 1e-5, None, out, scratch, nb, T, h, ff)
+    ctx.flush()
+    assert (out[T:] == 7.5).all()
+    ref = expert_outputs(x, *(values(O, w, 1, r, c)[0] for w, r, c in zip(ws, (ff, ff, h), (h, h, ff))))
+    scale = torch.maximum(ref.abs(), (ref * ref).mean().sqrt())
+    assert ((out[:T].double() - ref).abs() / scale).max() <= 4e-3        # the bound of the block of few tokens: one bf16 rounding of an activation
