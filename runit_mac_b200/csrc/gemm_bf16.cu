@@ -516,9 +516,9 @@ static int32_t dispatch_tc(runit_ctx* ctx, const char* name, const GemmDesc& d, 
     }
 }
 
-// Token tile of a dense product: the one with the least (waves of tiles) x (time of a tile).  A tile's time hardly falls with
-// its width below 128 tokens (the MMA issue rate bounds it), hence the weights.
-static uint32_t dense_tile_tok(const runit_ctx* ctx, uint32_t nb, uint32_t T) {
+// Token tile of a dense product by single CTAs: the one with the least (waves of tiles) x (time of a tile), in times of a tile of 256.  A tile's time
+// hardly falls with its width below 128 tokens (the MMA issue rate bounds it), hence the weights.
+static uint32_t dense_tile_tok(const runit_ctx* ctx, uint32_t nb, uint32_t T, float& cost_out) {
     const uint32_t nt[3] = {256, 128, 64};
     const float cost[3] = {1.0f, 0.6f, 0.45f};
     uint32_t best = 64;
@@ -528,7 +528,16 @@ static uint32_t dense_tile_tok(const runit_ctx* ctx, uint32_t nb, uint32_t T) {
         const float c = (float)((tiles + ctx->sm_count - 1) / ctx->sm_count) * cost[i];
         if (c < best_c) { best_c = c; best = nt[i]; }
     }
+    cost_out = best_c;
     return best;
+}
+// The same for CTA pairs: half as many places for tiles of 256 rows, so an odd number of 128-row blocks can cost a wave more.  A wave takes as long as
+// one of single CTAs up to K = 1024, less behind that, and a launch of clusters some 0.3 us more (us, single / pair: 2048 tokens x 8192 rows, K 512 41.9 / 41.8,
+// 1024 46.5 / 45.8, 2048 66.7 / 62.8, 4096 127 / 115; 1024 x 8192 27.2 / 27.0, 36.0 / 33.6, 63 / 58 from K 1024 on; one wave, 512 x 8192: 17.3 / 17.6, 24.6 /
+// 22.8, 37.8 / 34.5; a wave more, 2048 x 4736: 23.5 / 31.9, 27.4 / 35.5, 36.5 / 47.9, 65 / 81).
+static float pair_cost(const runit_ctx* ctx, uint32_t rows, uint32_t K, uint64_t tok_tiles) {
+    const uint64_t tiles = (uint64_t)((rows + 255) / 256) * tok_tiles, pairs = (uint64_t)ctx->sm_count / 2;
+    return (float)((tiles + pairs - 1) / pairs) * (K >= 4096 ? 0.89f : K >= 2048 ? 0.94f : K >= 1024 ? 0.98f : 1.0f) + 0.03f;
 }
 
 }  // namespace gm
@@ -561,16 +570,22 @@ int32_t gemm_bf16(runit_ctx* ctx, const char* name, const GemmDesc& d, bool exac
     }
     RUNIT_REQUIRE(ctx, d.ldx % 8 == 0 && runit_aligned(d.x, 16) && runit_aligned(d.w, 16), "%s: operands must be 16-byte aligned", name);
     a.nb = (d.rows + gm::kRowsTile - 1) / gm::kRowsTile;
-    a.tile_tok = grouped ? d.tile_tok : gm::dense_tile_tok(ctx, a.nb, d.T);
-    const uint64_t items64 = (uint64_t)a.nb * (grouped ? d.max_tiles : (d.T + a.tile_tok - 1) / a.tile_tok);
-    const uint32_t items = items64 < 0x7fffffffull ? (uint32_t)items64 : 0x7fffffffu;
-    // pairs where the tiles take several waves or K is long: the cluster's launch and meeting cost a single wave of short ones 1.3 us (512 tokens x
-    // 8192 x 1024: 19.3 us without, 20.6 with; 2048 x 2048 x 4096 43.3 and 41.1, 2048 x 8192 x 2048 69.8 and 65)
-    if (a.tile_tok == 256 && d.rows > gm::kRowsTile && (items > (uint32_t)ctx->sm_count || d.K >= 2048)) {
+    // a grouped product's tiles are known on the device alone: as many as full ones, and half an unfilled one per expert
+    const uint64_t pair_tiles = grouped ? (uint64_t)(d.T / 256 + (d.n_experts + 1) / 2) : (d.T + 255) / 256;
+    float cost = 0.f;
+    if (grouped) {
+        a.tile_tok = d.tile_tok;
+        cost = (float)(((uint64_t)a.nb * pair_tiles + ctx->sm_count - 1) / ctx->sm_count);
+    } else a.tile_tok = gm::dense_tile_tok(ctx, a.nb, d.T, cost);
+    const bool can = d.rows > gm::kRowsTile && (!grouped || a.tile_tok == 256);
+    if (can && ctx->tune.gemm_pair != 2 && (ctx->tune.gemm_pair == 1 || gm::pair_cost(ctx, d.rows, d.K, pair_tiles) < cost)) {
+        a.tile_tok = 256;
         a.nb = (d.rows + 255) / 256;
-        const uint64_t n = (uint64_t)a.nb * (grouped ? d.max_tiles : (d.T + 255) / 256);
+        const uint64_t n = (uint64_t)a.nb * (grouped ? d.max_tiles : pair_tiles);
         return gm::dispatch_pair(ctx, name, d, a, n < 0x7fffffffull ? (uint32_t)n : 0x7fffffffu);
     }
+    const uint64_t items64 = (uint64_t)a.nb * (grouped ? d.max_tiles : (d.T + a.tile_tok - 1) / a.tile_tok);
+    const uint32_t items = items64 < 0x7fffffffull ? (uint32_t)items64 : 0x7fffffffu;
     if (a.tile_tok == 256) return gm::dispatch_tc<256>(ctx, name, d, a, items);
     if (a.tile_tok == 128) return gm::dispatch_tc<128>(ctx, name, d, a, items);
     RUNIT_REQUIRE(ctx, a.tile_tok == 64, "%s: token tiles of 64, 128 or 256 only", name);

@@ -33,6 +33,7 @@ struct runit_tuning {
     int32_t ep_fused_exchange = 0;   // expert-parallel decoder: 1 = exchange inside the GEMVs (no launches of its own; measured slower)
     int32_t moe_slots = 0;        // MoE layer of several tokens: 0 = slots sorted by expert by size, 1 = always (tests), 2 = never
     int32_t moe_piece = 0;        // tokens of a piece of it at most (tests); 0 = as many as the staging area holds
+    int32_t gemm_pair = 0;        // GEMM of many tokens: 0 = CTA pairs by size, 1 = wherever they apply (tests), 2 = never
     int32_t gemv_pro_ctas = 0;    // bf16 GEMV with a prologue of several vectors: CTAs per SM at most (0 = default)
     int32_t router_variant = 0;   // batched f32 router: 0 = by size, 1 = one warp per expert, 2 = tiled GEMM, 3 = GEMM with K split over the warps of a CTA (tests force each)
 };
@@ -69,7 +70,7 @@ struct runit_ctx {
     void* d_kq = nullptr;               // Q6_K GEMV with K split over CTAs: 2048 tile tickets (zero at rest), then 1 MiB of partial sums
     void* d_xq = nullptr;               // staging area of the batched GEMV's quantised activations
     size_t xq_bytes = 0;
-    void* d_tc = nullptr;               // batched Q8_0 GEMV: tickets (zero at rest) and partial sums of row tiles that CTAs share
+    void* d_tc = nullptr;               // batched Q8_0 GEMV, Q6_K GEMV of many rows: tickets (zero at rest) and partial sums of row tiles that CTAs share
     void* d_slots = nullptr;            // staging area of the MoE layer's slots sorted by expert
     size_t slots_bytes = 0;
     void* encode_tiled = nullptr;       // cuTensorMapEncodeTiled, resolved at context creation

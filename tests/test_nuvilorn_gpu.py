@@ -94,6 +94,83 @@ def test_gemm(ctx, T, m, k):
             close(got.reshape(T, n), ref, 3e-5 if f32 else 1e-2)
 
 
+@pytest.fixture
+def pairs(ctx):
+    """Sets which kernel takes products with 256-token tiles: 1 pairs of CTAs, 2 single ones, 0 the rule."""
+    yield lambda which: ctx.set_tuning("gemm_pair", which)
+    ctx.set_tuning("gemm_pair", 0)
+
+
+@pytest.mark.parametrize("T,m,k", [(1, 130, 64), (31, 257, 2056), (255, 256, 200), (257, 385, 2056), (287, 512, 4100), (289, 129, 72), (511, 641, 136), (767, 19330, 72)])
+def test_gemm_by_cta_pairs(ctx, pairs, T, m, k):
+    """Every epilogue of the kernel for CTA pairs: rows that end in the first or the second CTA of a pair, last token tiles of 1, 31, 33 and 255, a K that
+    ends inside a step, more steps than the ring has places, and (the last shape, 228 tiles for 74 pairs) several items per pair.  It sums the products of the single kernel
+    in another grouping at most: both are within f32 rounding of the 64-bit sum."""
+    import runit_mac_b200 as R
+    g = np.random.default_rng(T + m)
+    u, w = bf16_rows(g.normal(size=(m, k)) / np.sqrt(k))
+    xu, xv = bf16_rows(g.normal(size=(T, k)))
+    pre, post = g.uniform(0.2, 2, T).astype(np.float32), g.uniform(0.2, 2, T).astype(np.float32)
+    wb, xb, pb, qb = (ctx.buffer_from(a) for a in (u, xu, pre, post))
+    z = xv @ w.T
+    base = g.normal(size=(T, m)).astype(np.float32)
+    zp = z * pre[:, None]
+    refs = {R.EPI_F32: z, R.EPI_ADD: z + base, R.EPI_CAST: z, R.EPI_RELU2: np.maximum(zp, 0) ** 2 * post[:, None]}
+    if m % 2 == 0:
+        refs[R.EPI_SILU_GLU] = zp[:, 0::2] * N.sigmoid(zp[:, 0::2]) * zp[:, 1::2] * post[:, None]
+    for epi, ref in refs.items():
+        n, act = ref.shape[1], epi >= R.EPI_SILU_GLU
+        f32 = epi in (R.EPI_F32, R.EPI_ADD)
+        outs = []
+        for which in (1, 2):
+            pairs(which)
+            guard = np.full(64, 7.5, np.float32)          # behind the last output
+            y = ctx.new_buffer(T * n * (4 if f32 else 2) + guard.nbytes)
+            if epi == R.EPI_ADD:
+                y.upload(base)
+            y.upload(guard, T * n * (4 if f32 else 2))
+            R.gemm_bf16_rows(ctx, wb, xb, y, n, T, m, k, 0, epi, pb if act else None, qb if act else None)
+            ctx.flush()
+            outs.append((y.download(np.float32, T * n) if f32 else N.from_bf16(y.download(np.uint16, T * n))).reshape(T, n))
+            assert (y.download(np.float32, 64, T * n * (4 if f32 else 2)) == guard).all()
+            close(outs[-1], ref, 3e-5 if f32 else 1e-2)
+        close(outs[0], outs[1], 3e-5 if f32 else 1e-2)
+
+
+def test_experts_by_cta_pairs(ctx, tmp_path, pairs):
+    """Tiles of 256 tokens of neighbouring experts, which end inside a tile, one expert without tokens; 200 and 320 rows per expert, so that the second CTA of a
+    pair has a part of its rows, or none."""
+    cfg = M.config(320, 60, [(M.mixer(1, 8, 2, 8, 8), M.moe(200, 5, 2))])
+
+    def edit(w):
+        w["l0.mix.o"][:] = 0
+        w["embed"][:, 0] = 3.0
+        w["l0.mlp.router"][3] = 0
+        w["l0.mlp.router"][3, 0] = -40.0
+    s = Served(ctx, tmp_path, cfg, "bfloat16", max_seq=704, edit=edit)
+    t = M.tokens(cfg, 700)
+    counts = np.zeros(5, int)
+    real = N.route_sigmoid
+
+    def watch(h, w_router, top):
+        idx, sc = real(h, w_router, top)
+        counts[:] = np.bincount(np.asarray(idx).reshape(-1), minlength=5)
+        return idx, sc
+    N.route_sigmoid = watch
+    try:
+        ref = N.forward(cfg, s.w, t)
+    finally:
+        N.route_sigmoid = real
+    mg = M.routing_margins(cfg, s.w, t)
+    assert counts[3] == 0 and (np.delete(counts, 3) % 256 != 0).all() and counts.max() > 256
+    outs = []
+    for which in (1, 2):
+        pairs(which)
+        outs.append(s.run(t, [700]))
+        check_rows(outs[-1], ref, "bfloat16", mg)
+    assert M.row_errors(outs[0], outs[1]).max() <= 1e-2        # the same bf16 operands; a sum next to a rounding boundary may fall on either side of it
+
+
 def test_gemm_repeats_bit_for_bit(ctx):
     import runit_mac_b200 as R
     g = np.random.default_rng(0)
