@@ -1,5 +1,5 @@
-// Batched (2..8 activation rows) Q8_0 GEMV on tcgen05 (tc_rows.cuh): the weights stream once and are unpacked into tensor memory, the two halves
-// of the activations are the 16 columns of one product.
+// Batched (2..8 activation rows) Q8_0 GEMV on tcgen05 (tc_rows.cuh): the weights stream once and are unpacked into tensor memory, the first two of the
+// activations' three parts are the 16 columns of one product, the third goes through one of its own.
 //
 // A pre-pass splits the activations once per call.  Work is cut into items of (128 rows, share of K); the shares of a row depend on K alone
 // and are added in order, so an output's bits depend neither on the other matrices of a launch nor on how the items fall on the CTAs.  Each
@@ -11,12 +11,13 @@
 // 127 -> 87 us (5.1 TB/s).  There the warp that would copy images splits the one activation row itself, a unit per step, into images
 // whose other values stay zeros: a pre-pass cost 1.5 to 3.5 us a call (152064 x 3584 90 us, 18944 x 512 6.0 against 4.5).  Bound now by the
 // unpacking warps' instructions and the copies together (with the pre-pass, without the arithmetic 79, with an eighth of the copies 78).  Copying words with cp.async instead, 322; six teams 112, unpacking ahead of the wait for the place 96.
-// Error against 64 bits 1.0e-7 (before 2.8e-7).
+// Error against 64 bits 0.9e-7 to 1.1e-7 from K = 2048 on (the kernels before 2.7e-7), and with three parts below that 6.0e-8 to 7.0e-8 (8.3e-8 to 9.2e-8).
 //
 // Bound: the unpacking warps, about 1000 clocks per 128 x 256 weights and SM (2.1 TB/s), and some 4 us between dependent calls (the pre-pass and
-// its hand-over).  The packed f32 kernel that it replaces multiplies every weight 8 times on the CUDA cores.  Decoding steps, us, f32 -> now: width 3584, two layers
-// and a head of 30000 rows, 2 / 4 / 8 sequences 294 / 421 / 915 -> 173 / 175 / 183; width 2048, four layers, 274 / 365 / 693 -> 208 / 209 / 221.
-// Error against 64 bits 2.0e-7 (f32 sums: 2.0e-7).  The 4-bit formats stay with gemv_imma.cu: the same kernel for them took 362 us where that one
+// its hand-over).  The packed f32 kernel that it replaces multiplies every weight 8 times on the CUDA cores.  Decoding steps, us, f32 -> now: width 3584, two
+// layers and a head of 30000 rows, 2 / 4 / 8 sequences 293 / 420 / 906 -> 191 / 183 / 188; width 2048, four layers, 271 / 363 / 689 -> 227 / 225 / 233.  Error against 64 bits 5.9e-8 at K = 256, 7.7e-8 at 2048, 1.0e-7
+// at 18944 (f32 products 7.8e-8, 9.6e-8, 1.4e-7; the two halves of 22 bits that were here before, 4 to 8 % faster, 8.1e-8, 9.5e-8, 1.2e-7, and more
+// than f32 products where a few activations dominate).  The 4-bit formats stay with gemv_imma.cu: the same kernel for them took 362 us where that one
 // takes 350 (Q4_K, 7B, four layers and head, 8 sequences), 332 against 353 (Q4_0, 4 sequences) and 198 against 187 (width 2048).
 #include <cuda_fp16.h>
 
@@ -37,7 +38,7 @@ __global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x,
     grid_dependency_wait();
     float v[8];
     tcr::load8(x + (size_t)n * k + (size_t)u * 256 + 8 * lane, n < batch, v);
-    const float scale = tcr::split_column<kKind>(v, lane, out, 2 * n, out, 2 * n + 1, 2048, nullptr, 0);
+    const float scale = tcr::split_column<kKind>(v, lane, out, n, out, 8 + n, C::kPanel, nullptr, 0);
     if (lane == 0) scales[u * 8 + n] = scale;
     __syncthreads();
     uint4* dst = reinterpret_cast<uint4*>(images + (size_t)u * C::kBStage);
@@ -100,7 +101,7 @@ template <tcr::Kind K> struct Policy {
     }
     __device__ __forceinline__ void store(uint32_t tile, uint32_t warp, uint32_t lane) const {
         const int s = segment(tile);
-        const uint32_t t = (warp & 3) * 32 + lane, row = (tile - a.tile0[s]) * 128 + (K == tcr::Q6K_8 ? tcr::q6k_row(t) : t), m = a.m[s];
+        const uint32_t t = (warp & 3) * 32 + lane, row = (tile - a.tile0[s]) * 128 + (C::kQ6 ? tcr::q6k_row(t) : t), m = a.m[s];
         if (row >= m) return;
 #pragma unroll
         for (uint32_t j = 0; j < kAcc; j++) {
@@ -160,7 +161,7 @@ __global__ void __launch_bounds__(tcr::Cfg<K>::kThreads, 1) gemv_tc_kernel(const
         // raw blocks: the first steps' ahead of the dependency wait; the columns' scales behind it
         uint32_t s = 0, early = 0;
         auto load = [&](const tcr::Run& r, uint32_t u, uint32_t step) {
-            if (K == tcr::Q6K_8) {
+            if (C::kQ6) {
                 const uint32_t row_bytes = a.units * 210;
                 if (blk.lane == 0) {
                     *reinterpret_cast<volatile uint32_t*>(blk.base_p + C::kOffAt + 4 * (step % C::kW)) = (u * 210 & 15) | (row_bytes & 15) << 8;
@@ -187,19 +188,19 @@ __global__ void __launch_bounds__(tcr::Cfg<K>::kThreads, 1) gemv_tc_kernel(const
                     if (!blk.raw_free(s)) break;
                     load(r, u, s);
                 }
-                if (K != tcr::Q6K_8 && elect_one()) bulk_load_1d(blk.scales(s), r.xs + (size_t)(u - r.u0) * r.n, r.n * 4, blk.raw_bar(s));
+                if (!C::kQ6 && elect_one()) bulk_load_1d(blk.scales(s), r.xs + (size_t)(u - r.u0) * r.n, r.n * 4, blk.raw_bar(s));
                 __syncwarp();
             }
         }
         // whatever was requested arrives before the CTA leaves, whichever role gives up, and when (weights whose step's scales were never requested can only
         // be waited for until the limit)
         mbar_drain(blk.w_full, C::kW, s > early ? s : early);
-    } else if (blk.warp == C::kCopyB && K == tcr::Q6K_8) {
-        // One activation row is split here, a unit per step: block b into rows 2 b and 2 b + 1 of an image whose other values stay zeros.
-        uint4* const images = reinterpret_cast<uint4*>(blk.base_p);
+    } else if (blk.warp == C::kCopyB && C::kQ6) {
+        // One activation row is split here, a unit per step: block b into rows b, 8 + b (and 16 + b) of an image whose other values stay zeros.
+        uint4* const images = reinterpret_cast<uint4*>(blk.base_p + C::kOffB);
         for (uint32_t i = blk.lane; i < C::kB * C::kBStage / 16; i += 32) images[i] = make_uint4(0, 0, 0, 0);
         __syncwarp();
-        const uint32_t steps = p.steps(), row = 2 * (blk.lane >> 2);
+        const uint32_t steps = p.steps(), row = blk.lane >> 2;
         uint32_t unit = p.run(p.begin()).u0;
         float next[8];
         grid_dependency_wait();
@@ -211,8 +212,8 @@ __global__ void __launch_bounds__(tcr::Cfg<K>::kThreads, 1) gemv_tc_kernel(const
             if (++unit == a.units) unit = 0;
             tcr::load8(a.x + (size_t)unit * 256 + 8 * blk.lane, true, next);
             if (!blk.image_free(c)) break;
-            uint8_t* const image = blk.base_p + c % C::kB * C::kBStage;
-            const float scale = tcr::split_column<K>(v, blk.lane, image, row, image, row + 1, 2048, nullptr, 0);
+            uint8_t* const image = blk.base_p + C::kOffB + c % C::kB * C::kBStage;
+            const float scale = tcr::split_column<K>(v, blk.lane, image, row, image, 8 + row, C::kPanel, nullptr, 0);
             if (blk.lane == 0) reinterpret_cast<float*>(blk.base_p + C::kOffXs)[c % C::kXs * C::kCols] = scale;
             fence_proxy_async();
             __syncwarp();
@@ -270,7 +271,7 @@ template <tcr::Kind K> static int32_t launch(runit_ctx* ctx, const char* name, A
     cfg.numAttrs = !ctx->foreign_kernels && !ctx->weights_written && ctx->tune.pdl != 0 ? 1 : 0;
     ctx->weights_written = false;
     cudaError_t e;
-    if (K != tcr::Q6K_8) {
+    if (!tcr::Cfg<K>::kQ6) {
         cfg.gridDim = dim3(a.units);
         cfg.blockDim = dim3(256);
         e = cudaLaunchKernelEx(&cfg, split_kernel, x, (uint8_t*)ctx->d_xq, (float*)a.scales, k, batch);
@@ -290,7 +291,7 @@ template <tcr::Kind K> static int32_t launch(runit_ctx* ctx, const char* name, A
 }  // namespace tcg
 
 bool gemv_tc_applies(const runit_ctx* ctx, int fmt, uint32_t k, uint32_t batch) {
-    if (fmt != RUNIT_FMT_Q8_0 || batch < 2 || batch > 8 || k % 256 != 0 || ctx->tune.gemv_math == 1 || !ctx->encode_tiled || !ctx->d_xq || !ctx->d_tc) return false;
+    if (fmt != RUNIT_FMT_Q8_0 || batch < 2 || batch > 8 || k == 0 || k % 256 != 0 || ctx->tune.gemv_math == 1 || !ctx->encode_tiled || !ctx->d_xq || !ctx->d_tc) return false;
     return (size_t)(k / 256) * (tcg::C::kBStage + 32) <= ctx->xq_bytes;
 }
 
@@ -318,7 +319,7 @@ int32_t gemv_tc_multi(runit_ctx* ctx, uint32_t n_mats, const void* const* w, con
             maps.m[i] = maps.m[0];
         }
     }
-    a.items = (uint32_t)tiles;         // at most 3 * 2^25, times ten shares
+    a.items = (uint32_t)tiles;         // times ten shares: far below 2^32 / 10, where the quotient by shares ends, for matrices that fit a GPU
     return launch<kKind>(ctx, "gemv_batched_tc", a, maps, x, k, batch);
 }
 
@@ -346,7 +347,9 @@ int32_t gemv_q6k_tc(runit_ctx* ctx, const char* name, const void* w, const float
     a.m[1] = m - whole;
     a.tile0[1] = (whole + 127) / 128;
     a.items = a.tile0[1] + a.nseg - 1;
-    return launch<tcr::Q6K_8>(ctx, name, a, maps, x, k, 1);
+    // Three parts of an activation where the kernel that this one replaces (one warp per row) multiplied f32 values; its others held them in three 8-bit limbs
+    // per 32 (2.7e-7 against 64 bits at K = 3584, two parts here 1.0e-7; 5 % of 152064 x 3584's time are saved).
+    return k < 2048 ? launch<tcr::Q6K_8R>(ctx, name, a, maps, x, k, 1) : launch<tcr::Q6K_8>(ctx, name, a, maps, x, k, 1);
 }
 
 }  // namespace runit

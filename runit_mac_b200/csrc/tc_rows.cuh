@@ -5,9 +5,13 @@
 //   * Q4_K: a weight is d * (sc * q) - dmin * m.  sc * q is an integer of at most 945, exact in f16, so one AND-OR and one f16x2 multiply-add turn
 //     two nibbles into the operand (1024 + q) * sc - 1024 * sc without rounding (a high nibble stays in place as 16 q).  d and dmin
 //     meet the 256-weight sums in f32.  Q8_0, Q6_K: the integers themselves; the scales meet the sums of 32 in f32.
-//   * an activation is x = 2^e * (hi + lo) with f16 hi and lo and one power of two per 256 elements of a column: 22 bits, error at most
+//   * Q4_K, Q6_K: an activation is x = 2^e * (hi + lo) with f16 hi and lo and one power of two per 256 elements of a column: 22 bits, error at most
 //     2^-22 of the value or 2^-35 of the largest of the 256 (which is brought near the top of f16's range, because the halves that meet high
 //     nibbles are stored as x / 16 and end at its smallest step).
+//   * Q8_0, Q6_K of K < 2048: x = 2^e * (hi + 2^-14 * (lo + rest)), hi an integer of at most 2^11: the sum of 32 products with a weight's integer stays below 2^24 and
+//     is exact, however the tensor cores round their sums; lo and rest are the other bits, as f16, and share their sums, which are 2^-11 of
+//     the others.  All 24 bits of a value down to 2^-11 of the largest of the 256 are kept, and 23 down to 2^-25.  Two halves alone (22 bits and sums
+//     that the tensor cores cut off) were 4 % further from 64 bits than f32 products at K = 256, and up to 40 % with a few large channels.
 //   * Q4_K: sum_j m_j * (sum of x over block j) is one more product of K = 16 per 256: A = 32 m twice, B = both halves of the block sums / 32.
 // Q4_K: an Inf or a NaN among a column's 256 activations makes its scale, and with it the column, NaN.  Sums per block: it is a half like others.
 //
@@ -34,47 +38,52 @@ namespace tcr {
 // What a step looks like:
 //   Q4K_8   up to 8 columns, both halves side by side as the 16 columns of one product
 //   Q4K_48  up to 48 columns in multiples of 16, the halves in turn into the same sums
-//   Q8_0_8  up to 8 columns, both halves of a column side by side; a sum for each of the eight blocks, because their scales are f16 values that
+//   Q8_0_8  up to 8 columns, hi and lo side by side; a sum for each of the eight blocks, because their scales are f16 values that
 //           no integer factor expresses
-//   Q6K_8   one column; block b of it has columns 2 b (hi) and 2 b + 1 (lo) of one product to itself, with zeros in the others' rows: one
-//           load of sixteen sums and not eight
+//   Q6K_8   one column; block b of it has columns b (hi) and 8 + b (lo) of one product to itself, with zeros in the others' rows: one load of sixteen
+//           sums and not eight
+//   Q6K_8R  the same with the rest in columns 16 + b (24 to 31 are not used: their rows are whatever lies behind the image's)
 // Image of 256 activations of N columns (128-byte swizzled rows of 64 elements, in the order of split_column):
 //   Q4K_8   4 panels of 16 rows (8 hi, 8 lo), then a panel whose row n holds the block sums of column n
 //   Q4K_48  4 panels of N rows of hi, 4 of lo, one of block sums
-//   else    4 panels of 16 rows (hi and lo of a column in neighbouring rows)
-enum Kind { Q4K_8, Q4K_48, Q8_0_8, Q6K_8 };
+//   else    4 panels of 16 or 24 rows: 8 hi, 8 lo, 8 rest (Q8_0: the rest in a product of its own with the columns of lo; the columns of hi meet rows of
+//           zeros there, which lie ahead of the images)
+enum Kind { Q4K_8, Q4K_48, Q8_0_8, Q6K_8, Q6K_8R };
 
 template <Kind K> struct Cfg {
-    static constexpr bool kBlocks = K == Q8_0_8 || K == Q6K_8;                  // sums per block
+    static constexpr bool kQ6 = K == Q6K_8 || K == Q6K_8R, kBlocks = K == Q8_0_8 || kQ6, kRest = K == Q8_0_8 || K == Q6K_8R;      // sums per block; three parts of an activation
     static constexpr uint32_t kCols = K == Q4K_48 ? 48 : 8;
     // kParts: a step is unpacked in one piece, or in halves (an empty tensor memory holds two steps, not three)
-    static constexpr uint32_t kParts = K == Q4K_48 || K == Q6K_8 ? 2 : 1, kTeams = K == Q4K_8 ? 3 : K == Q6K_8 ? 4 : 2, kSumWarps = K == Q4K_48 ? 12 : K == Q8_0_8 ? 8 : 4;
+    static constexpr uint32_t kParts = K == Q4K_48 || kQ6 ? 2 : 1, kTeams = K == Q4K_8 ? 3 : kQ6 ? 4 : 2, kSumWarps = K == Q4K_48 ? 12 : K == Q8_0_8 ? 8 : 4;
     static constexpr uint32_t kSum0 = 4 * kTeams, kMma = kSum0 + kSumWarps, kMmaWarps = K == Q4K_8 ? 3 : 2, kCopyW = kMma + kMmaWarps, kCopyB = kCopyW + 1, kThreads = 32 * (kCopyB + 1);      // warps by role
-    static constexpr uint32_t kUnit = K == Q8_0_8 ? 272 : K == Q6K_8 ? 240 : 144, kWBytes = 128 * kUnit;      // bytes of 256 weights; raw superblocks of a step
+    static constexpr uint32_t kUnit = K == Q8_0_8 ? 272 : kQ6 ? 240 : 144, kWBytes = 128 * kUnit;      // bytes of 256 weights; raw superblocks of a step
     // rings: raw steps, activations' images, unpacked pieces (kSteps steps) in tensor memory, sums; columns' scales and rows' scales (see the bounds below)
     static constexpr uint32_t kW = K == Q4K_8 ? 6 : 4, kB = K == Q4K_48 ? 2 : 4, kSteps = K == Q4K_8 ? 3 : 2, kA = kSteps * kParts, kD = kSteps;
     static constexpr uint32_t kXs = K == Q4K_48 ? 8 : 16, kRows = 8, kMins = kSteps;
-    static constexpr uint32_t kBRow = K == Q4K_8 ? 1280 : K == Q4K_48 ? 1152 : 1024;       // bytes of an image per column
-    static constexpr uint32_t kBStage = kCols * kBRow;
+    static constexpr uint32_t kBRow = K == Q4K_8 ? 1280 : K == Q4K_48 ? 1152 : kRest ? 1536 : 1024;       // bytes of an image per column
+    static constexpr uint32_t kBStage = kCols * kBRow, kOffB = K == Q8_0_8 ? 1024 : 0;     // eight rows of zeros, then the images
+    static constexpr uint32_t kPanel = (kRest ? 24 : 16) * 128;                                           // of an image with sums per block
     static constexpr uint32_t kMinCol = 128 * kSteps, kDCol = kMinCol + (kBlocks ? 0 : 32);
-    static constexpr uint32_t kDCols = K == Q4K_8 ? 32 : K == Q4K_48 ? 96 : K == Q6K_8 ? 16 : 128, kMOff = kDCols / 2;          // sums of a step: products, then minimums; or of its blocks
+    static constexpr uint32_t kDCols = K == Q4K_48 ? 96 : K == Q8_0_8 ? 128 : K == Q6K_8 ? 16 : 32, kMOff = kDCols / 2;          // sums of a step: products, then minimums; or of its blocks
     static constexpr uint32_t kRowScale = kBlocks ? 16 : 4;                                // bytes of a row's scales: eight d; d and dmin
-    static constexpr uint32_t kOffW = kB * kBStage, kOffXs = kOffW + kW * kWBytes, kOffRows = kOffXs + kXs * kCols * 4, kOffBar = kOffRows + kRows * 128 * kRowScale;
+    static constexpr uint32_t kOffW = kOffB + kB * kBStage, kOffXs = kOffW + kW * kWBytes, kOffRows = kOffXs + kXs * kCols * 4, kOffBar = kOffRows + kRows * 128 * kRowScale;
     static constexpr uint32_t kBars = 2 * (kA + kW + kB + kD) + kMmaWarps;
     static constexpr uint32_t kOffAt = kOffBar + kBars * 8 + 16;                 // Q6_K: where a raw step's rows start (row_start)
     static constexpr uint32_t kSmem = kOffAt + 4 * kW + 1024;
-    static constexpr int kAcc = K == Q4K_8 ? 8 : K == Q4K_48 ? 16 : K == Q6K_8 ? 1 : 4;           // sums of a thread and tile
+    static constexpr int kAcc = K == Q4K_8 ? 8 : K == Q4K_48 ? 16 : kQ6 ? 1 : 4;           // sums of a thread and tile
     static_assert(kBStage % 1024 == 0 && kWBytes % 128 == 0 && kOffRows % 16 == 0 && kOffBar % 8 == 0 && kSmem <= 227 * 1024, "shared memory");
     static_assert((kBlocks || kMinCol + 8 * kMins <= kDCol) && kMinCol <= kDCol && kDCol + kD * kDCols <= 512, "tensor memory");
     // A piece is unpacked once that of the step kSteps before has been multiplied, the minimums of that step with it.  Its sums had a place then, so
     // the sums up to step s - kSteps - kD have been read (one group of warps reads them in order), and with them the rows' scales that step s
     // replaces.  The copies of a step's columns' scales wait for the raw steps kW before to have been unpacked.
     // A team and an issuing warp have their own places in the rings that they wait on: a parity tells two phases of a place apart and not three.
-    static_assert(kA % kTeams == 0 && kW * kParts % kTeams == 0 && kMmaWarps == kSteps, "places of a team, of an issuing warp");
-    static_assert(K != Q6K_8 || (kTeams <= kA && kTeams <= kW * kParts), "a team's first piece waits for weights alone");
+    static_assert(kA % kTeams == 0 && kW * kParts % kTeams == 0 && kMmaWarps == kSteps && kD == kMmaWarps, "places of a team, of an issuing warp");
+    static_assert(!kQ6 || (kTeams <= kA && kTeams <= kW * kParts), "a team's first piece waits for weights alone");
     static_assert(kRows > kSteps + kD && kMins == kSteps && kXs * (K == Q4K_48 ? 2 : 1) > kW + kSteps + kD, "rings of scales");
 };
 
+// The products with hi, and those with lo and the rest.
+__device__ __forceinline__ float with_low(float hi, float lo) { return fmaf(lo, 6.103515625e-5f, hi); }      // 2^-14
 __device__ __forceinline__ __half2 as_half2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
 __device__ __forceinline__ uint32_t as_u32(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
 // 1024 + the field, as f16x2: one LOP3
@@ -111,7 +120,7 @@ __device__ __forceinline__ void load8(const float* x, bool live, float (&v)[8]) 
     }
 }
 // One column's 256 activations by a warp (load8) into the panels of an image: panels of hi from `hi` on, of lo from `lo`, `panel` bytes apart, and for
-// Q4_K the block sums' panel `sums`, in the rows given.  Returns the column's scale.
+// Q4_K the block sums' panel `sums`, in the rows given (else the rest eight rows behind lo).  Returns the column's scale.
 template <Kind K>
 __device__ __forceinline__ float split_column(const float (&v)[8], uint32_t lane, uint8_t* hi, uint32_t hi_row, uint8_t* lo, uint32_t lo_row, uint32_t panel,
                                               uint8_t* sums, uint32_t sum_row) {
@@ -126,13 +135,13 @@ __device__ __forceinline__ float split_column(const float (&v)[8], uint32_t lane
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     bad = __any_sync(0xffffffffu, bad);
-    // 2^e such that the largest |x| / 2^e lies in [2^14, 2^15): so does a 32nd of a block's sum.  e is held above -116 so that both powers
-    // are normal numbers.
-    int e = (int)((__float_as_uint(amax) >> 23) & 255u) - 127 - 14;
+    // 2^e such that the largest |x| / 2^e lies in [2^14, 2^15): so does a 32nd of a block's sum (with a rest: [2^10, 2^11)).  e is held above
+    // -116 so that both powers are normal numbers.
+    int e = (int)((__float_as_uint(amax) >> 23) & 255u) - 127 - (Cfg<K>::kRest ? 10 : 14);
     e = e < -116 ? -116 : e;
     const float inv = __uint_as_float((uint32_t)(127 - e) << 23);
     const uint32_t block = lane >> 2, half = block & 1;
-    __half h[8], l[8];
+    __half h[8], l[8], rest[8];
     float sum = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; i++) {
@@ -140,8 +149,11 @@ __device__ __forceinline__ float split_column(const float (&v)[8], uint32_t lane
         const bool finite = !Cfg<K>::kBlocks || fabsf(v[i]) <= 3.4028235e38f;
         const float w = bad ? 0.f : finite ? v[i] * inv : v[i];
         const float ws = !Cfg<K>::kBlocks && half ? w * 0.0625f : w;       // meets 16 q
-        h[i] = __float2half_rn(ws);
-        l[i] = __float2half_rn(finite ? ws - __half2float(h[i]) : 0.f);
+        h[i] = __float2half_rn(Cfg<K>::kRest ? rintf(ws) : ws);
+        float r = finite ? ws - __half2float(h[i]) : 0.f;
+        if (Cfg<K>::kRest) r *= 16384.f;
+        l[i] = __float2half_rn(r);
+        rest[i] = __float2half_rn(r - __half2float(l[i]));
         sum += w;
     }
     hi += (block >> 1) * panel;
@@ -150,6 +162,7 @@ __device__ __forceinline__ float split_column(const float (&v)[8], uint32_t lane
         const uint32_t c = 4 * half + (lane & 3);
         *reinterpret_cast<uint4*>(hi + chunk_offset(hi_row, c)) = *reinterpret_cast<const uint4*>(h);
         *reinterpret_cast<uint4*>(lo + chunk_offset(lo_row, c)) = *reinterpret_cast<const uint4*>(l);
+        if (Cfg<K>::kRest) *reinterpret_cast<uint4*>(lo + chunk_offset(lo_row + 8, c)) = *reinterpret_cast<const uint4*>(rest);
     } else {
 #pragma unroll
         for (int i = 0; i < 2; i++) {
@@ -333,6 +346,10 @@ template <Kind K, int SUBS> struct Block {
             *abort_flag = 0;
             fence_mbar_init();
         }
+        if (tid < C::kOffB / 16) {
+            reinterpret_cast<uint4*>(base_p)[tid] = make_uint4(0, 0, 0, 0);
+            fence_proxy_async();
+        }
         if (warp == C::kMma) {
             tmem_alloc(base + C::kOffBar + C::kBars * 8, 512);
             tmem_relinquish();
@@ -354,7 +371,7 @@ template <Kind K, int SUBS> struct Block {
     __device__ __forceinline__ uint32_t raw_bar(uint32_t s) const { return w_full + 8 * (s % C::kW); }
     __device__ __forceinline__ bool raw_free(uint32_t s) { return s < C::kW || wait(w_empty + 8 * (s % C::kW), (s / C::kW - 1) & 1); }
     __device__ __forceinline__ uint32_t scales(uint32_t c) const { return base + C::kOffXs + c % C::kXs * COLS * 4; }
-    __device__ __forceinline__ uint32_t image(uint32_t c) const { return base + c % C::kB * C::kBStage; }
+    __device__ __forceinline__ uint32_t image(uint32_t c) const { return base + C::kOffB + c % C::kB * C::kBStage; }
     __device__ __forceinline__ uint32_t image_bar(uint32_t c) const { return b_full + 8 * (c % C::kB); }
     __device__ __forceinline__ bool image_free(uint32_t c) { return c < C::kB || wait(b_empty + 8 * (c % C::kB), (c / C::kB - 1) & 1); }
 
@@ -365,7 +382,10 @@ template <Kind K, int SUBS> struct Block {
         grid_dependency_wait();                    // bounded waits begin behind it: the grid before may take as long as it likes
         auto step = [&](uint32_t s, uint32_t c, uint32_t n) {
             const uint32_t panel = n * 128, idesc = umma_idesc_f16(128, n, 0), bs = c % C::kB, ds = s % C::kD, d = tmem + C::kDCol + ds * C::kDCols;
-            const uint64_t img = umma_desc_sw128(base + bs * C::kBStage);
+            const uint32_t img_at = C::kOffB + bs * C::kBStage;
+            const uint64_t img = umma_desc_sw128(base + img_at);
+            // eight rows of zeros, and that far behind them the rest (of panel 0)
+            const uint64_t apart = umma_desc_sw128(base, img_at + 2048);
             if (!wait(b_full + 8 * bs, (c / C::kB) & 1)) return;
             if (s >= C::kD && !wait(d_empty + 8 * ds, (s / C::kD - 1) & 1)) return;
 #pragma unroll
@@ -377,11 +397,11 @@ template <Kind K, int SUBS> struct Block {
                 if (elect_one()) {
 #pragma unroll
                     for (uint32_t j = 0; j < kK; j++) {
-                        const uint32_t k = h * kK + j;
-                        const uint64_t b = img + (((k >> 2) * panel + (k & 3) * 32) >> 4);
-                        if (K == Q8_0_8) umma_f16_ts(d + 16 * (k >> 1), at + 8 * j, b, idesc, k & 1);
-                        else umma_f16_ts(d, at + 8 * j, b, idesc, k);
-                        if (K == Q4K_48) umma_f16_ts(d, at + 8 * j, b + (4 * panel >> 4), idesc, 1);
+                        const uint32_t k = h * kK + j, p0 = (k >> 2) * (C::kBlocks ? C::kPanel : panel), sum = K == Q8_0_8 ? d + 16 * (k >> 1) : d;
+                        const uint64_t in = (k & 3) * 2, b = img + (p0 >> 4) + in;
+                        umma_f16_ts(sum, at + 8 * j, b, idesc, K == Q8_0_8 ? k & 1 : k);
+                        if (K == Q4K_48) umma_f16_ts(sum, at + 8 * j, b + (4 * panel >> 4), idesc, 1);
+                        if (K == Q8_0_8) umma_f16_ts(sum, at + 8 * j, apart + ((uint64_t)(p0 >> 4) << 32) + in, idesc, 1);
                     }
                     if (!C::kBlocks && h == 0)
                         umma_f16_ts(d + C::kMOff, tmem + C::kMinCol + 8 * (s % C::kMins), img + ((K == Q4K_8 ? 4 : 8) * panel >> 4), idesc, 0);
@@ -404,7 +424,7 @@ template <Kind K, int SUBS> struct Block {
             }
         } else {
             const uint32_t steps = p.steps();
-            for (uint32_t s = w; s < steps && ok; s += C::kMmaWarps) step(s, s / SUBS, 16);
+            for (uint32_t s = w; s < steps && ok; s += C::kMmaWarps) step(s, s / SUBS, K == Q6K_8R ? 32 : 16);
         }
         // whoever gives up, and when: no product is in flight when the tensor memory goes back
         if (elect_one()) umma_commit(drain + 8 * w);
@@ -416,12 +436,12 @@ template <Kind K, int SUBS> struct Block {
         const uint32_t row = (warp & 3) * 32 + lane, lanes = ((warp & 3) * 32) << 16, pieces = steps * C::kParts;
         // Q6_K: a team's first piece needs nothing but weights, which come ahead of the dependency wait; a raw step of the others waits for its
         // columns' scales as well.  Every bounded wait for something else begins behind it.
-        if (K != Q6K_8) grid_dependency_wait();
+        if (!C::kQ6) grid_dependency_wait();
         for (uint32_t e = warp >> 2; e < pieces; e += C::kTeams) {
             const uint32_t s = e / C::kParts, h = e % C::kParts, ws = s % C::kW;
-            if (K == Q6K_8 && e >= C::kTeams && e < 2 * C::kTeams) grid_dependency_wait();
+            if (C::kQ6 && e >= C::kTeams && e < 2 * C::kTeams) grid_dependency_wait();
             if (!wait(w_full + 8 * ws, (s / C::kW) & 1)) break;
-            const uint8_t* raw = base_p + C::kOffW + ws * C::kWBytes + (K == Q6K_8 ? 0 : row * C::kUnit);
+            const uint8_t* raw = base_p + C::kOffW + ws * C::kWBytes + (C::kQ6 ? 0 : row * C::kUnit);
             uint8_t* const scales = base_p + C::kOffRows + ((s % C::kRows) * 128 + row) * C::kRowScale;
             const uint32_t as = e % C::kA, at = tmem + lanes + 128 / C::kParts * as;
             uint4 head = make_uint4(0, 0, 0, 0);
@@ -429,7 +449,7 @@ template <Kind K, int SUBS> struct Block {
             const Q4KScales sc = q4k_unpack_scales(head.y, head.z, head.w);
             if (e >= C::kA && !wait(a_empty + 8 * as, (e / C::kA - 1) & 1)) break;
             tc_fence_after_sync();
-            if constexpr (K == Q6K_8) {
+            if constexpr (C::kQ6) {
                 const uint32_t r = q6k_row(row) & 7, start = row_start(*reinterpret_cast<volatile uint32_t*>(base_p + C::kOffAt + 4 * ws), r), shift = 8 * (start & 2);
                 raw += (16 * r + (q6k_row(row) >> 3)) * C::kUnit + (start & ~3u);
                 *reinterpret_cast<uint32_t*>(scales + 4 * h) = unpack_q6k(raw, h, shift, at);
@@ -477,49 +497,58 @@ template <Kind K, int SUBS> struct Block {
                     float* to = acc[sub];
                     if (!wait(d_full + 8 * ds, (s / C::kD) & 1)) break;
                     tc_fence_after_sync();
-                    if constexpr (K == Q6K_8) {
+                    if constexpr (C::kQ6) {
                         const uint4 d4 = *reinterpret_cast<const uint4*>(scales);
                         const float d = half_bits_to_float(d4.z);
                         uint32_t v[16];
-                        float t = 0.f;
+                        float rest[8], t = 0.f;
                         tmem_ld16(dt, v);
+                        if (C::kRest) tmem_ld8(dt + 16, rest);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int b = 0; b < 8; b++) t = fmaf(d * (float)(int8_t)((b < 4 ? d4.x : d4.y) >> (8 * (b & 3))), __uint_as_float(v[2 * b]) + __uint_as_float(v[2 * b + 1]), t);
+                        for (int b = 0; b < 8; b++) {
+                            const float hi = __uint_as_float(v[b]), lo = __uint_as_float(v[8 + b]);
+                            t = fmaf(d * (float)(int8_t)((b < 4 ? d4.x : d4.y) >> (8 * (b & 3))), C::kRest ? with_low(hi, lo + rest[b]) : hi + lo, t);
+                        }
                         to[0] = fmaf(xs[0], t, to[0]);
                     } else if constexpr (C::kBlocks) {
                         const uint4 d4 = *reinterpret_cast<const uint4*>(scales);
                         const uint32_t dw[4] = {d4.x, d4.y, d4.z, d4.w};
-                        // columns (hi, lo) of four users, or of two
-                        const uint32_t users = p.few() ? 2 : 4;
+                        // four users, or two: four blocks at a time
+                        const uint32_t users = p.few() ? 2 : 4, col = users * part;
+                        float t[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                        for (int q = 0; q < 2; q++) {
-                            if (2 * q >= (int)users) break;
-                            float v[8][4], t[2] = {0.f, 0.f};
+                        for (int h = 0; h < 2; h++) {
+                            float hi[4][4], lo[4][4];
 #pragma unroll
-                            for (int b = 0; b < 8; b++) tmem_ld4(dt + 16 * b + 2 * users * part + 4 * q, v[b]);
+                            for (int b = 0; b < 4; b++) {
+                                tmem_ld4(dt + 16 * (4 * h + b) + col, hi[b]);
+                                tmem_ld4(dt + 16 * (4 * h + b) + 8 + col, lo[b]);
+                            }
                             tmem_ld_wait();
 #pragma unroll
-                            for (int b = 0; b < 8; b++) {
-                                const float db = half_bits_to_float(b & 1 ? dw[b >> 1] >> 16 : dw[b >> 1]);
-                                t[0] = fmaf(db, v[b][0] + v[b][1], t[0]);
-                                t[1] = fmaf(db, v[b][2] + v[b][3], t[1]);
+                            for (int b = 0; b < 4; b++) {
+                                const uint32_t w = dw[2 * h + (b >> 1)];
+                                const float db = half_bits_to_float(b & 1 ? w >> 16 : w);
+#pragma unroll
+                                for (uint32_t j = 0; j < 4; j++)
+                                    if (j < users) t[j] = fmaf(db, with_low(hi[b][j], lo[b][j]), t[j]);
                             }
-                            const float2 x2 = *reinterpret_cast<const float2*>(xs + users * part + 2 * q);
-                            to[2 * q] = fmaf(x2.x, t[0], to[2 * q]);
-                            to[2 * q + 1] = fmaf(x2.y, t[1], to[2 * q + 1]);
                         }
+#pragma unroll
+                        for (uint32_t j = 0; j < 4; j++)
+                            if (j < users) to[j] = fmaf(xs[col + j], t[j], to[j]);
                     } else {
                         const uint32_t dd = *reinterpret_cast<const uint32_t*>(scales);
                         const float d = half_bits_to_float(dd & 0xFFFFu), dm = -half_bits_to_float(dd >> 16);
                         if constexpr (K == Q4K_8) {
-                            float hi[8], lo[8], mm[8];
-                            tmem_ld8(dt, hi);
-                            tmem_ld8(dt + 8, lo);
+                            float v0[8], v1[8], mm[8];
+                            tmem_ld8(dt, v0);
+                            tmem_ld8(dt + 8, v1);
                             tmem_ld8(dt + C::kMOff, mm);
                             tmem_ld_wait();
 #pragma unroll
-                            for (int j = 0; j < 8; j++) to[j] = fmaf(xs[j], fmaf(d, hi[j] + lo[j], dm * mm[j]), to[j]);
+                            for (int j = 0; j < 8; j++) to[j] = fmaf(xs[j], fmaf(d, v0[j] + v1[j], dm * mm[j]), to[j]);
                         } else {
 #pragma unroll
                             for (int q = 0; q < 2; q++) {

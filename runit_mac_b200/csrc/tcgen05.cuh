@@ -29,13 +29,13 @@ __device__ __forceinline__ void tc_fence_after_sync() { asm volatile("tcgen05.fe
 
 // ── operand descriptors ──
 // Shared-memory matrix descriptor of a K-major tile in the 128-byte swizzled layout: rows of 64 16-bit elements
-// (128 bytes), groups of 8 rows 1024 bytes apart, 16-byte chunk c of row r stored at chunk position c ^ (r % 8).
+// (128 bytes), groups of 8 rows `stride` bytes apart (a multiple of 1024, below 256 KB), 16-byte chunk c of row r stored at chunk position c ^ (r % 8).
 // `addr` = shared address of the tile (1024-byte aligned) plus 32 bytes per 16-element K step inside the row.
 //   bits  0-13 start address >> 4      bits 16-29 leading byte offset >> 4 (unused for swizzled K-major: 1)
-//   bits 32-45 stride byte offset >> 4 (1024 >> 4)      bits 46-47 descriptor version (1 on sm_100)
+//   bits 32-45 stride byte offset >> 4      bits 46-47 descriptor version (1 on sm_100)
 //   bits 61-63 layout (2 = 128-byte swizzle)
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t addr) {
-    return (uint64_t)((addr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t addr, uint32_t stride = 1024) {
+    return (uint64_t)((addr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(stride >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
 // Instruction descriptor for kind::f16 with bf16 A and B (both K-major), f32 accumulator, tile M x N.
 //   bits 4-5 D format (1 = f32)   bits 7-9 A format (1 = bf16)   bits 10-12 B format (1 = bf16)

@@ -115,4 +115,4 @@ def test_bounded_waits_begin_behind_the_dependency_wait(role):
     assert not re.search(r"!wait\(", body[:body.index("grid_dependency_wait()")])
     if role == "unpack":
         loop = body[body.index("for (uint32_t e"):]
-        assert re.search(r"K == Q6K_8 && e >= C::kTeams && e < 2 \* C::kTeams\) grid_dependency_wait\(\)", loop[:loop.index("!wait(")])
+        assert re.search(r"C::kQ6 && e >= C::kTeams && e < 2 \* C::kTeams\) grid_dependency_wait\(\)", loop[:loop.index("!wait(")])
