@@ -5,8 +5,10 @@
 // which most serve an expert that another slot has just streamed.  Here the slots are sorted by expert (slots_table_kernel),
 // their activations are split into two f16 halves (split_slots_kernel), and a group of slots of one expert meets its matrices on tcgen05
 // (tc_rows.cuh): up to 8 slots per group where an expert has a few, up to 48 where it has many.
-// The layer of width 2048, 64 experts of 1024, top 8 (us; mma.sync with tiles of 8 columns -> now): 16 tokens 95 -> 68, 32 114 -> 77, 64 146 -> 93, 128
-// 200 -> 116, 256 285 -> 142; 60 experts of 768, top 4, 256 tokens 171 -> 106; 8 of 512, top 2, 64 tokens 53 -> 37.  Error against 64 bits 1.2e-7, as before.
+// The layer of width 2048, 64 experts of 1024, top 8 (us; mma.sync with tiles of 8 columns -> now): 16 tokens 86 -> 65, 32 112 -> 76, 64 144 -> 89, 128
+// 199 -> 114, 256 272 -> 139; 60 experts of 768, top 4, 256 tokens 171 -> 106; 8 of 512, top 2, 64 tokens 53 -> 37.  Error against 64 bits, of the output with a
+// residual of 1: 16 tokens 5.5e-8 -> 4.1e-8, 64 of 60 experts 4.9e-8 -> 4.0e-8, 256 1.12e-7 -> 0.89e-7.  (tcgen05 cuts its sums off where mma.sync did, a little
+// more: with hi and lo in turn for all of K, or side by side to its end, 5.6e-8, 5.1e-8 and 1.15e-7, 1 % faster.)
 #include <cuda_fp16.h>
 
 #include "moe_internal.h"

@@ -36,7 +36,7 @@ namespace runit {
 namespace tcr {
 
 // What a step looks like:
-//   Q4K_8   up to 8 columns, both halves side by side as the 16 columns of one product
+//   Q4K_8   up to 8 columns, both halves side by side as the 16 columns of one product; hi of the last 64 K behind all of lo, in the columns of lo
 //   Q4K_48  up to 48 columns in multiples of 16, the halves in turn into the same sums
 //   Q8_0_8  up to 8 columns, hi and lo side by side; a sum for each of the eight blocks, because their scales are f16 values that
 //           no integer factor expresses
@@ -61,7 +61,7 @@ template <Kind K> struct Cfg {
     static constexpr uint32_t kW = K == Q4K_8 ? 6 : 4, kB = K == Q4K_48 ? 2 : 4, kSteps = K == Q4K_8 ? 3 : 2, kA = kSteps * kParts, kD = kSteps;
     static constexpr uint32_t kXs = K == Q4K_48 ? 8 : 16, kRows = 8, kMins = kSteps;
     static constexpr uint32_t kBRow = K == Q4K_8 ? 1280 : K == Q4K_48 ? 1152 : kRest ? 1536 : 1024;       // bytes of an image per column
-    static constexpr uint32_t kBStage = kCols * kBRow, kOffB = K == Q8_0_8 ? 1024 : 0;     // eight rows of zeros, then the images
+    static constexpr uint32_t kBStage = kCols * kBRow, kOffB = K == Q4K_8 || K == Q8_0_8 ? 1024 : 0;     // eight rows of zeros, then the images
     static constexpr uint32_t kPanel = (kRest ? 24 : 16) * 128;                                           // of an image with sums per block
     static constexpr uint32_t kMinCol = 128 * kSteps, kDCol = kMinCol + (kBlocks ? 0 : 32);
     static constexpr uint32_t kDCols = K == Q4K_48 ? 96 : K == Q8_0_8 ? 128 : K == Q6K_8 ? 16 : 32, kMOff = kDCols / 2;          // sums of a step: products, then minimums; or of its blocks
@@ -384,8 +384,8 @@ template <Kind K, int SUBS> struct Block {
             const uint32_t panel = n * 128, idesc = umma_idesc_f16(128, n, 0), bs = c % C::kB, ds = s % C::kD, d = tmem + C::kDCol + ds * C::kDCols;
             const uint32_t img_at = C::kOffB + bs * C::kBStage;
             const uint64_t img = umma_desc_sw128(base + img_at);
-            // eight rows of zeros, and that far behind them the rest (of panel 0)
-            const uint64_t apart = umma_desc_sw128(base, img_at + 2048);
+            // eight rows of zeros, and that far behind them eight rows of the image: Q8_0 the rest (of panel 0), Q4_K hi of the last panel
+            const uint64_t apart = umma_desc_sw128(base, img_at + (K == Q4K_8 ? 3 * 2048 : 2048));
             if (!wait(b_full + 8 * bs, (c / C::kB) & 1)) return;
             if (s >= C::kD && !wait(d_empty + 8 * ds, (s / C::kD - 1) & 1)) return;
 #pragma unroll
@@ -399,9 +399,16 @@ template <Kind K, int SUBS> struct Block {
                     for (uint32_t j = 0; j < kK; j++) {
                         const uint32_t k = h * kK + j, p0 = (k >> 2) * (C::kBlocks ? C::kPanel : panel), sum = K == Q8_0_8 ? d + 16 * (k >> 1) : d;
                         const uint64_t in = (k & 3) * 2, b = img + (p0 >> 4) + in;
-                        umma_f16_ts(sum, at + 8 * j, b, idesc, K == Q8_0_8 ? k & 1 : k);
-                        if (K == Q4K_48) umma_f16_ts(sum, at + 8 * j, b + (4 * panel >> 4), idesc, 1);
+                        if (K == Q4K_8 && k >= 12) umma_f16_ts(d, at + 8 * j, apart + (64ull << 32) + in, idesc, 1);
+                        else umma_f16_ts(sum, at + 8 * j, K == Q4K_48 ? b + (4 * panel >> 4) : b, idesc, K == Q8_0_8 ? k & 1 : k);
                         if (K == Q8_0_8) umma_f16_ts(sum, at + 8 * j, apart + ((uint64_t)(p0 >> 4) << 32) + in, idesc, 1);
+                    }
+                    // hi behind lo: the tensor cores cut a sum off at each product, and as long as there is only lo in it, at 2^-11 of the others
+#pragma unroll
+                    for (uint32_t j = 0; j < kK; j++) {
+                        const uint32_t k = h * kK + j;
+                        if (K == Q4K_48) umma_f16_ts(d, at + 8 * j, img + ((k >> 2) * panel >> 4) + (k & 3) * 2, idesc, 1);
+                        if (K == Q4K_8 && k >= 12) umma_f16_ts(d, at + 8 * j, apart + (k & 3) * 2, idesc, 1);
                     }
                     if (!C::kBlocks && h == 0)
                         umma_f16_ts(d + C::kMOff, tmem + C::kMinCol + 8 * (s % C::kMins), img + ((K == Q4K_8 ? 4 : 8) * panel >> 4), idesc, 0);

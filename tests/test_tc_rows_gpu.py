@@ -219,3 +219,34 @@ def test_error_is_that_of_f32_products_at_most(ctx, oracle, fmt, k, heavy):
                 ctx.set_tuning(key, 0)
         errors.append(rms_error(y, ref))
     assert errors[0] <= 1.1 * errors[1], errors
+
+
+@pytest.mark.parametrize("T,most", [(32, 9.0e-7), (96, 1.9e-6)])
+def test_error_of_the_sorted_moe_layer(ctx, oracle, T, most):
+    """Groups of 8 and of 48 slots against 64 bits: below what the products measured with mma.sync (most), because the sums that the tensor cores cut off
+    are kept short or small."""
+    import torch
+    import runit_mac_b200 as R
+    E, k, h, ff = 8, 2, 1024, 512
+    rng = np.random.default_rng(T)
+    router, x = rng.normal(0, 0.02, (E, h)).astype(np.float32), rng.normal(0, 1, (T, h)).astype(np.float32)
+    weights = [oracle.rand_q4k(rng, E * r, c) for r, c in ((ff, h), (ff, h), (h, ff))]
+    out, idx, w = ctx.new_buffer(T * h * 4), ctx.new_buffer(T * k * 4), ctx.new_buffer(T * k * 4)
+    nbytes = R.moe_scratch_bytes(ctx, T, h, ff, E, k)
+    scratch = ctx.new_buffer(nbytes)
+    bufs = [ctx.buffer_from(a) for a in (router, *weights, x)]
+    ctx.set_tuning("moe_slots", 1)
+    try:
+        R.moe_layer_q4k(ctx, *bufs, None, out, idx, w, scratch, nbytes, T, h, ff, E, k, 0)
+        ctx.flush()
+    finally:
+        ctx.set_tuning("moe_slots", 0)
+    gate, up, down = (torch.from_numpy(oracle.dequant_rows(2, a, E * r, c)).cuda().double().reshape(E, r, c) for a, (r, c) in zip(weights, ((ff, h), (ff, h), (h, ff))))
+    idx, w = (torch.from_numpy(b.download(t, T * k).reshape(T, k)).cuda() for b, t in ((idx, np.int32), (w, np.float32)))
+    xd, ref = torch.from_numpy(x).cuda().double(), torch.zeros(T, h, device="cuda", dtype=torch.float64)
+    for e in range(E):
+        t, i = torch.nonzero(idx == e, as_tuple=True)
+        act = torch.nn.functional.silu(xd[t] @ gate[e].T) * (xd[t] @ up[e].T)
+        ref.index_add_(0, t, w[t, i, None].double() * (act @ down[e].T))
+    error = rms_error(torch.from_numpy(out.download(np.float32, T * h).reshape(T, h)).cuda(), ref)
+    assert error <= most, error
