@@ -193,7 +193,9 @@ int32_t runit_fused_qkv_q4k_f32(runit_ctx_t*, const void* w_q, const void* w_k, 
 int32_t runit_fused_ffn_q4k_f32(runit_ctx_t*, const void* w_gate, const void* w_up, const void* x_vec, void* act_out,
                                 uint32_t ff_dim, uint32_t k);
 /* Batched fused-dequant GEMV: x [batch][k] f32, y [batch][m] f32 (+ residual [batch][m], may be
- * NULL); weights streamed once for the whole batch; batch in 1..8. */
+ * NULL); weights streamed once for the whole batch; batch in 1..8.  Which kernel serves a product depends on its sizes, on the batch and on the
+ * matrices that share the call, so its last bits can too.  Q8_0 of 2 to 8 rows keeps 24 bits of an activation down to 2^-11 of the largest
+ * of its 256 neighbours and 23 down to 2^-25, or multiplies f32 values. */
 int32_t runit_gemv_batched_f32(runit_ctx_t*, int32_t fmt, const void* weight, const void* input, void* output,
                                const void* residual, uint32_t m, uint32_t k, uint32_t batch);
 /* The same for up to three matrices that share the input (q | k | v, gate | up): one launch, the activations are

@@ -242,6 +242,7 @@ int32_t runit_set_tuning(runit_ctx_t* ctx, const char* key, int32_t value) {
     else if (!strcmp(key, "stream_dynamic")) ctx->tune.stream_dynamic = value;
     else if (!strcmp(key, "moe_slots")) ctx->tune.moe_slots = value;
     else if (!strcmp(key, "moe_piece")) ctx->tune.moe_piece = value;
+    else if (!strcmp(key, "gemv_tc")) ctx->tune.gemv_tc = value;
     else if (!strcmp(key, "gemm_pair")) ctx->tune.gemm_pair = value;
     else if (!strcmp(key, "router_variant")) ctx->tune.router_variant = value;
     else if (!strcmp(key, "ep_fused_exchange")) ctx->tune.ep_fused_exchange = value;

@@ -502,7 +502,7 @@ int32_t runit_gemv_batched_multi_f32(runit_ctx_t* ctx, int32_t fmt, uint32_t n_m
         RUNIT_REQUIRE(ctx, weights[i] && outputs[i] && rows[i] > 0, "gemv_batched_multi_f32: null matrix or output %u", i);
         ok = ok && runit_aligned(weights[i], 16) && runit_aligned(outputs[i], 4);
     }
-    if (ok && gemv_tc_applies(ctx, fmt, k, batch))
+    if (ok && gemv_tc_applies(ctx, fmt, n_mats, rows, k, batch))
         return gemv_tc_multi(ctx, n_mats, weights, (const float*)input, (float* const*)outputs, nullptr, rows, k, batch);
     if (ok && gemv_imma_applies(ctx, fmt, k, batch) && (k / 256 * 144) % 16 == 0)
         return gemv_imma_multi(ctx, fmt, n_mats, weights, (const float*)input, (float* const*)outputs, nullptr, rows, k, batch);
@@ -521,7 +521,7 @@ int32_t runit_gemv_batched_f32(runit_ctx_t* ctx, int32_t fmt, const void* weight
     // batch 2..8: Q8_0 on tcgen05, the 4-bit formats on the integer tensor-core path (activations prepared once, weights streamed once)
     const bool aligned = weight && input && output && runit_aligned(weight, 16) && runit_aligned(input, 16) && runit_aligned(output, 4) &&
                          runit_aligned(residual, 4) && ctx->tune.gemv_variant != 1;
-    if (aligned && gemv_tc_applies(ctx, fmt, k, batch)) {
+    if (aligned && gemv_tc_applies(ctx, fmt, 1, &m, k, batch)) {
         const float* res = (const float*)residual;
         float* y = (float*)output;
         return gemv_tc_multi(ctx, 1, &weight, (const float*)input, &y, &res, &m, k, batch);

@@ -14,8 +14,9 @@
 // Error against 64 bits 0.9e-7 to 1.1e-7 from K = 2048 on (the kernels before 2.7e-7), and with three parts below that 6.0e-8 to 7.0e-8 (8.3e-8 to 9.2e-8).
 //
 // Bound: the unpacking warps, about 1000 clocks per 128 x 256 weights and SM (2.1 TB/s), and some 4 us between dependent calls (the pre-pass and
-// its hand-over).  The packed f32 kernel that it replaces multiplies every weight 8 times on the CUDA cores.  Decoding steps, us, f32 -> now: width 3584, two
-// layers and a head of 30000 rows, 2 / 4 / 8 sequences 293 / 420 / 906 -> 191 / 183 / 188; width 2048, four layers, 271 / 363 / 689 -> 227 / 225 / 233.  Error against 64 bits 5.9e-8 at K = 256, 7.7e-8 at 2048, 1.0e-7
+// its hand-over).  The packed f32 kernel, which still serves small ones of 2 to 4 rows (gemv_tc_pays), multiplies every weight 8 times on the CUDA cores.
+// Decoding steps, us, f32 -> now: width 3584, two layers and a head of 30000 rows, 2 / 4 / 8 sequences 293 / 420 / 906 -> 183 / 183 / 188; width 2048, four layers,
+// 271 / 363 / 689 -> 219 / 225 / 233; width 1024, eight layers, 211 / 273 / 511 -> 197 / 230 / 262.  Error against 64 bits 5.9e-8 at K = 256, 7.7e-8 at 2048, 1.0e-7
 // at 18944 (f32 products 7.8e-8, 9.6e-8, 1.4e-7; the two halves of 22 bits that were here before, 4 to 8 % faster, 8.1e-8, 9.5e-8, 1.2e-7, and more
 // than f32 products where a few activations dominate).  The 4-bit formats stay with gemv_imma.cu: the same kernel for them took 362 us where that one
 // takes 350 (Q4_K, 7B, four layers and head, 8 sequences), 332 against 353 (Q4_0, 4 sequences) and 198 against 187 (width 2048).
@@ -290,9 +291,27 @@ template <tcr::Kind K> static int32_t launch(runit_ctx* ctx, const char* name, A
 
 }  // namespace tcg
 
-bool gemv_tc_applies(const runit_ctx* ctx, int fmt, uint32_t k, uint32_t batch) {
+// Where it is the faster one.  The packed f32 kernel takes a launch per matrix and power of two in the batch (3 = 2 + 1), 2 to 4 us each and then some 5e12
+// multiply-adds a second; this one takes 4 to 7 us (the pre-pass and its hand-over) and 3.4e12 weights a second, whatever the batch.  So it wins with
+// eight rows or three launches, with two nearly always, and against one from the sizes below on, which lie where the two meet (us, f32 / this: batch 2,
+// K 256 8192 rows 2.8 / 4.5, 16384 5.1 / 4.6; K 1024 16384 9.2 / 11.1, 32768 15.3 / 13.3; K 2048 4096 6.2 / 7.7, 8192 12.1 / 10.5; K 3584 2048 6.4 / 7.7, 4096
+// 12.3 / 10.4; K 12288 512 9.2 / 10.5, 1024 14.3 / 10.5; batch 4, K 1024 8192 6.1 / 7.4, 16384 12.1 / 11.2; K 2048 2048 6.3 / 7.5, but a step of width 2048 with it 231 / 225, 4096 7.7 / 7.7; K 3584 2048 7.8 / 7.8; K 8192 512 9.5 /
+// 9.5; two launches, K 1024: two matrices of 2816, batch 2, 6.5 / 7.3; one of 1024, batch 3, 6.3 / 7.1, of 2048 7.6 / 7.2; batch 3 stays here throughout, because its third
+// row would meet 16-bit activations there).
+static bool gemv_tc_pays(uint32_t n_mats, uint64_t rows, uint32_t k, uint32_t batch) {
+    const uint32_t launches = n_mats * (uint32_t)__builtin_popcount(batch);
+    if (batch == 8 || launches > 2) return true;
+    if (launches == 2) return batch != 2 || k < 512 || k > 1024 || rows >= 8192;
+    if (batch == 2) return rows >= (k <= 512 ? 12288u : k <= 1024 ? 24576u : k <= 2048 ? 6144u : k <= 8192 ? 3072u : k <= 12288 ? 768u : 0u);
+    return rows >= (k <= 512 ? 10240u : k <= 1024 ? 12288u : k <= 5120 ? 2048u : k <= 8192 ? 512u : 0u);
+}
+
+bool gemv_tc_applies(const runit_ctx* ctx, int fmt, uint32_t n_mats, const uint32_t* m, uint32_t k, uint32_t batch) {
     if (fmt != RUNIT_FMT_Q8_0 || batch < 2 || batch > 8 || k == 0 || k % 256 != 0 || ctx->tune.gemv_math == 1 || !ctx->encode_tiled || !ctx->d_xq || !ctx->d_tc) return false;
-    return (size_t)(k / 256) * (tcg::C::kBStage + 32) <= ctx->xq_bytes;
+    if ((size_t)(k / 256) * (tcg::C::kBStage + 32) > ctx->xq_bytes) return false;
+    uint64_t rows = 0;
+    for (uint32_t i = 0; i < n_mats; i++) rows += m[i];
+    return ctx->tune.gemv_tc == 1 || gemv_tc_pays(n_mats, rows, k, batch);
 }
 
 // n_mats (1..3) matrices over the same activations in one launch.

@@ -33,6 +33,7 @@ struct runit_tuning {
     int32_t ep_fused_exchange = 0;   // expert-parallel decoder: 1 = exchange inside the GEMVs (no launches of its own; measured slower)
     int32_t moe_slots = 0;        // MoE layer of several tokens: 0 = slots sorted by expert by size, 1 = always (tests), 2 = never
     int32_t moe_piece = 0;        // tokens of a piece of it at most (tests); 0 = as many as the staging area holds
+    int32_t gemv_tc = 0;          // batched Q8_0 GEMV on tcgen05: 0 = by size, 1 = wherever it applies (tests)
     int32_t gemm_pair = 0;        // GEMM of many tokens: 0 = CTA pairs by size, 1 = wherever they apply (tests), 2 = never
     int32_t gemv_pro_ctas = 0;    // bf16 GEMV with a prologue of several vectors: CTAs per SM at most (0 = default)
     int32_t router_variant = 0;   // batched f32 router: 0 = by size, 1 = one warp per expert, 2 = tiled GEMM, 3 = GEMM with K split over the warps of a CTA (tests force each)
@@ -192,7 +193,7 @@ namespace tcg {
 constexpr uint32_t kMaxShares = 10, kMaxCtas = 160, kTickets = kMaxCtas * 8, kPartBytes = 4096;      // a share's sums of a tile
 constexpr size_t kTicketBytes = kTickets * 4, kContextBytes = kTicketBytes + (size_t)kMaxCtas * kMaxShares * kPartBytes;
 }  // namespace tcg
-bool gemv_tc_applies(const runit_ctx* ctx, int fmt, uint32_t k, uint32_t batch);
+bool gemv_tc_applies(const runit_ctx* ctx, int fmt, uint32_t n_mats, const uint32_t* m, uint32_t k, uint32_t batch);
 int32_t gemv_tc_multi(runit_ctx* ctx, uint32_t n_mats, const void* const* w, const float* x, float* const* y, const float* const* res, const uint32_t* m,
                       uint32_t k, uint32_t batch);
 // the same for Q6_K and one activation row

@@ -12,8 +12,16 @@ from test_moe_slots_gpu import run
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture
+def on_tc(ctx):
+    """Small batches and matrices too, which the packed f32 kernel serves faster."""
+    ctx.set_tuning("gemv_tc", 1)
+    yield
+    ctx.set_tuning("gemv_tc", 0)
+
+
 @pytest.mark.parametrize("m,k,batch", [(1, 256, 2), (127, 512, 8), (128, 256, 3), (129, 1280, 4), (1000, 2560, 5), (300, 18944, 8), (19100, 768, 7), (40, 5376, 6)])
-def test_batched_q8_0(ctx, oracle, m, k, batch):
+def test_batched_q8_0(ctx, oracle, on_tc, m, k, batch):
     import runit_mac_b200 as R
     O = oracle
     rng = np.random.default_rng(m + k + batch)
@@ -45,7 +53,7 @@ def test_batched_q8_0(ctx, oracle, m, k, batch):
 
 
 @pytest.mark.parametrize("k", [256, 1536, 3584])
-def test_batched_q8_0_bits_do_not_depend_on_the_launch(ctx, oracle, k):
+def test_batched_q8_0_bits_do_not_depend_on_the_launch(ctx, oracle, on_tc, k):
     """A matrix alone, in one launch with two others, and as the first rows of a larger one: the same bits."""
     import runit_mac_b200 as R
     O = oracle
@@ -69,7 +77,7 @@ def test_batched_q8_0_bits_do_not_depend_on_the_launch(ctx, oracle, k):
     assert np.array_equal(large[:, 640:], outs[2].download(np.float32, batch * 2000).reshape(batch, 2000))
 
 
-def test_batched_q8_0_value_that_is_not_finite_stays_with_its_row(ctx, oracle):
+def test_batched_q8_0_value_that_is_not_finite_stays_with_its_row(ctx, oracle, on_tc):
     import runit_mac_b200 as R
     O = oracle
     m, k, batch = 200, 1024, 5
@@ -147,7 +155,7 @@ def test_q6k(ctx, oracle, m, k):
 
 
 @pytest.mark.parametrize("fmt", [0, 5])
-def test_infinities_and_nan(ctx, oracle, fmt):
+def test_infinities_and_nan(ctx, oracle, on_tc, fmt):
     """An infinite activation gives infinities of the weights' signs (NaN where the weight is 0), a NaN gives NaN, in its own row of activations."""
     import torch
     import runit_mac_b200 as R
@@ -185,7 +193,7 @@ def rms_error(got, ref):
 @pytest.mark.parametrize("heavy", [False, True])
 @pytest.mark.parametrize("k", [256, 1792, 3584])
 @pytest.mark.parametrize("fmt", [0, 5])
-def test_error_is_that_of_f32_products_at_most(ctx, oracle, fmt, k, heavy):
+def test_error_is_that_of_f32_products_at_most(ctx, oracle, on_tc, fmt, k, heavy):
     """Against 64 bits, over rows enough that the root mean square stands to a few per cent, with activations as they come and with a few channels that
     dominate, as hidden states of large models have.  (A tenth of room: it lies 10 to 40 % below.)"""
     import torch

@@ -49,6 +49,7 @@ def test_callers_kernel_before_a_batched_gemv(rows, k, batch):
     import runit_mac_b200 as R
     stream = torch.cuda.Stream()
     ctx = R.Context(0, stream=stream.cuda_stream)
+    ctx.set_tuning("gemv_tc", 1)
     try:
         with torch.cuda.stream(stream):
             g = torch.Generator(device="cuda").manual_seed(k)
@@ -86,6 +87,7 @@ def test_fill_before_a_gemv(ctx, batch):
     m, k = 896, 896 if batch == 1 else 1024
     w, x = ctx.new_buffer(m * k // 32 * 34), ctx.buffer_from(np.random.default_rng(0).normal(0, 1, batch * k).astype(np.float32))
     outs = []
+    ctx.set_tuning("gemv_tc", 1)
     for wait in (True, False):
         ys = [ctx.new_buffer(batch * m * 4) for _ in range(20)]
         for i, y in enumerate(ys):
@@ -98,6 +100,7 @@ def test_fill_before_a_gemv(ctx, batch):
                 R.gemv_batched_f32(ctx, R.FMT_Q8_0, w, x, y, None, m, k, batch)
         ctx.flush()
         outs.append([y.download(np.float32, batch * m) for y in ys])
+    ctx.set_tuning("gemv_tc", 0)
     assert not np.array_equal(outs[0][0], outs[0][1])
     for a, b in zip(*outs):
         assert np.array_equal(a, b)
