@@ -1,7 +1,7 @@
 """Packed rows times a few columns on tcgen05 (tc_rows.cuh): the batched Q8_0 GEMV and the MoE layer with its slots sorted by expert, at the edges of their
 tiles and rings.
 
-Bound: an activation keeps 24 bits (Q4_K 22: two f16 halves of x / 2^e, error <= 2^-22 of it or 2^-35 of the largest of its 256), products are exact, sums
+Bound: an activation keeps 24 bits (Q4_K, and Q6_K from K = 2048 on, 22: two f16 halves of x / 2^e, error <= 2^-22 of it or 2^-35 of the largest of its 256), products are exact, sums
 are f32: 2^-24 of the running sum per addition along 32 products, 8 blocks and K / 256 units.  2e-5 of max(|ref|, rms) holds with room."""
 import numpy as np
 import pytest
